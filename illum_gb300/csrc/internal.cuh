@@ -96,6 +96,7 @@ struct MeshDesc {
   CondScalars cs;
   int tile0, ntiles;           // radiosity row tiles (0: no radiosity)
   double tol2;                 // squared residual tolerance
+  float res_unit;              // FP64 solve: residual units (2^20 / tol2) per unit of squared change
   int max_sweeps;
   int refine_every;            // mixed solve: 0 = refinement rounds to tol each step; K >= 1 = one
                                // pass per step, with fl(F) every K-th step (k_radiosity_lagged)
@@ -356,6 +357,8 @@ int radiosity_threads();
 // unsigned words of a view's barrier buffer: the grid barrier's counter and
 // the per-mesh residual accumulators of the radiosity kernels
 size_t radiosity_barrier_words(int nmesh);
+// residual units of the FP64 solve per unit of squared change (radiosity.cu)
+float radiosity_res_unit(double tol2);
 int radiosity_launch(const StepView& v, double* x, int warm, int precision, int grid, int inner, bool lagged,
                      cudaStream_t s);
 int radiosity_barrier_probe(unsigned* bar, int* derr, int blocks, long long polls, int unreachable, cudaStream_t s);

@@ -443,6 +443,24 @@ __device__ __forceinline__ void stage_halo(const StepView& v, const RowTile& T, 
   cbar();
 }
 
+// As stage_halo, x = eh + s formed from its two parts.
+__device__ __forceinline__ void stage_halo_sum(const StepView& v, const RowTile& T, const float2* eh, const float2* s,
+                                               float2* sx) {
+  const uint32_t* hp = v.t_halo + T.h0;
+  int h = threadIdx.x;
+  for (; h + RAD_THREADS < T.nhalo; h += 2 * RAD_THREADS) {
+    const uint32_t a = __ldg(hp + h), b = __ldg(hp + h + RAD_THREADS);
+    const float2 ea = ld_it(eh + a), eb = ld_it(eh + b), sa = ld_it(s + a), sb = ld_it(s + b);
+    sx[h] = df_add(ea, sa);
+    sx[h + RAD_THREADS] = df_add(eb, sb);
+  }
+  if (h < T.nhalo) {
+    const uint32_t a = __ldg(hp + h);
+    sx[h] = df_add(ld_it(eh + a), ld_it(s + a));
+  }
+  cbar();
+}
+
 // One tile: thread t owns entries [t*lam, (t+1)*lam) of the tile's entry
 // stream (rows in order, each row's entries in column order), stored so that
 // a group of 4 RAD_THREADS entries is contiguous: entry k of thread t at
@@ -532,15 +550,19 @@ __device__ __forceinline__ float block_sum(float d, float* red) {
 // and a mesh's decisions are the same alone and in a batch. A mesh stops
 // when its total is <= 2^20 units, i.e. sum of partials <= tol^2 (at most
 // ntiles units conservative). The accumulators follow the barrier's two
-// counter words, three buffers of nmesh by residual number mod 3: buffer
-// k + 1 is cleared during residual k (its last reader, decision k - 2,
-// finished before the barrier that precedes residual k), and the accumulators
-// of residual 0 are cleared before the first barrier.
+// counter words, three buffers of RES_LEVELS x nmesh by residual number
+// mod 3: buffer k + 1 is cleared during residual k (its last reader,
+// decision k - 2, finished before the barrier that precedes residual k), and
+// the accumulators of residual 0 are cleared before the first barrier. The
+// FP64 solve also needs totals far above the cap (it tracks how much the
+// change has shrunk): it counts a partial of more than 2^40 units in units
+// of 2^40 (level 1) or 2^80 (level 2), the mixed solves use level 0 only.
 constexpr unsigned long long RES_UNITS = 1ull << 20;
 constexpr unsigned long long RES_CAP = 1ull << 40;
+constexpr int RES_LEVELS = 3;
 
-__device__ __forceinline__ unsigned long long* res_acc(const StepView& v, int k) {
-  return reinterpret_cast<unsigned long long*>(v.barrier + 2) + (size_t)(k % 3) * v.nmesh;
+__device__ __forceinline__ unsigned long long* res_acc(const StepView& v, int k, int level = 0) {
+  return reinterpret_cast<unsigned long long*>(v.barrier + 2) + (size_t)((k % 3) * RES_LEVELS + level) * v.nmesh;
 }
 
 // done[m]: 0 running; 1 + (parity of the mesh's last residual) once
@@ -624,6 +646,143 @@ __device__ __forceinline__ void record_residuals(const StepView& v, const MeshSt
   }
 }
 
+// ---- the FP64 solve's sweeps ----
+//
+// A sweep evaluates s' = F x for x = E + s. Written as a change, with
+// d = s - (the previous s), the same sweep is d' = F d, s' = s + d': the
+// iterates are Jacobi's either way. A full sweep evaluates F x in
+// double-float (10 B per entry, ~20 FP32 operations, 8 B halos); a change
+// sweep evaluates F d in FP32 with the high parts of the values (6 B, one
+// FMA, 4 B halos) and adds it to the double-float s, with a rounding error
+// of about 2^-24 |F| |d|, relative to the change and not to x. So the solve
+// begins with a full sweep, continues with change sweeps while those errors
+// are small against the change, and returns to a full sweep, which
+// recomputes s from x and so removes them:
+//   after a full sweep: |d| <= tol stops, else a change sweep follows;
+//   after a change sweep, with A = the sum of |d| over the change sweeps
+//   since the last full one (the errors' scale, bounded by 2^-23 A): |d| <=
+//   15/16 tol with 2^-23 A <= tol / 16 stops (the residual is then <= tol);
+//   |d| <= 2^-20 A, or |d| <= 15/16 tol without the second condition, is
+//   followed by a full sweep; anything else by another change sweep.
+// The last sweep of a budget is a full one, so that a solve which reaches tol
+// within its budget by full sweeps alone still does. |d| comes from the integer residual totals, so the choice is the same in
+// every block, on every run, and alone or in a batch. A tolerance of zero
+// (or one whose units overflow) runs full sweeps only.
+struct MeshState64 {
+  int sweeps[RAD_MAX_MESH];
+  float acc[RAD_MAX_MESH];             // A in units of tol
+  unsigned char done[RAD_MAX_MESH];    // as MeshState::done
+  unsigned char mode[RAD_MAX_MESH];    // bit 0: the next sweep is a change sweep; bit 1: s is in S1
+};
+constexpr float CHG_STOP = 15.f / 16.f, CHG_NOISE_STOP = 1.f / 16.f;   // units of tol
+constexpr float CHG_NOISE = 1.1920929e-7f;                             // 2^-23
+constexpr float CHG_REFRESH = 9.5367432e-7f;                           // 2^-20
+constexpr float CHG_RANGE = 5.6294995e14f;   // 2^49: above it the totals are at their cap
+
+// Thread 0, after block_sum: record tile t's partial of residual k.
+__device__ __forceinline__ void post_partial64(const StepView& v, const RowTile& T, int t, int k, float unit,
+                                               float d2) {
+  if (threadIdx.x != 0) return;
+  v.tile_d2[(size_t)(k & 1) * v.ntiles + t] = (double)d2;
+  int level = 2;
+  unsigned long long u = RES_CAP;      // NaN and anything beyond level 2
+  if (!isnan(d2)) {
+    const float q = d2 > 0.f ? __fmul_ru(d2, unit) : 0.f;
+    const float cap = (float)RES_CAP;   // 2^40, exact
+    if (q < cap) {
+      level = 0;
+      u = (unsigned long long)ceilf(q);
+    } else if (q < cap * cap) {
+      level = 1;
+      u = (unsigned long long)ceilf(q * (1.f / cap));
+    } else if (q * (1.f / cap) * (1.f / cap) < cap) {
+      u = (unsigned long long)ceilf(q * (1.f / cap) * (1.f / cap));
+    }
+  }
+  if (u) atomicAdd(res_acc(v, k, level) + T.mesh, u);
+  for (int l = 0; l < RES_LEVELS; ++l) res_acc(v, k + 1, l)[T.mesh] = 0ull;
+}
+
+__device__ __forceinline__ void init_meshes64(const StepView& v, MeshState64& st) {
+  for (int m = threadIdx.x; m < v.nmesh; m += blockDim.x) {
+    const MeshDesc& M = v.md[m];
+    st.done[m] = (M.active && M.ntiles > 0) ? 0 : 1;
+    st.mode[m] = 0;
+    st.sweeps[m] = 0;
+    st.acc[m] = 0.f;
+  }
+  const int gt = blockIdx.x * blockDim.x + threadIdx.x;
+  for (int m = gt; m < RES_LEVELS * v.nmesh; m += gridDim.x * blockDim.x) res_acc(v, 0)[m] = 0ull;
+}
+
+// Every block, after the barrier that completes sweep k: stop decisions,
+// the kind of the next sweep, and the number of meshes still running.
+__device__ __forceinline__ int decide_meshes64(const StepView& v, MeshState64& st, int k) {
+  int running = 0;
+  for (int m0 = 0; m0 < v.nmesh; m0 += blockDim.x) {
+    const int m = m0 + threadIdx.x;
+    bool run = m < v.nmesh && !st.done[m];
+    if (run) {
+      const unsigned long long q0 = __ldcg(res_acc(v, k, 0) + m), q1 = __ldcg(res_acc(v, k, 1) + m),
+                               q2 = __ldcg(res_acc(v, k, 2) + m);
+      const float cap = (float)RES_CAP;
+      const float dn = sqrtf((float)q0 + cap * ((float)q1 + cap * (float)q2)) * (1.f / 1024.f);   // |d| / tol
+      const bool change = st.mode[m] & 1;
+      const int sw = ++st.sweeps[m];
+      float acc = st.acc[m];
+      bool stop, next_change;
+      if (change) {
+        const bool small = dn <= CHG_STOP;
+        stop = small && CHG_NOISE * acc <= CHG_NOISE_STOP;
+        next_change = !small && dn > CHG_REFRESH * acc && dn < CHG_RANGE;
+        acc += dn;
+      } else {
+        stop = q1 == 0 && q2 == 0 && q0 <= RES_UNITS;
+        next_change = dn < CHG_RANGE;
+        acc = dn;
+        st.mode[m] ^= 2;
+      }
+      const int budget = v.md[m].max_sweeps;
+      st.mode[m] = (st.mode[m] & 2) | (next_change && sw + 1 < budget ? 1 : 0);
+      if (stop || sw >= budget) {
+        st.done[m] = 1 + (k & 1);
+        run = false;
+        // the errors of a change sweep that was the last (A without the last |d|)
+        st.acc[m] = change ? acc - dn : 0.f;
+      } else {
+        st.acc[m] = acc;
+      }
+      if (blockIdx.x == 0) v.md[m].sweeps = sw;
+    }
+    running += __syncthreads_count(run);
+  }
+  return running;
+}
+
+// Block 0, at the end of the launch: each solved mesh's last residual into
+// the mesh table: the root of the sum of its tiles' partials (lane-strided
+// then a fixed warp tree), plus the bound on the change sweeps' errors.
+__device__ __forceinline__ void record_residuals64(const StepView& v, const MeshState64& st) {
+  if (blockIdx.x != 0 || threadIdx.x >= RAD_THREADS) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int m = warp; m < v.nmesh; m += RAD_THREADS / 32) {
+    const MeshDesc& M = v.md[m];
+    if (!M.active || M.ntiles == 0) continue;
+    const double* d2 = v.tile_d2 + (size_t)(st.done[m] - 1) * v.ntiles;
+    double t = 0.0;
+    for (int j = lane; j < M.ntiles; j += 32) t += ld_it(d2 + M.tile0 + j);
+    t = warp_sum(t);
+    if (lane == 0) {
+      const float err = CHG_NOISE * st.acc[m];   // units of tol
+      if (err > 0.f) {
+        const double r = sqrt(t) + (double)err * sqrt(M.tol2);
+        t = r * r;
+      }
+      v.md[m].res2 = t;
+    }
+  }
+}
+
 // The solve works on radiosity positions (Morton order within each mesh),
 // gathered through rperm at entry: EP = E (FP64), S0 / S1 = the iterates'
 // scattered parts s = x - E (double-floats), H0 / H1 = the iterates
@@ -637,9 +796,13 @@ __device__ __forceinline__ void record_residuals(const StepView& v, const MeshSt
 // instead of dE. sprev holds S(n) and, after it, its last change; for the
 // one-pass mixed solve (predicted) the predicted change F (E(n+1) - E(n))
 // instead, so that s0 = S(n) + P from the second step on.
+// The FP64 solve keeps s in S0 or S1 (a full sweep writes the other one, a
+// change sweep adds in place) and its last change d, as floats by sweep
+// parity, in D0 / D1 (H0's memory); a full sweep's halos form x = EH + s.
 struct RadBufs {
   double* EP;
   float2 *S0, *S1, *H0, *H1, *EH;
+  float *D0, *D1;
   __device__ __forceinline__ explicit RadBufs(const StepView& v) {
     EP = v.rbuf;
     S0 = reinterpret_cast<float2*>(v.rbuf + v.nt);
@@ -647,6 +810,8 @@ struct RadBufs {
     H0 = reinterpret_cast<float2*>(v.rbuf + 3 * (size_t)v.nt);
     H1 = H0 + v.nt;
     EH = H1 + v.nt;
+    D0 = reinterpret_cast<float*>(H0);
+    D1 = D0 + v.nt;
   }
 };
 
@@ -661,7 +826,8 @@ constexpr int RAD_ILP = 4;
 // free_rows (the mixed solve): also write the result of the rows without
 // entries (x = E, s = 0) and their warm-start record, for a kernel that
 // scatters its tile rows itself; that solve reads only EP, S0 and H0 (and
-// x32), the FP64 sweeps also S1, H1 and EH.
+// x32), the FP64 sweeps EP, S0, S1, EH and the rows' changes D0 / D1, which
+// stay zero for rows without entries.
 // kind (the one-pass mixed solve, per mesh: 0 bf16 step, 1 reference step, 2
 // first reference step): the warm start is S(n) + P, and the pass's halo
 // vector EH = (x - x_ref, E(n+1) - E(n)) and the reference iterate H1 are
@@ -727,7 +893,7 @@ __device__ __forceinline__ void init_x(const StepView& v, double* x, int warm, i
       const float2 x0 = df_add(eh, s0);
       B.EP[p] = e;
       B.S0[p] = s0;
-      B.H0[p] = x0;
+      if (free_rows) B.H0[p] = x0;
       if (predicted) {
         // x - x_ref, high parts first (exact when within a factor of 2)
         const int kd = kind[mi[k]];
@@ -745,19 +911,21 @@ __device__ __forceinline__ void init_x(const StepView& v, double* x, int warm, i
         v.x32[p] = 0.f;
         v.x32[v.nt + p] = 0.f;
       } else {
-        B.S1[p] = make_float2(0.f, 0.f);
-        B.H1[p] = x0;
         B.EH[p] = eh;
+        if (!act[k]) {
+          B.S1[p] = make_float2(0.f, 0.f);
+          B.D0[p] = 0.f;
+          B.D1[p] = 0.f;
+        }
       }
     }
   }
 }
 
 // Scatter the solved meshes' last iterate x = E + s back to facet order
-// (FP64; the FP64 solve's result is in S1 after an odd number of sweeps);
-// warm solves also record s and its change for the next step's start. Rows
+// (FP64); warm solves also record s and its change for the next step's start. Rows
 // without entries keep s = 0 in both buffers.
-__device__ __forceinline__ void scatter_x(const StepView& v, const MeshState& st, double* x, int warm, int gt,
+__device__ __forceinline__ void scatter_x(const StepView& v, const MeshState64& st, double* x, int warm, int gt,
                                           int nthreads) {
   const RadBufs B(v);
   for (int p0 = gt; p0 < v.nt; p0 += RAD_ILP * nthreads) {
@@ -775,7 +943,7 @@ __device__ __forceinline__ void scatter_x(const StepView& v, const MeshState& st
       if (!M.active || M.ntiles == 0) continue;
       ok[k] = true;
       g[k] = (int)v.rperm[p];
-      s[k] = ld_it(((st.sweeps[m] & 1) ? B.S1 : B.S0) + p);
+      s[k] = ld_it(((st.mode[m] & 2) ? B.S1 : B.S0) + p);
       e[k] = B.EP[p];
       sp[k] = warm ? v.sprev[p] : make_float2(0.f, 0.f);
     }
@@ -883,9 +1051,10 @@ __device__ __forceinline__ void produce_pass(Pipe& p, const StepView& v, const M
   }
 }
 
-// FP64 Jacobi to each mesh's tolerance. x: solution (and warm start).
+// FP64 Jacobi to each mesh's tolerance, full and change sweeps as above.
+// x: solution (and warm start).
 __global__ void __launch_bounds__(RAD_BLOCK, 1) k_radiosity64(StepView v, double* x, int warm) {
-  __shared__ MeshState st;
+  __shared__ MeshState64 st;
   __shared__ float red[32];
   __shared__ int bad;
   const RadSmem sm = rad_smem();
@@ -894,47 +1063,72 @@ __global__ void __launch_bounds__(RAD_BLOCK, 1) k_radiosity64(StepView v, double
   const int nthreads = gridDim.x * RAD_THREADS;
   unsigned gen = 0;
   Pipe pipe = make_pipe(sm, RAD_NST64, RAD_STAGE64, &bad);
-  init_meshes(v, st);
+  init_meshes64(v, st);
   if (!producer) init_x(v, x, warm, gt, nthreads, false);
   if (!grid_barrier(v.barrier, gridDim.x, gen, v.derr)) return;
   const uint64_t pol = l2_keep_policy(v.l2_stream);
   const ValsDF vals{v.t_vhi, v.t_vlo};
+  const ValsHiF vhi{v.t_vhi};
+  const int b0 = v.blk_start[blockIdx.x], b1 = v.blk_start[blockIdx.x + 1];
   for (int it = 0;; ++it) {
     if (producer) {
-      produce_pass(pipe, v, st, vals, pol);
+      if ((threadIdx.x & 31) == 0)
+        for (int k = b0; k < b1; ++k) {
+          const RowTile T = v.tiles[v.blk_tile[k]];
+          if (st.done[T.mesh]) continue;
+          if (st.mode[T.mesh] & 1) produce_tile(pipe, v, T, vhi, pol);
+          else produce_tile(pipe, v, T, vals, pol);
+        }
       __syncwarp();
     } else {
-      for (int k = v.blk_start[blockIdx.x]; k < v.blk_start[blockIdx.x + 1]; ++k) {
-    const int t = v.blk_tile[k];
+      const RadBufs B(v);
+      const float* dcur = (it & 1) ? B.D1 : B.D0;   // the change of the sweep before
+      float* dnxt = (it & 1) ? B.D0 : B.D1;
+      for (int k = b0; k < b1; ++k) {
+        const int t = v.blk_tile[k];
         const RowTile T = v.tiles[t];
         if (st.done[T.mesh]) continue;
-        const RadBufs B(v);
-        stage_halo(v, T, (it & 1) ? B.H1 : B.H0, sm.sx);
-        tile_rows<AccDF>(v, T, t, pipe, vals, sm.sx, sm.tail, sm.tnew, sm.rs);
+        const int mode = st.mode[T.mesh];
+        const float unit = v.md[T.mesh].res_unit;
+        float2* cur = (mode & 2) ? B.S1 : B.S0;
         const uint32_t* rows = v.t_row + T.r0;
-        const float2* cur = (it & 1) ? B.S1 : B.S0;
-        float2* nxt = (it & 1) ? B.S0 : B.S1;
-        float2* nxth = (it & 1) ? B.H0 : B.H1;
         float d2 = 0.f;
-        for (int r = threadIdx.x; r < T.nrows; r += RAD_THREADS) {
-          uint32_t i = __ldg(rows + r);
-          const float2 sn = sm.rs[r];          // s' = F x
-          const float2 sc = ld_it(cur + i);
-          // s' - s: exact high-part difference when the two are within a
-          // factor of two, else rounded relative to the change itself
-          const float df = __fadd_rn(__fsub_rn(sn.x, sc.x), __fsub_rn(sn.y, sc.y));
-          nxt[i] = sn;
-          nxth[i] = df_add(__ldg(B.EH + i), sn);
-          d2 = __fmaf_rn(df, df, d2);
+        if (mode & 1) {
+          float* sxf = reinterpret_cast<float*>(sm.sx);
+          float* rsf = reinterpret_cast<float*>(sm.rs);
+          stage_halo(v, T, dcur, sxf);
+          tile_rows<AccF32>(v, T, t, pipe, vhi, sxf, reinterpret_cast<float*>(sm.tail), sm.tnew, rsf);
+          for (int r = threadIdx.x; r < T.nrows; r += RAD_THREADS) {
+            const uint32_t i = __ldg(rows + r);
+            const float d = rsf[r];              // d' = F d
+            cur[i] = df_add(ld_it(cur + i), make_float2(d, 0.f));
+            dnxt[i] = d;
+            d2 = __fmaf_rn(d, d, d2);
+          }
+        } else {
+          float2* nxt = (mode & 2) ? B.S0 : B.S1;
+          stage_halo_sum(v, T, B.EH, cur, sm.sx);
+          tile_rows<AccDF>(v, T, t, pipe, vals, sm.sx, sm.tail, sm.tnew, sm.rs);
+          for (int r = threadIdx.x; r < T.nrows; r += RAD_THREADS) {
+            const uint32_t i = __ldg(rows + r);
+            const float2 sn = sm.rs[r];          // s' = F x
+            const float2 sc = ld_it(cur + i);
+            // s' - s: exact high-part difference when the two are within a
+            // factor of two, else rounded relative to the change itself
+            const float d = __fadd_rn(__fsub_rn(sn.x, sc.x), __fsub_rn(sn.y, sc.y));
+            nxt[i] = sn;
+            dnxt[i] = d;
+            d2 = __fmaf_rn(d, d, d2);
+          }
         }
-        post_partial(v, st, T, t, it, block_sum(d2, red));
+        post_partial64(v, T, t, it, unit, block_sum(d2, red));
       }
     }
     if (!grid_barrier(v.barrier, gridDim.x, gen, v.derr)) return;
-    if (decide_meshes(v, st, 1, 0, it) == 0) break;
+    if (decide_meshes64(v, st, it) == 0) break;
   }
   if (!producer) scatter_x(v, st, x, warm, gt, nthreads);
-  record_residuals(v, st);
+  record_residuals64(v, st);
 }
 
 // Mixed precision: outer refinement with the residual r = E - (I - fl(F)) x
@@ -1659,7 +1853,11 @@ int radiosity_threads() { return RAD_THREADS; }
 // when it would not stay in the 126 MB L2 between passes.
 int radiosity_l2_stream(int64_t stored) { return stored * 10 > (int64_t)96 << 20 ? 1 : 0; }
 
-size_t radiosity_barrier_words(int nmesh) { return 2 + 2 * 3 * (size_t)(nmesh > 0 ? nmesh : 1); }
+float radiosity_res_unit(double tol2) {
+  return tol2 > 0.0 ? (float)((double)RES_UNITS / tol2 * (1.0 + 1.0 / 65536.0)) : INFINITY;
+}
+
+size_t radiosity_barrier_words(int nmesh) { return 2 + 2 * 3 * RES_LEVELS * (size_t)(nmesh > 0 ? nmesh : 1); }
 
 // Cooperative grid size for ntiles tiles (at most the co-resident blocks).
 // Both solves launch the same block shape and shared memory, so one grid
