@@ -607,8 +607,8 @@ int ilg_ctx_device_bytes(const ilg_ctx* ctx, int64_t* bytes) {
            nbytes(c.H32, c.row_scale, c.t_vhi, c.t_vlo, c.t_scale, c.coef32, c.rho32, c.T32, c.disk32, c.x32) +
            nbytes(c.hmm32, c.coefdf, c.Tdf) + nbytes(c.rowptr) + nbytes(c.col) + nbytes(c.tiles) +
            nbytes(c.t_cf) + nbytes(c.t_vbf) + nbytes(c.row_act) +
-           nbytes(c.morton_order, c.t_row, c.t_halo, c.t_start, c.rperm) +
-           nbytes(c.work, c.counters, c.derr, c.mesh_flag) + nbytes(c.barrier) + nbytes(c.sun_aux) + nbytes(c.md) +
+           nbytes(c.morton_order, c.leaf_rank, c.t_row, c.t_halo, c.t_start, c.rperm) +
+           nbytes(c.work, c.counters, c.derr, c.mesh_flag, c.parent) + nbytes(c.barrier) + nbytes(c.sun_aux) + nbytes(c.md) +
            nbytes(c.scan.a, c.scan.b, c.scan.c, c.sort.keys_alt, c.sort.hist, c.sort.scan.a, c.sort.scan.b,
                   c.sort.scan.c) +
            nbytes(c.sort.vals_alt);

@@ -6,11 +6,12 @@
 //                             nrm    float4 (normal xyz, 0)
 //                             area   double
 //                             frame  9 doubles per facet (b, t, n columns)
-//   LBVH (Karras, BVH2):      nodes  4 x float4 per internal node: both
-//                                    children's boxes + child codes
-//                                    (>= 0 internal, ~k leaf k)
+//   LBVH (Karras, BVH2):      nodes  6 x float4 per internal node: both
+//                                    children's boxes, oriented slabs and
+//                                    child codes (>= 0 internal, ~k leaf k)
 //                             tri_s  3 x float4 per leaf in Morton order,
-//                                    v0.w = original facet index (int bits)
+//                                    v0.w = original facet index (int bits),
+//                                    v1.w, v2.w = l1 norms of its edges
 //   horizons:                 H      nphi doubles per facet (= the reference's
 //                                    nphi x N column-major matrix)
 //   form factors:             CSR by receiver row (rowptr int64, col int32,
@@ -29,6 +30,7 @@
 namespace ilg {
 
 constexpr int TRACE_STACK = 64;
+constexpr int NODE_W = 6;   // float4 per LBVH node
 
 struct HorizonNode {   // one node of the zenith-angle bisection tree
   double mid, s, c;    // mid angle and its sin / cos (geom.h sincos_x)
@@ -197,8 +199,11 @@ struct Context {
   dbuf<float4> nodes, tri_s;
   int root = 0;             // child code of the root (0, or ~0 for one facet)
   dbuf<uint32_t> morton_order;   // facet at each position of the LBVH's Morton order
+  dbuf<uint32_t> leaf_rank;      // that position of each facet
+  dbuf<int> parent;              // LBVH parents: internal nodes, then leaves by Morton position (-1: root)
   int64_t bvh_nodes = 0;
   int bvh_depth = 0;
+  int bvh_longest = 0;      // levels above the deepest leaf
 
   // horizons
   int nphi = 0;

@@ -1373,11 +1373,6 @@ __global__ void k_row_scale(const int64_t* __restrict__ rowptr, const double* __
   rscale[i] = m > 0.0 ? (float)m : 1.f;
 }
 
-__global__ void k_rank(const uint32_t* __restrict__ order, int nt, uint32_t* rank) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < nt) rank[order[p]] = (uint32_t)p;
-}
-
 // key = row << rb | Morton position of the column; value = CSR entry.
 __global__ void k_row_keys(const int64_t* __restrict__ rowptr, const int32_t* __restrict__ col,
                            const uint32_t* __restrict__ rank, int nt, int rb, unsigned long long* key,
@@ -1551,15 +1546,10 @@ int radiosity_prepare(Context& c) {
   ILG_CUDA(cudaMemcpyAsync(order.data(), c.morton_order.p, (size_t)nt * 4, cudaMemcpyDeviceToHost, s));
   dbuf<unsigned long long> dkey;
   dbuf<uint32_t> dsv;
-  const unsigned long long cmask = (1ull << rb) - 1;
   if (nnz > 0) {
-    dbuf<uint32_t> drank;
-    ILG_TRY(drank.alloc(nt));
     ILG_TRY(dkey.alloc(nnz));
     ILG_TRY(dsv.alloc(nnz));
-    k_rank<<<div_up(nt, 256), 256, 0, s>>>(c.morton_order.p, nt, drank.p);
-    ILG_CUDA(cudaGetLastError());
-    k_row_keys<<<div_up(nt, 256), 256, 0, s>>>(c.rowptr.p, c.col.p, drank.p, nt, rb, dkey.p, dsv.p);
+    k_row_keys<<<div_up(nt, 256), 256, 0, s>>>(c.rowptr.p, c.col.p, c.leaf_rank.p, nt, rb, dkey.p, dsv.p);
     ILG_CUDA(cudaGetLastError());
     ILG_TRY(radix_sort_u64(dkey.p, dsv.p, nnz, 2 * rb, c.sort, s));
   }

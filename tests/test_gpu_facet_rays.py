@@ -1,0 +1,38 @@
+"""GPU parity: horizon and visibility rays cast by whole warps from a facet.
+
+A warp's rays share their facet's path through the LBVH and its lanes are
+refilled as rays end, so the cases that could go wrong are the ones that
+leave lanes without work or put several facets into a warp: azimuth counts
+around a warp's 32 lanes, and meshes around the 32-facet leaf groups.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _mesh(n_faces):
+    """The first n_faces facets (Morton-coherent pieces of a cratered body)."""
+    from illum_gb300 import meshgen
+    v, f = meshgen.icosphere_craters(3, seed=8, n_craters=8, dmin_m=200.0, dmax_m=600.0)
+    return v, np.ascontiguousarray(f[:n_faces])
+
+
+@pytest.mark.parametrize("nphi", [2, 3, 7, 8, 15, 16, 31, 32, 33, 47, 64, 65])
+def test_horizons_any_azimuth_count(ilg, oracle_mod, nphi):
+    v, f = _mesh(320)
+    ctx = ilg.IllumContext(v, f)
+    ctx.make_horizons(nphi=nphi)
+    assert np.array_equal(ctx.horizons, oracle_mod.horizons(v, f, nphi).T)
+
+
+@pytest.mark.parametrize("n_faces", [1, 2, 3, 31, 32, 33, 64, 97, 1025])
+@pytest.mark.parametrize("cutoff", [None, 0.35])
+def test_form_factors_around_leaf_groups(ilg, oracle_mod, n_faces, cutoff):
+    v, f = _mesh(n_faces)
+    ctx = ilg.IllumContext(v, f)
+    rp, col, val = ctx.compute_F(albedo=0.3, cutoff=cutoff)
+    ro, co, vo, rays = oracle_mod.form_factors(v, f, albedo_scalar=0.3, cutoff=-1.0 if cutoff is None else cutoff)
+    rpo, cpo, vpo = oracle_mod.coo_to_csr(n_faces, ro, co, vo)
+    assert np.array_equal(rp, rpo) and np.array_equal(col, cpo) and np.array_equal(val, vpo)
+    assert ctx.visibility_rays == rays
