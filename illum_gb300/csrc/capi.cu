@@ -892,7 +892,7 @@ int ilg_radiosity_solve_gs(ilg_ctx* ctx, const double* E, int gs_steps, double* 
   if (!c.have_F) { set_error("no form factors"); return ILG_ERR_ARG; }
   ILG_TRY(gs_prepare(c));
   ILG_TRY(ensure_step_buffers(c, ILG_PREC_FP64));
-  double* Ed = c.gs_x.p + 2 * (size_t)c.nt;
+  double* Ed = gs_rhs(c);
   ILG_CUDA(cudaMemcpyAsync(Ed, E, (size_t)c.nt * 8, cudaMemcpyHostToDevice, c.stream));
   ILG_TRY(gs_solve_launch(c, Ed, c.Q.p, gs_steps, c.stream));
   std::vector<double> r2;
@@ -902,7 +902,7 @@ int ilg_radiosity_solve_gs(ilg_ctx* ctx, const double* E, int gs_steps, double* 
     ILG_CUDA(cudaMemcpyAsync(r2.data(), c.gs_x.p, (size_t)c.nt * 8, cudaMemcpyDeviceToHost, c.stream));
   }
   ILG_CUDA(cudaMemcpyAsync(x, c.Q.p, (size_t)c.nt * 8, cudaMemcpyDeviceToHost, c.stream));
-  ILG_CUDA(cudaStreamSynchronize(c.stream));
+  ILG_TRY(read_device_errors(c));   // also waits for the copies
   if (res) {
     double acc = 0.0;   // row order, as the CPU oracle sums
     for (double q : r2) acc += q;

@@ -246,7 +246,9 @@ struct Context {
   bool gs_ready = false;          // gs_rows / gs_lptr describe the current form factors
   dbuf<uint32_t> gs_rows;         // rows in dependency-level order
   std::vector<int> gs_lptr;       // level boundaries in gs_rows
-  dbuf<double> gs_x;              // 3 x N: two iterates and the right-hand side
+  dbuf<int> gs_nlow;              // per row: entries left of the diagonal
+  dbuf<double> gs_x;              // 6 x N: two iterates as (value, sweep) words, E + U x, the right-hand side
+  int gs_grid = 0;                // co-resident blocks of a sweep
 
   // thermal
   bool have_thermal = false;
@@ -372,6 +374,7 @@ int radiosity_barrier_probe(unsigned* bar, int* derr, int blocks, long long poll
 int radiosity_inner(int max_sweeps);
 
 // ---- gauss_seidel.cu ----
+double* gs_rhs(const Context& c);   // the right-hand side's place (N doubles)
 int gs_prepare(Context& c);       // dependency levels of the current form factors (once per F)
 int gs_levels(const Context& c);
 // 1 + gs_steps natural-order sweeps from zero for right-hand side E (device,

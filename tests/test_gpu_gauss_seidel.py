@@ -105,3 +105,30 @@ def test_fixed_sweep_mode_limits(ilg, c0_mesh):
         ilg.Batch([ctx], [mixed])
     with pytest.raises(ilg.IlgError):
         ctx.set_radiosity_mode(7, 1)
+
+
+@pytest.mark.parametrize("level,seed", [(3, 0), (4, 1)])
+def test_fixed_sweeps_row_lengths_around_a_warp(ilg, oracle_mod, level, seed):
+    """Rows of 0, 1, 31, 32, 33, 64, 65 and 300 lower and upper entries, far
+    and near: the warps that add a row's columns 32 at a time, in order, and
+    wait for rows of other warps, give the oracle's sums bit for bit."""
+    v, f = meshgen.icosphere_craters(level, seed=seed)
+    n = f.shape[0]
+    g = np.random.default_rng(seed)
+    rp, cols, vals = [0], [], []
+    for i in range(n):
+        lo = min(i, int(g.choice([0, 0, 1, 31, 32, 33, 64, 65, 300])))
+        up = min(n - 1 - i, int(g.choice([0, 1, 31, 32, 33, 64, 65, 300])))
+        near = np.arange(i - lo, i) if i % 2 else np.sort(g.choice(i, lo, replace=False)) if lo else np.zeros(0, int)
+        c = np.concatenate([near, i + 1 + np.sort(g.choice(n - 1 - i, up, replace=False)) if up else np.zeros(0, int)])
+        cols.append(c)
+        vals.append(g.uniform(0.0, 0.3 / max(1, c.size), c.size))
+        rp.append(rp[-1] + c.size)
+    rp, col, val = np.array(rp, np.int64), np.concatenate(cols).astype(np.int32), np.concatenate(vals)
+    ctx = ilg.IllumContext(v, f)
+    ctx.set_F(rp, col, val)
+    E = g.uniform(0.0, 600.0, n)
+    for steps in (0, 1, 4):
+        x, res = ctx.radiosity_solve_gs(E, steps)
+        xo, reso, _ = oracle_mod.gauss_seidel(rp, col, val, E, mode=0, gs_steps=steps)
+        assert np.array_equal(x, xo) and res == reso
