@@ -103,14 +103,13 @@ constexpr int RAD_NST_MAX = 8;
 constexpr size_t RAD_RING = (size_t)(RAD_NST64 * RAD_STAGE64 > RAD_NSTM * RAD_STAGEM ? RAD_NST64 * RAD_STAGE64
                                                                                         : RAD_NSTM * RAD_STAGEM);
 static_assert(RAD_CF_BYTES % 16 == 0 && RAD_F32_BYTES % 16 == 0, "bulk copies move multiples of 16 bytes");
-static_assert(RAD_NST64 <= RAD_NST_MAX && RAD_NSTM <= RAD_NST_MAX, "stage barriers");
+static_assert(RAD_NST64 + RAD_NSTM <= RAD_NST_MAX, "stage barriers");
 constexpr size_t RAD_SMEM = RAD_RING + (size_t)RAD_HALO * sizeof(float2) + RAD_THREADS * sizeof(float2) +
                             RAD_ROWS * sizeof(float2) + RAD_THREADS + 2 * RAD_NST_MAX * sizeof(unsigned long long);
 
-// Most polls of one grid-barrier wait (about 2^26 x 32 ns before it gives
-// up). A device variable so that a test can shrink it (ilg_debug_barrier_
+// Most polls of one grid-barrier wait (an L2 round trip each, ~0.4 us). A device variable so that a test can shrink it (ilg_debug_barrier_
 // timeout) and watch a wait run out without a long stall.
-constexpr long long BARRIER_POLLS = 1LL << 26;
+constexpr long long BARRIER_POLLS = 1LL << 23;
 __device__ long long g_barrier_polls = BARRIER_POLLS;
 
 // Grid barrier for a cooperative launch (all blocks co-resident) on an
@@ -120,8 +119,13 @@ __device__ long long g_barrier_polls = BARRIER_POLLS;
 // the others with its own increment (no reset on the critical path). The
 // wait is bounded: after g_barrier_polls polls it records DERR_BARRIER and
 // returns false (as does every block that sees the flag while waiting).
-// The fences make the iterates written before the barrier visible to the
-// loads after it.
+// The fence before the arrival and the acquiring load (or fence) after it
+// make the iterates written before the barrier visible to the loads after it.
+__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+  unsigned x;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(x) : "l"(p) : "memory");
+  return x;
+}
 __device__ bool grid_barrier(unsigned* bar, unsigned nblocks, unsigned& gen, int* derr) {
   __shared__ int ok;
   ++gen;
@@ -133,16 +137,16 @@ __device__ bool grid_barrier(unsigned* bar, unsigned nblocks, unsigned& gen, int
     __threadfence();
     if (atomicAdd(bar, 1u) + 1u < target) {
       long long it = 0;
-      while (*(volatile unsigned*)bar < target) {
-        if (++it > limit || *(volatile int*)&derr[DERR_BARRIER]) {
+      while (ld_acquire(bar) < target) {
+        if (++it > limit || ((it & 63) == 0 && *(volatile int*)&derr[DERR_BARRIER])) {
           atomicExch(&derr[DERR_BARRIER], 1);
           ok = 0;
           break;
         }
-        __nanosleep(32);
       }
+    } else {
+      __threadfence();
     }
-    __threadfence();
   }
   __syncthreads();
   return ok != 0;
@@ -169,9 +173,9 @@ __device__ __forceinline__ uint64_t l2_keep_policy(int stream) {
 // waits until a stage is free (its empty barrier), announces the bytes on the
 // stage's full barrier and issues the copies; consumers wait on the full
 // barrier, read their four entries and arrive on the empty barrier. Both
-// sides walk the same sequence of (tile, group) pairs, numbered q from the
-// start of the launch: stage q % nst, use number q / nst, so each wait is on
-// the parity of that use. Every wait is bounded: after RAD_MBAR_POLLS polls
+// sides walk the same sequence of (tile, group) pairs from the start of the
+// launch, stage by stage, so each wait is on the parity of the stage's use.
+// Every wait is bounded: after RAD_MBAR_POLLS polls
 // it records DERR_STREAM, and from then on the block's waits return at once
 // and its consumers treat the stream as empty (all-zero entries, which index
 // no halo value beyond slot 0 and end no row).
@@ -187,17 +191,21 @@ __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
 __device__ __forceinline__ void mbar_expect(unsigned long long* bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
+// true if the use with this parity has completed (the hardware may wait a
+// little for it)
+__device__ __forceinline__ bool mbar_try(unsigned long long* bar, unsigned parity) {
+  unsigned done;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+               "selp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+  return done != 0;
+}
 // true once the use with this parity has completed; false after the poll
 // limit (flagged) or when the block's stream has already failed
 __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity, int* bad, int* derr) {
   if (*(volatile int*)bad) return false;
-  const unsigned a = smem_u32(bar);
   for (long long it = 0; it < RAD_MBAR_POLLS; ++it) {
-    unsigned done;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                 "selp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(done) : "r"(a), "r"(parity) : "memory");
-    if (done) return true;
+    if (mbar_try(bar, parity)) return true;
     if (*(volatile int*)bad) return false;
   }
   *(volatile int*)bad = 1;
@@ -271,8 +279,9 @@ template <> __device__ __forceinline__ void zero_vals(float (&w)[4]) {
   for (int j = 0; j < 4; ++j) w[j] = 0.f;
 }
 
-// The block's stream ring and its sequence position (per thread; every
-// consumer and the producer lane advance it identically).
+// The block's stream ring and its position in it (per thread; every
+// consumer and the producer lane advance it identically): the stage, and the
+// parity of its current use.
 struct Pipe {
   unsigned char* ring;
   unsigned long long* full;
@@ -280,41 +289,50 @@ struct Pipe {
   int* bad;
   int nst;
   int stage_bytes;
-  unsigned q;
+  int s;
+  unsigned parity;
+  __device__ __forceinline__ void advance() {
+    if (++s == nst) {
+      s = 0;
+      parity ^= 1u;
+    }
+  }
 };
 
-// Producer (lane 0 of the producer warp): the copies of every group of tile T.
+// Producer (lane 0 of the producer warp): the copies of every group of tile
+// T. A stage is free once its previous use has been read; the wait on a
+// stage's first use passes at once (the phase before an mbarrier's first
+// counts as completed).
 template <class V>
 __device__ __forceinline__ void produce_tile(Pipe& p, const StepView& v, const RowTile& T, V vals, uint64_t pol) {
   const int ng = T.lam >> 2;
   const unsigned bytes = (unsigned)RAD_CF_BYTES + vals_bytes(vals);
-  for (int g = 0; g < ng; ++g, ++p.q) {
-    const unsigned s = p.q % (unsigned)p.nst, n = p.q / (unsigned)p.nst;
-    if (n > 0 && !mbar_wait(p.empty + s, (n - 1) & 1u, p.bad, v.derr)) continue;
+  for (int g = 0; g < ng; ++g, p.advance()) {
+    if (!mbar_wait(p.empty + p.s, p.parity ^ 1u, p.bad, v.derr)) continue;
     if (*(volatile int*)p.bad) continue;
-    const unsigned dst = smem_u32(p.ring + (size_t)s * p.stage_bytes);
+    const unsigned dst = smem_u32(p.ring + (size_t)p.s * p.stage_bytes);
     const size_t e = (size_t)T.e0 + (size_t)g * RAD_GROUP;
-    mbar_expect(p.full + s, bytes);
-    bulk_copy(dst, v.t_cf + e, RAD_CF_BYTES, p.full + s, pol);
-    copy_vals(vals, dst + RAD_CF_BYTES, e, p.full + s, pol);
+    mbar_expect(p.full + p.s, bytes);
+    bulk_copy(dst, v.t_cf + e, RAD_CF_BYTES, p.full + p.s, pol);
+    copy_vals(vals, dst + RAD_CF_BYTES, e, p.full + p.s, pol);
   }
 }
 
 // Consumer: the next group's four entries of this thread (columns and
-// values), then the stage is released.
+// values), then the stage is released (one arrival per warp).
 template <class V, class W>
 __device__ __forceinline__ void take_group(Pipe& p, const StepView& v, V vals, uint2& c, W (&w)[4]) {
-  const unsigned s = p.q % (unsigned)p.nst, n = p.q / (unsigned)p.nst;
-  ++p.q;
-  const unsigned char* st = p.ring + (size_t)s * p.stage_bytes;
-  if (mbar_wait(p.full + s, n & 1u, p.bad, v.derr)) {
+  const unsigned char* st = p.ring + p.s * p.stage_bytes;
+  if (mbar_try(p.full + p.s, p.parity) || mbar_wait(p.full + p.s, p.parity, p.bad, v.derr)) {
     c = *reinterpret_cast<const uint2*>(st + 8 * threadIdx.x);
     read_vals(vals, st + RAD_CF_BYTES, threadIdx.x, w);
   } else {
     c = make_uint2(0u, 0u);
     zero_vals(w);
   }
-  mbar_arrive(p.empty + s);
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(p.empty + p.s);
+  p.advance();
 }
 
 // Barrier of the consumer threads only (the producer warp does not take
@@ -461,7 +479,12 @@ __device__ __forceinline__ void stage_halo_sum(const StepView& v, const RowTile&
   cbar();
 }
 
-// One tile: thread t owns entries [t*lam, (t+1)*lam) of the tile's entry
+// The thread's first row in tile t (t_start), loaded ahead of its use.
+__device__ __forceinline__ uint32_t tile_start(const StepView& v, int t) {
+  return __ldg(v.t_start + (size_t)t * RAD_THREADS + threadIdx.x);
+}
+
+// One tile (s0: tile_start): thread t owns entries [t*lam, (t+1)*lam) of the tile's entry
 // stream (rows in order, each row's entries in column order), stored so that
 // a group of 4 RAD_THREADS entries is contiguous: entry k of thread t at
 // e0 + (k/4)*RAD_GROUP + 4t + k%4. The groups arrive in shared memory by
@@ -472,44 +495,52 @@ __device__ __forceinline__ void stage_halo_sum(const StepView& v, const RowTile&
 // order, then its own part. Ends with a consumer barrier: rs holds every
 // row sum of the tile.
 template <class Acc, class V>
-__device__ __forceinline__ void tile_rows(const StepView& v, const RowTile& T, int t, Pipe& p, V vals,
+__device__ __forceinline__ void tile_rows(const StepView& v, const RowTile& T, uint32_t s0, Pipe& p, V vals,
                                           const typename Acc::X* sx, typename Acc::Part* tail, unsigned char* tnew,
                                           typename Acc::Sum* rs) {
   typedef typename Acc::W W;
   const int tid = threadIdx.x;
-  const uint32_t s0 = __ldg(v.t_start + (size_t)t * RAD_THREADS + tid);
-  int r = (int)(s0 & 0x7fffffffu);
+  const int r = (int)(s0 & 0x7fffffffu);
   const bool cont = (s0 >> 31) != 0;
-  bool any = false, has_head = false;
-  int head_row = 0;
-  Acc acc, head;
+  // where the open row's sum goes when the row ends: rs, or for a row that
+  // began in an earlier thread the thread's own tail slot (read back below)
+  typename Acc::Sum* const first = cont ? tail + tid : rs + r;
+  typename Acc::Sum *dst = first, *next = rs + r + 1;
+  Acc acc;
   acc.zero();
-  head.zero();
   const int ng = T.lam >> 2;
+  // without a branch: a warp has a row end in most groups, but few lanes do
+  // (eight lanes per run, with neighbouring halo values and segmented scans at
+  // the row ends, were 1.6 times slower)
   auto elem = [&](uint32_t c, W w) {
     acc.add(w, sx[c & 0x7fffu]);
     if (c & 0x8000u) {
-      if (cont && !any) {
-        head = acc;
-        head_row = r;
-        has_head = true;
-      } else {
-        rs[r] = acc.get();
-      }
-      ++r;
+      *dst = acc.get();
+      dst = next;
+      ++next;
       acc.zero();
-      any = true;
     }
   };
   for (int g = 0; g < ng; ++g) {
     uint2 c;
     W w[4];
     take_group(p, v, vals, c, w);
-    elem(c.x & 0xffffu, w[0]);
-    elem(c.x >> 16, w[1]);
-    elem(c.y & 0xffffu, w[2]);
-    elem(c.y >> 16, w[3]);
+    if (__any_sync(0xffffffffu, ((c.x | c.y) & 0x80008000u) != 0)) {
+      elem(c.x & 0xffffu, w[0]);
+      elem(c.x >> 16, w[1]);
+      elem(c.y & 0xffffu, w[2]);
+      elem(c.y >> 16, w[3]);
+    } else {
+      acc.add(w[0], sx[c.x & 0x7fffu]);
+      acc.add(w[1], sx[c.x >> 16]);
+      acc.add(w[2], sx[c.y & 0x7fffu]);
+      acc.add(w[3], sx[c.y >> 16]);
+    }
   }
+  const bool any = dst != first, has_head = cont && any;
+  Acc head;
+  head.zero();
+  if (has_head) head.merge(tail[tid]);
   tail[tid] = acc.part();
   tnew[tid] = (any || !cont) ? 1 : 0;
   cbar();
@@ -520,7 +551,7 @@ __device__ __forceinline__ void tile_rows(const StepView& v, const RowTile& T, i
     s.zero();
     for (; u < tid; ++u) s.merge(tail[u]);
     s.merge(head.part());
-    rs[head_row] = s.get();
+    rs[r] = s.get();
   }
   cbar();
 }
@@ -549,8 +580,8 @@ __device__ __forceinline__ float block_sum(float d, float* red) {
 // total after the grid barrier and takes the same decision with one load,
 // and a mesh's decisions are the same alone and in a batch. A mesh stops
 // when its total is <= 2^20 units, i.e. sum of partials <= tol^2 (at most
-// ntiles units conservative). The accumulators follow the barrier's two
-// counter words, three buffers of RES_LEVELS x nmesh by residual number
+// ntiles units conservative). The accumulators lie in the barrier's buffer,
+// three buffers of RES_LEVELS x nmesh by residual number
 // mod 3: buffer k + 1 is cleared during residual k (its last reader,
 // decision k - 2, finished before the barrier that precedes residual k), and
 // the accumulators of residual 0 are cleared before the first barrier. The
@@ -561,8 +592,13 @@ constexpr unsigned long long RES_UNITS = 1ull << 20;
 constexpr unsigned long long RES_CAP = 1ull << 40;
 constexpr int RES_LEVELS = 3;
 
+// Words of the barrier buffer before the solo solve's sweep words (grid <=
+// RAD_MAX_GRID blocks, 2 x 16 bytes each), and before the accumulators.
+constexpr int RAD_MAX_GRID = 1024;
+constexpr int RAD_BAR_WORDS0 = 4;
+constexpr int RAD_BAR_WORDS1 = RAD_BAR_WORDS0 + RAD_MAX_GRID * 8;
 __device__ __forceinline__ unsigned long long* res_acc(const StepView& v, int k, int level = 0) {
-  return reinterpret_cast<unsigned long long*>(v.barrier + 2) + (size_t)((k % 3) * RES_LEVELS + level) * v.nmesh;
+  return reinterpret_cast<unsigned long long*>(v.barrier + RAD_BAR_WORDS1) + (size_t)((k % 3) * RES_LEVELS + level) * v.nmesh;
 }
 
 // done[m]: 0 running; 1 + (parity of the mesh's last residual) once
@@ -679,28 +715,54 @@ constexpr float CHG_NOISE = 1.1920929e-7f;                             // 2^-23
 constexpr float CHG_REFRESH = 9.5367432e-7f;                           // 2^-20
 constexpr float CHG_RANGE = 5.6294995e14f;   // 2^49: above it the totals are at their cap
 
+// A partial in residual units, and the level they are counted at.
+__device__ __forceinline__ unsigned long long res_units64(float d2, float unit, int& level) {
+  level = 2;
+  if (isnan(d2)) return RES_CAP;
+  const float q = d2 > 0.f ? __fmul_ru(d2, unit) : 0.f;
+  const float cap = (float)RES_CAP;   // 2^40, exact
+  if (q < cap) {
+    level = 0;
+    return (unsigned long long)ceilf(q);
+  }
+  if (q < cap * cap) {
+    level = 1;
+    return (unsigned long long)ceilf(q * (1.f / cap));
+  }
+  const float q2 = q * (1.f / cap) * (1.f / cap);
+  return q2 < cap ? (unsigned long long)ceilf(q2) : RES_CAP;
+}
+
 // Thread 0, after block_sum: record tile t's partial of residual k.
 __device__ __forceinline__ void post_partial64(const StepView& v, const RowTile& T, int t, int k, float unit,
                                                float d2) {
   if (threadIdx.x != 0) return;
   v.tile_d2[(size_t)(k & 1) * v.ntiles + t] = (double)d2;
-  int level = 2;
-  unsigned long long u = RES_CAP;      // NaN and anything beyond level 2
-  if (!isnan(d2)) {
-    const float q = d2 > 0.f ? __fmul_ru(d2, unit) : 0.f;
-    const float cap = (float)RES_CAP;   // 2^40, exact
-    if (q < cap) {
-      level = 0;
-      u = (unsigned long long)ceilf(q);
-    } else if (q < cap * cap) {
-      level = 1;
-      u = (unsigned long long)ceilf(q * (1.f / cap));
-    } else if (q * (1.f / cap) * (1.f / cap) < cap) {
-      u = (unsigned long long)ceilf(q * (1.f / cap) * (1.f / cap));
-    }
-  }
+  int level;
+  const unsigned long long u = res_units64(d2, unit, level);
   if (u) atomicAdd(res_acc(v, k, level) + T.mesh, u);
   for (int l = 0; l < RES_LEVELS; ++l) res_acc(v, k + 1, l)[T.mesh] = 0ull;
+}
+
+// What follows a sweep (see above): dn and the flags from the totals.
+struct Sweep64 {
+  bool stop, next_change;
+  float dn;   // |d| / tol
+};
+__device__ __forceinline__ Sweep64 sweep_decision(unsigned long long q0, unsigned long long q1, unsigned long long q2,
+                                                  bool change, float acc) {
+  const float cap = (float)RES_CAP;
+  Sweep64 r;
+  r.dn = sqrtf((float)q0 + cap * ((float)q1 + cap * (float)q2)) * (1.f / 1024.f);
+  if (change) {
+    const bool small = r.dn <= CHG_STOP;
+    r.stop = small && CHG_NOISE * acc <= CHG_NOISE_STOP;
+    r.next_change = !small && r.dn > CHG_REFRESH * acc && r.dn < CHG_RANGE;
+  } else {
+    r.stop = q1 == 0 && q2 == 0 && q0 <= RES_UNITS;
+    r.next_change = r.dn < CHG_RANGE;
+  }
+  return r;
 }
 
 __device__ __forceinline__ void init_meshes64(const StepView& v, MeshState64& st) {
@@ -725,38 +787,34 @@ __device__ __forceinline__ int decide_meshes64(const StepView& v, MeshState64& s
     if (run) {
       const unsigned long long q0 = __ldcg(res_acc(v, k, 0) + m), q1 = __ldcg(res_acc(v, k, 1) + m),
                                q2 = __ldcg(res_acc(v, k, 2) + m);
-      const float cap = (float)RES_CAP;
-      const float dn = sqrtf((float)q0 + cap * ((float)q1 + cap * (float)q2)) * (1.f / 1024.f);   // |d| / tol
       const bool change = st.mode[m] & 1;
       const int sw = ++st.sweeps[m];
-      float acc = st.acc[m];
-      bool stop, next_change;
-      if (change) {
-        const bool small = dn <= CHG_STOP;
-        stop = small && CHG_NOISE * acc <= CHG_NOISE_STOP;
-        next_change = !small && dn > CHG_REFRESH * acc && dn < CHG_RANGE;
-        acc += dn;
-      } else {
-        stop = q1 == 0 && q2 == 0 && q0 <= RES_UNITS;
-        next_change = dn < CHG_RANGE;
-        acc = dn;
-        st.mode[m] ^= 2;
-      }
+      const float acc0 = st.acc[m];
+      const Sweep64 dec = sweep_decision(q0, q1, q2, change, acc0);
+      if (!change) st.mode[m] ^= 2;
       const int budget = v.md[m].max_sweeps;
-      st.mode[m] = (st.mode[m] & 2) | (next_change && sw + 1 < budget ? 1 : 0);
-      if (stop || sw >= budget) {
+      st.mode[m] = (st.mode[m] & 2) | (dec.next_change && sw + 1 < budget ? 1 : 0);
+      if (dec.stop || sw >= budget) {
         st.done[m] = 1 + (k & 1);
         run = false;
         // the errors of a change sweep that was the last (A without the last |d|)
-        st.acc[m] = change ? acc - dn : 0.f;
+        st.acc[m] = change ? acc0 : 0.f;
       } else {
-        st.acc[m] = acc;
+        st.acc[m] = change ? acc0 + dec.dn : dec.dn;
       }
       if (blockIdx.x == 0) v.md[m].sweeps = sw;
     }
     running += __syncthreads_count(run);
   }
   return running;
+}
+
+// Squared residual plus the bound on the change sweeps' errors.
+__device__ __forceinline__ double with_errors(double r2, float acc, double tol2) {
+  const float err = CHG_NOISE * acc;   // units of tol
+  if (!(err > 0.f)) return r2;
+  const double r = sqrt(r2) + (double)err * sqrt(tol2);
+  return r * r;
 }
 
 // Block 0, at the end of the launch: each solved mesh's last residual into
@@ -772,14 +830,7 @@ __device__ __forceinline__ void record_residuals64(const StepView& v, const Mesh
     double t = 0.0;
     for (int j = lane; j < M.ntiles; j += 32) t += ld_it(d2 + M.tile0 + j);
     t = warp_sum(t);
-    if (lane == 0) {
-      const float err = CHG_NOISE * st.acc[m];   // units of tol
-      if (err > 0.f) {
-        const double r = sqrt(t) + (double)err * sqrt(M.tol2);
-        t = r * r;
-      }
-      v.md[m].res2 = t;
-    }
+    if (lane == 0) v.md[m].res2 = with_errors(t, st.acc[m], M.tol2);
   }
 }
 
@@ -923,10 +974,11 @@ __device__ __forceinline__ void init_x(const StepView& v, double* x, int warm, i
 }
 
 // Scatter the solved meshes' last iterate x = E + s back to facet order
-// (FP64); warm solves also record s and its change for the next step's start. Rows
-// without entries keep s = 0 in both buffers.
-__device__ __forceinline__ void scatter_x(const StepView& v, const MeshState64& st, double* x, int warm, int gt,
-                                          int nthreads) {
+// (FP64); warm solves also record s and its change for the next step's start.
+// Rows without entries keep s = 0 in both buffers. src(p): the buffer of
+// position p's s, or nullptr where its mesh was not solved.
+template <class Src>
+__device__ __forceinline__ void scatter_from(const StepView& v, Src src, double* x, int warm, int gt, int nthreads) {
   const RadBufs B(v);
   for (int p0 = gt; p0 < v.nt; p0 += RAD_ILP * nthreads) {
     int g[RAD_ILP];
@@ -938,12 +990,11 @@ __device__ __forceinline__ void scatter_x(const StepView& v, const MeshState64& 
       const int p = p0 + k * nthreads;
       ok[k] = false;
       if (p >= v.nt) continue;
-      const int m = mesh_of_facet(v, p);
-      const MeshDesc& M = v.md[m];
-      if (!M.active || M.ntiles == 0) continue;
+      const float2* S = src(p);
+      if (!S) continue;
       ok[k] = true;
       g[k] = (int)v.rperm[p];
-      s[k] = ld_it(((st.mode[m] & 2) ? B.S1 : B.S0) + p);
+      s[k] = ld_it(S + p);
       e[k] = B.EP[p];
       sp[k] = warm ? v.sprev[p] : make_float2(0.f, 0.f);
     }
@@ -958,6 +1009,20 @@ __device__ __forceinline__ void scatter_x(const StepView& v, const MeshState64& 
       }
     }
   }
+}
+__device__ __forceinline__ void scatter_x(const StepView& v, const MeshState64& st, double* x, int warm, int gt,
+                                          int nthreads) {
+  const RadBufs B(v);
+  scatter_from(v, [&](int p) -> const float2* {
+    const int m = mesh_of_facet(v, p);
+    const MeshDesc& M = v.md[m];
+    if (!M.active || M.ntiles == 0) return nullptr;
+    return (st.mode[m] & 2) ? B.S1 : B.S0;
+  }, x, warm, gt, nthreads);
+}
+__device__ __forceinline__ void scatter_solo(const StepView& v, const float2* S, double* x, int warm, int gt,
+                                             int nthreads) {
+  scatter_from(v, [&](int) { return S; }, x, warm, gt, nthreads);
 }
 
 // The rows of this block's tiles whose mesh stopped at the latest decision
@@ -996,7 +1061,7 @@ struct RadSmem {
   float2* rs;                // row sums of the tile (RAD_ROWS double-floats, or floats)
   unsigned char* tnew;       // per thread: its last open row began in its run
   unsigned long long* full;  // per stage: its copies have landed
-  unsigned long long* empty; // per stage: every consumer has read it
+  unsigned long long* empty; // per stage: every consumer warp has read it
 };
 
 __device__ __forceinline__ RadSmem rad_smem() {
@@ -1016,12 +1081,13 @@ static_assert((RAD_RING + (size_t)(RAD_HALO + RAD_THREADS + RAD_ROWS) * 8 + RAD_
 
 // The ring's barriers, set up by thread 0 before the launch's first block
 // barrier (inside init_meshes' caller): full counts the producer's one
-// arrival plus the copied bytes, empty one arrival per consumer thread.
-__device__ __forceinline__ Pipe make_pipe(const RadSmem& m, int nst, int stage_bytes, int* bad) {
+// arrival plus the copied bytes, empty one arrival per consumer warp.
+// first: the first of its barriers (pipes that share the ring take turns).
+__device__ __forceinline__ Pipe make_pipe(const RadSmem& m, int nst, int stage_bytes, int* bad, int first = 0) {
   if (threadIdx.x == 0) {
-    for (int s = 0; s < nst; ++s) {
+    for (int s = first; s < first + nst; ++s) {
       mbar_init(m.full + s, 1);
-      mbar_init(m.empty + s, RAD_THREADS);
+      mbar_init(m.empty + s, RAD_THREADS / 32);
     }
     *bad = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1029,12 +1095,13 @@ __device__ __forceinline__ Pipe make_pipe(const RadSmem& m, int nst, int stage_b
   __syncthreads();
   Pipe p;
   p.ring = m.ring;
-  p.full = m.full;
-  p.empty = m.empty;
+  p.full = m.full + first;
+  p.empty = m.empty + first;
   p.bad = bad;
   p.nst = nst;
   p.stage_bytes = stage_bytes;
-  p.q = 0;
+  p.s = 0;
+  p.parity = 0;
   return p;
 }
 
@@ -1096,8 +1163,9 @@ __global__ void __launch_bounds__(RAD_BLOCK, 1) k_radiosity64(StepView v, double
         if (mode & 1) {
           float* sxf = reinterpret_cast<float*>(sm.sx);
           float* rsf = reinterpret_cast<float*>(sm.rs);
+          const uint32_t s0 = tile_start(v, t);
           stage_halo(v, T, dcur, sxf);
-          tile_rows<AccF32>(v, T, t, pipe, vhi, sxf, reinterpret_cast<float*>(sm.tail), sm.tnew, rsf);
+          tile_rows<AccF32>(v, T, s0, pipe, vhi, sxf, reinterpret_cast<float*>(sm.tail), sm.tnew, rsf);
           for (int r = threadIdx.x; r < T.nrows; r += RAD_THREADS) {
             const uint32_t i = __ldg(rows + r);
             const float d = rsf[r];              // d' = F d
@@ -1107,8 +1175,9 @@ __global__ void __launch_bounds__(RAD_BLOCK, 1) k_radiosity64(StepView v, double
           }
         } else {
           float2* nxt = (mode & 2) ? B.S0 : B.S1;
+          const uint32_t s0 = tile_start(v, t);
           stage_halo_sum(v, T, B.EH, cur, sm.sx);
-          tile_rows<AccDF>(v, T, t, pipe, vals, sm.sx, sm.tail, sm.tnew, sm.rs);
+          tile_rows<AccDF>(v, T, s0, pipe, vals, sm.sx, sm.tail, sm.tnew, sm.rs);
           for (int r = threadIdx.x; r < T.nrows; r += RAD_THREADS) {
             const uint32_t i = __ldg(rows + r);
             const float2 sn = sm.rs[r];          // s' = F x
@@ -1129,6 +1198,231 @@ __global__ void __launch_bounds__(RAD_BLOCK, 1) k_radiosity64(StepView v, double
   }
   if (!producer) scatter_x(v, st, x, warm, gt, nthreads);
   record_residuals64(v, st);
+}
+
+// ---- the FP64 solve of one mesh with one tile per block ----
+//
+// The same sweeps on the same tiles, bit for bit, for the usual single-mesh
+// solve. A sweep of such a mesh is short (about 1 us of entries per block for
+// 5,120 facets, 5 us for 81,920), so what it waits for decides: after a grid
+// barrier the L1 is empty and every load is an L2 round trip. Here
+// everything that does not change from sweep to sweep (the tile, the halo's
+// and rows' positions, each thread's first row) and the block's own s stay in
+// registers, and the barrier carries the residual: each block publishes its
+// partial with the sweep's number in one 128-bit word, and every block reads
+// all of them, instead of an atomic counter to wait for and a total to load
+// after it.
+// tile_d2 and the totals are those of k_radiosity64, so the decisions are.
+// 81,920 facets, 8.1 M entries: a change sweep takes 11.6 us (7 us of it the
+// entries, bound by integer and LDS issue: the copies alone run at 10.9 TB/s
+// from L2; 2.4 us the spread between blocks), 16.8 us a full one; in
+// k_radiosity64 they took 12.5 and 18.3 us.
+struct __align__(16) SweepWord {
+  unsigned long long units, tag;   // residual units; level << 32 | sweep number (from 1)
+};
+__device__ __forceinline__ SweepWord* sweep_words(const StepView& v) {
+  return reinterpret_cast<SweepWord*>(v.barrier + RAD_BAR_WORDS0);
+}
+__device__ __forceinline__ void word_store(SweepWord* p, unsigned long long a, unsigned long long b) {
+  asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}"
+               ::"l"(p), "l"(a), "l"(b) : "memory");
+}
+__device__ __forceinline__ SweepWord word_load(const SweepWord* p) {
+  SweepWord w;
+  asm volatile("{\n\t.reg .b128 t;\n\tld.acquire.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+               : "=l"(w.units), "=l"(w.tag) : "l"(p) : "memory");
+  return w;
+}
+
+struct SoloShared {
+  float red[32];
+  int bad, ok, mode, stop;   // mode as MeshState64::mode
+  float acc;
+};
+
+constexpr int SOLO_ROWS = (RAD_ROWS + RAD_THREADS - 1) / RAD_THREADS;   // rows of a thread (4)
+constexpr int SOLO_HALO = 4;                                            // halo positions kept per thread
+
+// End of sweep `it` of the block whose partial is d2 (thread 0's): publish,
+// wait for every block's, and decide. All threads; false once a wait ran out.
+// A word is written after a fence and read by an acquiring load, so what the
+// other blocks stored before theirs is visible to the loads after this (a
+// fence after the wait instead: 0.2 us a sweep more).
+__device__ __forceinline__ bool solo_sweep_end(const StepView& v, SoloShared& S, int it, float d2, float unit,
+                                               int budget) {
+  __syncthreads();   // the block's stores of this sweep come before its word
+  const unsigned nb = gridDim.x;
+  SweepWord* words = sweep_words(v);
+  if (threadIdx.x == 0) {
+    int level;
+    const unsigned long long u = res_units64(d2, unit, level);
+    __threadfence();
+    word_store(words + 2 * blockIdx.x + (it & 1), u, ((unsigned long long)level << 32) | (unsigned)(it + 1));
+  }
+  if (threadIdx.x < 32) {
+    unsigned long long q0 = 0, q1 = 0, q2 = 0;
+    bool ok = true;
+    const long long limit = g_barrier_polls;
+    for (unsigned b = threadIdx.x; b < nb && ok; b += 32) {
+      SweepWord w;
+      for (long long poll = 0;; ++poll) {
+        w = word_load(words + 2 * b + (it & 1));
+        if ((unsigned)w.tag == (unsigned)(it + 1)) break;
+        if (poll > limit || ((poll & 255) == 255 && *(volatile int*)&v.derr[DERR_BARRIER])) {
+          atomicExch(&v.derr[DERR_BARRIER], 1);
+          ok = false;
+          break;
+        }
+      }
+      const int level = (int)(w.tag >> 32);
+      q0 += level == 0 ? w.units : 0ull;
+      q1 += level == 1 ? w.units : 0ull;
+      q2 += level == 2 ? w.units : 0ull;
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    for (int o = 16; o; o >>= 1) {
+      q0 += __shfl_xor_sync(0xffffffffu, q0, o);
+      q1 += __shfl_xor_sync(0xffffffffu, q1, o);
+      q2 += __shfl_xor_sync(0xffffffffu, q2, o);
+    }
+    if (threadIdx.x == 0) {
+      const bool change = S.mode & 1;
+      const float acc0 = S.acc;
+      const Sweep64 dec = sweep_decision(q0, q1, q2, change, acc0);
+      const int cur = change ? S.mode & 2 : (S.mode & 2) ^ 2;
+      const int sw = it + 1;
+      S.mode = cur | (dec.next_change && sw + 1 < budget ? 1 : 0);
+      S.stop = dec.stop || sw >= budget;
+      if (S.stop) S.acc = change ? acc0 : 0.f;
+      else S.acc = change ? acc0 + dec.dn : dec.dn;
+      S.ok = ok;
+    }
+  }
+  __syncthreads();
+  return S.ok != 0;
+}
+
+__global__ void __launch_bounds__(RAD_BLOCK, 1) k_radiosity64_solo(StepView v, double* x, int warm) {
+  __shared__ SoloShared S;
+  const RadSmem sm = rad_smem();
+  const bool producer = threadIdx.x >= RAD_THREADS;
+  const int gt = blockIdx.x * RAD_THREADS + threadIdx.x;
+  const int nthreads = gridDim.x * RAD_THREADS;
+  const int t = v.blk_tile[v.blk_start[blockIdx.x]];
+  const RowTile T = v.tiles[t];
+  const float unit = v.md[0].res_unit;
+  const int budget = v.md[0].max_sweeps;
+  if (!v.md[0].active) return;
+  // the ring holds three groups of a full sweep or five of a change sweep
+  // (every group of a sweep is taken before the next sweep's first copy)
+  Pipe pipe = make_pipe(sm, RAD_NST64, RAD_STAGE64, &S.bad);
+  Pipe pipe32 = make_pipe(sm, RAD_NSTM, RAD_STAGEM, &S.bad, RAD_NST64);
+  if (threadIdx.x == 0) {
+    S.mode = 0;
+    S.acc = 0.f;
+  }
+  const RadBufs B(v);
+  const ValsDF vals{v.t_vhi, v.t_vlo};
+  const ValsHiF vhi{v.t_vhi};
+  const uint64_t pol = l2_keep_policy(v.l2_stream);
+  uint32_t s0 = 0, hpos[SOLO_HALO], rpos[SOLO_ROWS];
+  if (!producer) {
+    init_x(v, x, warm, gt, nthreads, false);
+    s0 = tile_start(v, t);
+#pragma unroll
+    for (int q = 0; q < SOLO_HALO; ++q) {
+      const int h = threadIdx.x + q * RAD_THREADS;
+      hpos[q] = h < T.nhalo ? __ldg(v.t_halo + T.h0 + h) : 0u;
+    }
+#pragma unroll
+    for (int q = 0; q < SOLO_ROWS; ++q) {
+      const int r = threadIdx.x + q * RAD_THREADS;
+      rpos[q] = r < T.nrows ? __ldg(v.t_row + T.r0 + r) : 0u;
+    }
+  }
+  unsigned gen = 0;
+  if (!grid_barrier(v.barrier, gridDim.x, gen, v.derr)) return;
+  float2 sown[SOLO_ROWS];
+  if (!producer) {
+#pragma unroll
+    for (int q = 0; q < SOLO_ROWS; ++q)
+      sown[q] = threadIdx.x + q * RAD_THREADS < T.nrows ? ld_it(B.S0 + rpos[q]) : make_float2(0.f, 0.f);
+  }
+  int it = 0;
+  for (;; ++it) {
+    const int mode = S.mode;
+    float d2 = 0.f;
+    if (producer) {
+      if ((threadIdx.x & 31) == 0) {
+        if (mode & 1) produce_tile(pipe32, v, T, vhi, pol);
+        else produce_tile(pipe, v, T, vals, pol);
+      }
+      __syncwarp();
+    } else {
+      float2* cur = (mode & 2) ? B.S1 : B.S0;
+      const float* dcur = (it & 1) ? B.D1 : B.D0;
+      float* dnxt = (it & 1) ? B.D0 : B.D1;
+      if (mode & 1) {
+        float* sxf = reinterpret_cast<float*>(sm.sx);
+        float* rsf = reinterpret_cast<float*>(sm.rs);
+        float g[SOLO_HALO];
+#pragma unroll
+        for (int q = 0; q < SOLO_HALO; ++q)
+          if (threadIdx.x + q * RAD_THREADS < T.nhalo) g[q] = ld_it(dcur + hpos[q]);
+#pragma unroll
+        for (int q = 0; q < SOLO_HALO; ++q)
+          if (threadIdx.x + q * RAD_THREADS < T.nhalo) sxf[threadIdx.x + q * RAD_THREADS] = g[q];
+        for (int h = threadIdx.x + SOLO_HALO * RAD_THREADS; h < T.nhalo; h += RAD_THREADS)
+          sxf[h] = ld_it(dcur + __ldg(v.t_halo + T.h0 + h));
+        cbar();
+        tile_rows<AccF32>(v, T, s0, pipe32, vhi, sxf, reinterpret_cast<float*>(sm.tail), sm.tnew, rsf);
+#pragma unroll
+        for (int q = 0; q < SOLO_ROWS; ++q) {
+          const int r = threadIdx.x + q * RAD_THREADS;
+          if (r < T.nrows) {
+            const float d = rsf[r];
+            sown[q] = df_add(sown[q], make_float2(d, 0.f));
+            cur[rpos[q]] = sown[q];
+            dnxt[rpos[q]] = d;
+            d2 = __fmaf_rn(d, d, d2);
+          }
+        }
+      } else {
+        float2* nxt = (mode & 2) ? B.S0 : B.S1;
+        stage_halo_sum(v, T, B.EH, cur, sm.sx);
+        tile_rows<AccDF>(v, T, s0, pipe, vals, sm.sx, sm.tail, sm.tnew, sm.rs);
+#pragma unroll
+        for (int q = 0; q < SOLO_ROWS; ++q) {
+          const int r = threadIdx.x + q * RAD_THREADS;
+          if (r < T.nrows) {
+            const float2 sn = sm.rs[r];
+            const float d = __fadd_rn(__fsub_rn(sn.x, sown[q].x), __fsub_rn(sn.y, sown[q].y));
+            sown[q] = sn;
+            nxt[rpos[q]] = sn;
+            dnxt[rpos[q]] = d;
+            d2 = __fmaf_rn(d, d, d2);
+          }
+        }
+      }
+      d2 = block_sum(d2, S.red);
+      if (threadIdx.x == 0) v.tile_d2[(size_t)(it & 1) * v.ntiles + t] = (double)d2;
+    }
+    if (!solo_sweep_end(v, S, it, d2, unit, budget)) return;
+    if (S.stop) break;
+  }
+  if (!producer) {
+    scatter_solo(v, (S.mode & 2) ? B.S1 : B.S0, x, warm, gt, nthreads);
+    if (blockIdx.x == 0 && threadIdx.x < 32) {
+      double r2 = 0.0;
+      const double* d2 = v.tile_d2 + (size_t)(it & 1) * v.ntiles;
+      for (int j = threadIdx.x; j < v.ntiles; j += 32) r2 += ld_it(d2 + j);
+      r2 = warp_sum(r2);
+      if (threadIdx.x == 0) {
+        v.md[0].sweeps = it + 1;
+        v.md[0].res2 = with_errors(r2, S.acc, v.md[0].tol2);
+      }
+    }
+  }
 }
 
 // Mixed precision: outer refinement with the residual r = E - (I - fl(F)) x
@@ -1171,8 +1465,9 @@ __global__ void __launch_bounds__(RAD_BLOCK, 1) k_radiosity_mixed(StepView v, do
     const int t = v.blk_tile[k];
         const RowTile T = v.tiles[t];
         if (st.done[T.mesh]) continue;
+        const uint32_t s0 = tile_start(v, t);
         stage_halo(v, T, XH, sm.sx);
-        tile_rows<AccDF>(v, T, t, pipe, vhi, sm.sx, sm.tail, sm.tnew, sm.rs);
+        tile_rows<AccDF>(v, T, s0, pipe, vhi, sm.sx, sm.tail, sm.tnew, sm.rs);
         const uint32_t* rows = v.t_row + T.r0;
         float d2 = 0.f;
         for (int r = threadIdx.x; r < T.nrows; r += RAD_THREADS) {
@@ -1205,8 +1500,9 @@ __global__ void __launch_bounds__(RAD_BLOCK, 1) k_radiosity_mixed(StepView v, do
     const int t = v.blk_tile[k];
           const RowTile T = v.tiles[t];
           if (st.done[T.mesh]) continue;
+          const uint32_t s0 = tile_start(v, t);
           stage_halo(v, T, cur, sxf);
-          tile_rows<AccF32>(v, T, t, pipe, vbf, sxf, tailf, sm.tnew, rsf);
+          tile_rows<AccF32>(v, T, s0, pipe, vbf, sxf, tailf, sm.tnew, rsf);
           const uint32_t* rows = v.t_row + T.r0;
           const float* scale = v.t_scale + T.r0;
           if (it + 1 < inner) {
@@ -1323,9 +1619,10 @@ __global__ void __launch_bounds__(RAD_BLOCK, 1) k_radiosity_lagged(StepView v, d
       const RowTile T = v.tiles[t];
       if (st.done[T.mesh]) continue;
       const int kd = kind[T.mesh];
+      const uint32_t s0t = tile_start(v, t);
       stage_halo(v, T, XD, sm.sx);
-      if (kd) tile_rows<AccF2>(v, T, t, pipe, vhi, sm.sx, sm.tail, sm.tnew, sm.rs);
-      else tile_rows<AccF2>(v, T, t, pipe, vbf, sm.sx, sm.tail, sm.tnew, sm.rs);
+      if (kd) tile_rows<AccF2>(v, T, s0t, pipe, vhi, sm.sx, sm.tail, sm.tnew, sm.rs);
+      else tile_rows<AccF2>(v, T, s0t, pipe, vbf, sm.sx, sm.tail, sm.tnew, sm.rs);
       const uint32_t* rows = v.t_row + T.r0;
       const float* scale = v.t_scale + T.r0;
       float d2 = 0.f;
@@ -1502,10 +1799,14 @@ int radiosity_setup() {
   ILG_CUDA(cudaGetDevice(&dev));
   ILG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   ILG_CUDA(cudaFuncSetAttribute(k_radiosity64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RAD_SMEM));
+  ILG_CUDA(cudaFuncSetAttribute(k_radiosity64_solo, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RAD_SMEM));
   ILG_CUDA(cudaFuncSetAttribute(k_radiosity_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RAD_SMEM));
   ILG_CUDA(cudaFuncSetAttribute(k_radiosity_lagged, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RAD_SMEM));
   ILG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_rad_per_sm64, k_radiosity64, RAD_BLOCK, RAD_SMEM));
   ILG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_rad_per_smm, k_radiosity_mixed, RAD_BLOCK, RAD_SMEM));
+  int per_solo = 0;     // the two FP64 kernels share the grid
+  ILG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_solo, k_radiosity64_solo, RAD_BLOCK, RAD_SMEM));
+  g_rad_per_sm64 = std::min(g_rad_per_sm64, per_solo);
   int per_lagged = 0;   // the two mixed kernels share the grid
   ILG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_lagged, k_radiosity_lagged, RAD_BLOCK, RAD_SMEM));
   g_rad_per_smm = std::min(g_rad_per_smm, per_lagged);
@@ -1847,7 +2148,7 @@ float radiosity_res_unit(double tol2) {
   return tol2 > 0.0 ? (float)((double)RES_UNITS / tol2 * (1.0 + 1.0 / 65536.0)) : INFINITY;
 }
 
-size_t radiosity_barrier_words(int nmesh) { return 2 + 2 * 3 * RES_LEVELS * (size_t)(nmesh > 0 ? nmesh : 1); }
+size_t radiosity_barrier_words(int nmesh) { return RAD_BAR_WORDS1 + 2 * 3 * RES_LEVELS * (size_t)(nmesh > 0 ? nmesh : 1); }
 
 // Cooperative grid size for ntiles tiles (at most the co-resident blocks).
 // Both solves launch the same block shape and shared memory, so one grid
@@ -1955,7 +2256,10 @@ int radiosity_launch(const StepView& v, double* x, int warm, int precision, int 
     set_error("radiosity grid %d has no tile schedule (made for %d blocks)", grid, v.sched_grid);
     return ILG_ERR_ARG;
   }
-  ILG_CUDA(cudaMemsetAsync(v.barrier, 0, 2 * sizeof(unsigned), s));
+  // one mesh, one tile per block (the schedule gives every block one when
+  // there are as many tiles as blocks)
+  const bool solo = precision != ILG_PREC_MIXED && v.nmesh == 1 && v.ntiles == grid && grid <= RAD_MAX_GRID;
+  ILG_CUDA(cudaMemsetAsync(v.barrier, 0, (RAD_BAR_WORDS0 + (solo ? 8 * (size_t)grid : 0)) * sizeof(unsigned), s));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(RAD_BLOCK);
@@ -1970,6 +2274,8 @@ int radiosity_launch(const StepView& v, double* x, int warm, int precision, int 
     ILG_CUDA(cudaLaunchKernelEx(&cfg, k_radiosity_lagged, v, x, warm));
   else if (precision == ILG_PREC_MIXED)
     ILG_CUDA(cudaLaunchKernelEx(&cfg, k_radiosity_mixed, v, x, warm, radiosity_inner(inner)));
+  else if (solo)
+    ILG_CUDA(cudaLaunchKernelEx(&cfg, k_radiosity64_solo, v, x, warm));
   else
     ILG_CUDA(cudaLaunchKernelEx(&cfg, k_radiosity64, v, x, warm));
   return ILG_OK;
