@@ -31,6 +31,7 @@
 // (linearised or Newton) is solved in FP64. The mixed step uses the same
 // increment form in plain FP32; the standalone column entry points
 // (conductionq_, ilg_conductionq_batch) run the reference's rows in FP64.
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <mutex>
@@ -46,7 +47,7 @@ namespace {
 
 constexpr int COND_THREADS = 128;       // standalone column entry points
 constexpr int COND_STEP_THREADS = 64;   // scene steps: 7 blocks of 60-layer columns per SM
-constexpr int TAB_W = 5;            // g, m, al, f, inv_beta per layer
+constexpr int TAB_W = 5;            // g, m (increment form: g inv_beta), al, f, inv_beta per layer
 constexpr size_t SMEM_LIMIT = 160 * 1024;
 
 // Double-float number: value = h + l with |l| <= ulp(h) / 2. The
@@ -84,9 +85,31 @@ __device__ __forceinline__ dfloat operator*(dfloat a, dfloat b) {
   return df_norm(p, e);
 }
 
+// Products kept as exact pairs until the sum they enter is renormalised
+// (one renormalisation instead of two or three, and a shorter chain from b or
+// y to the result; no less accurate than the separate operations).
+// c + a * b
+__device__ __forceinline__ dfloat df_fma(dfloat a, dfloat b, dfloat c) {
+  const float p = __fmul_rn(a.h, b.h);
+  float e = __fmaf_rn(a.h, b.h, -p);
+  e = __fmaf_rn(a.h, b.l, e);
+  e = __fmaf_rn(a.l, b.h, e);
+  const float s = __fadd_rn(c.h, p);
+  const float bb = __fsub_rn(s, c.h);
+  const float t = __fadd_rn(__fsub_rn(c.h, __fsub_rn(s, bb)), __fsub_rn(p, bb));   // TwoSum error
+  return df_norm(s, __fadd_rn(t, __fadd_rn(c.l, e)));
+}
+// a * b + x * y
+__device__ __forceinline__ dfloat df_dot2(dfloat a, dfloat b, dfloat x, dfloat y) {
+  const float q = __fmul_rn(x.h, y.h);
+  float e = __fmaf_rn(x.h, y.h, -q);
+  e = __fmaf_rn(x.h, y.l, e);
+  e = __fmaf_rn(x.l, y.h, e);
+  return df_fma(a, b, dfloat(q, e));
+}
+
 // 2x, exact
 __device__ __forceinline__ double twice(double a) { return 2.0 * a; }
-__device__ __forceinline__ float twice(float a) { return 2.f * a; }
 __device__ __forceinline__ dfloat twice(dfloat a) { return dfloat(2.f * a.h, 2.f * a.l); }
 
 // Layer loads bypass L1 (each value is read once per pass), so the small
@@ -206,11 +229,166 @@ __device__ __forceinline__ float sr_add(float a, float b, uint32_t key) {
   return fabsf(e) > u * fabsf(__fsub_rn(n, s)) ? n : s;
 }
 
+// The surface row of one column. Ti, Tip1: the top two layers at time n;
+// rho_next: the eliminated right-hand side of the layer below the top one (in
+// increment form the increment's); Ts_prev, Q: surface temperature at n and
+// absorbed flux (prescribed temperature for conductionT) at n + 1. Returns
+// T1(n+1) and its increment in the state's type, the new surface temperature
+// and the conducted flux; false (with the flag set) on a zero pivot.
+template <class R> struct TopRow { R top, dtop; double Tsn, Fs; };
+template <class R>
+__device__ __forceinline__ bool top_row(const StepView& v, const CondScalars& cs, int g, R Ti, R Tip1, R rho_next,
+                                        double Ts_prev, double Q, TopRow<R>& out) {
+  constexpr bool INC = !std::is_same<R, double>::value;
+  double T0n, Tsn, Fs;
+  R top, dtop;
+  bool done_top = false;
+  if constexpr (!std::is_same<R, double>::value) {
+    if (cs.bc == 1) {
+      // FP32 and double-float states: P, A and the top layer in double-float
+      // (P = T1(n+1) - S_top Ts(n+1) is a small difference of
+      // temperature-sized terms), the root by FP32 Newton steps, polished in
+      // double-float for the FP64 step (no FP64 arithmetic)
+      // the double-float step takes Ts and Q to 48 bits; the FP32 step in
+      // FP32 (its layers are FP32), converting each once
+      constexpr bool DF = std::is_same<R, dfloat>::value;
+      const dfloat Tsd = DF ? dfloat(Ts_prev) : dfloat(__double2float_rn(Ts_prev), 0.f);
+      const dfloat Qd = DF ? dfloat(Q) : dfloat(__double2float_rn(Q), 0.f);
+      const TopResult tr = newton_top(cs, to_df(Ti), to_df(Tip1), to_df(rho_next), Tsd, Qd, DF);
+      const dfloat fsd = (tr.top - tr.tsn) * to_df(cs.d_kz);
+      Tsn = DF ? df_to_double(tr.tsn) : (double)__fadd_rn(tr.tsn.h, tr.tsn.l);
+      top = from_df<R>(tr.top);
+      dtop = from_df<R>(tr.dtop);
+      Fs = DF ? -df_to_double(fsd) : -(double)__fadd_rn(fsd.h, fsd.l);
+      T0n = 0.0;
+      done_top = true;
+    }
+  }
+  if (!done_top) {
+  double T0 = (double)Ti, T1 = (double)Tip1, rho1 = (double)rho_next;
+  double Ts = Ts_prev;
+  if (cs.bc == 0) {
+    double Qn = v.Qprev[g];
+    double Tr3 = Ts * Ts * Ts;
+    double arad = -3.0 * cs.es * Tr3 * Ts;
+    double brad = 2.0 * cs.es * Tr3;
+    double den = cs.k1 + brad;
+    double ann = (Qn - arad) / den, annp1 = (Q - arad) / den, bn = (cs.k1 - brad) / den;
+    double b0 = 1.0 + cs.alpha0 + cs.gamma0 - cs.gamma0 * bn;
+    double r0 = cs.gamma0 * (annp1 + ann) + (1.0 - cs.alpha0 - cs.gamma0 + cs.gamma0 * bn) * T0 + cs.alpha0 * T1;
+    double piv = b0 + cs.f0 * cs.gamma1;
+    if (piv == 0.0) { atomicExch(&v.derr[DERR_PIVOT], 1); return false; }
+    if (INC) r0 -= b0 * T0 - cs.alpha0 * T1;   // the row applied to T(n)
+    T0n = (r0 - cs.f0 * rho1) / piv;
+    if (INC) T0n += T0;
+    Tsn = 0.5 * (annp1 + bn * T0n + T0n);
+  } else if (cs.bc == 1) {
+    double R0 = (1.0 - cs.alpha0 - cs.gamma0) * T0 + cs.alpha0 * T1 + cs.gamma0 * (2.0 * Ts - T0);
+    if (INC) R0 = 2.0 * cs.alpha0 * (T1 - T0) + 4.0 * cs.gamma0 * (Ts - T0) - 2.0 * cs.gamma0 * Ts;
+    double P = (R0 - cs.f0 * rho1) * cs.inv_Ap;
+    if (INC) P += T0;
+    // Root of g(x) = Q + 2 k1 (P + (S - 1) x) - es x^4 = A + B x - es x^4
+    // (g' = B - 4 es x^3 < 0): Newton in FP32 to ~1e-6, then FP64 steps
+    // whose g is exact to FP64 and whose step uses an FP32 reciprocal of
+    // g' (relative error ~6e-8, so each step gains ~7 digits). The FP32
+    // stage leaves x within ~1e-7 of the root (its rounding floor), so one
+    // FP64 step that moves x by at most 1e-7 |x| leaves ~6e-8 |dT| +
+    // 2 |dT|^2 / |x| < 1e-11 K and ends the polish; a larger first step
+    // (an FP32 stage that did not converge) continues to the FP64 tolerance.
+    const double A = Q + 2.0 * cs.k1 * P;
+    float xf = (float)Ts;
+    {
+      const float Af = (float)A, Bf = (float)cs.B_top, esf = (float)cs.es;
+      for (int it = 0; it < 30; ++it) {
+        float x3 = xf * xf * xf;
+        float dT = (Af + Bf * xf - esf * x3 * xf) / (Bf - 4.f * esf * x3);
+        xf -= dT;
+        if (fabsf(dT) <= 1e-6f * fabsf(xf)) break;
+      }
+    }
+    double x = (double)xf;
+    double tolr = std::is_same<R, float>::value ? 1e-12 : 1e-13;
+    for (int it = 0; it < 8; ++it) {
+      double x3 = x * x * x;
+      double gx = A + cs.B_top * x - cs.es * x3 * x;
+      double dT = gx * (double)__frcp_rn((float)(cs.B_top - 4.0 * cs.es * x3));
+      x -= dT;
+      if (fabs(dT) <= (it == 0 ? 1e-7 : tolr) * fabs(x)) break;
+    }
+    Tsn = x;
+    T0n = P + cs.S_top * Tsn;
+  } else {
+    // prescribed surface temperature: Ts at n, Q holds Ts at n+1
+    double b0 = 1.0 + cs.alpha0 + cs.gamma0;
+    double r0 = cs.alpha0 * T1 + (1.0 - cs.alpha0 - cs.gamma0) * T0 + cs.gamma0 * (Ts + Q);
+    if (INC) r0 -= b0 * T0 - cs.alpha0 * T1;
+    T0n = (r0 - cs.f0 * rho1) / (b0 + cs.f0 * cs.gamma1);
+    if (INC) T0n += T0;
+    Tsn = Q;
+  }
+  Fs = -(T0n - Tsn) * cs.kz;
+  top = (R)T0n;
+  dtop = (R)(T0n - T0);
+  }
+  out.top = top;
+  out.dtop = dtop;
+  out.Tsn = Tsn;
+  out.Fs = Fs;
+  return true;
+}
+
+__device__ __forceinline__ uint32_t sr_key(int facet, int layer, int frame) {
+  return (uint32_t)facet * 0x9E3779B9u + (uint32_t)layer * 0x85EBCA6Bu + (uint32_t)frame * 0xC2B2AE35u;
+}
+
+// The facet's outputs after its column: conducted flux, and for a scene step
+// the surface state and the running means.
+__device__ __forceinline__ void store_surface(const StepView& v, const MeshDesc& M, const CondScalars& cs, int g,
+                                              double Q, double Tsn, double Fs, int upd) {
+  v.Fsurf[g] = Fs;
+  if (cs.bc != 2) {
+    v.Tsurf[g] = Tsn;
+    v.Qprev[g] = Q;
+  }
+  if (upd) {
+    // running means: 1/(frame + 1) by an FP32 reciprocal and two FP64
+    // Newton steps (no FP64 division; computing it here is cheaper than
+    // loading a per-mesh value at the end of the column)
+    const double n = (double)(M.frame + 1);
+    double rn = (double)__frcp_rn((float)n);
+    rn = rn * (2.0 - n * rn);
+    rn = rn * (2.0 - n * rn);
+    v.rad_avg[g] += (Q - v.rad_avg[g]) * rn;
+    v.therm_avg[g] += (Tsn - v.therm_avg[g]) * rn;
+    if (M.frame > 50) v.therm_max[g] = fmax(v.therm_max[g], Tsn);
+  }
+}
+
+// One layer of the increment form's passes, shared by the two column kernels
+// (a column's result does not depend on which one runs it; the FP32 forms
+// are spelled out so that the compiler cannot contract them differently).
+// up: rho_i = 2 (gamma dm - alpha dn) - f rho_{i+1}, dm = T_{i-1} - T_i, dn =
+// T_i - T_{i+1}; down: d_i = rho_i / beta_i + (gamma / beta_i) d_{i-1}.
+__device__ __forceinline__ float up_layer(float g, float al, float f, float dm, float dn, float rho) {
+  return __fmaf_rn(-f, rho, 2.f * __fmaf_rn(g, dm, -(__fmul_rn(al, dn))));
+}
+__device__ __forceinline__ dfloat up_layer(dfloat g, dfloat al, dfloat f, dfloat dm, dfloat dn, dfloat rho) {
+  return df_fma(-f, rho, twice(df_dot2(g, dm, -al, dn)));
+}
+__device__ __forceinline__ float down_layer(float gb, float ib, float rho, float d) {
+  return __fmaf_rn(gb, d, __fmul_rn(rho, ib));
+}
+// gb = gamma / beta: off the chain of the increments, rho / beta is
+__device__ __forceinline__ dfloat down_layer(dfloat gb, dfloat ib, dfloat rho, dfloat d) { return df_fma(gb, d, rho * ib); }
+
 // One thread per facet column. Block b covers facets [cb.y, cb.y + BS) of
 // mesh cb.x. Q: the new time level's flux per facet. SR: the FP32 layers'
 // updates rounded without bias (sr_add).
+// At least one block per SM: shared memory limits the blocks, and without the
+// bound the compiler gives the passes fewer registers than their loads ahead
+// need (57 us instead of 49).
 template <class R, bool SMEM, int BS, bool SR = false>
-__global__ void __launch_bounds__(BS)
+__global__ void __launch_bounds__(BS, 1)
 k_conduct(StepView v, const double* __restrict__ Qnp1, int upd) {
   extern __shared__ unsigned char smem_raw[];
   R* rho_s = reinterpret_cast<R*>(smem_raw);
@@ -268,26 +446,30 @@ k_conduct(StepView v, const double* __restrict__ Qnp1, int upd) {
         if (i0 + j < nz) RHO(i0 + j) = t[j];
     }
   }
-  // upward pass
+  // upward pass (eight layers per iteration in both passes: the coefficient
+  // loads of a layer need to be that far ahead of its serial chain; 81,920
+  // double-float columns of 60 layers took 69 / 59 / 53 / 49 / 52 us at 1 / 2 /
+  // 4 / 8 / 16)
   R Tip1 = RHO(nz - 1);
   R Ti = RHO(nz - 2);
   const R* cb_t = tab + (size_t)(nz - 1) * TAB_W;
   R dn = Ti - Tip1;   // increment form: layer differences d_i = T(i-1) - T(i), each formed once
-  R rho_next = INC ? twice(cb_t[0] * dn) + (R)cs.cgeo : cb_t[0] * Ti + cb_t[1] * Tip1 + (R)cs.cgeo;
+  R rho_next;
+  if constexpr (INC) rho_next = up_layer(cb_t[0], (R)0, (R)-1, dn, (R)0, (R)cs.cgeo);
+  else rho_next = cb_t[0] * Ti + cb_t[1] * Tip1 + (R)cs.cgeo;
   RHO(nz - 1) = rho_next;
-#pragma unroll 4
+#pragma unroll 8
   for (int i = nz - 2; i >= 1; --i) {
     R Tim1 = RHO(i - 1);
     const R* c = tab + (size_t)i * TAB_W;
-    R r;
-    if (INC) {
+    R rh;
+    if constexpr (INC) {
       R dm = Tim1 - Ti;
-      r = twice(c[0] * dm - c[2] * dn);
+      rh = up_layer(c[0], c[2], c[3], dm, dn, rho_next);
       dn = dm;
     } else {
-      r = c[0] * Tim1 + c[1] * Ti + c[2] * Tip1;
+      rh = c[0] * Tim1 + c[1] * Ti + c[2] * Tip1 - c[3] * rho_next;
     }
-    R rh = r - c[3] * rho_next;
     RHO(i) = rh;
     rho_next = rh;
     Tip1 = Ti;
@@ -300,104 +482,18 @@ k_conduct(StepView v, const double* __restrict__ Qnp1, int upd) {
     if (M.coupling == ILG_COUPLE_REFERENCE) Q = -Fs_prev + Qsrc;
     v.rad[g] = Q;
   }
-  double T0n, Tsn, Fs;
-  R top, dtop;   // T1(n+1) and its increment, in the state's type
-  bool done_top = false;
-  if constexpr (!std::is_same<R, double>::value) {
-    if (cs.bc == 1) {
-      // FP32 and double-float states: P, A and the top layer in double-float
-      // (P = T1(n+1) - S_top Ts(n+1) is a small difference of
-      // temperature-sized terms), the root by FP32 Newton steps, polished in
-      // double-float for the FP64 step (no FP64 arithmetic)
-      // the double-float step takes Ts and Q to 48 bits; the FP32 step in
-      // FP32 (its layers are FP32), converting each once
-      constexpr bool DF = std::is_same<R, dfloat>::value;
-      const dfloat Tsd = DF ? dfloat(Ts_prev) : dfloat(__double2float_rn(Ts_prev), 0.f);
-      const dfloat Qd = DF ? dfloat(Q) : dfloat(__double2float_rn(Q), 0.f);
-      const TopResult tr = newton_top(cs, to_df(Ti), to_df(Tip1), to_df(rho_next), Tsd, Qd, DF);
-      const dfloat fsd = (tr.top - tr.tsn) * to_df(cs.d_kz);
-      Tsn = DF ? df_to_double(tr.tsn) : (double)__fadd_rn(tr.tsn.h, tr.tsn.l);
-      top = from_df<R>(tr.top);
-      dtop = from_df<R>(tr.dtop);
-      Fs = DF ? -df_to_double(fsd) : -(double)__fadd_rn(fsd.h, fsd.l);
-      T0n = 0.0;
-      done_top = true;
-    }
-  }
-  if (!done_top) {
-  double T0 = (double)Ti, T1 = (double)Tip1, rho1 = (double)rho_next;
-  double Ts = Ts_prev;
-  if (cs.bc == 0) {
-    double Qn = v.Qprev[g];
-    double Tr3 = Ts * Ts * Ts;
-    double arad = -3.0 * cs.es * Tr3 * Ts;
-    double brad = 2.0 * cs.es * Tr3;
-    double den = cs.k1 + brad;
-    double ann = (Qn - arad) / den, annp1 = (Q - arad) / den, bn = (cs.k1 - brad) / den;
-    double b0 = 1.0 + cs.alpha0 + cs.gamma0 - cs.gamma0 * bn;
-    double r0 = cs.gamma0 * (annp1 + ann) + (1.0 - cs.alpha0 - cs.gamma0 + cs.gamma0 * bn) * T0 + cs.alpha0 * T1;
-    double piv = b0 + cs.f0 * cs.gamma1;
-    if (piv == 0.0) { atomicExch(&v.derr[DERR_PIVOT], 1); return; }
-    if (INC) r0 -= b0 * T0 - cs.alpha0 * T1;   // the row applied to T(n)
-    T0n = (r0 - cs.f0 * rho1) / piv;
-    if (INC) T0n += T0;
-    Tsn = 0.5 * (annp1 + bn * T0n + T0n);
-  } else if (cs.bc == 1) {
-    double R0 = (1.0 - cs.alpha0 - cs.gamma0) * T0 + cs.alpha0 * T1 + cs.gamma0 * (2.0 * Ts - T0);
-    if (INC) R0 = 2.0 * cs.alpha0 * (T1 - T0) + 4.0 * cs.gamma0 * (Ts - T0) - 2.0 * cs.gamma0 * Ts;
-    double P = (R0 - cs.f0 * rho1) * cs.inv_Ap;
-    if (INC) P += T0;
-    // Root of g(x) = Q + 2 k1 (P + (S - 1) x) - es x^4 = A + B x - es x^4
-    // (g' = B - 4 es x^3 < 0): Newton in FP32 to ~1e-6, then FP64 steps
-    // whose g is exact to FP64 and whose step uses an FP32 reciprocal of
-    // g' (relative error ~6e-8, so each step gains ~7 digits). The FP32
-    // stage leaves x within ~1e-7 of the root (its rounding floor), so one
-    // FP64 step that moves x by at most 1e-7 |x| leaves ~6e-8 |dT| +
-    // 2 |dT|^2 / |x| < 1e-11 K and ends the polish; a larger first step
-    // (an FP32 stage that did not converge) continues to the FP64 tolerance.
-    const double A = Q + 2.0 * cs.k1 * P;
-    float xf = (float)Ts;
-    {
-      const float Af = (float)A, Bf = (float)cs.B_top, esf = (float)cs.es;
-      for (int it = 0; it < 30; ++it) {
-        float x3 = xf * xf * xf;
-        float dT = (Af + Bf * xf - esf * x3 * xf) / (Bf - 4.f * esf * x3);
-        xf -= dT;
-        if (fabsf(dT) <= 1e-6f * fabsf(xf)) break;
-      }
-    }
-    double x = (double)xf;
-    double tolr = std::is_same<R, float>::value ? 1e-12 : 1e-13;
-    for (int it = 0; it < 8; ++it) {
-      double x3 = x * x * x;
-      double gx = A + cs.B_top * x - cs.es * x3 * x;
-      double dT = gx * (double)__frcp_rn((float)(cs.B_top - 4.0 * cs.es * x3));
-      x -= dT;
-      if (fabs(dT) <= (it == 0 ? 1e-7 : tolr) * fabs(x)) break;
-    }
-    Tsn = x;
-    T0n = P + cs.S_top * Tsn;
-  } else {
-    // prescribed surface temperature: Ts at n, Q holds Ts at n+1
-    double b0 = 1.0 + cs.alpha0 + cs.gamma0;
-    double r0 = cs.alpha0 * T1 + (1.0 - cs.alpha0 - cs.gamma0) * T0 + cs.gamma0 * (Ts + Q);
-    if (INC) r0 -= b0 * T0 - cs.alpha0 * T1;
-    T0n = (r0 - cs.f0 * rho1) / (b0 + cs.f0 * cs.gamma1);
-    if (INC) T0n += T0;
-    Tsn = Q;
-  }
-  Fs = -(T0n - Tsn) * cs.kz;
-  top = (R)T0n;
-  dtop = (R)(T0n - T0);
-  }
+  TopRow<R> tr;
+  if (!top_row<R>(v, cs, g, Ti, Tip1, rho_next, Ts_prev, Q, tr)) return;
+  const double Tsn = tr.Tsn, Fs = tr.Fs;
+  const R top = tr.top, dtop = tr.dtop;
   // downward pass
-  if (INC) {
+  if constexpr (INC) {
     R dprev = dtop;
     T[0] = top;
-#pragma unroll 4
+#pragma unroll 8
     for (int i = 1; i < nz; ++i) {   // the increments, into the rho slots
       const R* c = tab + (size_t)i * TAB_W;
-      R d = (RHO(i) + c[0] * dprev) * c[4];
+      R d = down_layer(c[1], c[4], RHO(i), dprev);
       RHO(i) = d;
       dprev = d;
     }
@@ -410,9 +506,7 @@ k_conduct(StepView v, const double* __restrict__ Qnp1, int upd) {
       for (int j = 0; j < 16; ++j)
         if (i0 + j < nz) {
           if constexpr (SR && std::is_same<R, float>::value)
-            T[(size_t)(i0 + j) * N] = sr_add(t[j], RHO(i0 + j),
-                                             (uint32_t)fl * 0x9E3779B9u + (uint32_t)(i0 + j) * 0x85EBCA6Bu +
-                                                 (uint32_t)M.frame * 0xC2B2AE35u);
+            T[(size_t)(i0 + j) * N] = sr_add(t[j], RHO(i0 + j), sr_key(fl, i0 + j, M.frame));
           else
             T[(size_t)(i0 + j) * N] = t[j] + RHO(i0 + j);
         }
@@ -428,23 +522,116 @@ k_conduct(StepView v, const double* __restrict__ Qnp1, int upd) {
     }
   }
 #undef RHO
-  v.Fsurf[g] = Fs;
-  if (cs.bc != 2) {
-    v.Tsurf[g] = Tsn;
-    v.Qprev[g] = Q;
+  store_surface(v, M, cs, g, Q, Tsn, Fs, upd);
+}
+
+// The increment form with the whole column in registers: one thread per
+// column, one array slot per layer (T_i, then rho_i, then the increment),
+// loops unrolled over NZ >= nz layers in chunks that a shallower mesh skips.
+// Every layer's load is in flight at once and nothing goes through shared
+// memory but the layer coefficients, which a block stages once (one 16-byte
+// broadcast per layer and pass, instead of five loads through L1 and six
+// shared-memory accesses of the column). T(n) is read again for the update
+// (from L2): a second register per layer would halve the columns in flight.
+// Layers beyond nz in the last chunk have gamma = alpha = 0 and f = -1, which
+// carry the bottom flux term unchanged up to layer nz - 1.
+// Bound by HBM and the latency of a column's chain together.
+constexpr int COL_CHUNK = 8;
+constexpr int COL_THREADS = 64;    // most threads per block
+// Blocks per SM that the registers have to allow (65,536 / (64 blocks)): the
+// 81,920-column, 60-layer step is then one wave.
+constexpr int col_blocks(int nz) { return nz <= 32 ? 12 : nz <= 48 ? 10 : nz <= 64 ? 9 : 8; }
+
+template <class R> struct UpCoef { R g, al, f, pad; };
+template <class R> struct DownCoef { R gb, ib; };
+
+template <class R, int NZ, bool SR>
+__global__ void __launch_bounds__(COL_THREADS, col_blocks(NZ))
+k_conduct_col(StepView v, const double* __restrict__ Qnp1, int upd) {
+  __shared__ __align__(16) UpCoef<R> up[NZ];
+  __shared__ __align__(16) DownCoef<R> down[NZ];
+  const int2 cb = v.cblocks ? v.cblocks[blockIdx.x] : make_int2(0, blockIdx.x * blockDim.x);
+  const MeshDesc& M = v.md[cb.x];
+  if (!M.active) return;
+  const int nz = M.cs.nz;
+  {
+    const R* __restrict__ tab = coef_tab<R>(v) + M.coef0;
+    for (int i = threadIdx.x; i < NZ; i += blockDim.x) {
+      const R* c = tab + (size_t)i * TAB_W;
+      const bool in = i < nz, mid = i < nz - 1;
+      up[i].g = in ? c[0] : (R)0;
+      up[i].al = mid ? c[2] : (R)0;
+      up[i].f = mid ? c[3] : (R)-1;
+      down[i].gb = in ? c[1] : (R)0;
+      down[i].ib = in ? c[4] : (R)0;
+    }
   }
-  if (upd) {
-    // running means: 1/(frame + 1) by an FP32 reciprocal and two FP64
-    // Newton steps (no FP64 division; computing it here is cheaper than
-    // loading a per-mesh value at the end of the column)
-    const double n = (double)(M.frame + 1);
-    double rn = (double)__frcp_rn((float)n);
-    rn = rn * (2.0 - n * rn);
-    rn = rn * (2.0 - n * rn);
-    v.rad_avg[g] += (Q - v.rad_avg[g]) * rn;
-    v.therm_avg[g] += (Tsn - v.therm_avg[g]) * rn;
-    if (M.frame > 50) v.therm_max[g] = fmax(v.therm_max[g], Tsn);
+  const int fl = cb.y + threadIdx.x;
+  const bool on = fl < M.nfacet;
+  const int g = M.facet0 + fl;
+  const size_t N = (size_t)M.nfacet;
+  R* __restrict__ T = state_T<R>(v) + M.T0 + fl;
+  R a[NZ];
+  if (on) {
+#pragma unroll
+    for (int i = 0; i < NZ; ++i) a[i] = i < nz ? ld_layer(T + (size_t)i * N) : (R)0;
   }
+  __syncthreads();
+  if (!on) return;
+  const CondScalars& cs = M.cs;
+  // the facet's scalars (see k_conduct)
+  const bool direct_only = upd && M.ntiles == 0;
+  const double Qsrc = direct_only ? v.E[e_slot(M.frame) * v.nt + g] : Qnp1[g];
+  const double Fs_prev = (direct_only && M.coupling == ILG_COUPLE_REFERENCE) ? v.Fsurf[g] : 0.0;
+  const double Ts_prev = v.Tsurf[g];
+  // upward pass
+  R rho = (R)cs.cgeo, dn = (R)0;
+#pragma unroll
+  for (int c = NZ - COL_CHUNK; c >= 0; c -= COL_CHUNK) {
+    if (c < nz) {
+#pragma unroll
+      for (int i = c + COL_CHUNK - 1; i >= c; --i) {
+        if (i == 0) continue;
+        const R dm = a[i - 1] - a[i];
+        rho = up_layer(up[i].g, up[i].al, up[i].f, dm, dn, rho);
+        // the layer below is T_i of the next row up
+        dn = dm;
+        if (i == 1) continue;   // a[1] = T_1 until the top row has read it
+        a[i] = rho;
+      }
+    }
+  }
+  double Q = Qsrc;
+  if (direct_only) {
+    if (M.coupling == ILG_COUPLE_REFERENCE) Q = -Fs_prev + Qsrc;
+    v.rad[g] = Q;
+  }
+  TopRow<R> tr;
+  if (!top_row<R>(v, cs, g, a[0], a[1], rho, Ts_prev, Q, tr)) return;
+  a[1] = rho;
+  // downward pass and update
+  T[0] = tr.top;
+  R d = tr.dtop;
+#pragma unroll
+  for (int c = 0; c < NZ; c += COL_CHUNK) {
+    if (c < nz) {
+      R t[COL_CHUNK];
+#pragma unroll
+      for (int j = 0; j < COL_CHUNK; ++j)
+        if (c + j > 0 && c + j < nz) t[j] = ld_layer(T + (size_t)(c + j) * N);
+#pragma unroll
+      for (int j = 0; j < COL_CHUNK; ++j) {
+        const int i = c + j;
+        if (i == 0) continue;
+        d = down_layer(down[i].gb, down[i].ib, a[i], d);
+        if (i < nz) {
+          if constexpr (SR) T[(size_t)i * N] = sr_add(t[j], d, sr_key(fl, i, M.frame));
+          else T[(size_t)i * N] = t[j] + d;
+        }
+      }
+    }
+  }
+  store_surface(v, M, cs, g, Q, tr.Tsn, tr.Fs, upd);
 }
 
 __global__ void k_df_to_f(const float2* __restrict__ in, float* __restrict__ out, size_t n) {
@@ -536,6 +723,25 @@ int build_tables(int nz, const double* z, const double* ti, const double* rhoc, 
   return ILG_OK;
 }
 
+// FP32 register columns: the smallest class that holds nz_max layers. Deeper
+// columns go through shared memory, and so do double-float ones: two
+// registers per layer leave 10 warps per SM, and the unrolled double-float
+// code (~60 instructions per layer) does not fit the instruction cache
+// (81,920 columns of 60 layers: 68 us against 50 us).
+constexpr int COL_MAX = 80;
+template <class R, bool SR>
+int launch_columns(const StepView& v, const double* Q, int upd, int nz_max, int bs, cudaStream_t s) {
+  bs = std::min(bs, COL_THREADS);
+  const int grid = v.cblocks ? v.ncblocks : div_up(v.nt, bs);
+  if (grid <= 0) return ILG_OK;
+  if (nz_max <= 32) k_conduct_col<R, 32, SR><<<grid, bs, 0, s>>>(v, Q, upd);
+  else if (nz_max <= 48) k_conduct_col<R, 48, SR><<<grid, bs, 0, s>>>(v, Q, upd);
+  else if (nz_max <= 64) k_conduct_col<R, 64, SR><<<grid, bs, 0, s>>>(v, Q, upd);
+  else k_conduct_col<R, COL_MAX, SR><<<grid, bs, 0, s>>>(v, Q, upd);
+  ILG_CUDA(cudaGetLastError());
+  return ILG_OK;
+}
+
 template <class R, int BS>
 int launch_conduct(const StepView& v, const double* Q, int upd, int nz_max, cudaStream_t s, bool sr = false) {
   size_t smem = (size_t)nz_max * BS * sizeof(R);
@@ -600,6 +806,7 @@ int conduction_prepare(Context& c, double dt, int precision) {
   std::vector<double> tab;
   CondScalars cs;
   ILG_TRY(build_tables(c.nz, c.z_h.data(), c.ti_h.data(), c.rhoc_h.data(), dt, c.emiss, c.Fgeo, c.bc_mode, tab, cs));
+  for (int i = 0; i < c.nz; ++i) tab[(size_t)i * TAB_W + 1] = tab[(size_t)i * TAB_W] * tab[(size_t)i * TAB_W + 4];
   if (precision == ILG_PREC_MIXED) {
     std::vector<float> t32(tab.size());
     for (size_t i = 0; i < tab.size(); ++i) t32[i] = (float)tab[i];
@@ -641,6 +848,10 @@ int conduction_launch(const StepView& v, const double* Q, int precision, int upd
                       bool sr) {
   int bs = v.cblocks ? COND_STEP_THREADS : v.tune.conduct_threads;
   if (bs != 32 && bs != 64 && bs != 128) { set_error("conduct_threads must be 32, 64 or 128"); return ILG_ERR_ARG; }
+  if (precision == ILG_PREC_MIXED && nz_max <= COL_MAX) {
+    return sr ? launch_columns<float, true>(v, Q, upd, nz_max, bs, s)
+              : launch_columns<float, false>(v, Q, upd, nz_max, bs, s);
+  }
   const size_t elt = precision == ILG_PREC_MIXED ? sizeof(float) : sizeof(dfloat);
   if ((size_t)nz_max * bs * elt > SMEM_LIMIT) bs = COND_STEP_THREADS;
   if (precision == ILG_PREC_MIXED) {
