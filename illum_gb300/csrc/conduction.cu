@@ -34,6 +34,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cstring>
 #include <mutex>
 #include <type_traits>
 #include <vector>
@@ -45,7 +46,8 @@ namespace ilg {
 
 namespace {
 
-constexpr int COND_THREADS = 128;       // standalone column entry points
+constexpr int COND_THREADS = 128;       // columns without allocation
+constexpr int COL_HOST_THREADS = 32;    // standalone column entry points (see run_columns)
 constexpr int COND_STEP_THREADS = 64;   // scene steps: 7 blocks of 60-layer columns per SM
 constexpr int TAB_W = 5;            // g, m (increment form: g inv_beta), al, f, inv_beta per layer
 constexpr size_t SMEM_LIMIT = 160 * 1024;
@@ -779,6 +781,8 @@ int conduction_setup() {
   if (done.load(std::memory_order_relaxed)) return ILG_OK;
   ILG_CUDA(cudaFuncSetAttribute(k_conduct<double, true, COND_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)SMEM_LIMIT));
+  ILG_CUDA(cudaFuncSetAttribute(k_conduct<double, true, COL_HOST_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)SMEM_LIMIT));
   ILG_CUDA(cudaFuncSetAttribute(k_conduct<dfloat, true, COND_STEP_THREADS>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_LIMIT));
   ILG_CUDA(cudaFuncSetAttribute(k_conduct<float, true, COND_STEP_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -989,8 +993,43 @@ int record_launch(const StepView& v, int precision, int ncblocks, cudaStream_t s
   return ILG_OK;
 }
 
+// Columns between the caller's layout (column f's nz layers contiguous) and
+// the layer-major one, by 32 x 32 tiles through shared memory: both sides
+// coalesced.
+template <bool TO_LAYERS>
+__global__ void __launch_bounds__(256) k_relayout(const double* __restrict__ in, int nz, int64_t ncol,
+                                                  double* __restrict__ out) {
+  __shared__ double t[32][33];   // [column][layer]
+  const int64_t f0 = (int64_t)blockIdx.x * 32;
+  const int i0 = blockIdx.y * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int k = ty; k < 32; k += 8) {
+    if (TO_LAYERS) {
+      if (f0 + k < ncol && i0 + tx < nz) t[k][tx] = in[(f0 + k) * nz + i0 + tx];
+    } else {
+      if (i0 + k < nz && f0 + tx < ncol) t[tx][k] = in[(int64_t)(i0 + k) * ncol + f0 + tx];
+    }
+  }
+  __syncthreads();
+  for (int k = ty; k < 32; k += 8) {
+    if (TO_LAYERS) {
+      if (i0 + k < nz && f0 + tx < ncol) out[(int64_t)(i0 + k) * ncol + f0 + tx] = t[tx][k];
+    } else {
+      if (f0 + k < ncol && i0 + tx < nz) out[(f0 + k) * nz + i0 + tx] = t[k][tx];
+    }
+  }
+}
+
 // Standalone batched columns (host arrays, reference layout: column-major
-// nz x ncol). Runs on the current device with a private stream.
+// nz x ncol). Runs on the current device with a private stream and one
+// stream-ordered allocation, which holds
+//   tab, the mesh record, the error flags    uploaded in one copy
+//   Qn, Qnp1, Ts, Fs                         ncol doubles each
+//   T                                        the caller's layout
+//   Tl                                       layer-major, as the kernel reads
+//   rho                                      for columns beyond shared memory
+// The layouts are exchanged on the device. One warp per block: FP64 work is
+// bound by the FP64 pipe of each SM it runs on, and 5,120 columns are 160
+// warps (40 blocks of four warps left three quarters of the SMs idle).
 static int run_columns(int ncol, int nz, const double* z, double dt, const double* Qn, const double* Qnp1, double* T,
                        const double* ti, const double* rhoc, double emiss, double* Tsurf, double Fgeo,
                        double* Fsurf, int bc) {
@@ -999,49 +1038,53 @@ static int run_columns(int ncol, int nz, const double* z, double dt, const doubl
   CondScalars cs;
   ILG_TRY(build_tables(nz, z, ti, rhoc, dt, emiss, Fgeo, bc, tab, cs));
   ILG_TRY(conduction_setup());
-  cudaStream_t s;
-  ILG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-  struct StreamGuard { cudaStream_t s; ~StreamGuard() { cudaStreamDestroy(s); } } guard{s};
-  dbuf<double> dtab, dT, dTs, dFs, dQn, dQ, rho;
-  dbuf<int> derr;
-  dbuf<MeshDesc> dmd;
-  ILG_TRY(dtab.alloc(tab.size()));
-  ILG_TRY(dT.alloc((size_t)nz * ncol));
-  ILG_TRY(dTs.alloc(ncol));
-  ILG_TRY(dFs.alloc(ncol));
-  ILG_TRY(dQn.alloc(ncol));
-  ILG_TRY(dQ.alloc(ncol));
-  ILG_TRY(derr.alloc(DERR_COUNT));
-  ILG_TRY(dmd.alloc(1));
-  size_t smem = (size_t)nz * 128 * sizeof(double);
-  if (smem > SMEM_LIMIT) ILG_TRY(rho.alloc((size_t)nz * ncol));
+  ILG_TRY(alloc_pool_setup());
+  OwnedStream os;   // destroyed after the buffer, which is freed on it
+  ILG_CUDA(cudaStreamCreateWithFlags(&os.s, cudaStreamNonBlocking));
+  cudaStream_t s = os.s;
+  AllocOn on(s);
+  const size_t n = (size_t)nz * ncol, nc = (size_t)ncol;
+  const size_t tab_b = (tab.size() * 8 + 255) & ~(size_t)255, md_b = (sizeof(MeshDesc) + 255) & ~(size_t)255;
+  const size_t head_b = tab_b + md_b + 256;
+  const bool deep = (size_t)nz * COL_HOST_THREADS * sizeof(double) > SMEM_LIMIT;
+  dbuf<unsigned char> buf;
+  ILG_TRY(buf.alloc(head_b + (4 * nc + (deep ? 3 : 2) * n) * 8));
+  double* const dtab = reinterpret_cast<double*>(buf.p);
+  MeshDesc* const dmd = reinterpret_cast<MeshDesc*>(buf.p + tab_b);
+  int* const derr = reinterpret_cast<int*>(buf.p + tab_b + md_b);
+  double* const dQn = reinterpret_cast<double*>(buf.p + head_b);
+  double *const dQ = dQn + nc, *const dTs = dQ + nc, *const dFs = dTs + nc, *const dT = dFs + nc, *const dTl = dT + n,
+               *const rho = dTl + n;
+  std::vector<unsigned char> head(head_b, 0);
   MeshDesc md{};
   md.facet0 = 0; md.nfacet = ncol; md.nz = nz; md.coef0 = 0; md.T0 = 0; md.cs = cs; md.active = 1;
-  std::vector<double> Tl((size_t)nz * ncol);
-  for (int f = 0; f < ncol; ++f)
-    for (int i = 0; i < nz; ++i) Tl[(size_t)i * ncol + f] = T[(size_t)f * nz + i];
-  ILG_CUDA(cudaMemcpyAsync(dmd.p, &md, sizeof(md), cudaMemcpyHostToDevice, s));
-  ILG_CUDA(cudaMemcpyAsync(dtab.p, tab.data(), tab.size() * 8, cudaMemcpyHostToDevice, s));
-  ILG_CUDA(cudaMemcpyAsync(dT.p, Tl.data(), Tl.size() * 8, cudaMemcpyHostToDevice, s));
-  ILG_CUDA(cudaMemcpyAsync(dTs.p, Tsurf, (size_t)ncol * 8, cudaMemcpyHostToDevice, s));
-  ILG_CUDA(cudaMemcpyAsync(dQ.p, Qnp1, (size_t)ncol * 8, cudaMemcpyHostToDevice, s));
-  if (Qn) ILG_CUDA(cudaMemcpyAsync(dQn.p, Qn, (size_t)ncol * 8, cudaMemcpyHostToDevice, s));
-  else ILG_CUDA(cudaMemsetAsync(dQn.p, 0, (size_t)ncol * 8, s));
-  ILG_CUDA(cudaMemsetAsync(derr.p, 0, DERR_COUNT * sizeof(int), s));
+  std::memcpy(head.data(), tab.data(), tab.size() * 8);
+  std::memcpy(head.data() + tab_b, &md, sizeof(md));
+  ILG_CUDA(cudaMemcpyAsync(buf.p, head.data(), head_b, cudaMemcpyHostToDevice, s));
+  ILG_CUDA(cudaMemcpyAsync(dT, T, n * 8, cudaMemcpyHostToDevice, s));
+  ILG_CUDA(cudaMemcpyAsync(dTs, Tsurf, nc * 8, cudaMemcpyHostToDevice, s));
+  ILG_CUDA(cudaMemcpyAsync(dQ, Qnp1, nc * 8, cudaMemcpyHostToDevice, s));
+  if (Qn) ILG_CUDA(cudaMemcpyAsync(dQn, Qn, nc * 8, cudaMemcpyHostToDevice, s));
+  else ILG_CUDA(cudaMemsetAsync(dQn, 0, nc * 8, s));
+  const dim3 tiles(div_up(ncol, 32), div_up(nz, 32));
+  k_relayout<true><<<tiles, 256, 0, s>>>(dT, nz, ncol, dTl);
+  ILG_CUDA(cudaGetLastError());
   StepView v{};
-  v.nt = ncol; v.nmesh = 1; v.md = dmd.p;
-  v.Tsurf = dTs.p; v.Fsurf = dFs.p; v.Qprev = dQn.p; v.T64 = dT.p; v.coef64 = dtab.p; v.rho64 = rho.p;
-  v.derr = derr.p;
-  ILG_TRY((launch_conduct<double, COND_THREADS>(v, dQ.p, 0, nz, s)));
+  v.nt = ncol; v.nmesh = 1; v.md = dmd;
+  v.Tsurf = dTs; v.Fsurf = dFs; v.Qprev = dQn; v.T64 = dTl; v.coef64 = dtab; v.rho64 = deep ? rho : nullptr;
+  v.derr = derr;
+  ILG_TRY((launch_conduct<double, COL_HOST_THREADS>(v, dQ, 0, nz, s)));
+  k_relayout<false><<<tiles, 256, 0, s>>>(dTl, nz, ncol, dT);
+  ILG_CUDA(cudaGetLastError());
   int herr[DERR_COUNT];
-  ILG_CUDA(cudaMemcpyAsync(Tl.data(), dT.p, Tl.size() * 8, cudaMemcpyDeviceToHost, s));
-  if (bc != 2) ILG_CUDA(cudaMemcpyAsync(Tsurf, dTs.p, (size_t)ncol * 8, cudaMemcpyDeviceToHost, s));
-  ILG_CUDA(cudaMemcpyAsync(Fsurf, dFs.p, (size_t)ncol * 8, cudaMemcpyDeviceToHost, s));
-  ILG_CUDA(cudaMemcpyAsync(herr, derr.p, sizeof(herr), cudaMemcpyDeviceToHost, s));
+  ILG_CUDA(cudaMemcpyAsync(herr, derr, sizeof(herr), cudaMemcpyDeviceToHost, s));
   ILG_CUDA(cudaStreamSynchronize(s));
+  // a zero pivot leaves the caller's arrays as they were
   if (herr[DERR_PIVOT]) { set_error("zero pivot in a conduction column"); return ILG_ERR_PIVOT; }
-  for (int f = 0; f < ncol; ++f)
-    for (int i = 0; i < nz; ++i) T[(size_t)f * nz + i] = Tl[(size_t)i * ncol + f];
+  ILG_CUDA(cudaMemcpyAsync(T, dT, n * 8, cudaMemcpyDeviceToHost, s));
+  if (bc != 2) ILG_CUDA(cudaMemcpyAsync(Tsurf, dTs, nc * 8, cudaMemcpyDeviceToHost, s));
+  ILG_CUDA(cudaMemcpyAsync(Fsurf, dFs, nc * 8, cudaMemcpyDeviceToHost, s));
+  ILG_CUDA(cudaStreamSynchronize(s));
   return ILG_OK;
 }
 
