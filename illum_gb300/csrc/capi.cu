@@ -199,15 +199,23 @@ int enqueue_serial_prologue(const StepView& v, const StepPlan& p, cudaStream_t s
 
 // The step's radiosity reads its frame's E slot (the one-pass mixed solve
 // also the next frame's); the direct insolation of the frame after those
-// then writes its own slot on s2 while the conduction runs on s (the two
-// share no array: the conduction reads the radiosity solution, or the
-// current slot for meshes without form factors). Both finish before the
-// advance. Results equal the serial order's bit for bit.
+// writes its own slot on s2 meanwhile (neither the solve nor the conduction
+// reads that slot or writes what the insolation reads). It starts with the
+// solve, which leaves it room on every SM; without one (or in the fixed-sweep
+// mode, whose launches fill the device) it runs beside the conduction. Both
+// finish before the advance. Results equal the serial order's bit for bit.
 int enqueue_step_pipe(const StepView& v, const StepPlan& p, cudaStream_t s, const StepPipe& pipe) {
-  if (p.rad_on) ILG_TRY(radiosity_phase(v, p, s));
+  const int mu32 = p.precision == ILG_PREC_MIXED ? 1 : 0, ahead = p.rad_lagged ? 2 : 1;
+  const bool beside = p.rad_on && !p.gs_ctx;
+  if (p.rad_on && !beside) ILG_TRY(radiosity_phase(v, p, s));
   ILG_CUDA(cudaEventRecord(pipe.fork, s));
   ILG_CUDA(cudaStreamWaitEvent(pipe.s2, pipe.fork, 0));
-  ILG_TRY(direct_launch(v, 0, p.precision == ILG_PREC_MIXED ? 1 : 0, p.rad_lagged ? 2 : 1, pipe.s2));
+  if (beside) {
+    ILG_TRY(radiosity_phase(v, p, s));
+    ILG_TRY(direct_beside_launch(v, mu32, ahead, pipe.s2));
+  } else {
+    ILG_TRY(direct_launch(v, 0, mu32, ahead, pipe.s2));
+  }
   ILG_CUDA(cudaEventRecord(pipe.join, pipe.s2));
   ILG_TRY(conduction_launch(v, v.rad, p.precision, 1, p.nz_max, s, p.layer_sr));
   if (p.rec_on) ILG_TRY(record_launch(v, p.precision, v.cblocks ? v.ncblocks : div_up(v.nt, conduction_step_threads()), s));

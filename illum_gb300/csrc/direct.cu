@@ -16,6 +16,8 @@
 //     per-sample evaluation of geom.h sample_lit in FP64, bit-identical to
 //     the CPU oracle.
 // Compiled with -fmad=false (geom.h requirement).
+#include <algorithm>
+
 #include "geom.h"
 #include "internal.cuh"
 
@@ -81,8 +83,8 @@ __device__ __forceinline__ bool thr_range(const float* __restrict__ h, int nphi,
 // mu32: the cosine of the sun centre in FP32 (n . u, u the unit sun vector;
 // relative error ~2e-7) instead of the reference's FP64 value; the lit
 // sample count stays exact either way.
-__global__ void k_direct_classify(StepView v, int dropin, int mu32_flux, int ahead) {
-  int f = blockIdx.x * blockDim.x + threadIdx.x;
+// Returns whether facet f is left undecided.
+__device__ __forceinline__ bool classify_facet(const StepView& v, int f, int dropin, int mu32_flux, int ahead) {
   bool amb = false;
   const MeshDesc* Mp = nullptr;
   if (f < v.nt) {
@@ -163,6 +165,12 @@ __global__ void k_direct_classify(StepView v, int dropin, int mu32_flux, int ahe
     }
     amb = !decided;
   }
+  return amb;
+}
+
+__global__ void k_direct_classify(StepView v, int dropin, int mu32_flux, int ahead) {
+  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool amb = classify_facet(v, f, dropin, mu32_flux, ahead);
   // warp-aggregated append of undecided facets
   unsigned m = __ballot_sync(0xffffffffu, amb);
   if (m) {
@@ -280,91 +288,137 @@ __device__ __forceinline__ void dx_exact_sample(const StepView& v, DxFacet& F, i
   if (sample_lit(p, disk, BTN, hl, M.nphi, M.dphi, M.interp)) atomicAdd(&F.count, 1);
 }
 
+// The fluxes of the facets work[0, nf), nf <= 32, by a block of THREADS
+// threads. list: LIST entries, nlist: shared. Ends with a block barrier.
+template <int THREADS, int LIST>
+__device__ __forceinline__ void exact_facets(const StepView& v, DxFacet* fs, int* list, int& nlist, const int* work,
+                                             int nf, int dropin, int mu32_flux, int ahead) {
+  const int nsamp = v.ndisk - 1;   // samples per facet (the meshes of a view share the disk)
+  const int FT = THREADS - 32;     // filter threads (warps 1..)
+  const int total = nf * nsamp;
+  if (threadIdx.x < 32) {
+    // FP64 set-up, one lane per facet (overlaps the filter below)
+    if (threadIdx.x < nf) {
+      DxFacet& F = fs[threadIdx.x];
+      int f = work[threadIdx.x];
+      const MeshDesc& M = v.md[v.mesh_of ? v.mesh_of[f] : 0];
+      const SunAux* S = mesh_sun(v, M, ahead);
+      float4 c4 = v.cen[f];
+      d3 p = mkd((double)c4.x, (double)c4.y, (double)c4.z);
+      d3 Sv = mkd(S->sx, S->sy, S->sz);
+      d3 SP = sub(Sv, p);
+      double dist = norm(SP);
+      d3 N = mkd(SP.x / dist, SP.y / dist, SP.z / dist);   // = geom.h normalise(S - p)
+      d3 T, B;
+      sun_frame(N, &T, &B);
+      F.Tx = T.x; F.Ty = T.y; F.Tz = T.z;
+      F.Bx = B.x; F.By = B.y; F.Bz = B.z;
+      if (mu32_flux) {
+        float4 n4 = v.nrm[f];
+        F.mu = (double)((n4.x * S->ux + n4.y * S->uy) + n4.z * S->uz);
+      } else {
+        const double* fr = v.frame + 9 * (int64_t)f;
+        F.mu = sun_mu(Sv, p, mkd(fr[6], fr[7], fr[8]));
+      }
+    }
+  } else {
+    if (threadIdx.x - 32 < nf) dx_setup32(v, fs[threadIdx.x - 32], work[threadIdx.x - 32], ahead);
+    if (threadIdx.x == 32) nlist = 0;
+    asm volatile("bar.sync 1, %0;" ::"r"(FT));   // the filter warps only
+    const int q1 = min(total, LIST);
+    for (int q = threadIdx.x - 32; q < q1; q += FT) {
+      const int j = q / nsamp, s = q - j * nsamp;
+      int lit = dx_classify(v, v.md[fs[j].mesh], fs[j], s);
+      if (lit == 1) atomicAdd(&fs[j].count, 1);
+      if (lit < 0) list[atomicAdd(&nlist, 1)] = q;
+    }
+  }
+  __syncthreads();
+  for (int q0 = 0;;) {
+    const int nl = nlist;
+    for (int a = threadIdx.x; a < nl; a += THREADS) {
+      const int q = list[a];
+      const int j = q / nsamp;
+      dx_exact_sample(v, fs[j], q - j * nsamp, ahead);
+    }
+    q0 += LIST;
+    if (q0 >= total) break;
+    // more pairs than one round holds
+    __syncthreads();
+    if (threadIdx.x == 0) nlist = 0;
+    __syncthreads();
+    const int q1 = min(total, q0 + LIST);
+    for (int q = q0 + threadIdx.x; q < q1; q += THREADS) {
+      const int j = q / nsamp, s = q - j * nsamp;
+      int lit = dx_classify(v, v.md[fs[j].mesh], fs[j], s);
+      if (lit == 1) atomicAdd(&fs[j].count, 1);
+      if (lit < 0) list[atomicAdd(&nlist, 1)] = q;
+    }
+    __syncthreads();
+  }
+  __syncthreads();
+  // the facet's flux, one thread per facet
+  if (threadIdx.x < nf) {
+    const DxFacet& F = fs[threadIdx.x];
+    const MeshDesc& M = v.md[F.mesh];
+    const SunAux* S = mesh_sun(v, M, ahead);
+    double dv = (double)F.count / M.denom;
+    double mu = F.mu;
+    dv *= (mu > 0.0 ? mu : 0.0);
+    dv *= S->flux;
+    store_direct(v, M, F.f, dv, dropin, ahead);
+  }
+  __syncthreads();
+}
+
 template <int NF>
 __global__ void __launch_bounds__(DX_THREADS) k_direct_exact(StepView v, int dropin, int mu32_flux, int ahead) {
   __shared__ DxFacet fs[NF];
   __shared__ int list[DX_LIST];
   __shared__ int nlist;
   const int nw = v.counters[0];
-  const int nsamp = v.ndisk - 1;   // samples per facet (the meshes of a view share the disk)
-  const int FT = DX_THREADS - 32;  // filter threads (warps 1..)
-  for (int base = blockIdx.x * NF; base < nw; base += gridDim.x * NF) {
-    const int nf = min(NF, nw - base);
-    const int total = nf * nsamp;
-    if (threadIdx.x < 32) {
-      // FP64 set-up, one lane per facet (overlaps the filter below)
-      if (threadIdx.x < nf) {
-        DxFacet& F = fs[threadIdx.x];
-        int f = v.work[base + threadIdx.x];
-        const MeshDesc& M = v.md[v.mesh_of ? v.mesh_of[f] : 0];
-        const SunAux* S = mesh_sun(v, M, ahead);
-        float4 c4 = v.cen[f];
-        d3 p = mkd((double)c4.x, (double)c4.y, (double)c4.z);
-        d3 Sv = mkd(S->sx, S->sy, S->sz);
-        d3 SP = sub(Sv, p);
-        double dist = norm(SP);
-        d3 N = mkd(SP.x / dist, SP.y / dist, SP.z / dist);   // = geom.h normalise(S - p)
-        d3 T, B;
-        sun_frame(N, &T, &B);
-        F.Tx = T.x; F.Ty = T.y; F.Tz = T.z;
-        F.Bx = B.x; F.By = B.y; F.Bz = B.z;
-        if (mu32_flux) {
-          float4 n4 = v.nrm[f];
-          F.mu = (double)((n4.x * S->ux + n4.y * S->uy) + n4.z * S->uz);
-        } else {
-          const double* fr = v.frame + 9 * (int64_t)f;
-          F.mu = sun_mu(Sv, p, mkd(fr[6], fr[7], fr[8]));
-        }
-      }
-    } else {
-      if (threadIdx.x - 32 < nf) dx_setup32(v, fs[threadIdx.x - 32], v.work[base + threadIdx.x - 32], ahead);
-      if (threadIdx.x == 32) nlist = 0;
-      asm volatile("bar.sync 1, %0;" ::"r"(FT));   // the filter warps only
-      const int q1 = min(total, DX_LIST);
-      for (int q = threadIdx.x - 32; q < q1; q += FT) {
-        const int j = q / nsamp, s = q - j * nsamp;
-        int lit = dx_classify(v, v.md[fs[j].mesh], fs[j], s);
-        if (lit == 1) atomicAdd(&fs[j].count, 1);
-        if (lit < 0) list[atomicAdd(&nlist, 1)] = q;
-      }
+  for (int base = blockIdx.x * NF; base < nw; base += gridDim.x * NF)
+    exact_facets<DX_THREADS, DX_LIST>(v, fs, list, nlist, v.work + base, min(NF, nw - base), dropin, mu32_flux, ahead);
+}
+
+// Both passes in one kernel that fits beside a radiosity solve: one block of
+// 128 (FP64) or 256 (mixed) threads of 64 registers per SM, a few KB of shared
+// memory (the solve's 1,024 threads and its ring take the rest). A pipelined
+// step runs a later frame's insolation this way while its own radiosity
+// solve streams the matrix: the solve leaves the FP64 pipe and half of the
+// issue slots idle. Blocks take a facet per thread at a time, in turn, and pass their
+// own undecided ones to the exact test, DXB_FACETS at a time.
+// Alone it takes longer than the two launches (81,920 facets: 64 against 45 us
+// in FP64, 47 against 31 us mixed), but they ran beside a conduction that
+// leaves them no registers until its last blocks: a step took 235 us in FP64
+// (solve 154, conduction 49, both with the insolation 75) and 73 us mixed,
+// now 207 and 58 us.
+constexpr int DXB_FACETS = 8;
+constexpr int DXB_LIST = 1024;
+
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_direct_beside(StepView v, int mu32_flux, int ahead) {
+  __shared__ DxFacet fs[DXB_FACETS];
+  __shared__ int list[DXB_LIST];
+  __shared__ int work[DXB_FACETS + THREADS];   // undecided facets
+  __shared__ int nlist, nwork;
+  if (threadIdx.x == 0) nwork = 0;
+  __syncthreads();
+  for (int64_t f0 = (int64_t)blockIdx.x * THREADS; f0 < v.nt; f0 += (int64_t)gridDim.x * THREADS) {
+    const int f = (int)min(f0 + threadIdx.x, (int64_t)v.nt);
+    if (classify_facet(v, f, 0, mu32_flux, ahead)) work[atomicAdd(&nwork, 1)] = f;
+    __syncthreads();
+    int n = nwork;
+    while (n >= DXB_FACETS) {
+      exact_facets<THREADS, DXB_LIST>(v, fs, list, nlist, work + n - DXB_FACETS, DXB_FACETS, 0, mu32_flux, ahead);
+      n -= DXB_FACETS;
     }
     __syncthreads();
-    for (int q0 = 0;;) {
-      const int nl = nlist;
-      for (int a = threadIdx.x; a < nl; a += DX_THREADS) {
-        const int q = list[a];
-        const int j = q / nsamp;
-        dx_exact_sample(v, fs[j], q - j * nsamp, ahead);
-      }
-      q0 += DX_LIST;
-      if (q0 >= total) break;
-      // more pairs than one round holds (more than DX_LIST / DX_FACETS samples per facet)
-      __syncthreads();
-      if (threadIdx.x == 0) nlist = 0;
-      __syncthreads();
-      const int q1 = min(total, q0 + DX_LIST);
-      for (int q = q0 + threadIdx.x; q < q1; q += DX_THREADS) {
-        const int j = q / nsamp, s = q - j * nsamp;
-        int lit = dx_classify(v, v.md[fs[j].mesh], fs[j], s);
-        if (lit == 1) atomicAdd(&fs[j].count, 1);
-        if (lit < 0) list[atomicAdd(&nlist, 1) ] = q;
-      }
-      __syncthreads();
-    }
-    __syncthreads();
-    // the facet's flux, one thread per facet
-    if (threadIdx.x < nf) {
-      const DxFacet& F = fs[threadIdx.x];
-      const MeshDesc& M = v.md[F.mesh];
-      const SunAux* S = mesh_sun(v, M, ahead);
-      double dv = (double)F.count / M.denom;
-      double mu = F.mu;
-      dv *= (mu > 0.0 ? mu : 0.0);
-      dv *= S->flux;
-      store_direct(v, M, F.f, dv, dropin, ahead);
-    }
+    if (threadIdx.x == 0) nwork = n;
     __syncthreads();
   }
+  const int n = nwork;
+  if (n > 0) exact_facets<THREADS, DXB_LIST>(v, fs, list, nlist, work, n, 0, mu32_flux, ahead);
 }
 
 }  // namespace
@@ -408,6 +462,21 @@ int direct_launch(const StepView& v, int dropin, int mu32_flux, int ahead, cudaS
     case 32: k_direct_exact<32><<<152 * 4, DX_THREADS, 0, s>>>(v, dropin, mu32_flux, ahead); break;
     default: set_error("exact_facets must be 4, 8, 16 or 32"); return ILG_ERR_ARG;
   }
+  ILG_CUDA(cudaGetLastError());
+  return ILG_OK;
+}
+
+// The same for a frame ahead, sized to run beside the radiosity solve.
+int direct_beside_launch(const StepView& v, int mu32_flux, int ahead, cudaStream_t s) {
+  // the solve's split of the SM between shared memory and L1: a kernel that
+  // asks for another one waits until the SM is empty
+  auto go = [&](auto kern, int threads) -> int {
+    ILG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    kern<<<std::min(div_up(v.nt, threads), 152), threads, 0, s>>>(v, mu32_flux, ahead);   // one block per SM
+    return ILG_OK;
+  };
+  if (mu32_flux) ILG_TRY(go(k_direct_beside<256>, 256));
+  else ILG_TRY(go(k_direct_beside<128>, 128));
   ILG_CUDA(cudaGetLastError());
   return ILG_OK;
 }

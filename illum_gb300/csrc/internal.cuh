@@ -348,6 +348,7 @@ SunAux make_sun_aux(const double* s, double solar_const, double scene_mag, doubl
 // ahead = 1: the flux of the frame after each mesh's current one (the
 // pipelined step computes it beside the current frame's conduction).
 int direct_launch(const StepView& v, int dropin, int mu32_flux, int ahead, cudaStream_t s);
+int direct_beside_launch(const StepView& v, int mu32_flux, int ahead, cudaStream_t s);
 
 // ---- radiosity.cu ----
 int radiosity_prepare(Context& c);
@@ -389,8 +390,8 @@ int read_device_errors(Context& c);
 int check_run(Context& c, const ilg_run_opts* o, bool host_driven);
 MeshDesc solo_desc(const Context& c, const ilg_run_opts* o, int first_sun);
 int enqueue_step(const StepView& v, const StepPlan& p, cudaStream_t s, cudaEvent_t* ev);
-// Pipelined step: radiosity of the current frame, then its conduction on s
-// beside the next frame's direct insolation on pipe.s2, then the advance.
+// Pipelined step: radiosity of the current frame and its conduction on s,
+// beside a later frame's direct insolation on pipe.s2, then the advance.
 // The current frame's direct flux must be in its E slot already: from the
 // previous pipelined step or from enqueue_prologue at the start of a run.
 int enqueue_step_pipe(const StepView& v, const StepPlan& p, cudaStream_t s, const StepPipe& pipe);

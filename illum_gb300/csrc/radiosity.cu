@@ -74,10 +74,17 @@ namespace ilg {
 namespace {
 
 constexpr int RAD_THREADS = 992;             // consumer threads (31 warps): one entry run each
+// Registers per thread: 1,024 threads leave 8,192 of the SM's in the FP64 and
+// 16,384 in the mixed solve, one block of 128 or 256 threads of the direct
+// insolation that runs beside it (direct.cu k_direct_beside). The FP64 solves
+// are long enough to hide the smaller block and lose 8% at 48 registers.
+#define RAD_REGS64 56
+#define RAD_REGSM 48
 constexpr int RAD_BLOCK = RAD_THREADS + 32;  // and one producer warp that issues the entry-stream copies
 constexpr int RAD_HALO = 8192;           // halo values per tile (double-float: 64 KB of shared memory)
 constexpr int RAD_ROWS = 3072;           // rows per tile (their sums: 24 KB of shared memory)
 constexpr int RAD_MAX_MESH = 1024;
+constexpr int RAD_MESH_BYTES = 13;       // shared memory per mesh of the view (MeshState)
 constexpr int RAD_INNER = 2;             // most fp32 sweeps per refinement of the mixed solve: the bf16 error
                                          // (~4e-3 of the correction) already dominates rho^(k+1), rho ~ 0.013
 constexpr int64_t RAD_MIN_TILE = 16384;  // entries: smaller tiles cost more in staging than they balance
@@ -605,11 +612,14 @@ __device__ __forceinline__ unsigned long long* res_acc(const StepView& v, int k,
 // stopped; 1 for meshes that never ran. unit[m]: residual units per unit of
 // squared change, 2^20 / tol^2 enlarged by 2^-16 so that the FP32 products
 // below never round a partial's units down (+inf when tol is 0).
+// The arrays follow the tile buffers in dynamic shared memory, sized for the
+// view's meshes (a kernel beside this one needs what they leave).
 struct MeshState {
-  int done[RAD_MAX_MESH];
-  int sweeps[RAD_MAX_MESH];
-  float unit[RAD_MAX_MESH];
-  unsigned char now[RAD_MAX_MESH];   // stopped at the latest decision
+  int* done;
+  int* sweeps;
+  float* unit;
+  unsigned char* now;   // stopped at the latest decision
+  __device__ __forceinline__ explicit MeshState(int nmesh);
 };
 
 __device__ __forceinline__ unsigned long long res_units(float d2, float unit) {
@@ -705,10 +715,11 @@ __device__ __forceinline__ void record_residuals(const StepView& v, const MeshSt
 // every block, on every run, and alone or in a batch. A tolerance of zero
 // (or one whose units overflow) runs full sweeps only.
 struct MeshState64 {
-  int sweeps[RAD_MAX_MESH];
-  float acc[RAD_MAX_MESH];             // A in units of tol
-  unsigned char done[RAD_MAX_MESH];    // as MeshState::done
-  unsigned char mode[RAD_MAX_MESH];    // bit 0: the next sweep is a change sweep; bit 1: s is in S1
+  int* sweeps;
+  float* acc;             // A in units of tol
+  unsigned char* done;    // as MeshState::done
+  unsigned char* mode;    // bit 0: the next sweep is a change sweep; bit 1: s is in S1
+  __device__ __forceinline__ explicit MeshState64(int nmesh);
 };
 constexpr float CHG_STOP = 15.f / 16.f, CHG_NOISE_STOP = 1.f / 16.f;   // units of tol
 constexpr float CHG_NOISE = 1.1920929e-7f;                             // 2^-23
@@ -1078,6 +1089,23 @@ __device__ __forceinline__ RadSmem rad_smem() {
 }
 static_assert((RAD_RING + (size_t)(RAD_HALO + RAD_THREADS + RAD_ROWS) * 8 + RAD_THREADS) % 8 == 0,
               "stage barriers are 8-byte aligned");
+// Dynamic shared memory of a launch over nmesh meshes.
+constexpr size_t rad_smem_bytes(int nmesh) { return RAD_SMEM + (((size_t)nmesh * RAD_MESH_BYTES + 15) & ~(size_t)15); }
+
+__device__ __forceinline__ MeshState::MeshState(int nmesh) {
+  extern __shared__ __align__(128) unsigned char rad_dyn[];
+  done = reinterpret_cast<int*>(rad_dyn + RAD_SMEM);
+  sweeps = done + nmesh;
+  unit = reinterpret_cast<float*>(sweeps + nmesh);
+  now = reinterpret_cast<unsigned char*>(unit + nmesh);
+}
+__device__ __forceinline__ MeshState64::MeshState64(int nmesh) {
+  extern __shared__ __align__(128) unsigned char rad_dyn[];
+  sweeps = reinterpret_cast<int*>(rad_dyn + RAD_SMEM);
+  acc = reinterpret_cast<float*>(sweeps + nmesh);
+  done = reinterpret_cast<unsigned char*>(acc + nmesh);
+  mode = done + nmesh;
+}
 
 // The ring's barriers, set up by thread 0 before the launch's first block
 // barrier (inside init_meshes' caller): full counts the producer's one
@@ -1120,8 +1148,8 @@ __device__ __forceinline__ void produce_pass(Pipe& p, const StepView& v, const M
 
 // FP64 Jacobi to each mesh's tolerance, full and change sweeps as above.
 // x: solution (and warm start).
-__global__ void __launch_bounds__(RAD_BLOCK, 1) k_radiosity64(StepView v, double* x, int warm) {
-  __shared__ MeshState64 st;
+__global__ void __maxnreg__(RAD_REGS64) k_radiosity64(StepView v, double* x, int warm) {
+  MeshState64 st(v.nmesh);
   __shared__ float red[32];
   __shared__ int bad;
   const RadSmem sm = rad_smem();
@@ -1240,8 +1268,7 @@ struct SoloShared {
   float acc;
 };
 
-constexpr int SOLO_ROWS = (RAD_ROWS + RAD_THREADS - 1) / RAD_THREADS;   // rows of a thread (4)
-constexpr int SOLO_HALO = 4;                                            // halo positions kept per thread
+constexpr int SOLO_HALO = 3;   // halo positions kept per thread (81,920 facets: 2,050 per tile on average)
 
 // End of sweep `it` of the block whose partial is d2 (thread 0's): publish,
 // wait for every block's, and decide. All threads; false once a wait ran out.
@@ -1302,7 +1329,7 @@ __device__ __forceinline__ bool solo_sweep_end(const StepView& v, SoloShared& S,
   return S.ok != 0;
 }
 
-__global__ void __launch_bounds__(RAD_BLOCK, 1) k_radiosity64_solo(StepView v, double* x, int warm) {
+__global__ void __maxnreg__(RAD_REGS64) k_radiosity64_solo(StepView v, double* x, int warm) {
   __shared__ SoloShared S;
   const RadSmem sm = rad_smem();
   const bool producer = threadIdx.x >= RAD_THREADS;
@@ -1325,7 +1352,10 @@ __global__ void __launch_bounds__(RAD_BLOCK, 1) k_radiosity64_solo(StepView v, d
   const ValsDF vals{v.t_vhi, v.t_vlo};
   const ValsHiF vhi{v.t_vhi};
   const uint64_t pol = l2_keep_policy(v.l2_stream);
-  uint32_t s0 = 0, hpos[SOLO_HALO], rpos[SOLO_ROWS];
+  // a thread's first row stays in registers (most tiles have fewer rows than
+  // threads), further ones are loaded again every sweep
+  uint32_t s0 = 0, hpos[SOLO_HALO], rpos = 0;
+  const bool has_row = !producer && threadIdx.x < T.nrows;
   if (!producer) {
     init_x(v, x, warm, gt, nthreads, false);
     s0 = tile_start(v, t);
@@ -1334,20 +1364,11 @@ __global__ void __launch_bounds__(RAD_BLOCK, 1) k_radiosity64_solo(StepView v, d
       const int h = threadIdx.x + q * RAD_THREADS;
       hpos[q] = h < T.nhalo ? __ldg(v.t_halo + T.h0 + h) : 0u;
     }
-#pragma unroll
-    for (int q = 0; q < SOLO_ROWS; ++q) {
-      const int r = threadIdx.x + q * RAD_THREADS;
-      rpos[q] = r < T.nrows ? __ldg(v.t_row + T.r0 + r) : 0u;
-    }
+    if (has_row) rpos = __ldg(v.t_row + T.r0 + threadIdx.x);
   }
   unsigned gen = 0;
   if (!grid_barrier(v.barrier, gridDim.x, gen, v.derr)) return;
-  float2 sown[SOLO_ROWS];
-  if (!producer) {
-#pragma unroll
-    for (int q = 0; q < SOLO_ROWS; ++q)
-      sown[q] = threadIdx.x + q * RAD_THREADS < T.nrows ? ld_it(B.S0 + rpos[q]) : make_float2(0.f, 0.f);
-  }
+  float2 sown = has_row ? ld_it(B.S0 + rpos) : make_float2(0.f, 0.f);
   int it = 0;
   for (;; ++it) {
     const int mode = S.mode;
@@ -1376,32 +1397,34 @@ __global__ void __launch_bounds__(RAD_BLOCK, 1) k_radiosity64_solo(StepView v, d
           sxf[h] = ld_it(dcur + __ldg(v.t_halo + T.h0 + h));
         cbar();
         tile_rows<AccF32>(v, T, s0, pipe32, vhi, sxf, reinterpret_cast<float*>(sm.tail), sm.tnew, rsf);
-#pragma unroll
-        for (int q = 0; q < SOLO_ROWS; ++q) {
-          const int r = threadIdx.x + q * RAD_THREADS;
-          if (r < T.nrows) {
-            const float d = rsf[r];
-            sown[q] = df_add(sown[q], make_float2(d, 0.f));
-            cur[rpos[q]] = sown[q];
-            dnxt[rpos[q]] = d;
-            d2 = __fmaf_rn(d, d, d2);
-          }
+        auto finish = [&](uint32_t i, float d, float2& so) {
+          so = df_add(so, make_float2(d, 0.f));
+          cur[i] = so;
+          dnxt[i] = d;
+          d2 = __fmaf_rn(d, d, d2);
+        };
+        if (has_row) finish(rpos, rsf[threadIdx.x], sown);
+        for (int r = threadIdx.x + RAD_THREADS; r < T.nrows; r += RAD_THREADS) {
+          const uint32_t i = __ldg(v.t_row + T.r0 + r);
+          float2 so = ld_it(cur + i);
+          finish(i, rsf[r], so);
         }
       } else {
         float2* nxt = (mode & 2) ? B.S0 : B.S1;
         stage_halo_sum(v, T, B.EH, cur, sm.sx);
         tile_rows<AccDF>(v, T, s0, pipe, vals, sm.sx, sm.tail, sm.tnew, sm.rs);
-#pragma unroll
-        for (int q = 0; q < SOLO_ROWS; ++q) {
-          const int r = threadIdx.x + q * RAD_THREADS;
-          if (r < T.nrows) {
-            const float2 sn = sm.rs[r];
-            const float d = __fadd_rn(__fsub_rn(sn.x, sown[q].x), __fsub_rn(sn.y, sown[q].y));
-            sown[q] = sn;
-            nxt[rpos[q]] = sn;
-            dnxt[rpos[q]] = d;
-            d2 = __fmaf_rn(d, d, d2);
-          }
+        auto finish = [&](uint32_t i, float2 sn, float2& so) {
+          const float d = __fadd_rn(__fsub_rn(sn.x, so.x), __fsub_rn(sn.y, so.y));
+          so = sn;
+          nxt[i] = sn;
+          dnxt[i] = d;
+          d2 = __fmaf_rn(d, d, d2);
+        };
+        if (has_row) finish(rpos, sm.rs[threadIdx.x], sown);
+        for (int r = threadIdx.x + RAD_THREADS; r < T.nrows; r += RAD_THREADS) {
+          const uint32_t i = __ldg(v.t_row + T.r0 + r);
+          float2 so = ld_it(cur + i);
+          finish(i, sm.rs[r], so);
         }
       }
       d2 = block_sum(d2, S.red);
@@ -1430,8 +1453,8 @@ __global__ void __launch_bounds__(RAD_BLOCK, 1) k_radiosity64_solo(StepView v, d
 // bf16 F~ (inner sweeps, 1..RAD_INNER), s += d. A mesh stops when
 // ||r||_2 <= tol, or after the update of the round that reaches max_sweeps;
 // each tile's block writes its rows' results.
-__global__ void __launch_bounds__(RAD_BLOCK, 1) k_radiosity_mixed(StepView v, double* x, int warm, int inner) {
-  __shared__ MeshState st;
+__global__ void __maxnreg__(RAD_REGSM) k_radiosity_mixed(StepView v, double* x, int warm, int inner) {
+  MeshState st(v.nmesh);
   __shared__ float red[32];
   __shared__ int bad;
   const RadSmem sm = rad_smem();
@@ -1571,8 +1594,8 @@ __global__ void __launch_bounds__(RAD_BLOCK, 1) k_radiosity_mixed(StepView v, do
 // halos of (x - x_ref, dE)), and the next step starts from s0 = s + P, off by
 // F^2 dE instead of F dE. The step's squared change |s - s0|^2 is recorded
 // as its residual.
-__global__ void __launch_bounds__(RAD_BLOCK, 1) k_radiosity_lagged(StepView v, double* x, int warm) {
-  __shared__ MeshState st;
+__global__ void __maxnreg__(RAD_REGSM) k_radiosity_lagged(StepView v, double* x, int warm) {
+  MeshState st(v.nmesh);
   __shared__ float red[32];
   __shared__ int bad;
   // each mesh's kind of pass (0: bf16 step, 1: reference step, 2: reference
@@ -1798,18 +1821,16 @@ int radiosity_setup() {
   int dev, nsm;
   ILG_CUDA(cudaGetDevice(&dev));
   ILG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  ILG_CUDA(cudaFuncSetAttribute(k_radiosity64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RAD_SMEM));
-  ILG_CUDA(cudaFuncSetAttribute(k_radiosity64_solo, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RAD_SMEM));
-  ILG_CUDA(cudaFuncSetAttribute(k_radiosity_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RAD_SMEM));
-  ILG_CUDA(cudaFuncSetAttribute(k_radiosity_lagged, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RAD_SMEM));
-  ILG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_rad_per_sm64, k_radiosity64, RAD_BLOCK, RAD_SMEM));
-  ILG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_rad_per_smm, k_radiosity_mixed, RAD_BLOCK, RAD_SMEM));
-  int per_solo = 0;     // the two FP64 kernels share the grid
-  ILG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_solo, k_radiosity64_solo, RAD_BLOCK, RAD_SMEM));
-  g_rad_per_sm64 = std::min(g_rad_per_sm64, per_solo);
-  int per_lagged = 0;   // the two mixed kernels share the grid
-  ILG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_lagged, k_radiosity_lagged, RAD_BLOCK, RAD_SMEM));
-  g_rad_per_smm = std::min(g_rad_per_smm, per_lagged);
+  const size_t most = rad_smem_bytes(RAD_MAX_MESH);
+  for (const void* k : {(const void*)k_radiosity64, (const void*)k_radiosity64_solo, (const void*)k_radiosity_mixed,
+                        (const void*)k_radiosity_lagged}) {
+    int per = 0;   // one grid (and tile schedule) serves every kernel
+    ILG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    ILG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, RAD_BLOCK, most));
+    const bool fp64 = k == (const void*)k_radiosity64 || k == (const void*)k_radiosity64_solo;
+    int& least = fp64 ? g_rad_per_sm64 : g_rad_per_smm;
+    least = least > 0 ? std::min(least, per) : per;
+  }
   if (g_rad_per_sm64 < 1 || g_rad_per_smm < 1) { set_error("radiosity kernel cannot be resident"); return ILG_ERR_CUDA; }
   g_rad_nsm = nsm;
   g_rad_ready.store(true, std::memory_order_release);
@@ -2263,7 +2284,7 @@ int radiosity_launch(const StepView& v, double* x, int warm, int precision, int 
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(RAD_BLOCK);
-  cfg.dynamicSmemBytes = RAD_SMEM;
+  cfg.dynamicSmemBytes = rad_smem_bytes(v.nmesh);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;   // all blocks co-resident: the grid barrier is safe
