@@ -268,8 +268,8 @@ class IllumContext:
         return {"per_source": per, "within_radius": within[:rad.shape[0]], "rays": rays.value}
 
     def get_F(self):
-        rowptr = np.zeros(self.num_faces + 1, np.int64)
-        col = np.zeros(max(self.nnz, 1), np.int32); val = np.zeros(max(self.nnz, 1), np.float64)
+        rowptr = np.empty(self.num_faces + 1, np.int64)
+        col = np.empty(max(self.nnz, 1), np.int32); val = np.empty(max(self.nnz, 1), np.float64)
         _check(lib().ilg_get_F(self._h, _p(rowptr), _p(col), _p(val)))
         return rowptr, col[:self.nnz], val[:self.nnz]
 
@@ -315,7 +315,7 @@ class IllumContext:
     @property
     def horizons(self) -> np.ndarray:
         """nphi x N (one column of zenith angles per facet)."""
-        out = np.zeros((self.num_faces, self.nphi), np.float64)
+        out = np.empty((self.num_faces, self.nphi), np.float64)
         _check(lib().ilg_get_horizons(self._h, _p(out)))
         return out.T
 
@@ -334,14 +334,14 @@ class IllumContext:
         s = _f64(sun_position).reshape(3)
         d = np.asarray(disk_xy, np.float64)
         dcm = np.ascontiguousarray(d.T)     # column-major n x 2
-        out = np.zeros(self.num_faces, np.float64)
+        out = np.empty(self.num_faces, np.float64)
         _check(lib().ilg_direct_radiosity(self._h, _p(s), _p(dcm), d.shape[0], _p(out)))
         return out
 
     # -- radiosity
     def radiosity_solve(self, E, tol=1e-10, max_sweeps=200):
         E = _f64(E)
-        x = np.zeros(self.num_faces, np.float64)
+        x = np.empty(self.num_faces, np.float64)
         res = C.c_double(); sw = C.c_int()
         _check(lib().ilg_radiosity_solve(self._h, _p(E), tol, max_sweeps, _p(x), C.byref(res), C.byref(sw)))
         return x, res.value, sw.value
@@ -354,7 +354,7 @@ class IllumContext:
         """The reference's solve: forward solve + gs_steps natural-order
         Gauss-Seidel sweeps (src/cpp/illum_cli.cpp:425-433). Returns (x, res)."""
         E = _f64(E)
-        x = np.zeros(self.num_faces, np.float64)
+        x = np.empty(self.num_faces, np.float64)
         res = C.c_double()
         _check(lib().ilg_radiosity_solve_gs(self._h, _p(E), int(gs_steps), _p(x), C.byref(res)))
         return x, res.value
@@ -382,13 +382,13 @@ class IllumContext:
         _check(lib().ilg_set_suns(self._h, s.shape[0], _p(s), _p(dcm), d.shape[0]))
 
     def run_steps(self, opts: RunOpts, first_sun: int, nsteps: int, record_tsurf=False):
-        out = np.zeros((nsteps, self.num_faces), np.float64) if record_tsurf else None
+        out = np.empty((nsteps, self.num_faces), np.float64) if record_tsurf else None
         _check(lib().ilg_run_steps(self._h, C.byref(opts), first_sun, nsteps, _p(out)))
         return out
 
     def run_steps_host(self, opts: RunOpts, suns, record_tsurf=True):
         s = _f64(suns).reshape(-1, 3)
-        out = np.zeros((s.shape[0], self.num_faces), np.float64) if record_tsurf else None
+        out = np.empty((s.shape[0], self.num_faces), np.float64) if record_tsurf else None
         _check(lib().ilg_run_steps_host(self._h, C.byref(opts), s.shape[0], _p(s), _p(out)))
         return out
 
@@ -402,7 +402,7 @@ class IllumContext:
 
     def outputs(self):
         n = self.num_faces
-        r, ra, ta, tm = (np.zeros(n) for _ in range(4))
+        r, ra, ta, tm = (np.empty(n) for _ in range(4))
         _check(lib().ilg_get_outputs(self._h, _p(r), _p(ra), _p(ta), _p(tm)))
         return {"rad": r, "rad_avg": ra, "therm_avg": ta, "therm_max": tm}
 
@@ -498,7 +498,7 @@ class ThermalModel:
         return {"per_source": per, "within_radius": within[:rad.shape[0]], "rays": rays.value}
 
     def get_F(self):
-        F = np.zeros(self.ctx.num_faces)
+        F = np.empty(self.ctx.num_faces)
         _check(lib().ilg_thermal_get(self.ctx._h, None, _p(F), None))
         return F
 
@@ -562,7 +562,7 @@ class Batch:
         _check(lib().ilg_batch_set_active(self._h, member, int(active)))
 
     def tsurf(self, member):
-        out = np.zeros(self.contexts[member].num_faces)
+        out = np.empty(self.contexts[member].num_faces)
         _check(lib().ilg_batch_get_tsurf(self._h, member, _p(out)))
         return out
 

@@ -23,6 +23,7 @@
 
 #include <cuda_bf16.h>
 
+#include <initializer_list>
 #include <vector>
 
 #include "common.cuh"
@@ -400,6 +401,12 @@ int enqueue_prologue(const StepView& v, const StepPlan& p, cudaStream_t s);
 int enqueue_serial_prologue(const StepView& v, const StepPlan& p, cudaStream_t s);
 int advance_launch(const StepView& v, cudaStream_t s);
 int flush_launch(float4* buf, size_t n, unsigned salt, cudaStream_t s);
+
+// ---- capi.cu ----
+// Makes the pages of caller arrays that a copy from the device will fill
+// resident first (see the definition).
+struct HostRange { void* p; size_t bytes; };
+void fault_in(std::initializer_list<HostRange> ranges);
 
 // ---- conduction.cu ----
 int conduction_prepare(Context& c, double dt, int precision);
