@@ -87,7 +87,6 @@ constexpr int RAD_MAX_MESH = 1024;
 constexpr int RAD_MESH_BYTES = 13;       // shared memory per mesh of the view (MeshState)
 constexpr int RAD_INNER = 2;             // most fp32 sweeps per refinement of the mixed solve: the bf16 error
                                          // (~4e-3 of the correction) already dominates rho^(k+1), rho ~ 0.013
-constexpr int64_t RAD_MIN_TILE = 16384;  // entries: smaller tiles cost more in staging than they balance
 constexpr int64_t RAD_SPLIT_MIN = 131072;  // entries: tiles above twice the split target are halved
 // Tile balance, in stored entries: a block's sweep time is about
 // c + 1.35e-4 us per stored entry + 8.8e-4 us per row + 1.5e-4 us per halo
@@ -96,6 +95,13 @@ constexpr int64_t RAD_SPLIT_MIN = 131072;  // entries: tiles above twice the spl
 constexpr int64_t RAD_ROW_COST = 7;
 constexpr int64_t RAD_HALO_COST = 1;
 constexpr int64_t RAD_GROUP = 4 * RAD_THREADS;  // stored entries per group (4 per thread): a tile's stream is whole groups
+// Smallest tile, in entries: one group. A small mesh's sweep is bound by its
+// longest tile (each further group ~1 us) and a barrier whose cost does not
+// grow from 3 blocks to 94, so it takes as many blocks as it has groups: FP64
+// steps of 5,120 facets (45,577 entries) take 57 us in 12 tiles of one group,
+// 60 in 6, 70 in 4, 77 in 3 and 96 in 2; of 20,480 facets (728,586) 83 us in
+// 94 tiles, 90 in 38, 106 in 21; in mixed precision 34 / 42 and 37 / 39 us.
+constexpr int64_t RAD_MIN_TILE = RAD_GROUP;
 // One group in shared memory: its columns (u16), then its values (f32 hi,
 // f32 lo for the FP64 sweeps; f32 hi for the mixed residual; bf16 for the
 // mixed inner sweeps). Every piece is a multiple of 16 bytes, and a group
