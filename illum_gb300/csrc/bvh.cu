@@ -482,9 +482,9 @@ constexpr int PATH_MOST = 64;              // bits of a lane's mask of path entr
 constexpr int LANE_IDLE = 0x7fffffff;      // no node left (codes of internal nodes are < 2^31 - 1)
 // Lanes at internal nodes below which pending leaves are tested, and idle
 // lanes from which new rays begin (form factors of 81,920 facets: 8..20 lanes
-// with 4..28 idle ones took 268..169 ms, fewer registers aside).
+// with 4..28 idle ones took 268..145 ms; lanes wait cheaply).
 constexpr int NODE_LANES = 16;
-constexpr int REFILL_LANES = 24;
+constexpr int REFILL_LANES = 28;
 
 struct PathEntry {
   float4 a, b, c;   // box (lo.xyz, hi.x), (hi.y, hi.z, child code as int bits, dmin - m . o), slab (m, dmax - m . o)
@@ -1019,21 +1019,55 @@ __global__ void __launch_bounds__(128) k_count_pairs(LeafGroups G, const float4*
 // possibly more than once (it is sorted and made unique afterwards); hits
 // that the warp has seen lately for the same source are dropped.
 //
-// A warp takes one source at a time (from a counter) and keeps its lanes
-// filled from the source's enumeration. Every ray begins with the triangle
+// A warp takes one unit at a time (from a counter): a source, or a part of
+// one with many candidates, and keeps its lanes filled from the source's
+// enumeration. Every ray begins with the triangle
 // it is aimed at, which bounds its length before any box is tested, and with
 // its own facet; the order of the tests does not change the closest hit.
 // Bound by issue (62%, 17 of 32 lanes active) and L1 bandwidth (54%). Form
-// factors of 81,920 facets (766 M rays) 234 -> 164 ms, of a 256 x 256 terrain
-// within 30 m (92 M rays) 53 -> 39 ms against a candidate list in device
-// memory (a counting and a filling walk per source, 0.4 and 0.17 of the ray
-// kernel's time) and one root-to-leaf walk over boxes per ray.
+// factors of 81,920 facets (766 M rays) 234 -> 145 ms, of a 256 x 256 terrain
+// within 30 m (92 M rays) 53 -> 37 ms, of 20,480 facets (7.4 M) 7.1 -> 2.3 ms
+// against a candidate list in device memory (a counting and a filling walk per
+// source, 0.4 and 0.17 of the ray kernel's time) and one root-to-leaf walk
+// over boxes per ray. The enumeration waits in shared memory, which leaves the
+// walk without spills at seven blocks per SM (five: 13% slower, six 4%).
 constexpr int VIS_THREADS = 128;
 constexpr int VIS_QUEUE = 64;      // candidates waiting (at most 31 + 32)
 constexpr int VIS_KEYS = 64;       // keys waiting to be written (at most 31 + 32)
 constexpr int VIS_SEEN = 128;      // recent hits per warp
 
+// Candidates per unit. A facet deep in a crater has twenty times the
+// candidates of one outside, and as one unit its rays would keep one warp
+// busy after the others have run out: 20,480 facets (7.4 M rays, at most
+// 4,522 of one source, 229 in the middle) took 2.23 ms that way, with SMs at
+// work for 72% of it on average, and 1.4 ms in parts. A part first counts through the candidates before it
+// and loads the path anew, so sources are only split where the mean warp has
+// few units: at VIS_SHARES parts of a warp's share of the rays, at least
+// VIS_PART_MIN.
+constexpr int VIS_PART_MIN = 256;
+constexpr int VIS_SHARES = 8;
+
+// The units of sources [a, b): (source, its part), in any order.
+__global__ void k_vis_units(const uint32_t* __restrict__ count, int a, int b, uint32_t part, uint2* units,
+                            unsigned* nunits) {
+  const int q = a + blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const unsigned n = q < b ? (count[q] + part - 1) / part : 0;
+  unsigned at = n;
+  for (int o = 1; o < 32; o *= 2) {
+    const unsigned t = __shfl_up_sync(0xffffffffu, at, o);
+    if (lane >= o) at += t;
+  }
+  unsigned base = 0;
+  if (lane == 31 && at) base = atomicAdd(nunits, at);
+  base = __shfl_sync(0xffffffffu, base, 31);
+  at += base - n;
+  for (unsigned k = 0; k < n; ++k) units[at + k] = make_uint2((unsigned)q, k);
+}
+
 struct VisWarp {
+  Enumerate en;              // the unit's enumeration, out of the walk's registers
+  unsigned passed;           // candidates it has passed
   int queue[VIS_QUEUE];
   int seen[VIS_SEEN];
   unsigned long long keys[VIS_KEYS];
@@ -1082,11 +1116,12 @@ __device__ __forceinline__ void test_closest(const float4* __restrict__ tri_s, i
   }
 }
 
-__global__ void __launch_bounds__(VIS_THREADS, 6)
+__global__ void __launch_bounds__(VIS_THREADS, 7)
 k_vis_rays(const float4* __restrict__ nodes, const float4* __restrict__ tri_s, const int* __restrict__ parent,
            const uint32_t* __restrict__ rank, LeafGroups G, const float4* __restrict__ cen,
-           const float4* __restrict__ nrm, const int* __restrict__ src, int q0, int q1, float offset, int bits,
-           int entries, int* next_source, unsigned long long* ukeys, unsigned long long* ucount, int* derr) {
+           const float4* __restrict__ nrm, const int* __restrict__ src, const uint2* __restrict__ units,
+           const unsigned* __restrict__ nunits, unsigned part, float offset, int bits, int entries,
+           unsigned* next_unit, unsigned long long* ukeys, unsigned long long* ucount, int* derr) {
   __shared__ VisWarp sh[VIS_THREADS / 32];
   extern __shared__ PathEntry vis_paths[];   // [warp][entries]
   PathEntry* path = vis_paths + (size_t)(threadIdx.x >> 5) * entries;
@@ -1103,25 +1138,53 @@ k_vis_rays(const float4* __restrict__ nodes, const float4* __restrict__ tri_s, c
     __syncwarp();
     nkeys = 0;
   };
+  const unsigned nu = __ldg(nunits);
   for (;;) {
-    int q = 0;
-    if (lane == 0) q = q0 + atomicAdd(next_source, 1);
-    q = __shfl_sync(0xffffffffu, q, 0);
-    if (q >= q1) break;
+    unsigned u = 0;
+    if (lane == 0) u = atomicAdd(next_unit, 1u);
+    u = __shfl_sync(0xffffffffu, u, 0);
+    if (u >= nu) break;
+    const uint2 unit = __ldg(units + u);
+    const int q = (int)unit.x;
     const int j = src ? src[q] : (int)G.order[q];
     const f3 p_j = f3of(cen[j]), n_j = f3of(nrm[j]);
     const f3 o = add(p_j, scl(n_j, offset));
-    Enumerate en;
-    en.start(G, j, p_j, n_j);
+    __syncwarp();
+    if (lane == 0) {
+      S.en.start(G, j, p_j, n_j);
+      S.passed = 0;
+    }
+    __syncwarp();
     int qn = 0;                 // candidates in the queue
+    // The next candidates into the queue, at least `want`; false: no more.
+    // The unit's are those of rank [first, first + part) in the source's
+    // enumeration.
+    auto fetch = [&](int want) -> bool {
+      Enumerate en = S.en;
+      unsigned at = S.passed;
+      const unsigned first = unit.y * part;
+      bool more = true;
+      while (qn < want) {
+        int k0;
+        unsigned pass;
+        more = at < first + part && en.next(G, lane, k0, pass);
+        if (!more) break;
+        const unsigned r = at + __popc(pass & lt);
+        const bool in = ((pass >> lane) & 1) && r >= first && r < first + part;
+        const unsigned take = __ballot_sync(0xffffffffu, in);
+        if (in) S.queue[qn + __popc(take & lt)] = k0 + lane;
+        qn += __popc(take);
+        at += __popc(pass);
+      }
+      __syncwarp();
+      if (lane == 0) {
+        S.en = en;
+        S.passed = at;
+      }
+      __syncwarp();
+      return more;
+    };
     bool more = true;
-    int k0;
-    unsigned pass;
-    // the first group before the path: many sources have no candidates
-    more = en.next(G, lane, k0, pass);
-    if (!more) continue;
-    if ((pass >> lane) & 1) S.queue[__popc(pass & lt)] = k0 + lane;
-    qn = __popc(pass);
     const int own = (int)__ldg(rank + j);
     const int ne = load_path(nodes, parent, G.nt, own, o, path, entries, lane);
     for (int t = lane; t < VIS_SEEN; t += 32) S.seen[t] = -1;
@@ -1155,13 +1218,7 @@ k_vis_rays(const float4* __restrict__ nodes, const float4* __restrict__ tri_s, c
       // fill the idle lanes
       const unsigned idle = __ballot_sync(0xffffffffu, !on);
       const int want = __popc(idle);
-      while (more && qn < want) {
-        more = en.next(G, lane, k0, pass);
-        if (!more) break;
-        if ((pass >> lane) & 1) S.queue[qn + __popc(pass & lt)] = k0 + lane;
-        qn += __popc(pass);
-        __syncwarp();
-      }
+      if (more && qn < want) more = fetch(want);
       const int take = min(want, qn);
       if (!on && __popc(idle & lt) < take) {
         target = S.queue[qn - 1 - __popc(idle & lt)];
@@ -1589,6 +1646,8 @@ int ff_set_chunk(int64_t pairs) {
 // The leaf groups of a build (LeafGroups over its own buffers).
 struct GroupBufs {
   dbuf<float4> cen_s, lo[3], hi[3];
+  dbuf<uint32_t> cnt;         // candidates per source (count_pairs)
+  dbuf<uint2> units;          // of the chunk being cast
   LeafGroups G{};
   int build(const Context& c, double cutoff, cudaStream_t s) {
     const int nt = c.nt;
@@ -1625,36 +1684,43 @@ struct GroupBufs {
 
 // Candidate pairs per source (of the facets src, or all of them by Morton
 // position): their exclusive sums, with the total behind them.
-static int count_pairs(Context& c, const GroupBufs& g, const int* src, int nsrc, std::vector<unsigned long long>& offs_h,
+static int count_pairs(Context& c, GroupBufs& g, const int* src, int nsrc, std::vector<unsigned long long>& offs_h,
                        cudaStream_t s) {
-  dbuf<uint32_t> cnt;
   dbuf<unsigned long long> offs;
-  ILG_TRY(cnt.alloc(nsrc));
+  ILG_TRY(g.cnt.alloc(nsrc));
   ILG_TRY(offs.alloc(nsrc));
-  k_count_pairs<<<div_up(nsrc, 4), 128, 0, s>>>(g.G, c.nrm.p, c.cen.p, src, nsrc, cnt.p);
+  k_count_pairs<<<div_up(nsrc, 4), 128, 0, s>>>(g.G, c.nrm.p, c.cen.p, src, nsrc, g.cnt.p);
   ILG_CUDA(cudaGetLastError());
-  ILG_TRY(scan_exclusive_u32_to_u64(cnt.p, offs.p, nsrc, c.scan, s));
+  ILG_TRY(scan_exclusive_u32_to_u64(g.cnt.p, offs.p, nsrc, c.scan, s));
   offs_h.resize((size_t)nsrc + 1);
   uint32_t last_cnt = 0;
   ILG_CUDA(cudaMemcpyAsync(offs_h.data(), offs.p, 8 * (size_t)nsrc, cudaMemcpyDeviceToHost, s));
-  ILG_CUDA(cudaMemcpyAsync(&last_cnt, cnt.p + (nsrc - 1), 4, cudaMemcpyDeviceToHost, s));
+  ILG_CUDA(cudaMemcpyAsync(&last_cnt, g.cnt.p + (nsrc - 1), 4, cudaMemcpyDeviceToHost, s));
   ILG_CUDA(cudaStreamSynchronize(s));
   offs_h[nsrc] = offs_h[nsrc - 1] + last_cnt;
   return ILG_OK;
 }
 
-// The rays of sources [a, b): keys into ukeys (room for every pair of the
-// range), their number in *nk. counters: two zeroed words, ucount and the
-// source counter.
-static int cast_visibility(Context& c, const GroupBufs& g, const int* src, int a, int b, float offset, int bits,
-                           unsigned long long* ukeys, unsigned long long* counters, unsigned long long* nk,
+// The rays of sources [a, b), npairs in all: keys into ukeys (room for every
+// pair), their number in *nk. counters: two words, ucount and (units, units
+// taken).
+static int cast_visibility(Context& c, GroupBufs& g, const int* src, int a, int b, int64_t npairs, float offset,
+                           int bits, unsigned long long* ukeys, unsigned long long* counters, unsigned long long* nk,
                            cudaStream_t s) {
   ILG_CUDA(cudaMemsetAsync(counters, 0, 16, s));
-  const int blocks = std::min(div_up(b - a, VIS_THREADS / 32), 152 * 16);   // warps take sources from a counter
+  unsigned* nunits = reinterpret_cast<unsigned*>(counters + 1);
+  const int warps = VIS_THREADS / 32, most = 152 * 16;   // blocks; warps take units from a counter
+  const uint32_t part = (uint32_t)std::min<int64_t>(
+      std::max<int64_t>(VIS_PART_MIN, npairs / ((int64_t)VIS_SHARES * 152 * 7 * warps)), 1 << 30);
+  const int64_t cap = (int64_t)(b - a) + npairs / part;   // sum of ceil(count / part)
+  ILG_TRY(g.units.reserve(cap));
+  k_vis_units<<<div_up(b - a, 256), 256, 0, s>>>(g.cnt.p, a, b, part, g.units.p, nunits);
+  ILG_CUDA(cudaGetLastError());
+  const int blocks = (int)std::min<int64_t>((cap + warps - 1) / warps, most);
   const int entries = path_entries(c);
-  const size_t smem = (size_t)(VIS_THREADS / 32) * entries * sizeof(PathEntry);
+  const size_t smem = (size_t)warps * entries * sizeof(PathEntry);
   k_vis_rays<<<blocks, VIS_THREADS, smem, s>>>(c.nodes.p, c.tri_s.p, c.parent.p, c.leaf_rank.p, g.G, c.cen.p, c.nrm.p,
-                                               src, a, b, offset, bits, entries, reinterpret_cast<int*>(counters + 1),
+                                               src, g.units.p, nunits, part, offset, bits, entries, nunits + 1,
                                                ukeys, counters, c.derr.p);
   ILG_CUDA(cudaGetLastError());
   ILG_CUDA(cudaMemcpyAsync(nk, counters, 8, cudaMemcpyDeviceToHost, s));
@@ -1712,7 +1778,7 @@ int form_factors_build(Context& c, const double* albedo_h, double albedo_scalar,
       const int64_t np = (int64_t)(offs_h[b] - offs_h[a]);
       if (np == 0) continue;
       unsigned long long nk = 0;
-      ILG_TRY(cast_visibility(c, groups, nullptr, a, b, (float)offset, bits, ukeys.p, ucount.p, &nk, s));
+      ILG_TRY(cast_visibility(c, groups, nullptr, a, b, np, (float)offset, bits, ukeys.p, ucount.p, &nk, s));
       if (nk == 0) continue;
       if (nk > 1) ILG_TRY(radix_sort_u64(ukeys.p, nullptr, (int64_t)nk, 2 * bits, c.sort, s));
       ILG_TRY(keep.reserve(nk));
@@ -1846,7 +1912,7 @@ int visibility_sample(Context& c, double cutoff, double offset, const int* src_h
     const int64_t np = (int64_t)(offs_h[b] - offs_h[a]);
     if (np == 0) continue;
     unsigned long long nk = 0;
-    ILG_TRY(cast_visibility(c, groups, dsrc.p, a, b, (float)offset, bits, ukeys.p, ucount.p, &nk, s));
+    ILG_TRY(cast_visibility(c, groups, dsrc.p, a, b, np, (float)offset, bits, ukeys.p, ucount.p, &nk, s));
     if (nk > 1) ILG_TRY(radix_sort_u64(ukeys.p, nullptr, (int64_t)nk, 2 * bits, c.sort, s));
     if (nk > 0) {
       k_sample_count<<<div_up((int64_t)nk, 256), 256, 0, s>>>(ukeys.p, (int64_t)nk, bits, c.cen.p, c.nrm.p, c.area.p,

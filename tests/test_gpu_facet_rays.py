@@ -36,3 +36,22 @@ def test_form_factors_around_leaf_groups(ilg, oracle_mod, n_faces, cutoff):
     rpo, cpo, vpo = oracle_mod.coo_to_csr(n_faces, ro, co, vo)
     assert np.array_equal(rp, rpo) and np.array_equal(col, cpo) and np.array_equal(val, vpo)
     assert ctx.visibility_rays == rays
+
+
+@pytest.mark.parametrize("n_seen", [255, 256, 257, 511, 512, 513, 1100])
+def test_form_factors_of_a_source_cast_in_parts(ilg, oracle_mod, n_seen):
+    """A facet that faces n_seen others: its rays are cast in parts of 256."""
+    g = np.random.default_rng(n_seen)
+    u = g.normal(size=(n_seen, 3))
+    u[:, 2] = np.abs(u[:, 2]) + 0.2
+    c = u / np.linalg.norm(u, axis=1)[:, None] * g.uniform(0.6, 1.0, (n_seen, 1))
+    tri = c[:, None, :] + 0.03 * g.normal(size=(n_seen, 3, 3))
+    floor = np.array([[[0.0, 0.0, 0.0], [0.05, 0.0, 0.0], [0.0, 0.05, 0.0]]])
+    v = np.concatenate([floor, tri]).reshape(-1, 3).astype(np.float32).astype(np.float64)
+    f = np.arange(3 * (n_seen + 1), dtype=np.int32).reshape(-1, 3)
+    ctx = ilg.IllumContext(v, f)
+    rp, col, val = ctx.compute_F(albedo=0.3)
+    ro, co, vo, rays = oracle_mod.form_factors(v, f, albedo_scalar=0.3, cutoff=-1.0)
+    rpo, cpo, vpo = oracle_mod.coo_to_csr(n_seen + 1, ro, co, vo)
+    assert np.array_equal(rp, rpo) and np.array_equal(col, cpo) and np.array_equal(val, vpo)
+    assert ctx.visibility_rays == rays
