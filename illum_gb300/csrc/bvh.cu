@@ -482,8 +482,9 @@ constexpr int PATH_MOST = 64;              // bits of a lane's mask of path entr
 constexpr int LANE_IDLE = 0x7fffffff;      // no node left (codes of internal nodes are < 2^31 - 1)
 // Lanes at internal nodes below which pending leaves are tested, and idle
 // lanes from which new rays begin (form factors of 81,920 facets: 8..20 lanes
-// with 4..28 idle ones took 268..145 ms; lanes wait cheaply).
-constexpr int NODE_LANES = 16;
+// with 4..28 idle ones took 268..145 ms; horizon maps are 1% faster with 12
+// than with 16).
+constexpr int NODE_LANES = 12;
 constexpr int REFILL_LANES = 28;
 
 struct PathEntry {
@@ -703,17 +704,26 @@ __device__ __forceinline__ void walk_nodes(Walk& w, int* stack, const float4* __
 // ------------------------------------------------------------------ horizons
 // One lane per (facet, azimuth): walk the precomputed bisection tree of
 // src/cpp/illum.cpp:304-316 (hit -> hi = mid, miss -> lo = mid), one any-hit
-// ray per level, until a terminal node. A warp holds 32 consecutive azimuths
-// of one or two facets (of up to HZ_FACETS when nphi < 32). A ray first
-// tests the triangle its lane's last ray hit: the next angle of the
-// bisection often hits it again.
-// Bound by issue (62%, 12 of 32 lanes active: rays of one facet differ most
-// in length) and the FP64 directions (38% of that pipe); 8 blocks per SM hide
-// the node loads (6 were 20% slower). 81,920 facets x 64 azimuths: 23.6 ms
-// with a root-to-leaf walk over boxes alone, 18.6 ms this way; 11.7 nodes and
-// 2.4 triangles per ray.
+// ray per level, until a terminal node. A warp has one facet (or HZ_FACETS
+// when nphi < 32), and a lane whose azimuth is done takes the next one: the
+// azimuths' work differs several times over, and with one per lane a warp
+// waited for its longest. A ray first tests the triangle its lane's last ray
+// hit: the next angle of the bisection often hits it again.
+// Bound by issue (rays of one facet differ most in length) and the FP64
+// directions (38% of that pipe); 8 blocks per SM hide the node loads (6 were
+// 20% slower, 7 6%, 9 spill). 81,920 facets x 64 azimuths: 23.6 ms with a
+// root-to-leaf walk over boxes alone, 18.9 ms with one azimuth per lane,
+// 16.6 ms this way; 20,480 x 32 1.03 -> 0.89 ms; a 256 x 256 terrain x 128
+// 68 -> 59 ms. With two or four facets per warp: 16.8 and 17.6, 1.04 and 1.19
+// (too few warps), 61 and 64 ms.
 constexpr int HZ_THREADS = 128;
-constexpr int HZ_FACETS = 4;      // most paths per warp
+constexpr int HZ_FACETS = 4;      // most facets per warp
+
+struct HzFacet {                  // one of a warp's facets
+  frame3 F;
+  f3 o;
+  int own, ne;                    // its leaf (-1: not in the tree) and path entries
+};
 
 __device__ __forceinline__ bool hit_any(const float4* __restrict__ tri_s, int k, f3 o, f3 d) {
   const float4 a = __ldg(&tri_s[3 * (int64_t)k]), b = __ldg(&tri_s[3 * (int64_t)k + 1]),
@@ -734,50 +744,35 @@ k_horizons(const float4* __restrict__ nodes, const float4* __restrict__ tri_s, i
            const double* __restrict__ cph, const double* __restrict__ sph, const HorizonNode* __restrict__ tree,
            int tree_size, float offset, int slots, int entries, double* H, int* derr) {
   extern __shared__ PathEntry hz_paths[];   // [warp][slots][entries]
+  __shared__ HzFacet hz_facets[HZ_THREADS / 32][HZ_FACETS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   PathEntry* paths = hz_paths + (size_t)warp * slots * entries;
-  const int64_t w = (int64_t)blockIdx.x * (HZ_THREADS / 32) + warp;
-  // the warp's first facet and the lane's (facet, azimuth)
-  int f0, nf, f, k;
-  bool on;
-  if (nphi >= 32) {
-    const int64_t g0 = 32 * w, g = g0 + lane, total = (int64_t)nt * nphi;
-    if (g0 >= total) return;
-    f0 = (int)(g0 / nphi);
-    nf = (int)((min(g0 + 31, total - 1)) / nphi) - f0 + 1;
-    on = g < total;
-    f = on ? (int)(g / nphi) : f0;
-    k = on ? (int)(g % nphi) : 0;
-  } else {
-    const int per = min(HZ_FACETS, 32 / nphi);
-    if (w * per >= nt) return;
-    f0 = (int)(w * per);
-    nf = min(per, nt - f0);
-    on = lane < nf * nphi;
-    f = f0 + (on ? lane / nphi : 0);
-    k = on ? lane % nphi : 0;
-  }
-  int ne = 0, own = -1;
+  HzFacet* facets = hz_facets[warp];
+  const int f0 = (blockIdx.x * (HZ_THREADS / 32) + warp) * slots;
+  if (f0 >= nt) return;
+  const int nf = min(slots, nt - f0), items = nf * nphi;
   for (int q = 0; q < nf; ++q) {
-    int m, kq = -1;
+    const f3 n = f3of(nrm[f0 + q]);
+    const f3 o = add(f3of(cen[f0 + q]), scl(n, offset));
+    int m, own = -1;
     if (SLAB) {
-      kq = (int)__ldg(rank + f0 + q);
-      m = load_path(nodes, parent, nt, kq, add(f3of(cen[f0 + q]), scl(f3of(nrm[f0 + q]), offset)),
-                    paths + q * entries, entries, lane);
+      own = (int)__ldg(rank + f0 + q);
+      m = load_path(nodes, parent, nt, own, o, paths + q * entries, entries, lane);
     } else {
       m = load_root(root, paths + q * entries, lane);
     }
-    if (f0 + q == f) {
-      ne = m;
-      own = kq;
+    if (lane == q) {
+      const int64_t f = f0 + q;
+      facets[q] = HzFacet{tri_frame(f3of(tri_o[3 * f]), f3of(tri_o[3 * f + 1]), n), o, own, m};
     }
   }
-  const PathEntry* path = paths + (f - f0) * entries;
-  const float4 c4 = cen[f], n4 = nrm[f];
-  const f3 n = f3of(n4);
-  const f3 o = add(f3of(c4), scl(n, offset));
-  const frame3 F = tri_frame(f3of(tri_o[3 * (int64_t)f]), f3of(tri_o[3 * (int64_t)f + 1]), n);
-  const double cp = cph[k], sp = sph[k];
+  __syncwarp();
+  // the lane's azimuth: item q * nphi + k of the warp's; the next one to take
+  int item = lane, next = 32;
+  bool on = item < items;
+  int q = on ? item / nphi : 0;
+  const PathEntry* path = paths + q * entries;
+  f3 o = facets[q].o;
   int node = 1, last = -1;
   RayF r = make_rayf(o, mk(0.f, 0.f, 1.f));
   Walk wk;
@@ -789,34 +784,45 @@ k_horizons(const float4* __restrict__ nodes, const float4* __restrict__ tri_s, i
   const float TMAX = 3.0e38f;
   for (;;) {
     if (fresh) {
-      bool go = true;
-      if (node >= tree_size) {
-        atomicExch(&derr[DERR_HORIZON], 1);
-        H[(int64_t)f * nphi + k] = 0.0;
-        go = false;
+      const HorizonNode* hn = tree + node;
+      const bool bad = node >= tree_size;
+      if (bad || hn->terminal) {
+        if (bad) atomicExch(&derr[DERR_HORIZON], 1);
+        H[(int64_t)f0 * nphi + item] = bad ? 0.0 : hn->mid;
         on = fresh = false;
       }
-      if (go) {
-        const HorizonNode hn = tree[node];
-        if (hn.terminal) {
-          H[(int64_t)f * nphi + k] = hn.mid;
-          on = fresh = false;
-        } else {
-          r = make_rayf(o, horizon_dir(F, cp, sp, hn.c, hn.s));
-          bool hit = last >= 0 && hit_any(tri_s, last, o, r.d);
-          if (!hit && own >= 0 && own != last) hit = hit_any(tri_s, own, o, r.d);
-          if (hit) {
-            node = 2 * node;              // still fresh: the next angle
-          } else {
-            fresh = false;
-            wk.sp = 0;
-            wk.mask = enter_mask(r, path, ne, TMAX);
-            walk_next<false>(wk, stack, r, path, TMAX);
-            if (wk.cur == LANE_IDLE) {    // enters nothing: a miss
-              node = 2 * node + 1;
-              fresh = true;
-            }
-          }
+    }
+    // lanes without an azimuth take the warp's next ones
+    if (next < items) {
+      const unsigned idle = __ballot_sync(0xffffffffu, !on);
+      const int mine = next + __popc(idle & ((1u << lane) - 1u));
+      next += __popc(idle);
+      if (!on && mine < items) {
+        item = mine;
+        q = item / nphi;
+        path = paths + q * entries;
+        o = facets[q].o;
+        node = 1;
+        last = -1;
+        on = fresh = true;
+      }
+    }
+    if (fresh && !tree[node].terminal) {   // (a tree may end at its root)
+      const int k = item - q * nphi, own = facets[q].own;
+      const HorizonNode hn = tree[node];
+      r = make_rayf(o, horizon_dir(facets[q].F, __ldg(cph + k), __ldg(sph + k), hn.c, hn.s));
+      bool hit = last >= 0 && hit_any(tri_s, last, o, r.d);
+      if (!hit && own >= 0 && own != last) hit = hit_any(tri_s, own, o, r.d);
+      if (hit) {
+        node = 2 * node;              // still fresh: the next angle
+      } else {
+        fresh = false;
+        wk.sp = 0;
+        wk.mask = enter_mask(r, path, facets[q].ne, TMAX);
+        walk_next<false>(wk, stack, r, path, TMAX);
+        if (wk.cur == LANE_IDLE) {    // enters nothing: a miss
+          node = 2 * node + 1;
+          fresh = true;
         }
       }
     }
@@ -1607,8 +1613,8 @@ int horizons_build(Context& c, int nphi, double theta_eps, double offset, const 
   // context's own (src/cpp/illum.cpp:333-360), where a facet's rays start at
   // its own leaf
   const Context& hb = hmesh ? *hmesh : c;
-  const int64_t warps = nphi >= 32 ? ((int64_t)c.nt * nphi + 31) / 32 : div_up(c.nt, std::min(HZ_FACETS, 32 / nphi));
-  const int slots = nphi >= 32 ? 2 : std::min(HZ_FACETS, 32 / nphi);
+  const int slots = nphi >= 32 ? 1 : HZ_FACETS;
+  const int warps = div_up(c.nt, slots);
   const int entries = hmesh ? 1 : path_entries(c);
   const size_t smem = (size_t)(HZ_THREADS / 32) * slots * entries * sizeof(PathEntry);
   auto kern = hmesh ? k_horizons<false> : k_horizons<true>;

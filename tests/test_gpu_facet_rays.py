@@ -26,6 +26,16 @@ def test_horizons_any_azimuth_count(ilg, oracle_mod, nphi):
     assert np.array_equal(ctx.horizons, oracle_mod.horizons(v, f, nphi).T)
 
 
+@pytest.mark.parametrize("n_faces", [1, 3, 5, 15, 18])
+@pytest.mark.parametrize("nphi", [9, 31, 32, 63, 97, 130])
+@pytest.mark.parametrize("theta_eps", [1e-3, 0.9, 4.0])   # 4: the bisection ends at its root
+def test_horizons_lanes_take_further_azimuths(ilg, oracle_mod, n_faces, nphi, theta_eps):
+    v, f = _mesh(n_faces)
+    ctx = ilg.IllumContext(v, f)
+    ctx.make_horizons(nphi=nphi, theta_eps=theta_eps)
+    assert np.array_equal(ctx.horizons, oracle_mod.horizons(v, f, nphi, theta_eps=theta_eps).T)
+
+
 @pytest.mark.parametrize("n_faces", [1, 2, 3, 31, 32, 33, 64, 97, 1025])
 @pytest.mark.parametrize("cutoff", [None, 0.35])
 def test_form_factors_around_leaf_groups(ilg, oracle_mod, n_faces, cutoff):
