@@ -751,6 +751,10 @@ k_horizons(const float4* __restrict__ nodes, const float4* __restrict__ tri_s, i
   const int f0 = (blockIdx.x * (HZ_THREADS / 32) + warp) * slots;
   if (f0 >= nt) return;
   const int nf = min(slots, nt - f0), items = nf * nphi;
+  if (tree_size > 1 && tree[1].terminal) {   // the bisection ends without a ray
+    for (int k = lane; k < items; k += 32) H[(int64_t)f0 * nphi + k] = tree[1].mid;
+    return;
+  }
   for (int q = 0; q < nf; ++q) {
     const f3 n = f3of(nrm[f0 + q]);
     const f3 o = add(f3of(cen[f0 + q]), scl(n, offset));
@@ -807,7 +811,7 @@ k_horizons(const float4* __restrict__ nodes, const float4* __restrict__ tri_s, i
         on = fresh = true;
       }
     }
-    if (fresh && !tree[node].terminal) {   // (a tree may end at its root)
+    if (fresh) {
       const int k = item - q * nphi, own = facets[q].own;
       const HorizonNode hn = tree[node];
       r = make_rayf(o, horizon_dir(facets[q].F, __ldg(cph + k), __ldg(sph + k), hn.c, hn.s));
