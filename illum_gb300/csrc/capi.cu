@@ -661,8 +661,7 @@ int ilg_ctx_device_bytes(const ilg_ctx* ctx, int64_t* bytes) {
            nbytes(c.t_cf) + nbytes(c.t_vbf) + nbytes(c.row_act) +
            nbytes(c.morton_order, c.leaf_rank, c.t_row, c.t_halo, c.t_start, c.rperm) +
            nbytes(c.work, c.counters, c.derr, c.mesh_flag, c.parent) + nbytes(c.barrier) + nbytes(c.sun_aux) + nbytes(c.md) +
-           nbytes(c.scan.a, c.scan.b, c.scan.c, c.sort.keys_alt, c.sort.hist, c.sort.scan.a, c.sort.scan.b,
-                  c.sort.scan.c) +
+           nbytes(c.scan.a, c.scan.b, c.scan.c, c.sort.keys_alt, c.sort.hist) +
            nbytes(c.sort.vals_alt);
   return ILG_OK;
 }

@@ -136,15 +136,12 @@ enum DevErr : int {
 };
 
 // ---- primitives (primitives.cu) ----
-// Exclusive prefix sum of n 64-bit counts; out may alias in. Uses tmp
-// scratch grown on demand. *total receives the sum when non-null (device->host
-// copy, synchronising the stream).
+// Exclusive prefix sum of n 32-bit counts, in 64 bits. Uses tmp scratch grown
+// on demand.
 struct ScanScratch {
   dbuf<unsigned long long> a, b, c;
   void release() { a.release(); b.release(); c.release(); }
 };
-int scan_exclusive_u64(const unsigned long long* in, unsigned long long* out, int64_t n,
-                       ScanScratch& tmp, cudaStream_t s);
 int scan_exclusive_u32_to_u64(const uint32_t* in, unsigned long long* out, int64_t n,
                               ScanScratch& tmp, cudaStream_t s);
 
@@ -153,9 +150,8 @@ int scan_exclusive_u32_to_u64(const uint32_t* in, unsigned long long* out, int64
 struct SortScratch {
   dbuf<unsigned long long> keys_alt;
   dbuf<uint32_t> vals_alt;
-  dbuf<unsigned long long> hist;
-  ScanScratch scan;
-  void release() { keys_alt.release(); vals_alt.release(); hist.release(); scan.release(); }
+  dbuf<unsigned long long> hist;   // digit counts, tile counters and states
+  void release() { keys_alt.release(); vals_alt.release(); hist.release(); }
 };
 int radix_sort_u64(unsigned long long* keys, uint32_t* vals, int64_t n, int bits, SortScratch& tmp,
                    cudaStream_t s);

@@ -2,6 +2,9 @@
 // LBVH build (Morton codes) and the form-factor CSR assembly (row/column
 // keys). Reduce-then-scan with 2048-element tiles; the radix sort ranks keys
 // inside a tile with warp match masks, which keeps it stable.
+#include <algorithm>
+#include <utility>
+
 #include "common.cuh"
 
 namespace ilg {
@@ -97,114 +100,258 @@ int scan_impl(const T* in, u64* out, int64_t n, ScanScratch& tmp, cudaStream_t s
 }
 
 // ---------------------------------------------------------------- radix sort
-constexpr int RS_THREADS = 256;
-constexpr int RS_WARPS = RS_THREADS / 32;
-constexpr int RS_ITEMS = 8;                       // per thread
-constexpr int RS_TILE = RS_THREADS * RS_ITEMS;    // 2048 keys per block
-constexpr int RS_WTILE = RS_TILE / RS_WARPS;      // 256 keys per warp
+// Stable LSD sort, 8 bits or less per pass. One launch counts the digits of
+// all passes; a pass then reads and writes every key once: a tile ranks its
+// keys, publishes its digit counts, adds up those of the tiles before it
+// (their own counts, or a running sum where one has been published: look-back)
+// and writes the tile out in digit order through shared memory, in runs of
+// about TILE / 128 keys. Tiles take their number from a counter, so the tiles
+// that one waits for are running or done. Bound by the ranking and the
+// look-back (33% issue, 27% of the copy rate) for large n and by the launches
+// for small n: 22 M keys of 34 bits with 32-bit values 1.28 ms, 20,480 keys of
+// 63 bits 80 us (a counting, three scan and a scatter launch per pass: 1.46 ms
+// and 210 us, the gaps between the launches aside).
+constexpr int RS_BINS = 256;
+constexpr int RS_PASSES = 8;
+constexpr int RS_LOOK = 4;          // tiles looked back at together: their loads overlap (1: 6% slower, 16: 5%)
+constexpr int RS_POLLS = 1 << 20;   // look-back polls before a tile counts for itself
 
-__global__ void k_radix_hist(const u64* __restrict__ keys, int64_t n, int shift, u64* __restrict__ hist,
-                             int nblocks) {
-  __shared__ unsigned h[256];
-  for (int i = threadIdx.x; i < 256; i += RS_THREADS) h[i] = 0;
+template <int THREADS_, int ITEMS_, int BLOCKS_>
+struct RadixTile {
+  static constexpr int BLOCKS = BLOCKS_, THREADS = THREADS_, ITEMS = ITEMS_, WARPS = THREADS / 32, TILE = THREADS * ITEMS;
+  static constexpr size_t SMEM = (size_t)TILE * 12;   // keys and values in digit order
+};
+typedef RadixTile<512, 12, 2> RadixLarge;
+typedef RadixTile<256, 8, 2> RadixSmall;   // up to RS_SMALL keys: more tiles than a few
+constexpr int64_t RS_SMALL = 1 << 19;
+
+// Digit counts of all passes: hist[pass][digit] += counts.
+__global__ void __launch_bounds__(256) k_radix_digits(const u64* __restrict__ keys, int64_t n, int passes, int width,
+                                                      u64* __restrict__ hist) {
+  __shared__ unsigned h[RS_PASSES * RS_BINS];
+  const int lane = threadIdx.x & 31;
+  const unsigned bins = 1u << width;
+  for (int i = threadIdx.x; i < passes * RS_BINS; i += 256) h[i] = 0;
   __syncthreads();
-  int64_t base = (int64_t)blockIdx.x * RS_TILE;
-  for (int i = 0; i < RS_ITEMS; ++i) {
-    int64_t idx = base + (int64_t)i * RS_THREADS + threadIdx.x;
-    if (idx < n) atomicAdd(&h[(unsigned)((keys[idx] >> shift) & 255ull)], 1u);
+  for (int64_t base = (int64_t)blockIdx.x * 256; base < n; base += (int64_t)gridDim.x * 256) {
+    const int64_t i = base + threadIdx.x;
+    const bool in = i < n;
+    const u64 k = in ? keys[i] : 0ull;
+    for (int p = 0; p < passes; ++p) {
+      const unsigned d = in ? (unsigned)(k >> (p * width)) & (bins - 1) : bins;
+      if (__all_sync(0xffffffffu, d == __shfl_sync(0xffffffffu, d, 0))) {   // neighbours often share their high digits
+        if (lane == 0 && in) atomicAdd(&h[p * RS_BINS + d], 32u);
+      } else if (in) {
+        atomicAdd(&h[p * RS_BINS + d], 1u);
+      }
+    }
   }
   __syncthreads();
-  for (int d = threadIdx.x; d < 256; d += RS_THREADS) hist[(int64_t)d * nblocks + blockIdx.x] = h[d];
+  for (int i = threadIdx.x; i < passes * RS_BINS; i += 256)
+    if (h[i]) atomicAdd(&hist[i], (u64)h[i]);
 }
 
-template <bool HASV>
-__global__ void k_radix_scatter(const u64* __restrict__ kin, const uint32_t* __restrict__ vin,
-                                u64* __restrict__ kout, uint32_t* __restrict__ vout, int64_t n, int shift,
-                                const u64* __restrict__ offs, int nblocks) {
-  __shared__ unsigned wcnt[RS_WARPS][256];
-  __shared__ u64 boff[256];
-  int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i < RS_WARPS * 256; i += RS_THREADS) (&wcnt[0][0])[i] = 0;
+// A tile's published digit count: value << 8 | code, the code 2 pass + 1 for
+// the tile's own count and 2 pass + 2 for the sum up to and with it.
+__device__ __forceinline__ void publish(u64* at, u64 value, int code) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(at), "l"((value << 8) | (u64)code) : "memory");
+}
+__device__ __forceinline__ u64 published(const u64* at) {
+  u64 v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(at) : "memory");
+  return v;
+}
+
+// Exclusive scans over the digits of two values, one digit per thread (the
+// first RS_BINS threads; every thread calls).
+template <int WARPS>
+__device__ __forceinline__ void scan_digits(unsigned a, u64 b, unsigned& ea, u64& eb, unsigned* wa, u64* wb) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned ia = a;
+  u64 ib = b;
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned ya = __shfl_up_sync(0xffffffffu, ia, o);
+    const u64 yb = __shfl_up_sync(0xffffffffu, ib, o);
+    if (lane >= o) {
+      ia += ya;
+      ib += yb;
+    }
+  }
+  if (lane == 31 && warp < RS_BINS / 32) {
+    wa[warp] = ia;
+    wb[warp] = ib;
+  }
   __syncthreads();
-  int64_t wbase = (int64_t)blockIdx.x * RS_TILE + (int64_t)warp * RS_WTILE;
-  u64 k[RS_ITEMS];
-  uint32_t v[RS_ITEMS];
-  unsigned rank[RS_ITEMS];
-  int dig[RS_ITEMS];
-  const unsigned lt_mask = (1u << lane) - 1u;
+  ea = ia - a;
+  eb = ib - b;
+  if (warp < RS_BINS / 32)
+    for (int w = 0; w < warp; ++w) {
+      ea += wa[w];
+      eb += wb[w];
+    }
+}
+
+template <class R, bool HASV>
+__global__ void __launch_bounds__(R::THREADS, R::BLOCKS)
+k_radix_pass(const u64* __restrict__ kin, const uint32_t* __restrict__ vin, u64* __restrict__ kout,
+             uint32_t* __restrict__ vout, int64_t n, int pass, int width, const u64* __restrict__ hist, u64* state,
+             unsigned* taken, int polls) {
+  constexpr int WARPS = R::WARPS, ITEMS = R::ITEMS, TILE = R::TILE;
+  extern __shared__ u64 rs_keys[];                              // [TILE], then the values
+  uint32_t* rs_vals = reinterpret_cast<uint32_t*>(rs_keys + TILE);
+  __shared__ unsigned wcnt[WARPS][RS_BINS];
+  __shared__ int64_t goff[RS_BINS];                             // digit's place in the output minus in the tile
+  __shared__ unsigned wa[RS_BINS / 32], tile_s;
+  __shared__ u64 wb[RS_BINS / 32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, shift = pass * width;
+  const unsigned mask = (1u << width) - 1u, lt = (1u << lane) - 1u;
+  if (threadIdx.x == 0) tile_s = atomicAdd(taken, 1u);
+  for (int i = threadIdx.x; i < WARPS * RS_BINS; i += R::THREADS) (&wcnt[0][0])[i] = 0;
+  __syncthreads();
+  const int64_t tile = tile_s, first = tile * TILE;
+  const int count = (int)min((int64_t)TILE, n - first);
+  u64 k[ITEMS];
+  uint32_t v[ITEMS];
+  unsigned rank[ITEMS];
 #pragma unroll
-  for (int it = 0; it < RS_ITEMS; ++it) {
-    int64_t idx = wbase + it * 32 + lane;
-    bool valid = idx < n;
-    k[it] = valid ? kin[idx] : 0ull;
-    if (HASV) v[it] = valid ? vin[idx] : 0u;
-    int d = valid ? (int)((k[it] >> shift) & 255ull) : 256;
-    dig[it] = d;
-    unsigned peers = __match_any_sync(0xffffffffu, d);
-    unsigned before = peers & lt_mask;
-    unsigned base = d < 256 ? wcnt[warp][d] : 0u;
+  for (int it = 0; it < ITEMS; ++it) {
+    const int i = warp * (32 * ITEMS) + it * 32 + lane;
+    k[it] = i < count ? kin[first + i] : ~0ull;
+    if (HASV) v[it] = i < count ? vin[first + i] : 0u;
+  }
+#pragma unroll
+  for (int it = 0; it < ITEMS; ++it) {
+    const bool in = warp * (32 * ITEMS) + it * 32 + lane < count;
+    const unsigned d = in ? (unsigned)(k[it] >> shift) & mask : mask + 1;
+    unsigned peers = 0xffffffffu;   // lanes with the same digit (a vote per bit: a third of match_any's time)
+    for (int b = 0; b <= width; ++b) {
+      const bool one = (d >> b) & 1;
+      const unsigned m = __ballot_sync(0xffffffffu, one);
+      peers &= one ? m : ~m;
+    }
+    const unsigned before = peers & lt;
+    const unsigned base = in ? wcnt[warp][d] : 0u;
     __syncwarp();
-    if (d < 256 && before == 0) wcnt[warp][d] = base + __popc(peers);
+    if (in && before == 0) wcnt[warp][d] = base + __popc(peers);
     __syncwarp();
     rank[it] = base + __popc(before);
   }
   __syncthreads();
-  for (int d = threadIdx.x; d < 256; d += RS_THREADS) {
-    unsigned run = 0;
-    for (int w = 0; w < RS_WARPS; ++w) {
-      unsigned c = wcnt[w][d];
-      wcnt[w][d] = run;
-      run += c;
+  const int d = threadIdx.x;
+  unsigned cnt = 0;
+  u64* mine = state + tile * RS_BINS + d;
+  if (d < RS_BINS) {
+    for (int w = 0; w < WARPS; ++w) {
+      const unsigned c = wcnt[w][d];
+      wcnt[w][d] = cnt;
+      cnt += c;
     }
-    boff[d] = offs[(int64_t)d * nblocks + blockIdx.x];
+    publish(mine, cnt, 2 * pass + (tile == 0 ? 2 : 1));
+  }
+  unsigned loc;
+  u64 gbase;
+  scan_digits<WARPS>(cnt, d < RS_BINS ? hist[d] : 0ull, loc, gbase, wa, wb);
+  // look-back
+  u64 before = 0;
+  bool lost = false;
+  if (d < RS_BINS && tile > 0) {
+    int64_t p = tile - 1;
+    int left = polls;
+    for (bool done = false; !done;) {
+      u64 w[RS_LOOK];
+      bool open = true;
+#pragma unroll
+      for (int q = 0; q < RS_LOOK; ++q) w[q] = p - q >= 0 ? published(state + (p - q) * RS_BINS + d) : 0ull;
+#pragma unroll
+      for (int q = 0; q < RS_LOOK; ++q) {
+        const int code = (int)(w[q] & 255ull) - 2 * pass;
+        open = open && !done && (code == 1 || code == 2);
+        if (open) {
+          before += w[q] >> 8;
+          --p;
+          done = code == 2;
+        }
+      }
+      if (!done && --left < 0) {
+        lost = true;
+        done = true;
+      }
+    }
+  }
+  if (__syncthreads_or(lost)) {   // count the keys before the tile directly
+    for (int i = threadIdx.x; i < RS_BINS; i += R::THREADS) goff[i] = 0;
+    __syncthreads();
+    for (int64_t i = threadIdx.x; i < first; i += R::THREADS)
+      atomicAdd(reinterpret_cast<u64*>(&goff[(unsigned)(kin[i] >> shift) & mask]), 1ull);
+    __syncthreads();
+    if (d < RS_BINS) before = (u64)goff[d];
+  }
+  if (d < RS_BINS) {
+    if (tile > 0) publish(mine, before + cnt, 2 * pass + 2);
+    goff[d] = (int64_t)(gbase + before) - (int64_t)loc;
+    for (int w = 0; w < WARPS; ++w) wcnt[w][d] += loc;
   }
   __syncthreads();
 #pragma unroll
-  for (int it = 0; it < RS_ITEMS; ++it) {
-    int d = dig[it];
-    if (d < 256) {
-      u64 pos = boff[d] + wcnt[warp][d] + rank[it];
-      kout[pos] = k[it];
-      if (HASV) vout[pos] = v[it];
+  for (int it = 0; it < ITEMS; ++it) {
+    if (warp * (32 * ITEMS) + it * 32 + lane < count) {
+      const unsigned at = wcnt[warp][(unsigned)(k[it] >> shift) & mask] + rank[it];
+      rs_keys[at] = k[it];
+      if (HASV) rs_vals[at] = v[it];
     }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < count; i += R::THREADS) {
+    const u64 key = rs_keys[i];
+    const int64_t at = goff[(unsigned)(key >> shift) & mask] + i;
+    kout[at] = key;
+    if (HASV) vout[at] = rs_vals[i];
   }
 }
 
-}  // namespace
-
-int scan_exclusive_u64(const u64* in, u64* out, int64_t n, ScanScratch& tmp, cudaStream_t s) {
-  return scan_impl<u64>(in, out, n, tmp, s, 0);
-}
-int scan_exclusive_u32_to_u64(const uint32_t* in, u64* out, int64_t n, ScanScratch& tmp, cudaStream_t s) {
-  return scan_impl<uint32_t>(in, out, n, tmp, s, 0);
-}
-
-int radix_sort_u64(u64* keys, uint32_t* vals, int64_t n, int bits, SortScratch& tmp, cudaStream_t s) {
-  if (n <= 1) return ILG_OK;
-  int nb = div_up(n, RS_TILE);
-  ILG_TRY(tmp.keys_alt.reserve((size_t)n));
-  if (vals) ILG_TRY(tmp.vals_alt.reserve((size_t)n));
-  ILG_TRY(tmp.hist.reserve((size_t)nb * 256));
+template <class R>
+int radix_passes(u64* keys, uint32_t* vals, int64_t n, int bits, SortScratch& tmp, cudaStream_t s) {
+  const int64_t tiles = (n + R::TILE - 1) / R::TILE;
+  const int passes = (bits + 7) / 8, width = (bits + passes - 1) / passes;
+  // digit counts, tile counters and tile states, all zero at first
+  const size_t head = (size_t)passes * RS_BINS + RS_PASSES;
+  ILG_TRY(tmp.hist.reserve(head + (size_t)tiles * RS_BINS));
+  u64* hist = tmp.hist.p;
+  unsigned* taken = reinterpret_cast<unsigned*>(hist + (size_t)passes * RS_BINS);
+  u64* state = hist + head;
+  ILG_CUDA(cudaMemsetAsync(hist, 0, (head + (size_t)tiles * RS_BINS) * 8, s));
+  k_radix_digits<<<(int)std::min<int64_t>((n + 2047) / 2048, 152 * 8), 256, 0, s>>>(keys, n, passes, width, hist);
+  ILG_CUDA(cudaGetLastError());
+  auto kern = vals ? k_radix_pass<R, true> : k_radix_pass<R, false>;
+  ILG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R::SMEM));
   u64 *ka = keys, *kb = tmp.keys_alt.p;
   uint32_t *va = vals, *vb = vals ? tmp.vals_alt.p : nullptr;
-  int passes = 0;
-  for (int shift = 0; shift < bits; shift += 8, ++passes) {
-    k_radix_hist<<<nb, RS_THREADS, 0, s>>>(ka, n, shift, tmp.hist.p, nb);
+  for (int p = 0; p < passes; ++p) {
+    kern<<<(int)tiles, R::THREADS, R::SMEM, s>>>(ka, va, kb, vb, n, p, width, hist + (size_t)p * RS_BINS, state,
+                                                 taken + p, RS_POLLS);
     ILG_CUDA(cudaGetLastError());
-    ILG_TRY(scan_exclusive_u64(tmp.hist.p, tmp.hist.p, (int64_t)nb * 256, tmp.scan, s));
-    if (vals)
-      k_radix_scatter<true><<<nb, RS_THREADS, 0, s>>>(ka, va, kb, vb, n, shift, tmp.hist.p, nb);
-    else
-      k_radix_scatter<false><<<nb, RS_THREADS, 0, s>>>(ka, nullptr, kb, nullptr, n, shift, tmp.hist.p, nb);
-    ILG_CUDA(cudaGetLastError());
-    u64* t = ka; ka = kb; kb = t;
-    uint32_t* tv = va; va = vb; vb = tv;
+    std::swap(ka, kb);
+    std::swap(va, vb);
   }
   if (passes & 1) {
     ILG_CUDA(cudaMemcpyAsync(keys, ka, (size_t)n * 8, cudaMemcpyDeviceToDevice, s));
     if (vals) ILG_CUDA(cudaMemcpyAsync(vals, va, (size_t)n * 4, cudaMemcpyDeviceToDevice, s));
   }
   return ILG_OK;
+}
+
+}  // namespace
+
+int scan_exclusive_u32_to_u64(const uint32_t* in, u64* out, int64_t n, ScanScratch& tmp, cudaStream_t s) {
+  return scan_impl<uint32_t>(in, out, n, tmp, s, 0);
+}
+
+int radix_sort_u64(u64* keys, uint32_t* vals, int64_t n, int bits, SortScratch& tmp, cudaStream_t s) {
+  if (n <= 1 || bits <= 0) return ILG_OK;
+  ILG_TRY(tmp.keys_alt.reserve((size_t)n));
+  if (vals) ILG_TRY(tmp.vals_alt.reserve((size_t)n));
+  return n <= RS_SMALL ? radix_passes<RadixSmall>(keys, vals, n, bits, tmp, s)
+                       : radix_passes<RadixLarge>(keys, vals, n, bits, tmp, s);
 }
 
 }  // namespace ilg

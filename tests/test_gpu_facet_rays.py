@@ -65,3 +65,14 @@ def test_form_factors_of_a_source_cast_in_parts(ilg, oracle_mod, n_seen):
     rpo, cpo, vpo = oracle_mod.coo_to_csr(n_seen + 1, ro, co, vo)
     assert np.array_equal(rp, rpo) and np.array_equal(col, cpo) and np.array_equal(val, vpo)
     assert ctx.visibility_rays == rays
+
+
+@pytest.mark.parametrize("n_faces", [2047, 2048, 2049, 4097])
+def test_leaf_order_around_sort_tiles(ilg, oracle_mod, n_faces):
+    """The Morton keys are sorted in tiles of 2,048."""
+    from illum_gb300 import meshgen
+    v, f = meshgen.icosphere_craters(4, seed=8, n_craters=8, dmin_m=200.0, dmax_m=600.0)
+    f = np.ascontiguousarray(f[::-1][:n_faces])
+    ctx = ilg.IllumContext(v, f)
+    ctx.make_horizons(nphi=2)
+    assert np.array_equal(ctx.horizons, oracle_mod.horizons(v, f, 2).T)
