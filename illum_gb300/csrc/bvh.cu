@@ -709,21 +709,28 @@ __device__ __forceinline__ void walk_nodes(Walk& w, int* stack, const float4* __
 // azimuths' work differs several times over, and with one per lane a warp
 // waited for its longest. A ray first tests the triangle its lane's last ray
 // hit: the next angle of the bisection often hits it again.
-// Bound by issue (rays of one facet differ most in length) and the FP64
-// directions (38% of that pipe); 8 blocks per SM hide the node loads (6 were
-// 20% slower, 7 6%, 9 spill). 81,920 facets x 64 azimuths: 23.6 ms with a
-// root-to-leaf walk over boxes alone, 18.9 ms with one azimuth per lane,
-// 16.6 ms this way; 20,480 x 32 1.03 -> 0.89 ms; a 256 x 256 terrain x 128
-// 68 -> 59 ms. With two or four facets per warp: 16.8 and 17.6, 1.04 and 1.19
-// (too few warps), 61 and 64 ms.
+// Bound by issue and node-load latency (rays of one facet differ most in
+// length); 8 blocks per SM hide the loads best (7 were 6% slower, 9 spill).
+// 81,920 facets x 64 azimuths: 23.6 ms with a root-to-leaf walk over boxes
+// alone, 18.9 ms with one azimuth per lane, 16.5 ms this way; 20,480 x 32
+// 1.03 -> 0.79 ms; a 256 x 256 terrain x 128 68 -> 60 ms. With two or four
+// facets per warp: 16.8 and 17.6, 1.04 and 1.19 (too few warps), 61 and 64 ms.
+// Ray directions in FP64 and a facet frame computed per warp kept that pipe
+// 54% busy (0.90 ms for 20,480 x 32): the frame is read instead, and a
+// direction is rounded from double-floats that know when they are not sure.
 constexpr int HZ_THREADS = 128;
 constexpr int HZ_FACETS = 4;      // most facets per warp
 
 struct HzFacet {                  // one of a warp's facets
   frame3 F;
+  float2 n[3];                    // F.n as double-floats
   f3 o;
   int own, ne;                    // its leaf (-1: not in the tree) and path entries
 };
+__device__ __forceinline__ float2 split_df(double x) {
+  const float hi = (float)x;
+  return make_float2(hi, (float)(x - (double)hi));
+}
 
 __device__ __forceinline__ bool hit_any(const float4* __restrict__ tri_s, int k, f3 o, f3 d) {
   const float4 a = __ldg(&tri_s[3 * (int64_t)k]), b = __ldg(&tri_s[3 * (int64_t)k + 1]),
@@ -734,27 +741,44 @@ __device__ __forceinline__ bool hit_any(const float4* __restrict__ tri_s, int k,
   return mt64(o, d, f3of(a), f3of(b), f3of(c), &th);
 }
 
+// fl(s g + c n) of one component of a ray's direction, s, c, g, n as
+// double-floats: geom.h horizon_dir rounds an FP64 value within 2^-50 of this
+// sum to float, so unless the sum (good to 2^-43) is as near as that to a
+// rounding boundary the float is the same. false: it may not be.
+__device__ __forceinline__ bool dir_component(float2 s, float2 g, float2 c, float2 n, float& out) {
+  const float p = __fmul_rn(s.x, g.x), q = __fmul_rn(c.x, n.x);
+  float e = __fmaf_rn(s.x, g.x, -p), f = __fmaf_rn(c.x, n.x, -q);
+  e = __fmaf_rn(s.x, g.y, e);
+  f = __fmaf_rn(c.x, n.y, f);
+  e = __fmaf_rn(s.y, g.x, e);
+  f = __fmaf_rn(c.y, n.x, f);
+  const float a = __fadd_rn(p, q), bb = __fsub_rn(a, p);
+  const float err = __fadd_rn(__fsub_rn(p, __fsub_rn(a, bb)), __fsub_rn(q, bb));   // TwoSum
+  const float lo = __fadd_rn(err, __fadd_rn(e, f));
+  const float h = __fadd_rn(a, lo), l = __fsub_rn(lo, __fsub_rn(h, a));
+  const float E = 2.2737368e-13f;   // 2^-42
+  out = h;
+  return __fadd_rn(h, __fadd_rn(l, E)) == h && __fadd_rn(h, __fsub_rn(l, E)) == h;
+}
+
 // SLAB: the facets are leaves of the tree (else the coordinates of the two
 // meshes may differ in magnitude, which the slabs' widening does not cover).
 template <bool SLAB>
 __global__ void __launch_bounds__(HZ_THREADS, 8)
 k_horizons(const float4* __restrict__ nodes, const float4* __restrict__ tri_s, int root,
-           const int* __restrict__ parent, const uint32_t* __restrict__ rank, const float4* __restrict__ tri_o,
+           const int* __restrict__ parent, const uint32_t* __restrict__ rank, const double* __restrict__ frame,
            const float4* __restrict__ cen, const float4* __restrict__ nrm, int nt, int nphi,
            const double* __restrict__ cph, const double* __restrict__ sph, const HorizonNode* __restrict__ tree,
            int tree_size, float offset, int slots, int entries, double* H, int* derr) {
   extern __shared__ PathEntry hz_paths[];   // [warp][slots][entries]
   __shared__ HzFacet hz_facets[HZ_THREADS / 32][HZ_FACETS];
+  __shared__ float2 hz_dir[3][HZ_THREADS];   // the lane's azimuth: cos b + sin t
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   PathEntry* paths = hz_paths + (size_t)warp * slots * entries;
   HzFacet* facets = hz_facets[warp];
   const int f0 = (blockIdx.x * (HZ_THREADS / 32) + warp) * slots;
   if (f0 >= nt) return;
   const int nf = min(slots, nt - f0), items = nf * nphi;
-  if (tree_size > 1 && tree[1].terminal) {   // the bisection ends without a ray
-    for (int k = lane; k < items; k += 32) H[(int64_t)f0 * nphi + k] = tree[1].mid;
-    return;
-  }
   for (int q = 0; q < nf; ++q) {
     const f3 n = f3of(nrm[f0 + q]);
     const f3 o = add(f3of(cen[f0 + q]), scl(n, offset));
@@ -766,8 +790,9 @@ k_horizons(const float4* __restrict__ nodes, const float4* __restrict__ tri_s, i
       m = load_root(root, paths + q * entries, lane);
     }
     if (lane == q) {
-      const int64_t f = f0 + q;
-      facets[q] = HzFacet{tri_frame(f3of(tri_o[3 * f]), f3of(tri_o[3 * f + 1]), n), o, own, m};
+      const double* fr = frame + 9 * (int64_t)(f0 + q);
+      const frame3 F{mkd(fr[0], fr[1], fr[2]), mkd(fr[3], fr[4], fr[5]), mkd(fr[6], fr[7], fr[8])};
+      facets[q] = HzFacet{F, {split_df(F.n.x), split_df(F.n.y), split_df(F.n.z)}, o, own, m};
     }
   }
   __syncwarp();
@@ -777,6 +802,14 @@ k_horizons(const float4* __restrict__ nodes, const float4* __restrict__ tri_s, i
   int q = on ? item / nphi : 0;
   const PathEntry* path = paths + q * entries;
   f3 o = facets[q].o;
+  auto aim = [&]() {
+    const frame3& F = facets[q].F;
+    const double cp = __ldg(cph + (item - q * nphi)), sp = __ldg(sph + (item - q * nphi));
+    hz_dir[0][threadIdx.x] = split_df(F.b.x * cp + F.t.x * sp);
+    hz_dir[1][threadIdx.x] = split_df(F.b.y * cp + F.t.y * sp);
+    hz_dir[2][threadIdx.x] = split_df(F.b.z * cp + F.t.z * sp);
+  };
+  if (on) aim();
   int node = 1, last = -1;
   RayF r = make_rayf(o, mk(0.f, 0.f, 1.f));
   Walk wk;
@@ -796,7 +829,8 @@ k_horizons(const float4* __restrict__ nodes, const float4* __restrict__ tri_s, i
         on = fresh = false;
       }
     }
-    // lanes without an azimuth take the warp's next ones
+    // lanes without an azimuth take the warp's next ones (the tree's root is
+    // never terminal: an azimuth has one ray at least)
     if (next < items) {
       const unsigned idle = __ballot_sync(0xffffffffu, !on);
       const int mine = next + __popc(idle & ((1u << lane) - 1u));
@@ -806,6 +840,7 @@ k_horizons(const float4* __restrict__ nodes, const float4* __restrict__ tri_s, i
         q = item / nphi;
         path = paths + q * entries;
         o = facets[q].o;
+        aim();
         node = 1;
         last = -1;
         on = fresh = true;
@@ -813,8 +848,15 @@ k_horizons(const float4* __restrict__ nodes, const float4* __restrict__ tri_s, i
     }
     if (fresh) {
       const int k = item - q * nphi, own = facets[q].own;
-      const HorizonNode hn = tree[node];
-      r = make_rayf(o, horizon_dir(facets[q].F, __ldg(cph + k), __ldg(sph + k), hn.c, hn.s));
+      const HorizonNode* hn = tree + node;
+      f3 dir;
+      const float2 sd = hn->sdf, cd = hn->cdf;
+      const HzFacet& fc = facets[q];
+      if (!(dir_component(sd, hz_dir[0][threadIdx.x], cd, fc.n[0], dir.x) &
+            dir_component(sd, hz_dir[1][threadIdx.x], cd, fc.n[1], dir.y) &
+            dir_component(sd, hz_dir[2][threadIdx.x], cd, fc.n[2], dir.z)))
+        dir = horizon_dir(fc.F, __ldg(cph + k), __ldg(sph + k), hn->c, hn->s);
+      r = make_rayf(o, dir);
       bool hit = last >= 0 && hit_any(tri_s, last, o, r.d);
       if (!hit && own >= 0 && own != last) hit = hit_any(tri_s, own, o, r.d);
       if (hit) {
@@ -1549,7 +1591,7 @@ int bvh_render(Context& c, int mode, double az_deg, double el_deg, int width, in
 // the reference's.
 static int build_horizon_tree(double theta_eps, std::vector<HorizonNode>& tree) {
   const int MAXD = 20;
-  tree.assign(2, HorizonNode{0, 0, 0, 0, 0});
+  tree.assign(2, HorizonNode{});
   struct St { double lo, hi, mid; };
   std::vector<St> st(2);
   st[1] = St{0.0, PI, PI / 2.0};
@@ -1598,6 +1640,10 @@ int horizons_build(Context& c, int nphi, double theta_eps, double offset, const 
   cudaStream_t s = c.stream;
   std::vector<HorizonNode> tree;
   ILG_TRY(build_horizon_tree(theta_eps, tree));
+  for (HorizonNode& nd : tree) {
+    nd.sdf = split_df_host(nd.s);
+    nd.cdf = split_df_host(nd.c);
+  }
   std::vector<double> cph(nphi), sph(nphi);
   double dphi = TWO_PI / (double)(nphi - 1);
   for (int k = 0; k < nphi; ++k) {
@@ -1624,7 +1670,7 @@ int horizons_build(Context& c, int nphi, double theta_eps, double offset, const 
   auto kern = hmesh ? k_horizons<false> : k_horizons<true>;
   ILG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kern<<<div_up(warps, HZ_THREADS / 32), HZ_THREADS, smem, s>>>(
-      hb.nodes.p, hb.tri_s.p, hb.root, hmesh ? nullptr : c.parent.p, c.leaf_rank.p, c.tri_o.p, c.cen.p, c.nrm.p, c.nt,
+      hb.nodes.p, hb.tri_s.p, hb.root, hmesh ? nullptr : c.parent.p, c.leaf_rank.p, c.frame.p, c.cen.p, c.nrm.p, c.nt,
       nphi, dc.p, ds.p, dtree.p, (int)tree.size(), (float)offset, slots, entries, c.H.p, c.derr.p);
   ILG_CUDA(cudaGetLastError());
   c.nphi = nphi;

@@ -37,6 +37,7 @@ struct HorizonNode {   // one node of the zenith-angle bisection tree
   double mid, s, c;    // mid angle and its sin / cos (geom.h sincos_x)
   int terminal;        // 1: the bisection returns mid here without a ray
   int pad;
+  float2 sdf, cdf;     // s and c as double-floats
 };
 
 // Scalars of a conduction table set (conduction.cu build_tables).

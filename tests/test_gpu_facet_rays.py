@@ -28,7 +28,7 @@ def test_horizons_any_azimuth_count(ilg, oracle_mod, nphi):
 
 @pytest.mark.parametrize("n_faces", [1, 3, 5, 15, 18])
 @pytest.mark.parametrize("nphi", [9, 31, 32, 63, 97, 130])
-@pytest.mark.parametrize("theta_eps", [1e-3, 0.9, 4.0])   # 4: the bisection ends at its root
+@pytest.mark.parametrize("theta_eps", [1e-3, 0.9, 4.0])   # 4: the bisection ends after one ray
 def test_horizons_lanes_take_further_azimuths(ilg, oracle_mod, n_faces, nphi, theta_eps):
     v, f = _mesh(n_faces)
     ctx = ilg.IllumContext(v, f)
@@ -76,3 +76,19 @@ def test_leaf_order_around_sort_tiles(ilg, oracle_mod, n_faces):
     ctx = ilg.IllumContext(v, f)
     ctx.make_horizons(nphi=2)
     assert np.array_equal(ctx.horizons, oracle_mod.horizons(v, f, 2).T)
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+def test_horizons_of_facets_along_an_axis(ilg, oracle_mod, axis):
+    """Direction components that are zero up to rounding: taken in FP64."""
+    n = 9
+    x, y = np.meshgrid(np.arange(n, dtype=np.float64), np.arange(n, dtype=np.float64), indexing="ij")
+    z = np.zeros((n, n))
+    z[4, 4] = 1.5
+    v = np.roll(np.stack([x.ravel(), y.ravel(), z.ravel()], axis=1), axis, axis=1)
+    i = (np.arange(n - 1)[:, None] * n + np.arange(n - 1)[None, :]).ravel()
+    f = np.concatenate([np.stack([i, i + n, i + 1], axis=1), np.stack([i + 1, i + n, i + n + 1], axis=1)])
+    f = np.ascontiguousarray(f, np.int32)
+    ctx = ilg.IllumContext(v, f)
+    ctx.make_horizons(nphi=17)
+    assert np.array_equal(ctx.horizons, oracle_mod.horizons(v, f, 17).T)
