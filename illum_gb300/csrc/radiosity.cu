@@ -87,6 +87,15 @@ constexpr int RAD_MAX_MESH = 1024;
 constexpr int RAD_MESH_BYTES = 13;       // shared memory per mesh of the view (MeshState)
 constexpr int RAD_INNER = 2;             // most fp32 sweeps per refinement of the mixed solve: the bf16 error
                                          // (~4e-3 of the correction) already dominates rho^(k+1), rho ~ 0.013
+// Largest tile, in entries, of a mesh that is cut for fewer blocks than the
+// device holds, to be solved beside others: blocks take several meshes' tiles,
+// longest first, and with few of them per block the longest block decides. A
+// tile costs as much as 26,000 entries besides its own, which speaks against
+// smaller ones. FP64 / mixed solves of a step, us, in tiles of 200,000, 128,000,
+// 64,000 and 32,000 entries: 16 meshes (36.7 M entries) 705 542 604 609 /
+// 100 87 95 98; 7 meshes 373 308 336 378 / 67 56 62 66; 3 meshes 360 263 178
+// 226 / 63 52 39 47; 12 meshes (2.3 M entries) 203 203 140 104 / 52 52 41 35.
+constexpr int64_t RAD_SHARED_TILE = 64000;
 constexpr int64_t RAD_SPLIT_MIN = 131072;  // entries: tiles above twice the split target are halved
 // Tile balance, in stored entries: a block's sweep time is about
 // c + 1.35e-4 us per stored entry + 8.8e-4 us per row + 1.5e-4 us per halo
@@ -108,17 +117,12 @@ constexpr int64_t RAD_MIN_TILE = RAD_GROUP;
 // starts at a multiple of RAD_GROUP entries, so each is one bulk copy.
 constexpr int RAD_CF_BYTES = (int)RAD_GROUP * 2;
 constexpr int RAD_F32_BYTES = (int)RAD_GROUP * 4;
-constexpr int RAD_STAGE64 = RAD_CF_BYTES + 2 * RAD_F32_BYTES;   // FP64 sweeps: 3 stages
-constexpr int RAD_STAGEM = RAD_CF_BYTES + RAD_F32_BYTES;        // mixed solve: 5 stages
-constexpr int RAD_NST64 = 3;
-constexpr int RAD_NSTM = 5;
-constexpr int RAD_NST_MAX = 8;
-constexpr size_t RAD_RING = (size_t)(RAD_NST64 * RAD_STAGE64 > RAD_NSTM * RAD_STAGEM ? RAD_NST64 * RAD_STAGE64
-                                                                                        : RAD_NSTM * RAD_STAGEM);
+constexpr int RAD_STAGE = RAD_CF_BYTES + RAD_F32_BYTES;
+constexpr int RAD_STAGES = 5;
+constexpr size_t RAD_RING = (size_t)RAD_STAGES * RAD_STAGE;
 static_assert(RAD_CF_BYTES % 16 == 0 && RAD_F32_BYTES % 16 == 0, "bulk copies move multiples of 16 bytes");
-static_assert(RAD_NST64 + RAD_NSTM <= RAD_NST_MAX, "stage barriers");
 constexpr size_t RAD_SMEM = RAD_RING + (size_t)RAD_HALO * sizeof(float2) + RAD_THREADS * sizeof(float2) +
-                            RAD_ROWS * sizeof(float2) + RAD_THREADS + 2 * RAD_NST_MAX * sizeof(unsigned long long);
+                            RAD_ROWS * sizeof(float2) + RAD_THREADS + 2 * RAD_STAGES * sizeof(unsigned long long);
 
 // Most polls of one grid-barrier wait (an L2 round trip each, ~0.4 us). A device variable so that a test can shrink it (ilg_debug_barrier_
 // timeout) and watch a wait run out without a long stall.
@@ -238,14 +242,9 @@ struct ValsDF { const float* hi; const float* lo; };   // double-float (hi, lo)
 struct ValsHi { const float* hi; };                    // fl(F) as a double-float with lo = 0
 struct ValsBF { const __nv_bfloat16* v; };             // bf16, scaled per row
 struct ValsHiF { const float* hi; };                   // fl(F) as a float
-__device__ __forceinline__ unsigned vals_bytes(ValsDF) { return 2 * RAD_F32_BYTES; }
 __device__ __forceinline__ unsigned vals_bytes(ValsHi) { return RAD_F32_BYTES; }
 __device__ __forceinline__ unsigned vals_bytes(ValsHiF) { return RAD_F32_BYTES; }
 __device__ __forceinline__ unsigned vals_bytes(ValsBF) { return RAD_CF_BYTES; }
-__device__ __forceinline__ void copy_vals(ValsDF s, unsigned dst, size_t e, unsigned long long* bar, uint64_t pol) {
-  bulk_copy(dst, s.hi + e, RAD_F32_BYTES, bar, pol);
-  bulk_copy(dst + RAD_F32_BYTES, s.lo + e, RAD_F32_BYTES, bar, pol);
-}
 __device__ __forceinline__ void copy_vals(ValsHi s, unsigned dst, size_t e, unsigned long long* bar, uint64_t pol) {
   bulk_copy(dst, s.hi + e, RAD_F32_BYTES, bar, pol);
 }
@@ -254,14 +253,6 @@ __device__ __forceinline__ void copy_vals(ValsHiF s, unsigned dst, size_t e, uns
 }
 __device__ __forceinline__ void copy_vals(ValsBF s, unsigned dst, size_t e, unsigned long long* bar, uint64_t pol) {
   bulk_copy(dst, s.v + e, RAD_CF_BYTES, bar, pol);
-}
-__device__ __forceinline__ void read_vals(ValsDF, const unsigned char* st, int tid, float2 (&w)[4]) {
-  const float4 h = *reinterpret_cast<const float4*>(st + 16 * tid);
-  const float4 l = *reinterpret_cast<const float4*>(st + RAD_F32_BYTES + 16 * tid);
-  w[0] = make_float2(h.x, l.x);
-  w[1] = make_float2(h.y, l.y);
-  w[2] = make_float2(h.z, l.z);
-  w[3] = make_float2(h.w, l.w);
 }
 __device__ __forceinline__ void read_vals(ValsHi, const unsigned char* st, int tid, float2 (&w)[4]) {
   const float4 h = *reinterpret_cast<const float4*>(st + 16 * tid);
@@ -300,12 +291,10 @@ struct Pipe {
   unsigned long long* full;
   unsigned long long* empty;
   int* bad;
-  int nst;
-  int stage_bytes;
   int s;
   unsigned parity;
   __device__ __forceinline__ void advance() {
-    if (++s == nst) {
+    if (++s == RAD_STAGES) {
       s = 0;
       parity ^= 1u;
     }
@@ -323,11 +312,29 @@ __device__ __forceinline__ void produce_tile(Pipe& p, const StepView& v, const R
   for (int g = 0; g < ng; ++g, p.advance()) {
     if (!mbar_wait(p.empty + p.s, p.parity ^ 1u, p.bad, v.derr)) continue;
     if (*(volatile int*)p.bad) continue;
-    const unsigned dst = smem_u32(p.ring + (size_t)p.s * p.stage_bytes);
+    const unsigned dst = smem_u32(p.ring + (size_t)p.s * RAD_STAGE);
     const size_t e = (size_t)T.e0 + (size_t)g * RAD_GROUP;
     mbar_expect(p.full + p.s, bytes);
     bulk_copy(dst, v.t_cf + e, RAD_CF_BYTES, p.full + p.s, pol);
     copy_vals(vals, dst + RAD_CF_BYTES, e, p.full + p.s, pol);
+  }
+}
+// Double-floats take two stages per group, the low parts in the second.
+__device__ __forceinline__ void produce_tile(Pipe& p, const StepView& v, const RowTile& T, ValsDF vals, uint64_t pol) {
+  const int ng = T.lam >> 2;
+  for (int q = 0; q < 2 * ng; ++q, p.advance()) {
+    if (!mbar_wait(p.empty + p.s, p.parity ^ 1u, p.bad, v.derr)) continue;
+    if (*(volatile int*)p.bad) continue;
+    const unsigned dst = smem_u32(p.ring + (size_t)p.s * RAD_STAGE);
+    const size_t e = (size_t)T.e0 + (size_t)(q >> 1) * RAD_GROUP;
+    if (q & 1) {
+      mbar_expect(p.full + p.s, RAD_F32_BYTES);
+      bulk_copy(dst, vals.lo + e, RAD_F32_BYTES, p.full + p.s, pol);
+    } else {
+      mbar_expect(p.full + p.s, RAD_CF_BYTES + RAD_F32_BYTES);
+      bulk_copy(dst, v.t_cf + e, RAD_CF_BYTES, p.full + p.s, pol);
+      bulk_copy(dst + RAD_CF_BYTES, vals.hi + e, RAD_F32_BYTES, p.full + p.s, pol);
+    }
   }
 }
 
@@ -335,7 +342,7 @@ __device__ __forceinline__ void produce_tile(Pipe& p, const StepView& v, const R
 // values), then the stage is released (one arrival per warp).
 template <class V, class W>
 __device__ __forceinline__ void take_group(Pipe& p, const StepView& v, V vals, uint2& c, W (&w)[4]) {
-  const unsigned char* st = p.ring + p.s * p.stage_bytes;
+  const unsigned char* st = p.ring + p.s * RAD_STAGE;
   if (mbar_try(p.full + p.s, p.parity) || mbar_wait(p.full + p.s, p.parity, p.bad, v.derr)) {
     c = *reinterpret_cast<const uint2*>(st + 8 * threadIdx.x);
     read_vals(vals, st + RAD_CF_BYTES, threadIdx.x, w);
@@ -346,6 +353,25 @@ __device__ __forceinline__ void take_group(Pipe& p, const StepView& v, V vals, u
   __syncwarp();
   if ((threadIdx.x & 31) == 0) mbar_arrive(p.empty + p.s);
   p.advance();
+}
+
+__device__ __forceinline__ void take_group(Pipe& p, const StepView& v, ValsDF vals, uint2& c, float2 (&w)[4]) {
+  float h[4], l[4];
+  take_group(p, v, ValsHiF{vals.hi}, c, h);
+  const float* st = reinterpret_cast<const float*>(p.ring + p.s * RAD_STAGE);
+  if (mbar_try(p.full + p.s, p.parity) || mbar_wait(p.full + p.s, p.parity, p.bad, v.derr)) {
+    const float4 q = *reinterpret_cast<const float4*>(st + 4 * threadIdx.x);
+    l[0] = q.x;
+    l[1] = q.y;
+    l[2] = q.z;
+    l[3] = q.w;
+  } else {
+    zero_vals(l);
+  }
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(p.empty + p.s);
+  p.advance();
+  for (int j = 0; j < 4; ++j) w[j] = make_float2(h[j], l[j]);
 }
 
 // Barrier of the consumer threads only (the producer warp does not take
@@ -368,6 +394,7 @@ __device__ __forceinline__ float2 split_df(double x) {
 // by TwoSum, l += e. Intrinsics keep the compiler from contracting or
 // reassociating the error-free steps.
 struct AccDF {
+  static constexpr bool CHEAP = false;
   typedef float2 W;
   typedef float2 X;
   typedef float2 Part;
@@ -414,6 +441,7 @@ __device__ __forceinline__ float2 df_neg(float2 a) { return make_float2(-a.x, -a
 
 // Plain fp32 sum (mixed inner sweeps: bf16 values, fp32 iterates).
 struct AccF32 {
+  static constexpr bool CHEAP = true;
   typedef float W;
   typedef float X;
   typedef float Part;
@@ -429,6 +457,7 @@ struct AccF32 {
 // Two fp32 sums over the same entries (the one-pass mixed solve: the
 // iterate's change and the next frame's change of the direct flux).
 struct AccF2 {
+  static constexpr bool CHEAP = true;
   typedef float W;
   typedef float2 X;
   typedef float2 Part;
@@ -497,6 +526,11 @@ __device__ __forceinline__ uint32_t tile_start(const StepView& v, int t) {
   return __ldg(v.t_start + (size_t)t * RAD_THREADS + threadIdx.x);
 }
 
+// Column codes: a pair of entries in 32 bits, the first one's halo index in
+// bits 0-12, the second one's in bits 16-28, and the row-end bits of both
+// beside the first, so that an index takes one operation.
+constexpr unsigned CF_INDEX = 0x1fffu, CF_END0 = 0x8000u, CF_END1 = 0x4000u;
+
 // One tile (s0: tile_start): thread t owns entries [t*lam, (t+1)*lam) of the tile's entry
 // stream (rows in order, each row's entries in column order), stored so that
 // a group of 4 RAD_THREADS entries is contiguous: entry k of thread t at
@@ -522,32 +556,31 @@ __device__ __forceinline__ void tile_rows(const StepView& v, const RowTile& T, u
   Acc acc;
   acc.zero();
   const int ng = T.lam >> 2;
-  // without a branch: a warp has a row end in most groups, but few lanes do
-  // (eight lanes per run, with neighbouring halo values and segmented scans at
-  // the row ends, were 1.6 times slower)
-  auto elem = [&](uint32_t c, W w) {
-    acc.add(w, sx[c & 0x7fffu]);
-    if (c & 0x8000u) {
-      *dst = acc.get();
-      dst = next;
-      ++next;
-      acc.zero();
-    }
+  auto end = [&]() {   // the row's last entry
+    *dst = acc.get();
+    dst = next;
+    ++next;
+    acc.zero();
   };
   for (int g = 0; g < ng; ++g) {
     uint2 c;
     W w[4];
     take_group(p, v, vals, c, w);
-    if (__any_sync(0xffffffffu, ((c.x | c.y) & 0x80008000u) != 0)) {
-      elem(c.x & 0xffffu, w[0]);
-      elem(c.x >> 16, w[1]);
-      elem(c.y & 0xffffu, w[2]);
-      elem(c.y >> 16, w[3]);
+    const typename Acc::X x0 = sx[c.x & CF_INDEX], x1 = sx[c.x >> 16], x2 = sx[c.y & CF_INDEX], x3 = sx[c.y >> 16];
+    if (Acc::CHEAP && ((c.x | c.y) & (CF_END0 | CF_END1)) == 0) {
+      acc.add(w[0], x0);
+      acc.add(w[1], x1);
+      acc.add(w[2], x2);
+      acc.add(w[3], x3);
     } else {
-      acc.add(w[0], sx[c.x & 0x7fffu]);
-      acc.add(w[1], sx[c.x >> 16]);
-      acc.add(w[2], sx[c.y & 0x7fffu]);
-      acc.add(w[3], sx[c.y >> 16]);
+      acc.add(w[0], x0);
+      if (c.x & CF_END0) end();
+      acc.add(w[1], x1);
+      if (c.x & CF_END1) end();
+      acc.add(w[2], x2);
+      if (c.y & CF_END0) end();
+      acc.add(w[3], x3);
+      if (c.y & CF_END1) end();
     }
   }
   const bool any = dst != first, has_head = cont && any;
@@ -1090,7 +1123,7 @@ __device__ __forceinline__ RadSmem rad_smem() {
   m.rs = m.tail + RAD_THREADS;
   m.tnew = reinterpret_cast<unsigned char*>(m.rs + RAD_ROWS);
   m.full = reinterpret_cast<unsigned long long*>(m.tnew + RAD_THREADS);
-  m.empty = m.full + RAD_NST_MAX;
+  m.empty = m.full + RAD_STAGES;
   return m;
 }
 static_assert((RAD_RING + (size_t)(RAD_HALO + RAD_THREADS + RAD_ROWS) * 8 + RAD_THREADS) % 8 == 0,
@@ -1117,9 +1150,9 @@ __device__ __forceinline__ MeshState64::MeshState64(int nmesh) {
 // barrier (inside init_meshes' caller): full counts the producer's one
 // arrival plus the copied bytes, empty one arrival per consumer warp.
 // first: the first of its barriers (pipes that share the ring take turns).
-__device__ __forceinline__ Pipe make_pipe(const RadSmem& m, int nst, int stage_bytes, int* bad, int first = 0) {
+__device__ __forceinline__ Pipe make_pipe(const RadSmem& m, int* bad) {
   if (threadIdx.x == 0) {
-    for (int s = first; s < first + nst; ++s) {
+    for (int s = 0; s < RAD_STAGES; ++s) {
       mbar_init(m.full + s, 1);
       mbar_init(m.empty + s, RAD_THREADS / 32);
     }
@@ -1129,11 +1162,9 @@ __device__ __forceinline__ Pipe make_pipe(const RadSmem& m, int nst, int stage_b
   __syncthreads();
   Pipe p;
   p.ring = m.ring;
-  p.full = m.full + first;
-  p.empty = m.empty + first;
+  p.full = m.full;
+  p.empty = m.empty;
   p.bad = bad;
-  p.nst = nst;
-  p.stage_bytes = stage_bytes;
   p.s = 0;
   p.parity = 0;
   return p;
@@ -1163,7 +1194,7 @@ __global__ void __maxnreg__(RAD_REGS64) k_radiosity64(StepView v, double* x, int
   const int gt = blockIdx.x * RAD_THREADS + threadIdx.x;
   const int nthreads = gridDim.x * RAD_THREADS;
   unsigned gen = 0;
-  Pipe pipe = make_pipe(sm, RAD_NST64, RAD_STAGE64, &bad);
+  Pipe pipe = make_pipe(sm, &bad);
   init_meshes64(v, st);
   if (!producer) init_x(v, x, warm, gt, nthreads, false);
   if (!grid_barrier(v.barrier, gridDim.x, gen, v.derr)) return;
@@ -1348,8 +1379,7 @@ __global__ void __maxnreg__(RAD_REGS64) k_radiosity64_solo(StepView v, double* x
   if (!v.md[0].active) return;
   // the ring holds three groups of a full sweep or five of a change sweep
   // (every group of a sweep is taken before the next sweep's first copy)
-  Pipe pipe = make_pipe(sm, RAD_NST64, RAD_STAGE64, &S.bad);
-  Pipe pipe32 = make_pipe(sm, RAD_NSTM, RAD_STAGEM, &S.bad, RAD_NST64);
+  Pipe pipe = make_pipe(sm, &S.bad);
   if (threadIdx.x == 0) {
     S.mode = 0;
     S.acc = 0.f;
@@ -1381,7 +1411,7 @@ __global__ void __maxnreg__(RAD_REGS64) k_radiosity64_solo(StepView v, double* x
     float d2 = 0.f;
     if (producer) {
       if ((threadIdx.x & 31) == 0) {
-        if (mode & 1) produce_tile(pipe32, v, T, vhi, pol);
+        if (mode & 1) produce_tile(pipe, v, T, vhi, pol);
         else produce_tile(pipe, v, T, vals, pol);
       }
       __syncwarp();
@@ -1402,7 +1432,7 @@ __global__ void __maxnreg__(RAD_REGS64) k_radiosity64_solo(StepView v, double* x
         for (int h = threadIdx.x + SOLO_HALO * RAD_THREADS; h < T.nhalo; h += RAD_THREADS)
           sxf[h] = ld_it(dcur + __ldg(v.t_halo + T.h0 + h));
         cbar();
-        tile_rows<AccF32>(v, T, s0, pipe32, vhi, sxf, reinterpret_cast<float*>(sm.tail), sm.tnew, rsf);
+        tile_rows<AccF32>(v, T, s0, pipe, vhi, sxf, reinterpret_cast<float*>(sm.tail), sm.tnew, rsf);
         auto finish = [&](uint32_t i, float d, float2& so) {
           so = df_add(so, make_float2(d, 0.f));
           cur[i] = so;
@@ -1474,7 +1504,7 @@ __global__ void __maxnreg__(RAD_REGSM) k_radiosity_mixed(StepView v, double* x, 
   float* xb = v.x32 + v.nt;
   float* r32 = v.x32 + 2 * (size_t)v.nt;
   unsigned gen = 0;
-  Pipe pipe = make_pipe(sm, RAD_NSTM, RAD_STAGEM, &bad);
+  Pipe pipe = make_pipe(sm, &bad);
   init_meshes(v, st);
   if (!producer) init_x(v, x, warm, gt, nthreads, true);
   if (!grid_barrier(v.barrier, gridDim.x, gen, v.derr)) return;
@@ -1617,7 +1647,7 @@ __global__ void __maxnreg__(RAD_REGSM) k_radiosity_lagged(StepView v, double* x,
   float2* XD = B.EH;            // by position: (x - x_ref, E(n+1) - E(n))
   float* pred = v.x32 + v.nt;   // by position: P, the predicted change of s
   unsigned gen = 0;
-  Pipe pipe = make_pipe(sm, RAD_NSTM, RAD_STAGEM, &bad);
+  Pipe pipe = make_pipe(sm, &bad);
   init_meshes(v, st);
   for (int m = threadIdx.x; m < v.nmesh; m += blockDim.x) {
     const MeshDesc& M = v.md[m];
@@ -1773,6 +1803,112 @@ __global__ void k_tile_slots(const unsigned long long* __restrict__ key, const u
   efac[off] = (uint32_t)g;
 }
 
+// Order of the entries within each piece of a row (the entries of one row in
+// one thread's run; their sum may be taken in any order): the 32 lanes of a
+// warp read one halo value each per step, from wherever their rows' columns
+// lie, and random columns hit the same bank of shared memory 3.5 times (two
+// words per value: 6.1). Each step's entries are chosen from the next
+// BANK_WINDOW of every lane's piece: lanes propose an entry whose bank is
+// still free (for one-word values: 32 banks; for two-word values, which the
+// hardware serves half a warp at a time: 16 pairs), the lowest lane of those
+// that propose the same one takes it, and the others look again; then the
+// same with banks used once; then the first entry. Random columns come to 2.1
+// and 4.1 accesses (windows of 16 or 32 entries: no fewer than 2.1 and 3.9).
+// One warp per warp of a tile, in place.
+constexpr int BANK_WINDOW = 8;
+constexpr int BANK_ROUNDS = 4;
+
+__global__ void __launch_bounds__(128) k_tile_banks(const RowTile* __restrict__ tiles, int ntiles, uint16_t* cf,
+                                                    uint32_t* esrc) {
+  constexpr int WARPS = RAD_THREADS / 32;
+  __shared__ uint32_t window[4][BANK_WINDOW][32];   // the candidates' CSR entries
+  const int lane = threadIdx.x & 31;
+  const int64_t w = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (w >= (int64_t)ntiles * WARPS) return;
+  uint32_t(&src)[BANK_WINDOW][32] = window[threadIdx.x >> 5];
+  const RowTile T = tiles[w / WARPS];
+  const int64_t base = T.e0 + 4 * (32 * (w % WARPS) + lane);
+  auto at = [&](int k) { return base + (int64_t)(k >> 2) * RAD_GROUP + (k & 3); };
+  unsigned c[BANK_WINDOW];   // the candidates' halo indices
+  unsigned have = 0;         // slots in use
+  bool open = true, ends = false;   // the piece has entries after the window; its last one ends its row
+  int next = 0;
+  unsigned pair = 0;   // the even entry's code
+  for (int k = 0; k < T.lam; ++k) {
+    if (!have) open = true;
+#pragma unroll
+    for (int i = 0; i < BANK_WINDOW; ++i)
+      if (open && !((have >> i) & 1)) {
+        const unsigned v = cf[at(next)];
+        c[i] = v & 0x7fffu;
+        src[i][lane] = esrc[at(next)];
+        have |= 1u << i;
+        ++next;
+        ends = (v & 0x8000u) != 0;
+        open = !ends && next < T.lam;
+      }
+    int q = -1;
+    unsigned loc = 0;
+    // banks (32) and, by half warp, bank pairs (2 x 16) in use: once, twice
+    unsigned b1 = 0, b2 = 0, h1 = 0, h2 = 0;
+    const int half = lane & 16;
+    for (int phase = 0; phase < 2; ++phase) {
+      for (int r = 0; r < BANK_ROUNDS; ++r) {
+        const unsigned bu = phase ? b2 : b1, hu = phase ? h2 : h1;
+        int want = -1;
+        unsigned wc = 0;
+        if (q < 0) {
+#pragma unroll
+          for (int i = 0; i < BANK_WINDOW; ++i)
+            if (want < 0 && ((have >> i) & 1) && !((bu >> (c[i] & 31)) & 1) &&
+                !((hu >> (half + (c[i] & 15))) & 1)) {
+              want = i;
+              wc = c[i];
+            }
+        }
+        const unsigned asking = __ballot_sync(0xffffffffu, want >= 0);
+        if (!asking) break;
+        unsigned same = asking;
+#pragma unroll
+        for (int bit = 0; bit < 4; ++bit) {
+          const bool one = (wc >> bit) & 1;
+          const unsigned m = __ballot_sync(0xffffffffu, one);
+          same &= one ? m : ~m;
+        }
+        // the same pair in this half of the warp, the same bank anywhere
+        const unsigned m4 = __ballot_sync(0xffffffffu, (wc >> 4) & 1);
+        const unsigned bank = same & (((wc >> 4) & 1) ? m4 : ~m4);
+        const unsigned rivals = (same & (half ? 0xffff0000u : 0xffffu)) | bank;
+        const bool win = want >= 0 && (rivals & ((1u << lane) - 1u)) == 0;
+        const unsigned nb = __reduce_or_sync(0xffffffffu, win ? 1u << (wc & 31) : 0u);
+        const unsigned nh = __reduce_or_sync(0xffffffffu, win ? 1u << (half + (wc & 15)) : 0u);
+        b2 |= b1 & nb;
+        b1 |= nb;
+        h2 |= h1 & nh;
+        h1 |= nh;
+        if (win) {
+          q = want;
+          loc = wc;
+        }
+      }
+    }
+    if (q < 0) {
+      q = __ffs(have) - 1;
+#pragma unroll
+      for (int i = 0; i < BANK_WINDOW; ++i)
+        if (i == q) loc = c[i];
+    }
+    have &= ~(1u << q);
+    const bool end = !have && !open && ends;
+    if (k & 1) {
+      *reinterpret_cast<uint32_t*>(cf + at(k - 1)) = pair | loc << 16 | (end ? CF_END1 : 0u);
+    } else {
+      pair = loc | (end ? CF_END0 : 0u);
+    }
+    esrc[at(k)] = src[q][lane];
+  }
+}
+
 // Each thread's first row (with a continuation bit when its run starts
 // inside the row): rowj0 holds each tile row's first entry index within the
 // tile, tile rows in order.
@@ -1914,7 +2050,9 @@ int radiosity_prepare(Context& c) {
   // halo exceeds the shared-memory capacity is split in two, until none
   // does.
   const int Gdev = g_rad_nsm * std::min(g_rad_per_sm64, g_rad_per_smm);
-  const int G = c.tile_blocks > 0 ? std::min(Gdev, c.tile_blocks) : Gdev;
+  const int G = c.tile_blocks > 0
+                    ? (int)std::min<int64_t>(Gdev, std::max<int64_t>(c.tile_blocks, (nnz + RAD_SHARED_TILE - 1) / RAD_SHARED_TILE))
+                    : Gdev;
   std::vector<RowTile> tiles;
   std::vector<size_t> tile_a;   // first active row of each tile
   std::vector<int64_t> tile_ne;  // entries of each tile
@@ -2129,6 +2267,8 @@ int radiosity_prepare(Context& c) {
     ILG_CUDA(cudaMemsetAsync(dfac.p, 0, (size_t)ns * 4, s));
     k_tile_slots<<<div_up(nnz, 256), 256, 0, s>>>(key2.p, idx2.p, flag.p, before.p, nnz, rb, dkey.p, dsv.p,
                                                   c.rowptr.p, drowoff.p, c.tiles.p, c.t_cf.p, dsrc.p, dfac.p);
+    ILG_CUDA(cudaGetLastError());
+    k_tile_banks<<<div_up((int64_t)ntile * (RAD_THREADS / 32), 4), 128, 0, s>>>(c.tiles.p, ntile, c.t_cf.p, dsrc.p);
     ILG_CUDA(cudaGetLastError());
     k_tile_starts<<<div_up((int64_t)ntile * RAD_THREADS, 256), 256, 0, s>>>(c.tiles.p, ntile, dne.p, drowj0.p,
                                                                             c.t_start.p);

@@ -68,3 +68,37 @@ def test_zero_and_tiny_tolerances_run_full_sweeps(ilg, tol):
         return
     r = np.linalg.norm(x - E - _apply(rp, col, val, x))
     assert r <= 2.0 ** -44 * np.linalg.norm(x - E) + 2.0 ** -50 * np.linalg.norm(x)
+
+
+@pytest.mark.parametrize("nnz", [1, 31, 3967, 3968, 3969, 63488, 63489, 63999, 64000, 64001, 128001])
+@pytest.mark.parametrize("blocks", [0, 1, 2])
+def test_tiles_of_any_entry_count(ilg, nnz, blocks):
+    """Row pieces of every length (entries are stored in a bank order within
+    a piece) and tiles around a group and around the largest shared tile, in
+    both precisions' sweeps."""
+    from illum_gb300 import meshgen
+    v, f = meshgen.icosphere_craters(3, 3, sigma_m=0.0, n_craters=0)
+    n = f.shape[0]
+    g = np.random.default_rng(nnz)
+    lens = np.zeros(n, np.int64)
+    left, i = nnz, 0
+    while left > 0:   # short and long rows in turn
+        k = i % n
+        add = min(left, int(g.integers(1, 10)) if i % 3 else int(g.integers(1, 400)), n - 1 - int(lens[k]))
+        lens[k] += add
+        left -= add
+        i += 1
+    rp = np.concatenate([[0], np.cumsum(lens)])
+    col = np.concatenate([np.sort(g.choice(n, int(m), replace=False)) for m in lens]).astype(np.int32)
+    val = g.uniform(0.1, 1.0, nnz) * 0.5 / max(1, lens.max())
+    ctx = ilg.IllumContext(v, f)
+    ctx.set_radiosity_blocks(blocks)
+    ctx.set_F(rp, col, val)
+    t = ctx.F_tiles()
+    assert (t["entries_per_thread"] * 992 >= 1).all() and t["rows"].sum() == (lens > 0).sum()
+    if blocks:
+        assert t["entries_per_thread"].max() <= max(4 * 17, -(-nnz // (992 * blocks)) + 8)
+    E = g.uniform(0.0, 600.0, n)
+    x, res, sweeps = ctx.radiosity_solve(E, tol=1e-9)
+    r = np.linalg.norm(x - E - _apply(rp, col, val, x))
+    assert res <= 1e-9 and r <= res + 2.0 ** -44 * np.linalg.norm(x - E) + 2.0 ** -50 * np.linalg.norm(x)
