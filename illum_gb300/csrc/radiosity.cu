@@ -1720,23 +1720,26 @@ __global__ void __maxnreg__(RAD_REGSM) k_radiosity_lagged(StepView v, double* x,
 }
 
 // Per-row fp32 scale = max |F_ij| of the row (the bf16 copy stores F/scale).
+// One warp per row, here and in k_row_keys: with one thread per row 22 M
+// entries in 130,050 rows took 134 and 463 us.
 __global__ void k_row_scale(const int64_t* __restrict__ rowptr, const double* __restrict__ val, int nt,
                             float* rscale) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (i >= nt) return;
   double m = 0.0;
-  for (int64_t k = rowptr[i]; k < rowptr[i + 1]; ++k) m = fmax(m, fabs(val[k]));
-  rscale[i] = m > 0.0 ? (float)m : 1.f;
+  for (int64_t k = rowptr[i] + lane; k < rowptr[i + 1]; k += 32) m = fmax(m, fabs(val[k]));
+  for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (lane == 0) rscale[i] = m > 0.0 ? (float)m : 1.f;
 }
 
 // key = row << rb | Morton position of the column; value = CSR entry.
 __global__ void k_row_keys(const int64_t* __restrict__ rowptr, const int32_t* __restrict__ col,
                            const uint32_t* __restrict__ rank, int nt, int rb, unsigned long long* key,
                            uint32_t* src) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (i >= nt) return;
-  unsigned long long hi = (unsigned long long)i << rb;
-  for (int64_t k = rowptr[i]; k < rowptr[i + 1]; ++k) {
+  const unsigned long long hi = (unsigned long long)i << rb;
+  for (int64_t k = rowptr[i] + lane; k < rowptr[i + 1]; k += 32) {
     key[k] = hi | rank[col[k]];
     src[k] = (uint32_t)k;
   }
@@ -1812,11 +1815,13 @@ __global__ void k_tile_slots(const unsigned long long* __restrict__ key, const u
 // still free (for one-word values: 32 banks; for two-word values, which the
 // hardware serves half a warp at a time: 16 pairs), the lowest lane of those
 // that propose the same one takes it, and the others look again; then the
-// same with banks used once; then the first entry. Random columns come to 2.1
-// and 4.1 accesses (windows of 16 or 32 entries: no fewer than 2.1 and 3.9).
+// same with banks used once; then the first entry. Random columns come to 2.2
+// and 4.2 accesses (a window of 32 entries and eight rounds: 2.1 and 3.9). The
+// one-pass mixed solve of 36.7 M entries takes 95 us instead of 103; the FP64
+// sweeps are bound by the stream from L2 and take what they took.
 // One warp per warp of a tile, in place.
-constexpr int BANK_WINDOW = 8;
-constexpr int BANK_ROUNDS = 4;
+constexpr int BANK_WINDOW = 4;
+constexpr int BANK_ROUNDS = 2;
 
 __global__ void __launch_bounds__(128) k_tile_banks(const RowTile* __restrict__ tiles, int ntiles, uint16_t* cf,
                                                     uint32_t* esrc) {
@@ -1992,7 +1997,7 @@ int radiosity_prepare(Context& c) {
   const int nt = c.nt;
   const int64_t nnz = c.nnz;
   ILG_TRY(c.row_scale.alloc(nt));
-  k_row_scale<<<div_up(nt, 256), 256, 0, s>>>(c.rowptr.p, c.val.p, nt, c.row_scale.p);
+  k_row_scale<<<div_up((int64_t)nt * 32, 256), 256, 0, s>>>(c.rowptr.p, c.val.p, nt, c.row_scale.p);
   ILG_CUDA(cudaGetLastError());
   ILG_TRY(c.rperm.alloc(nt));
   ILG_CUDA(cudaMemcpyAsync(c.rperm.p, c.morton_order.p, (size_t)nt * 4, cudaMemcpyDeviceToDevice, s));
@@ -2013,7 +2018,7 @@ int radiosity_prepare(Context& c) {
   if (nnz > 0) {
     ILG_TRY(dkey.alloc(nnz));
     ILG_TRY(dsv.alloc(nnz));
-    k_row_keys<<<div_up(nt, 256), 256, 0, s>>>(c.rowptr.p, c.col.p, c.leaf_rank.p, nt, rb, dkey.p, dsv.p);
+    k_row_keys<<<div_up((int64_t)nt * 32, 256), 256, 0, s>>>(c.rowptr.p, c.col.p, c.leaf_rank.p, nt, rb, dkey.p, dsv.p);
     ILG_CUDA(cudaGetLastError());
     ILG_TRY(radix_sort_u64(dkey.p, dsv.p, nnz, 2 * rb, c.sort, s));
   }
