@@ -383,6 +383,14 @@ __device__ __forceinline__ float down_layer(float gb, float ib, float rho, float
 // gb = gamma / beta: off the chain of the increments, rho / beta is
 __device__ __forceinline__ dfloat down_layer(dfloat gb, dfloat ib, dfloat rho, dfloat d) { return df_fma(gb, d, rho * ib); }
 
+// A layer coefficient, through the read-only path: it may move ahead of the
+// column's stores (without that the downward pass took 61 us instead of 45).
+__device__ __forceinline__ float ld_coef(const float* p) { return __ldg(p); }
+__device__ __forceinline__ dfloat ld_coef(const dfloat* p) {
+  const float2 q = __ldg(reinterpret_cast<const float2*>(p));
+  return dfloat(q.x, q.y);
+}
+
 // One thread per facet column. Block b covers facets [cb.y, cb.y + BS) of
 // mesh cb.x. Q: the new time level's flux per facet. SR: the FP32 layers'
 // updates rounded without bias (sr_add).
@@ -467,7 +475,7 @@ k_conduct(StepView v, const double* __restrict__ Qnp1, int upd) {
     R rh;
     if constexpr (INC) {
       R dm = Tim1 - Ti;
-      rh = up_layer(c[0], c[2], c[3], dm, dn, rho_next);
+      rh = up_layer(ld_coef(c), ld_coef(c + 2), ld_coef(c + 3), dm, dn, rho_next);
       dn = dm;
     } else {
       rh = c[0] * Tim1 + c[1] * Ti + c[2] * Tip1 - c[3] * rho_next;
@@ -492,27 +500,30 @@ k_conduct(StepView v, const double* __restrict__ Qnp1, int upd) {
   if constexpr (INC) {
     R dprev = dtop;
     T[0] = top;
-#pragma unroll 8
-    for (int i = 1; i < nz; ++i) {   // the increments, into the rho slots
+    // Eight layers of T(n) in flight while the chain runs through them: with
+    // the increments stored first and added afterwards the loads' latency came
+    // on top of the chain's (81,920 double-float columns of 60 layers 49.2 ->
+    // 45 us, 435,200 of 55 on average 213 -> 181 us; four or sixteen at a time
+    // 49 and 46 us).
+    constexpr int CH = 8;
+    auto layer = [&](int i, R t) {   // T(n+1) = T(n) + dT
       const R* c = tab + (size_t)i * TAB_W;
-      R d = down_layer(c[1], c[4], RHO(i), dprev);
-      RHO(i) = d;
+      const R d = down_layer(ld_coef(c + 1), ld_coef(c + 4), RHO(i), dprev);
       dprev = d;
-    }
-    for (int i0 = 1; i0 < nz; i0 += 16) {   // T(n+1) = T(n) + dT, sixteen layers in flight
-      R t[16];
+      if constexpr (SR && std::is_same<R, float>::value)
+        T[(size_t)i * N] = sr_add(t, d, sr_key(fl, i, M.frame));
+      else
+        T[(size_t)i * N] = t + d;
+    };
+    R t[CH];
+    int i0 = 1;
+    for (; i0 + CH <= nz; i0 += CH) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j)
-        if (i0 + j < nz) t[j] = ld_layer(T + (size_t)(i0 + j) * N);
+      for (int j = 0; j < CH; ++j) t[j] = ld_layer(T + (size_t)(i0 + j) * N);
 #pragma unroll
-      for (int j = 0; j < 16; ++j)
-        if (i0 + j < nz) {
-          if constexpr (SR && std::is_same<R, float>::value)
-            T[(size_t)(i0 + j) * N] = sr_add(t[j], RHO(i0 + j), sr_key(fl, i0 + j, M.frame));
-          else
-            T[(size_t)(i0 + j) * N] = t[j] + RHO(i0 + j);
-        }
+      for (int j = 0; j < CH; ++j) layer(i0 + j, t[j]);
     }
+    for (; i0 < nz; ++i0) layer(i0, ld_layer(T + (size_t)i0 * N));
   } else {
     R prev = top;
     T[0] = prev;
