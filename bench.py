@@ -483,7 +483,7 @@ def nested_batch(ig, meshgen, K, W):
             "phases_ms_per_step": mx["phases"], "fp64_phases_ms_per_step": d["phases"],
             "max_err_K_vs_fp64": err, "err_after_steps": W + K + P, "setup_s": t_setup, "roofline_radiosity": roof,
             "autotune": mx["autotune"], "fp64_autotune": d["autotune"],
-            "clocks": mx["clocks"], "fp64_clocks": d["clocks"], "gpu_launches": 5 * K}
+            "clocks": mx["clocks"], "fp64_clocks": d["clocks"], "gpu_launches": 4 * K}
 
 
 # ----------------------------------------------------------------- C3 terrain
@@ -695,7 +695,7 @@ def nested_terrain(ig, meshgen, n, cutoff_m, K, W, sample_frac=0.0025):
             "setup_s": {"mesh_s": t_mesh, "bvh_s": t_bvh, "horizons_s": t_hor, "form_factors_s": t_ff},
             "horizon_rays_per_s": N * c["nphi"] * 11 / t_hor, "visibility_rays_per_s": rays / t_ff,
             "cutoff_sizing": sizing, "base_build": base, "cutoff_fallback": fallback,
-            "clocks": m["clocks"], "fp64_clocks": d["clocks"], "gpu_launches": 5 * K}
+            "clocks": m["clocks"], "fp64_clocks": d["clocks"], "gpu_launches": 4 * K}
 
 
 # ----------------------------------------------------------------- C4 serving
@@ -901,7 +901,11 @@ def main():
     peak, peak_kind = _peaks()
     bytes_cond = N * (2 * nz * 8 + 6 * 8)
     nnz = W["setup"]["nnz"]
-    bytes_rad = sweeps_per_step * (nnz * (8 + 4) + N * (4 + 8 + 8 + 8))
+    # a full sweep (the first, and one about six sweeps in) reads F as 64-bit
+    # values, a change sweep as 32-bit ones
+    full = min(2.0, sweeps_per_step)
+    bytes_rad = (full * (nnz * (8 + 4) + N * (4 + 8 + 8 + 8)) +
+                 (sweeps_per_step - full) * (nnz * (4 + 4) + N * (4 + 4 + 8 + 8)))
     kern = {"conduction": (bytes_cond, ph["conduction"], "k_conduct_dfloat_c1"),
             "radiosity": (bytes_rad, ph["radiosity"], "k_radiosity64_c1")}
     dom = max(kern, key=lambda k: kern[k][1])
@@ -971,7 +975,7 @@ def main():
                           "conduction layer recurrences in double-float (FP32 pairs, ~2^-46 relative)",
             "config": {"workload": WORKLOAD_C1, "facets": N, "nnz": nnz, "l2": "256 MB flush before every timed step",
                        "parallelism": f"replicas x{world}"},
-            "e2e": e2e, "gpu_launches": 5 * args.steps, "roofline": roofline, "cpu_baseline": cpu,
+            "e2e": e2e, "gpu_launches": 4 * args.steps, "roofline": roofline, "cpu_baseline": cpu,
             "clocks": clk, "parity_vs_oracle": parity,
             "phases_ms_per_step": ph, "radiosity_sweeps_per_step": sweeps_per_step, "autotune": tune,
             "ambiguous_facets_per_step": amb_per_step,

@@ -2,8 +2,8 @@
 //
 // A batch concatenates its member contexts into one scene: facet arrays,
 // horizons, layer blocks ([nz][N] per mesh), conduction tables, sun tables
-// and the radiosity SELL slices (columns and rows shifted by the mesh's
-// first facet), plus a mesh table (MeshDesc) that every step kernel reads.
+// and the radiosity row tiles (halos and rows shifted by the mesh's first
+// facet), plus a mesh table (MeshDesc) that every step kernel reads.
 // One step is then one launch per phase for all active meshes. Each mesh
 // keeps its own dt, layer count, thermal profile, sun table, coupling and
 // radiosity tolerance; meshes switch off after their last sun position.

@@ -155,7 +155,7 @@ struct StepView {
   const int* blk_tile;
   int sched_grid;              // the radiosity grid the schedule was made for
   int l2_stream;               // 1: the stored matrix is much larger than L2 (stream it evict-first)
-  const uint16_t* t_cf;        // per stored entry: halo index | row end << 15
+  const uint16_t* t_cf;        // per stored entry: halo index; pairs with row ends (radiosity.cu CF_*)
   const float* t_vhi;          // double-float values: hi = fl(F)
   const float* t_vlo;          //   and lo = fl(F - hi)
   const __nv_bfloat16* t_vbf;  // value / row scale

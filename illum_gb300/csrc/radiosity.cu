@@ -10,7 +10,7 @@
 // Morton-consecutive rows with about nnz / (co-resident blocks) entries each.
 // A tile's rows see a compact set of facets (its halo), so a block first
 // gathers the halo's x values into shared memory and then streams the tile's
-// entries, each a 16-bit halo index (plus a row-end bit) and a value. The
+// entries, each a 16-bit halo index (with the pair's row-end bits) and a value. The
 // stream reaches shared memory by bulk copies (cp.async.bulk with mbarrier
 // completion) that one producer warp issues ahead of the 31 consumer warps,
 // so DRAM keeps working while the consumers gather the next tile's halo or
@@ -111,10 +111,12 @@ constexpr int64_t RAD_GROUP = 4 * RAD_THREADS;  // stored entries per group (4 p
 // 60 in 6, 70 in 4, 77 in 3 and 96 in 2; of 20,480 facets (728,586) 83 us in
 // 94 tiles, 90 in 38, 106 in 21; in mixed precision 34 / 42 and 37 / 39 us.
 constexpr int64_t RAD_MIN_TILE = RAD_GROUP;
-// One group in shared memory: its columns (u16), then its values (f32 hi,
-// f32 lo for the FP64 sweeps; f32 hi for the mixed residual; bf16 for the
-// mixed inner sweeps). Every piece is a multiple of 16 bytes, and a group
-// starts at a multiple of RAD_GROUP entries, so each is one bulk copy.
+// One group in shared memory: its columns (u16), then its values (f32 hi, or
+// bf16 for the mixed inner sweeps); the f32 lo of double-floats take a stage
+// of their own. Every piece is a multiple of 16 bytes, and a group starts at a
+// multiple of RAD_GROUP entries, so each is one bulk copy. (Three stages wide
+// enough for double-floats left the change sweeps, six of seven, with three
+// groups in flight: 605 us instead of 589 for 16 meshes.)
 constexpr int RAD_CF_BYTES = (int)RAD_GROUP * 2;
 constexpr int RAD_F32_BYTES = (int)RAD_GROUP * 4;
 constexpr int RAD_STAGE = RAD_CF_BYTES + RAD_F32_BYTES;
@@ -1278,10 +1280,12 @@ __global__ void __maxnreg__(RAD_REGS64) k_radiosity64(StepView v, double* x, int
 // all of them, instead of an atomic counter to wait for and a total to load
 // after it.
 // tile_d2 and the totals are those of k_radiosity64, so the decisions are.
-// 81,920 facets, 8.1 M entries: a change sweep takes 11.6 us (7 us of it the
-// entries, bound by integer and LDS issue: the copies alone run at 10.9 TB/s
-// from L2; 2.4 us the spread between blocks), 16.8 us a full one; in
-// k_radiosity64 they took 12.5 and 18.3 us.
+// 81,920 facets, 8.1 M entries: a change sweep takes 11.6 us, 7 us of it the
+// entries, which come from L2 at 8.5 TB/s (a full sweep's at 9.7, the copies
+// alone at 10.9: taking half the shared-memory accesses out, or the row-end
+// selections, changed nothing), 1.9 us the barrier even for the last block
+// and 1 us the spread between blocks; 16.8 us a full one. In k_radiosity64
+// they took 12.5 and 18.3 us.
 struct __align__(16) SweepWord {
   unsigned long long units, tag;   // residual units; level << 32 | sweep number (from 1)
 };

@@ -188,8 +188,9 @@ int ilg_set_radiosity_blocks(ilg_ctx* ctx, int blocks);
  * src/cpp/illum_cli.cpp:425-433; its default gs_steps is 1,
  * illum_cli.cpp:607-610). Each row sums in the reference's order, so x
  * equals the CPU restatement's bit for bit. *res (may be NULL) receives
- * ||(I - F) x - E||_2. Rows run level by level (rows whose lower columns
- * are all final); the levels are found on the first call after F changes. */
+ * ||(I - F) x - E||_2. Rows are taken in dependency-level order (rows whose lower
+ * columns are all final first), each waiting for the columns it needs; the
+ * order is found on the first call after F changes. */
 int ilg_radiosity_solve_gs(ilg_ctx* ctx, const double* E, int gs_steps, double* x, double* res);
 /* Number of dependency levels of the fixed-sweep solve (0 before its first
  * use on the current form factors). */
