@@ -407,42 +407,42 @@ static StepPlan solo_plan(Context& c, const ilg_run_opts& o) {
   return p;
 }
 
-// A result array is usually fresh memory without pages, and the copy into it
-// then stops at every page: 4 MB arrive in 740 us and 264 MB in 10.5 ms,
-// against 50 us and 1.5 ms where the pages exist (GB300 / Grace, 64 KB pages).
-// MADV_POPULATE_WRITE maps a whole range in one call, contents kept: with it
-// the same arrays take 177 us and 3.9 ms in all. One thread is as fast as
-// several up to 4 MB and four are the fastest from 16 MB (266 us against 485
-// alone, 726 with eight; 264 MB: 2.4, 8.3 and 3.9 ms), hence the line at 8 MB.
-// Only a hint: where the kernel does not know it (or the memory is not
-// ordinary memory), the copy maps the pages as before.
+// A large result array is fresh memory without pages (the C library maps
+// blocks above 32 MB anew each time; smaller ones usually come from memory it
+// has used before), and the copy into it stops at every page: 264 MB arrive in
+// 10.5 ms, 1.5 ms where the pages exist (GB300 / Grace, 64 KB pages).
+// MADV_POPULATE_WRITE maps a whole range in one call, contents kept: 3.9 ms in
+// all with four threads, 9.9 with one, 5.5 with eight. The form factors of a
+// 256 x 256 terrain 48.3 -> 43.6 ms; for the 4 MB arrays of a terrain's outputs
+// the calls cost more than they saved (four steps 3.41 -> 3.62 ms), hence the
+// line at 32 MB. Only a hint: where the kernel does not know it (or the memory
+// is not ordinary memory), the copy maps the pages as before.
 #ifndef MADV_POPULATE_WRITE
 #define MADV_POPULATE_WRITE 23
 #endif
-constexpr size_t FAULT_MIN = 128 << 10, FAULT_SPLIT = 8 << 20;
+constexpr size_t FAULT_MIN = 32 << 20, FAULT_PARTS = 4;
 
 void fault_in(std::initializer_list<HostRange> ranges) {
-  const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
-  size_t pages = 0;
+  size_t large = 0;
   for (const HostRange& r : ranges)
-    if (r.p) pages += r.bytes / page + 1;
-  if (pages * page < FAULT_MIN) return;
-  const size_t parts = pages * page < FAULT_SPLIT ? 1 : 4;
-  auto part = [&ranges, page, parts](size_t k) {   // the k-th part of every range
+    if (r.p && r.bytes >= FAULT_MIN) ++large;
+  if (!large) return;
+  const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+  auto part = [&ranges, page](size_t k) {   // the k-th part of every large range
     for (const HostRange& r : ranges) {
-      if (!r.p || !r.bytes) continue;
+      if (!r.p || r.bytes < FAULT_MIN) continue;
       const uintptr_t a = (uintptr_t)r.p / page, n = ((uintptr_t)r.p + r.bytes - 1) / page + 1 - a;
-      const uintptr_t x = a + n * k / parts, y = a + n * (k + 1) / parts;
+      const uintptr_t x = a + n * k / FAULT_PARTS, y = a + n * (k + 1) / FAULT_PARTS;
       if (x < y) (void)madvise((void*)(x * page), (y - x) * page, MADV_POPULATE_WRITE);
     }
   };
-  std::thread helper[3];
+  std::thread helper[FAULT_PARTS - 1];
   size_t k = 1;
   try {
-    for (; k < parts; ++k) helper[k - 1] = std::thread(part, k);
+    for (; k < FAULT_PARTS; ++k) helper[k - 1] = std::thread(part, k);
   } catch (...) {   // no thread to be had: its parts here
   }
-  for (size_t q = k; q < parts; ++q) part(q);
+  for (size_t q = k; q < FAULT_PARTS; ++q) part(q);
   part(0);
   for (std::thread& t : helper)
     if (t.joinable()) t.join();
@@ -868,7 +868,6 @@ int ilg_direct_radiosity(ilg_ctx* ctx, const double* sun, const double* disk_xy,
   M.host_sun = 1;
   ILG_TRY(upload_desc(c, M));
   ILG_TRY(direct_launch(solo_view(c, ILG_PREC_FP64), 1, 0, 0, c.stream));
-  fault_in({{out, (size_t)c.nt * 8}});
   ILG_CUDA(cudaMemcpyAsync(out, c.E.p, (size_t)c.nt * 8, cudaMemcpyDeviceToHost, c.stream));
   ILG_CUDA(cudaStreamSynchronize(c.stream));
   return read_device_errors(c);
@@ -899,7 +898,6 @@ int ilg_radiosity_solve(ilg_ctx* ctx, const double* E, double tol, int max_sweep
   StepView v = solo_view(c, ILG_PREC_FP64);
   ILG_TRY(radiosity_launch(v, c.Q.p, 0, ILG_PREC_FP64, radiosity_grid(c.ntiles, ILG_PREC_FP64), 1, false, c.stream));
   MeshDesc out;
-  fault_in({{x, (size_t)c.nt * 8}});
   ILG_CUDA(cudaMemcpyAsync(x, c.Q.p, (size_t)c.nt * 8, cudaMemcpyDeviceToHost, c.stream));
   ILG_CUDA(cudaMemcpyAsync(&out, c.md.p, sizeof(out), cudaMemcpyDeviceToHost, c.stream));
   ILG_CUDA(cudaStreamSynchronize(c.stream));
@@ -956,7 +954,6 @@ int ilg_radiosity_solve_gs(ilg_ctx* ctx, const double* E, int gs_steps, double* 
     r2.resize(c.nt);
     ILG_CUDA(cudaMemcpyAsync(r2.data(), c.gs_x.p, (size_t)c.nt * 8, cudaMemcpyDeviceToHost, c.stream));
   }
-  fault_in({{x, (size_t)c.nt * 8}});
   ILG_CUDA(cudaMemcpyAsync(x, c.Q.p, (size_t)c.nt * 8, cudaMemcpyDeviceToHost, c.stream));
   ILG_TRY(read_device_errors(c));   // also waits for the copies
   if (res) {

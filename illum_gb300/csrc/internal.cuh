@@ -404,8 +404,8 @@ int advance_launch(const StepView& v, cudaStream_t s);
 int flush_launch(float4* buf, size_t n, unsigned salt, cudaStream_t s);
 
 // ---- capi.cu ----
-// Makes the pages of caller arrays that a copy from the device will fill
-// resident first (see the definition).
+// Makes the pages of large caller arrays that a copy from the device will
+// fill resident first (see the definition).
 struct HostRange { void* p; size_t bytes; };
 void fault_in(std::initializer_list<HostRange> ranges);
 

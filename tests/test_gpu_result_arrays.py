@@ -12,9 +12,10 @@ from illum_gb300 import meshgen
 pytestmark = pytest.mark.gpu
 
 
-# bytes of the horizon map: below the smallest range that is populated, one
-# page or a few, on both sides of the split into parts, and well beyond it
-@pytest.mark.parametrize("level,nphi,shift", [(1, 3, 8), (3, 13, 24), (5, 51, 8), (5, 52, 65528), (5, 200, 4096)])
+# horizon maps of a few bytes up to 32 MB, the smallest range whose pages are
+# made resident in parts, on both sides of that line, and beyond it
+@pytest.mark.parametrize("level,nphi,shift", [(1, 3, 8), (3, 13, 24), (5, 51, 8), (5, 52, 65528), (5, 204, 4096),
+                                              (5, 205, 4096), (5, 301, 65528)])
 def test_horizons_into_a_fresh_unaligned_array(level, nphi, shift):
     ctx = ig.IllumContext(*meshgen.icosphere_craters(level, 3, sigma_m=0.0, n_craters=0))
     n = ctx.num_faces * nphi
