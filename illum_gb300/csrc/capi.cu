@@ -303,6 +303,7 @@ MeshDesc solo_desc(const Context& c, const ilg_run_opts* o, int first_sun) {
   M.rec_frame0 = c.rec_frame0;
   M.tol2 = o ? o->tol * o->tol : 0.0;
   M.res_unit = radiosity_res_unit(M.tol2);
+  M.rad_err = c.rad_err;
   M.max_sweeps = o ? o->max_sweeps : 1;
   M.refine_every = o ? o->refine_every : 0;
   M.ref_age = c.ref_age;

@@ -101,6 +101,7 @@ struct MeshDesc {
   int tile0, ntiles;           // radiosity row tiles (0: no radiosity)
   double tol2;                 // squared residual tolerance
   float res_unit;              // FP64 solve: residual units (2^20 / tol2) per unit of squared change
+  float rad_err;               // FP64 solve: a change sweep's errors per |d| (radiosity.cu)
   int max_sweeps;
   int refine_every;            // mixed solve: 0 = refinement rounds to tol each step; K >= 1 = one
                                // pass per step, with fl(F) every K-th step (k_radiosity_lagged)
@@ -239,6 +240,7 @@ struct Context {
   dbuf<double> tile_d2;
   dbuf<int> sched_start, sched_tile;   // per-block tile schedule (radiosity_schedule)
   int sched_grid = 0;
+  float rad_err = 0.f;                 // bound on a change sweep's errors (MeshDesc::rad_err)
   int tile_blocks = 0;                 // row tiles cut for this many blocks (0: every co-resident block)
   dbuf<uint8_t> row_act;
   dbuf<uint32_t> rperm;           // Morton position -> facet (radiosity's internal order)

@@ -62,6 +62,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cstring>
 #include <limits>
 #include <mutex>
 #include <thread>
@@ -742,31 +743,38 @@ __device__ __forceinline__ void record_residuals(const StepView& v, const MeshSt
 // iterates are Jacobi's either way. A full sweep evaluates F x in
 // double-float (10 B per entry, ~20 FP32 operations, 8 B halos); a change
 // sweep evaluates F d in FP32 with the high parts of the values (6 B, one
-// FMA, 4 B halos) and adds it to the double-float s, with a rounding error
-// of about 2^-24 |F| |d|, relative to the change and not to x. So the solve
-// begins with a full sweep, continues with change sweeps while those errors
-// are small against the change, and returns to a full sweep, which
-// recomputes s from x and so removes them:
-//   after a full sweep: |d| <= tol stops, else a change sweep follows;
-//   after a change sweep, with A = the sum of |d| over the change sweeps
-//   since the last full one (the errors' scale, bounded by 2^-23 A): |d| <=
-//   15/16 tol with 2^-23 A <= tol / 16 stops (the residual is then <= tol);
-//   |d| <= 2^-20 A, or |d| <= 15/16 tol without the second condition, is
-//   followed by a full sweep; anything else by another change sweep.
+// FMA, 4 B halos) and adds it to the double-float s. What FP32 loses stays in
+// s: at most c |d| per sweep, c = n 2^-24 || |F| ||_2 with n the longest chain
+// of additions to a row's sum (radiosity_prepare bounds both), so at most
+// c A in all, A = the sum of |d| over the change sweeps since the last full
+// one. So the solve begins with a full sweep, continues with change sweeps,
+// and stops when the residual is known to be small enough; a full sweep,
+// which recomputes s from x and so removes the errors, comes in between where
+// they would be too large for that:
+//   a solve stops after a full sweep with |d| <= tol, or after a change sweep
+//   with |d| + c A <= tol (which it reports as its residual);
+//   a full sweep follows when the errors may have reached the change, |d| <=
+//   4 c A; when c A > tol but a full sweep now would leave a sixteenth of tol
+//   at the rate of the last two sweeps; when |d| is small enough or expected
+//   to be after the next sweep (|d|^2 <= tol |d before|, at first |d| <= 8
+//   tol) and c A > tol / 2; and when |d| <= tol did not stop the solve;
+//   another change sweep follows otherwise.
+// The bound holds for any matrix, also one whose rounding errors all have the
+// same sign in every sweep. (Taken as 2^-23 A, whatever the row lengths: rows
+// of 8,000 equal entries were left with residuals above tol.)
 // The last sweep of a budget is a full one, so that a solve which reaches tol
-// within its budget by full sweeps alone still does. |d| comes from the integer residual totals, so the choice is the same in
-// every block, on every run, and alone or in a batch. A tolerance of zero
-// (or one whose units overflow) runs full sweeps only.
+// within its budget by full sweeps alone still does. |d| comes from the
+// integer residual totals, so the choice is the same in every block, on every
+// run, and alone or in a batch. A tolerance of zero (or one whose units
+// overflow) runs full sweeps only.
 struct MeshState64 {
   int* sweeps;
-  float* acc;             // A in units of tol
-  unsigned char* done;    // as MeshState::done
-  unsigned char* mode;    // bit 0: the next sweep is a change sweep; bit 1: s is in S1
+  float* acc;             // A in units of tol, with the last |d|
+  float* prev;            // the last |d| in units of tol
+  unsigned char* mode;    // bit 0: the next sweep is a change sweep; bit 1: s is in S1; from bit 2: as MeshState::done
   __device__ __forceinline__ explicit MeshState64(int nmesh);
 };
-constexpr float CHG_STOP = 15.f / 16.f, CHG_NOISE_STOP = 1.f / 16.f;   // units of tol
-constexpr float CHG_NOISE = 1.1920929e-7f;                             // 2^-23
-constexpr float CHG_REFRESH = 9.5367432e-7f;                           // 2^-20
+constexpr int MODE_DONE = 2;   // shift of the done bits
 constexpr float CHG_RANGE = 5.6294995e14f;   // 2^49: above it the totals are at their cap
 
 // A partial in residual units, and the level they are counted at.
@@ -798,34 +806,33 @@ __device__ __forceinline__ void post_partial64(const StepView& v, const RowTile&
   for (int l = 0; l < RES_LEVELS; ++l) res_acc(v, k + 1, l)[T.mesh] = 0ull;
 }
 
-// What follows a sweep (see above): dn and the flags from the totals.
+// What follows a sweep (see above), from its totals, the errors' factor c and
+// A and |d| before it (zero before the first).
 struct Sweep64 {
   bool stop, next_change;
-  float dn;   // |d| / tol
+  float dn, acc, err;   // |d|, A, and the errors in the result, in units of tol
 };
 __device__ __forceinline__ Sweep64 sweep_decision(unsigned long long q0, unsigned long long q1, unsigned long long q2,
-                                                  bool change, float acc) {
+                                                  bool change, float c, float acc, float prev) {
   const float cap = (float)RES_CAP;
   Sweep64 r;
   r.dn = sqrtf((float)q0 + cap * ((float)q1 + cap * (float)q2)) * (1.f / 1024.f);
-  if (change) {
-    const bool small = r.dn <= CHG_STOP;
-    r.stop = small && CHG_NOISE * acc <= CHG_NOISE_STOP;
-    r.next_change = !small && r.dn > CHG_REFRESH * acc && r.dn < CHG_RANGE;
-  } else {
-    r.stop = q1 == 0 && q2 == 0 && q0 <= RES_UNITS;
-    r.next_change = r.dn < CHG_RANGE;
-  }
+  r.err = change ? c * acc : 0.f;
+  r.acc = change ? acc + r.dn : r.dn;
+  r.stop = change ? r.dn + r.err <= 1023.f / 1024.f : q1 == 0 && q2 == 0 && q0 <= RES_UNITS;
+  const float e = c * r.acc;   // the errors after another change sweep
+  const bool last = r.dn <= 1.f || (e > 0.5f && r.dn * r.dn <= (prev > 0.f ? prev : 8.f * r.dn));
+  const bool renew = e > 1.f && 16.f * c * r.dn * prev <= prev - r.dn;
+  r.next_change = !last && !renew && r.dn > 4.f * e && r.dn < CHG_RANGE;
   return r;
 }
 
 __device__ __forceinline__ void init_meshes64(const StepView& v, MeshState64& st) {
   for (int m = threadIdx.x; m < v.nmesh; m += blockDim.x) {
     const MeshDesc& M = v.md[m];
-    st.done[m] = (M.active && M.ntiles > 0) ? 0 : 1;
-    st.mode[m] = 0;
+    st.mode[m] = (M.active && M.ntiles > 0) ? 0 : 1 << MODE_DONE;
     st.sweeps[m] = 0;
-    st.acc[m] = 0.f;
+    st.acc[m] = st.prev[m] = 0.f;
   }
   const int gt = blockIdx.x * blockDim.x + threadIdx.x;
   for (int m = gt; m < RES_LEVELS * v.nmesh; m += gridDim.x * blockDim.x) res_acc(v, 0)[m] = 0ull;
@@ -837,24 +844,22 @@ __device__ __forceinline__ int decide_meshes64(const StepView& v, MeshState64& s
   int running = 0;
   for (int m0 = 0; m0 < v.nmesh; m0 += blockDim.x) {
     const int m = m0 + threadIdx.x;
-    bool run = m < v.nmesh && !st.done[m];
+    bool run = m < v.nmesh && !(st.mode[m] >> MODE_DONE);
     if (run) {
       const unsigned long long q0 = __ldcg(res_acc(v, k, 0) + m), q1 = __ldcg(res_acc(v, k, 1) + m),
                                q2 = __ldcg(res_acc(v, k, 2) + m);
       const bool change = st.mode[m] & 1;
       const int sw = ++st.sweeps[m];
-      const float acc0 = st.acc[m];
-      const Sweep64 dec = sweep_decision(q0, q1, q2, change, acc0);
-      if (!change) st.mode[m] ^= 2;
+      const Sweep64 dec = sweep_decision(q0, q1, q2, change, v.md[m].rad_err, st.acc[m], st.prev[m]);
+      const int in_s1 = change ? st.mode[m] & 2 : (st.mode[m] & 2) ^ 2;
       const int budget = v.md[m].max_sweeps;
-      st.mode[m] = (st.mode[m] & 2) | (dec.next_change && sw + 1 < budget ? 1 : 0);
+      st.mode[m] = in_s1 | (dec.next_change && sw + 1 < budget ? 1 : 0);
+      st.acc[m] = dec.acc;
+      st.prev[m] = dec.dn;
       if (dec.stop || sw >= budget) {
-        st.done[m] = 1 + (k & 1);
+        st.mode[m] |= (1 + (k & 1)) << MODE_DONE;
         run = false;
-        // the errors of a change sweep that was the last (A without the last |d|)
-        st.acc[m] = change ? acc0 : 0.f;
-      } else {
-        st.acc[m] = change ? acc0 + dec.dn : dec.dn;
+        st.acc[m] = dec.err;   // for record_residuals64
       }
       if (blockIdx.x == 0) v.md[m].sweeps = sw;
     }
@@ -864,8 +869,7 @@ __device__ __forceinline__ int decide_meshes64(const StepView& v, MeshState64& s
 }
 
 // Squared residual plus the bound on the change sweeps' errors.
-__device__ __forceinline__ double with_errors(double r2, float acc, double tol2) {
-  const float err = CHG_NOISE * acc;   // units of tol
+__device__ __forceinline__ double with_errors(double r2, float err, double tol2) {
   if (!(err > 0.f)) return r2;
   const double r = sqrt(r2) + (double)err * sqrt(tol2);
   return r * r;
@@ -880,7 +884,7 @@ __device__ __forceinline__ void record_residuals64(const StepView& v, const Mesh
   for (int m = warp; m < v.nmesh; m += RAD_THREADS / 32) {
     const MeshDesc& M = v.md[m];
     if (!M.active || M.ntiles == 0) continue;
-    const double* d2 = v.tile_d2 + (size_t)(st.done[m] - 1) * v.ntiles;
+    const double* d2 = v.tile_d2 + (size_t)((st.mode[m] >> MODE_DONE) - 1) * v.ntiles;
     double t = 0.0;
     for (int j = lane; j < M.ntiles; j += 32) t += ld_it(d2 + M.tile0 + j);
     t = warp_sum(t);
@@ -1146,8 +1150,8 @@ __device__ __forceinline__ MeshState64::MeshState64(int nmesh) {
   extern __shared__ __align__(128) unsigned char rad_dyn[];
   sweeps = reinterpret_cast<int*>(rad_dyn + RAD_SMEM);
   acc = reinterpret_cast<float*>(sweeps + nmesh);
-  done = reinterpret_cast<unsigned char*>(acc + nmesh);
-  mode = done + nmesh;
+  prev = acc + nmesh;
+  mode = reinterpret_cast<unsigned char*>(prev + nmesh);
 }
 
 // The ring's barriers, set up by thread 0 before the launch's first block
@@ -1211,8 +1215,9 @@ __global__ void __maxnreg__(RAD_REGS64) k_radiosity64(StepView v, double* x, int
       if ((threadIdx.x & 31) == 0)
         for (int k = b0; k < b1; ++k) {
           const RowTile T = v.tiles[v.blk_tile[k]];
-          if (st.done[T.mesh]) continue;
-          if (st.mode[T.mesh] & 1) produce_tile(pipe, v, T, vhi, pol);
+          const int mode = st.mode[T.mesh];
+          if (mode >> MODE_DONE) continue;
+          if (mode & 1) produce_tile(pipe, v, T, vhi, pol);
           else produce_tile(pipe, v, T, vals, pol);
         }
       __syncwarp();
@@ -1223,8 +1228,8 @@ __global__ void __maxnreg__(RAD_REGS64) k_radiosity64(StepView v, double* x, int
       for (int k = b0; k < b1; ++k) {
         const int t = v.blk_tile[k];
         const RowTile T = v.tiles[t];
-        if (st.done[T.mesh]) continue;
         const int mode = st.mode[T.mesh];
+        if (mode >> MODE_DONE) continue;
         const float unit = v.md[T.mesh].res_unit;
         float2* cur = (mode & 2) ? B.S1 : B.S0;
         const uint32_t* rows = v.t_row + T.r0;
@@ -1308,7 +1313,7 @@ __device__ __forceinline__ SweepWord word_load(const SweepWord* p) {
 struct SoloShared {
   float red[32];
   int bad, ok, mode, stop;   // mode as MeshState64::mode
-  float acc;
+  float acc, prev, err;
 };
 
 constexpr int SOLO_HALO = 3;   // halo positions kept per thread (81,920 facets: 2,050 per tile on average)
@@ -1319,7 +1324,7 @@ constexpr int SOLO_HALO = 3;   // halo positions kept per thread (81,920 facets:
 // other blocks stored before theirs is visible to the loads after this (a
 // fence after the wait instead: 0.2 us a sweep more).
 __device__ __forceinline__ bool solo_sweep_end(const StepView& v, SoloShared& S, int it, float d2, float unit,
-                                               int budget) {
+                                               float c, int budget) {
   __syncthreads();   // the block's stores of this sweep come before its word
   const unsigned nb = gridDim.x;
   SweepWord* words = sweep_words(v);
@@ -1357,14 +1362,14 @@ __device__ __forceinline__ bool solo_sweep_end(const StepView& v, SoloShared& S,
     }
     if (threadIdx.x == 0) {
       const bool change = S.mode & 1;
-      const float acc0 = S.acc;
-      const Sweep64 dec = sweep_decision(q0, q1, q2, change, acc0);
+      const Sweep64 dec = sweep_decision(q0, q1, q2, change, c, S.acc, S.prev);
       const int cur = change ? S.mode & 2 : (S.mode & 2) ^ 2;
       const int sw = it + 1;
       S.mode = cur | (dec.next_change && sw + 1 < budget ? 1 : 0);
       S.stop = dec.stop || sw >= budget;
-      if (S.stop) S.acc = change ? acc0 : 0.f;
-      else S.acc = change ? acc0 + dec.dn : dec.dn;
+      S.acc = dec.acc;
+      S.prev = dec.dn;
+      S.err = dec.err;
       S.ok = ok;
     }
   }
@@ -1380,15 +1385,15 @@ __global__ void __maxnreg__(RAD_REGS64) k_radiosity64_solo(StepView v, double* x
   const int nthreads = gridDim.x * RAD_THREADS;
   const int t = v.blk_tile[v.blk_start[blockIdx.x]];
   const RowTile T = v.tiles[t];
-  const float unit = v.md[0].res_unit;
+  const float unit = v.md[0].res_unit, c = v.md[0].rad_err;
   const int budget = v.md[0].max_sweeps;
   if (!v.md[0].active) return;
-  // the ring holds three groups of a full sweep or five of a change sweep
+  // the ring holds two and a half groups of a full sweep or five of a change sweep
   // (every group of a sweep is taken before the next sweep's first copy)
   Pipe pipe = make_pipe(sm, &S.bad);
   if (threadIdx.x == 0) {
     S.mode = 0;
-    S.acc = 0.f;
+    S.acc = S.prev = 0.f;
   }
   const RadBufs B(v);
   const ValsDF vals{v.t_vhi, v.t_vlo};
@@ -1472,7 +1477,7 @@ __global__ void __maxnreg__(RAD_REGS64) k_radiosity64_solo(StepView v, double* x
       d2 = block_sum(d2, S.red);
       if (threadIdx.x == 0) v.tile_d2[(size_t)(it & 1) * v.ntiles + t] = (double)d2;
     }
-    if (!solo_sweep_end(v, S, it, d2, unit, budget)) return;
+    if (!solo_sweep_end(v, S, it, d2, unit, c, budget)) return;
     if (S.stop) break;
   }
   if (!producer) {
@@ -1484,7 +1489,7 @@ __global__ void __maxnreg__(RAD_REGS64) k_radiosity64_solo(StepView v, double* x
       r2 = warp_sum(r2);
       if (threadIdx.x == 0) {
         v.md[0].sweeps = it + 1;
-        v.md[0].res2 = with_errors(r2, S.acc, v.md[0].tol2);
+        v.md[0].res2 = with_errors(r2, S.err, v.md[0].tol2);
       }
     }
   }
@@ -1725,17 +1730,52 @@ __global__ void __maxnreg__(RAD_REGSM) k_radiosity_lagged(StepView v, double* x,
   record_residuals(v, st);
 }
 
+// Bounds of the change sweeps' errors (the FP64 solve): || |F| ||_2 is at most
+// the root of the largest row sum times the largest column sum of |F|. The
+// column sums are integers, in units of max |F| / 2^32, so that the result
+// does not depend on the order of the additions.
+struct FNorms {
+  unsigned long long max_abs, row_sum;   // as the bits of doubles, whose order is theirs (a NaN counts as largest)
+  unsigned long long col_sum;            // in units
+};
+__global__ void k_col_sums(const int32_t* __restrict__ col, const double* __restrict__ val, int64_t nnz,
+                           const FNorms* norms, unsigned long long* sums) {
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= nnz) return;
+  const double m = __longlong_as_double((long long)norms->max_abs);
+  if (m > 0.0) atomicAdd(sums + col[k], (unsigned long long)ceil(fabs(val[k]) / m * 4294967296.0));
+}
+__global__ void k_col_max(const unsigned long long* __restrict__ sums, int nt, FNorms* norms) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  unsigned long long m = j < nt ? sums[j] : 0ull;
+  for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0 && m) atomicMax(&norms->col_sum, m);
+}
+
 // Per-row fp32 scale = max |F_ij| of the row (the bf16 copy stores F/scale).
 // One warp per row, here and in k_row_keys: with one thread per row 22 M
 // entries in 130,050 rows took 134 and 463 us.
 __global__ void k_row_scale(const int64_t* __restrict__ rowptr, const double* __restrict__ val, int nt,
-                            float* rscale) {
+                            float* rscale, FNorms* norms) {
   const int i = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (i >= nt) return;
-  double m = 0.0;
-  for (int64_t k = rowptr[i] + lane; k < rowptr[i + 1]; k += 32) m = fmax(m, fabs(val[k]));
-  for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if (lane == 0) rscale[i] = m > 0.0 ? (float)m : 1.f;
+  double m = 0.0, sum = 0.0;
+  for (int64_t k = rowptr[i] + lane; k < rowptr[i + 1]; k += 32) {
+    const double a = fabs(val[k]);
+    m = fmax(m, a);
+    sum += a;
+  }
+  for (int o = 16; o; o >>= 1) {
+    m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  }
+  if (lane == 0) {
+    rscale[i] = m > 0.0 ? (float)m : 1.f;
+    if (sum != 0.0) {
+      atomicMax(&norms->max_abs, (unsigned long long)__double_as_longlong(m));
+      atomicMax(&norms->row_sum, (unsigned long long)__double_as_longlong(fabs(sum)));
+    }
+  }
 }
 
 // key = row << rb | Morton position of the column; value = CSR entry.
@@ -2003,8 +2043,22 @@ int radiosity_prepare(Context& c) {
   const int nt = c.nt;
   const int64_t nnz = c.nnz;
   ILG_TRY(c.row_scale.alloc(nt));
-  k_row_scale<<<div_up((int64_t)nt * 32, 256), 256, 0, s>>>(c.rowptr.p, c.val.p, nt, c.row_scale.p);
+  dbuf<FNorms> norms;
+  dbuf<unsigned long long> col_sums;
+  ILG_TRY(norms.alloc(1));
+  ILG_TRY(col_sums.alloc(nt));
+  ILG_CUDA(cudaMemsetAsync(norms.p, 0, sizeof(FNorms), s));
+  ILG_CUDA(cudaMemsetAsync(col_sums.p, 0, (size_t)nt * 8, s));
+  k_row_scale<<<div_up((int64_t)nt * 32, 256), 256, 0, s>>>(c.rowptr.p, c.val.p, nt, c.row_scale.p, norms.p);
   ILG_CUDA(cudaGetLastError());
+  if (nnz > 0) {
+    k_col_sums<<<div_up(nnz, 256), 256, 0, s>>>(c.col.p, c.val.p, nnz, norms.p, col_sums.p);
+    ILG_CUDA(cudaGetLastError());
+    k_col_max<<<div_up(nt, 256), 256, 0, s>>>(col_sums.p, nt, norms.p);
+    ILG_CUDA(cudaGetLastError());
+  }
+  FNorms norms_h;
+  ILG_CUDA(cudaMemcpyAsync(&norms_h, norms.p, sizeof(FNorms), cudaMemcpyDeviceToHost, s));
   ILG_TRY(c.rperm.alloc(nt));
   ILG_CUDA(cudaMemcpyAsync(c.rperm.p, c.morton_order.p, (size_t)nt * 4, cudaMemcpyDeviceToDevice, s));
 
@@ -2246,6 +2300,20 @@ int radiosity_prepare(Context& c) {
     if (!split) break;
     if (iter > 40) { set_error("row tiles: halos do not fit after %d splits", iter); return ILG_ERR_CUDA; }
   }
+  // errors of a change sweep's row sums: a row's entries in its threads' runs,
+  // then the runs, and the rounding of the values (see FNorms)
+  int64_t chain = 0;
+  for (int t = 0; t < ntile; ++t) {
+    int64_t longest = 0;
+    for (int q = 0; q < tiles[t].nrows; ++q) longest = std::max(longest, rlen(tile_a[t] + q));
+    const int64_t lam = tiles[t].lam;
+    chain = std::max(chain, std::min(longest, lam) + (longest + lam - 1) / lam + 3);
+  }
+  double max_abs, row_sum;
+  std::memcpy(&max_abs, &norms_h.max_abs, 8);
+  std::memcpy(&row_sum, &norms_h.row_sum, 8);
+  const double col_sum = (double)norms_h.col_sum * (max_abs / 4294967296.0);
+  c.rad_err = (float)((double)chain * std::ldexp(1.02, -24) * std::sqrt(row_sum * col_sum));
   if (ntile > 0) {
     c.ntiles = ntile;
     c.tile_elems = stored_total;
