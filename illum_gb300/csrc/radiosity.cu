@@ -1735,15 +1735,16 @@ __global__ void __maxnreg__(RAD_REGSM) k_radiosity_lagged(StepView v, double* x,
 // column sums are integers, in units of max |F| / 2^32, so that the result
 // does not depend on the order of the additions.
 struct FNorms {
-  unsigned long long max_abs, row_sum;   // as the bits of doubles, whose order is theirs (a NaN counts as largest)
-  unsigned long long col_sum;            // in units
+  unsigned max_abs, row_sum;    // rounded up, as the bits of floats, whose order is theirs (a NaN counts as largest)
+  unsigned long long col_sum;   // in units
 };
 __global__ void k_col_sums(const int32_t* __restrict__ col, const double* __restrict__ val, int64_t nnz,
                            const FNorms* norms, unsigned long long* sums) {
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nnz) return;
-  const double m = __longlong_as_double((long long)norms->max_abs);
-  if (m > 0.0) atomicAdd(sums + col[k], (unsigned long long)ceil(fabs(val[k]) / m * 4294967296.0));
+  const float m = __uint_as_float(norms->max_abs);
+  const float units = __fmul_ru(__fdiv_ru(__double2float_ru(fabs(val[k])), m), 4294967296.f);
+  atomicAdd(sums + col[k], __float2ull_ru(units));
 }
 __global__ void k_col_max(const unsigned long long* __restrict__ sums, int nt, FNorms* norms) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1759,21 +1760,22 @@ __global__ void k_row_scale(const int64_t* __restrict__ rowptr, const double* __
                             float* rscale, FNorms* norms) {
   const int i = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (i >= nt) return;
-  double m = 0.0, sum = 0.0;
+  double m = 0.0;
+  float sum = 0.f;
   for (int64_t k = rowptr[i] + lane; k < rowptr[i + 1]; k += 32) {
     const double a = fabs(val[k]);
     m = fmax(m, a);
-    sum += a;
+    sum = __fadd_ru(sum, __double2float_ru(a));
   }
   for (int o = 16; o; o >>= 1) {
     m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    sum = __fadd_ru(sum, __shfl_xor_sync(0xffffffffu, sum, o));
   }
   if (lane == 0) {
     rscale[i] = m > 0.0 ? (float)m : 1.f;
-    if (sum != 0.0) {
-      atomicMax(&norms->max_abs, (unsigned long long)__double_as_longlong(m));
-      atomicMax(&norms->row_sum, (unsigned long long)__double_as_longlong(fabs(sum)));
+    if (sum != 0.f) {
+      atomicMax(&norms->max_abs, __float_as_uint(__double2float_ru(m)));
+      atomicMax(&norms->row_sum, __float_as_uint(fabsf(sum)));
     }
   }
 }
@@ -2309,11 +2311,11 @@ int radiosity_prepare(Context& c) {
     const int64_t lam = tiles[t].lam;
     chain = std::max(chain, std::min(longest, lam) + (longest + lam - 1) / lam + 3);
   }
-  double max_abs, row_sum;
-  std::memcpy(&max_abs, &norms_h.max_abs, 8);
-  std::memcpy(&row_sum, &norms_h.row_sum, 8);
-  const double col_sum = (double)norms_h.col_sum * (max_abs / 4294967296.0);
-  c.rad_err = (float)((double)chain * std::ldexp(1.02, -24) * std::sqrt(row_sum * col_sum));
+  float max_abs, row_sum;
+  std::memcpy(&max_abs, &norms_h.max_abs, 4);
+  std::memcpy(&row_sum, &norms_h.row_sum, 4);
+  const double col_sum = (double)norms_h.col_sum * ((double)max_abs / 4294967296.0);
+  c.rad_err = (float)((double)chain * std::ldexp(1.02, -24) * std::sqrt((double)row_sum * col_sum));
   if (ntile > 0) {
     c.ntiles = ntile;
     c.tile_elems = stored_total;
