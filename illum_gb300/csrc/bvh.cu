@@ -537,20 +537,24 @@ __device__ __forceinline__ int load_path(const float4* __restrict__ nodes, const
   return e;
 }
 
-// The path of a facet that is not a leaf of the tree.
+// The path of rays that walk the tree from its root.
 __device__ __forceinline__ int load_root(int root, PathEntry* path, int lane) {
   if (lane == 0) whole_tree(path[0], root);
   __syncwarp();
   return 1;
 }
 
-// Slab test with the origin folded into a fused multiply-add, lo * inv + oi,
-// oi = -o * inv. Its rounding displaces a plane by at most ~2^-24 |o|, far
-// inside the boxes' padding of 1e-6 of the scene's magnitude, besides the
-// relative errors that the slack covers as in geom.h slab; so it never
-// rejects a box that contains an mt64 hit either. Direction components below
-// 1e-18 of a unit direction count as 1e-18 (a displacement of 1e-18 of the
-// ray's length), which keeps o * inv finite for coordinates up to 1e20.
+// Slab test of a ray that starts near the tree (rays_near), with the origin
+// folded into a fused multiply-add, lo * inv + oi, oi = -o * inv. Its rounding
+// displaces a plane by at most ~2^-24 |o|, far inside the boxes' padding of
+// 1e-6 of the scene's magnitude, besides the relative errors that the slack
+// covers as in geom.h slab; so it never rejects a box that contains an mt64
+// hit either. From further away 2^-24 |o| exceeds the padding (it was 16
+// times the scene's magnitude: hits were lost), so those rays (NEAR false)
+// take the differences, as geom.h slab does, whose errors stay relative.
+// Direction components below 1e-18 of a unit direction count as 1e-18 (a
+// displacement of 1e-18 of the ray's length), which keeps o * inv finite for
+// coordinates up to 1e20.
 struct RayF {
   f3 o, d, inv, oi;
 };
@@ -567,11 +571,15 @@ __device__ __forceinline__ RayF make_rayf(f3 o, f3 d) {
 }
 __device__ __forceinline__ float dotf(f3 a, f3 b) { return __fmaf_rn(a.z, b.z, __fmaf_rn(a.y, b.y, a.x * b.x)); }
 // Whether the ray meets the box within tmax; [tn, tf]: where.
+template <bool NEAR>
 __device__ __forceinline__ bool in_box(const RayF& r, float lx, float ly, float lz, float hx, float hy, float hz,
                                        float tmax, float& tn, float& tf) {
-  const float tx0 = __fmaf_rn(lx, r.inv.x, r.oi.x), tx1 = __fmaf_rn(hx, r.inv.x, r.oi.x);
-  const float ty0 = __fmaf_rn(ly, r.inv.y, r.oi.y), ty1 = __fmaf_rn(hy, r.inv.y, r.oi.y);
-  const float tz0 = __fmaf_rn(lz, r.inv.z, r.oi.z), tz1 = __fmaf_rn(hz, r.inv.z, r.oi.z);
+  auto plane = [](float x, float o, float inv, float oi) {
+    return NEAR ? __fmaf_rn(x, inv, oi) : __fmul_rn(__fsub_rn(x, o), inv);
+  };
+  const float tx0 = plane(lx, r.o.x, r.inv.x, r.oi.x), tx1 = plane(hx, r.o.x, r.inv.x, r.oi.x);
+  const float ty0 = plane(ly, r.o.y, r.inv.y, r.oi.y), ty1 = plane(hy, r.o.y, r.inv.y, r.oi.y);
+  const float tz0 = plane(lz, r.o.z, r.inv.z, r.oi.z), tz1 = plane(hz, r.o.z, r.inv.z, r.oi.z);
   tn = fmaxf(fmaxf(fminf(tx0, tx1), fminf(ty0, ty1)), fmaxf(fminf(tz0, tz1), 0.0f));
   tf = fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)), fminf(fmaxf(tz0, tz1), tmax)) * 1.0000005f;
   return tn <= tf;
@@ -585,9 +593,10 @@ __device__ __forceinline__ bool in_slab(const RayF& r, f3 m, float mo, float dmi
   const float a = __fmaf_rn(tn, md, mo), b = __fmaf_rn(tf, md, mo);
   return fminf(a, b) <= dmax && fmaxf(a, b) >= dmin;
 }
+template <bool NEAR>
 __device__ __forceinline__ bool in_entry(const RayF& r, const PathEntry& e, float tmax) {
   float tn, tf;
-  return in_box(r, e.a.x, e.a.y, e.a.z, e.a.w, e.b.x, e.b.y, tmax, tn, tf) &&
+  return in_box<NEAR>(r, e.a.x, e.a.y, e.a.z, e.a.w, e.b.x, e.b.y, tmax, tn, tf) &&
          in_slab(r, f3of(e.c), 0.f, e.b.w, e.c.w, tn, tf);
 }
 
@@ -626,10 +635,11 @@ struct Walk {
   int sp, cur;          // cur: internal node (>= 0), leaf (~k < 0), or LANE_IDLE
   u64 mask;
 };
+template <bool NEAR>
 __device__ __forceinline__ u64 enter_mask(const RayF& r, const PathEntry* path, int ne, float tmax) {
   unsigned lo = 0, hi = 0;
   for (int e = 0; e < ne; ++e)
-    if (in_entry(r, path[e], tmax)) {
+    if (in_entry<NEAR>(r, path[e], tmax)) {
       if (e < 32) lo |= 1u << e;
       else hi |= 1u << (e - 32);
     }
@@ -637,7 +647,7 @@ __device__ __forceinline__ u64 enter_mask(const RayF& r, const PathEntry* path, 
 }
 // The next node: the stack's top, else the nearest path entry (within tmax
 // where that has shrunk since the entries were tested).
-template <bool SHRINKS>
+template <bool SHRINKS, bool NEAR>
 __device__ __forceinline__ void walk_next(Walk& w, const int* stack, const RayF& r, const PathEntry* path, float tmax) {
   if (w.sp) {
     w.cur = stack[--w.sp];
@@ -646,7 +656,7 @@ __device__ __forceinline__ void walk_next(Walk& w, const int* stack, const RayF&
   while (w.mask) {
     const int e = __ffsll((long long)w.mask) - 1;
     w.mask &= w.mask - 1;
-    if (!SHRINKS || in_entry(r, path[e], tmax)) {
+    if (!SHRINKS || in_entry<NEAR>(r, path[e], tmax)) {
       w.cur = __float_as_int(path[e].b.z);
       return;
     }
@@ -654,16 +664,17 @@ __device__ __forceinline__ void walk_next(Walk& w, const int* stack, const RayF&
   w.cur = LANE_IDLE;
 }
 // One internal node: the nearer child that the ray enters is next, the other
-// one is pushed.
-template <bool SHRINKS, bool SLAB>
+// one is pushed. The slabs are for rays that start near the tree (the error
+// bound of in_slab).
+template <bool SHRINKS, bool NEAR>
 __device__ __forceinline__ void walk_visit(Walk& w, int* stack, const float4* __restrict__ nodes, const RayF& r,
                                            const PathEntry* path, float tmax, int* err) {
   const float4* nd = nodes + (int64_t)NODE_W * w.cur;
   const float4 a = __ldg(nd), b = __ldg(nd + 1), c = __ldg(nd + 2), d = __ldg(nd + 5);
   float tl, fl, tr, fr;
-  bool hl = in_box(r, a.x, a.y, a.z, a.w, b.x, b.y, tmax, tl, fl);
-  bool hr = in_box(r, b.z, b.w, c.x, c.y, c.z, c.w, tmax, tr, fr);
-  if (SLAB) {
+  bool hl = in_box<NEAR>(r, a.x, a.y, a.z, a.w, b.x, b.y, tmax, tl, fl);
+  bool hr = in_box<NEAR>(r, b.z, b.w, c.x, c.y, c.z, c.w, tmax, tr, fr);
+  if (NEAR) {
     const float4 ml = __ldg(nd + 3), mr = __ldg(nd + 4);
     hl = hl & in_slab(r, f3of(ml), dotf(f3of(ml), r.o), ml.w, d.x, tl, fl);
     hr = hr & in_slab(r, f3of(mr), dotf(f3of(mr), r.o), mr.w, d.y, tr, fr);
@@ -685,19 +696,19 @@ __device__ __forceinline__ void walk_visit(Walk& w, int* stack, const float4* __
   } else if (hr) {
     w.cur = right;
   } else {
-    walk_next<SHRINKS>(w, stack, r, path, tmax);
+    walk_next<SHRINKS, NEAR>(w, stack, r, path, tmax);
   }
 }
 // Visits by all lanes at internal nodes, until fewer than NODE_LANES are
 // left while others wait at a leaf (or none is).
-template <bool SHRINKS, bool SLAB>
+template <bool SHRINKS, bool NEAR>
 __device__ __forceinline__ void walk_nodes(Walk& w, int* stack, const float4* __restrict__ nodes, const RayF& r,
                                            const PathEntry* path, float tmax, int* err) {
   for (;;) {
     const bool in = w.cur >= 0 && w.cur != LANE_IDLE;
     const unsigned m = __ballot_sync(0xffffffffu, in);
     if (m == 0 || (__popc(m) < NODE_LANES && __any_sync(0xffffffffu, w.cur < 0))) break;
-    if (in) walk_visit<SHRINKS, SLAB>(w, stack, nodes, r, path, tmax, err);
+    if (in) walk_visit<SHRINKS, NEAR>(w, stack, nodes, r, path, tmax, err);
   }
 }
 
@@ -761,9 +772,10 @@ __device__ __forceinline__ bool dir_component(float2 s, float2 g, float2 c, floa
   return __fadd_rn(h, __fadd_rn(l, E)) == h && __fadd_rn(h, __fsub_rn(l, E)) == h;
 }
 
-// SLAB: the facets are leaves of the tree (else the coordinates of the two
-// meshes may differ in magnitude, which the slabs' widening does not cover).
-template <bool SLAB>
+// NEAR: the facets are leaves of the tree and the rays start near it. Else
+// (another mesh's tree, whose coordinates may differ in magnitude, or a large
+// offset) the walk begins at the root.
+template <bool NEAR>
 __global__ void __launch_bounds__(HZ_THREADS, 8)
 k_horizons(const float4* __restrict__ nodes, const float4* __restrict__ tri_s, int root,
            const int* __restrict__ parent, const uint32_t* __restrict__ rank, const double* __restrict__ frame,
@@ -783,7 +795,7 @@ k_horizons(const float4* __restrict__ nodes, const float4* __restrict__ tri_s, i
     const f3 n = f3of(nrm[f0 + q]);
     const f3 o = add(f3of(cen[f0 + q]), scl(n, offset));
     int m, own = -1;
-    if (SLAB) {
+    if (NEAR) {
       own = (int)__ldg(rank + f0 + q);
       m = load_path(nodes, parent, nt, own, o, paths + q * entries, entries, lane);
     } else {
@@ -864,8 +876,8 @@ k_horizons(const float4* __restrict__ nodes, const float4* __restrict__ tri_s, i
       } else {
         fresh = false;
         wk.sp = 0;
-        wk.mask = enter_mask(r, path, facets[q].ne, TMAX);
-        walk_next<false>(wk, stack, r, path, TMAX);
+        wk.mask = enter_mask<NEAR>(r, path, facets[q].ne, TMAX);
+        walk_next<false, NEAR>(wk, stack, r, path, TMAX);
         if (wk.cur == LANE_IDLE) {    // enters nothing: a miss
           node = 2 * node + 1;
           fresh = true;
@@ -878,7 +890,7 @@ k_horizons(const float4* __restrict__ nodes, const float4* __restrict__ tri_s, i
     // enough lanes (or all) that can begin a ray: begin them
     if (fm && (__popc(fm) >= REFILL_LANES || fm == onm)) continue;
     for (;;) {
-      walk_nodes<false, SLAB>(wk, stack, nodes, r, path, TMAX, &derr[DERR_STACK]);
+      walk_nodes<false, NEAR>(wk, stack, nodes, r, path, TMAX, &derr[DERR_STACK]);
       if (wk.cur < 0) {
         const int kl = ~wk.cur;
         if (hit_any(tri_s, kl, o, r.d)) {
@@ -887,7 +899,7 @@ k_horizons(const float4* __restrict__ nodes, const float4* __restrict__ tri_s, i
           fresh = true;
           wk.cur = LANE_IDLE;
         } else {
-          walk_next<false>(wk, stack, r, path, TMAX);
+          walk_next<false, NEAR>(wk, stack, r, path, TMAX);
         }
       }
       if (on && !fresh && wk.cur == LANE_IDLE) {
@@ -1168,8 +1180,10 @@ __device__ __forceinline__ void test_closest(const float4* __restrict__ tri_s, i
   }
 }
 
+// NEAR: the rays start near the tree. Else they walk it from the root.
+template <bool NEAR>
 __global__ void __launch_bounds__(VIS_THREADS, 7)
-k_vis_rays(const float4* __restrict__ nodes, const float4* __restrict__ tri_s, const int* __restrict__ parent,
+k_vis_rays(const float4* __restrict__ nodes, const float4* __restrict__ tri_s, int root, const int* __restrict__ parent,
            const uint32_t* __restrict__ rank, LeafGroups G, const float4* __restrict__ cen,
            const float4* __restrict__ nrm, const int* __restrict__ src, const uint2* __restrict__ units,
            const unsigned* __restrict__ nunits, unsigned part, float offset, int bits, int entries,
@@ -1238,7 +1252,7 @@ k_vis_rays(const float4* __restrict__ nodes, const float4* __restrict__ tri_s, c
     };
     bool more = true;
     const int own = (int)__ldg(rank + j);
-    const int ne = load_path(nodes, parent, G.nt, own, o, path, entries, lane);
+    const int ne = NEAR ? load_path(nodes, parent, G.nt, own, o, path, entries, lane) : load_root(root, path, lane);
     for (int t = lane; t < VIS_SEEN; t += 32) S.seen[t] = -1;
     __syncwarp();
     bool on = false;            // this lane has a ray
@@ -1280,8 +1294,8 @@ k_vis_rays(const float4* __restrict__ nodes, const float4* __restrict__ tri_s, c
         test_closest(tri_s, target, o, r.d, B);
         test_closest(tri_s, own, o, r.d, B);
         wk.sp = 0;
-        wk.mask = enter_mask(r, path, ne, B.tmax);
-        walk_next<true>(wk, stack, r, path, B.tmax);
+        wk.mask = enter_mask<NEAR>(r, path, ne, B.tmax);
+        walk_next<true, NEAR>(wk, stack, r, path, B.tmax);
       }
       qn -= take;
       __syncwarp();
@@ -1289,10 +1303,10 @@ k_vis_rays(const float4* __restrict__ nodes, const float4* __restrict__ tri_s, c
       if (!onm) break;
       const bool refillable = more || qn > 0;
       for (;;) {
-        walk_nodes<true, true>(wk, stack, nodes, r, path, B.tmax, &derr[DERR_STACK]);
+        walk_nodes<true, NEAR>(wk, stack, nodes, r, path, B.tmax, &derr[DERR_STACK]);
         if (wk.cur < 0) {
           if (~wk.cur != target) test_closest(tri_s, ~wk.cur, o, r.d, B);
-          walk_next<true>(wk, stack, r, path, B.tmax);
+          walk_next<true, NEAR>(wk, stack, r, path, B.tmax);
         }
         const int run = __popc(__ballot_sync(0xffffffffu, wk.cur != LANE_IDLE));
         if (run == 0 || (refillable && 32 - run >= REFILL_LANES)) break;
@@ -1401,6 +1415,14 @@ __global__ void k_rowptr(const int32_t* __restrict__ rows, int64_t nnz, int nt, 
 
 // Padding of the boxes (see slabf for what it has to cover).
 static float box_pad(const Context& c) { return 1e-6f * c.scene_mag; }
+// Whether rays from the facets' centroids, `offset` along the normals, start
+// near the context's own tree: within a quarter of the scene's magnitude of
+// it, where the folded plane tests displace a plane by 0.1e-6 of the scene's
+// magnitude (padding 1e-6) and the slabs' heights are good to 1.3e-6 of it
+// (widened by 2e-6); and coordinates small enough for o * inv.
+static bool rays_near(const Context& c, float offset) {
+  return std::fabs(offset) * c.nrm_max <= 0.25f * c.scene_mag && c.scene_mag < 1e19f;
+}
 // Most path entries of a facet: one per level, as many as the mask's bits.
 static int path_entries(const Context& c) { return std::max(1, std::min(c.bvh_longest, PATH_MOST)); }
 
@@ -1419,6 +1441,11 @@ int bvh_build(Context& c, const float* verts_h, int nv, const int32_t* tris_h, c
   for (int t = 0; t < 3 * nt; ++t)
     if (tris_h[t] < 0 || tris_h[t] >= nv) { set_error("triangle %d has vertex index %d out of range", t / 3, tris_h[t]); return ILG_ERR_ARG; }
   c.scene_mag = mag > 0.f ? mag : 1.f;
+  c.nrm_max = 1.f;
+  for (int t = 0; normals_h && t < nt; ++t) {
+    const float* n = normals_h + 3 * (size_t)t;
+    c.nrm_max = std::max(c.nrm_max, std::sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]));
+  }
 
   dbuf<float> dverts, dnormals;
   dbuf<int32_t> dtris;
@@ -1665,12 +1692,13 @@ int horizons_build(Context& c, int nphi, double theta_eps, double offset, const 
   const Context& hb = hmesh ? *hmesh : c;
   const int slots = nphi >= 32 ? 1 : HZ_FACETS;
   const int warps = div_up(c.nt, slots);
-  const int entries = hmesh ? 1 : path_entries(c);
+  const bool near = !hmesh && rays_near(c, (float)offset);
+  const int entries = near ? path_entries(c) : 1;
   const size_t smem = (size_t)(HZ_THREADS / 32) * slots * entries * sizeof(PathEntry);
-  auto kern = hmesh ? k_horizons<false> : k_horizons<true>;
+  auto kern = near ? k_horizons<true> : k_horizons<false>;
   ILG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kern<<<div_up(warps, HZ_THREADS / 32), HZ_THREADS, smem, s>>>(
-      hb.nodes.p, hb.tri_s.p, hb.root, hmesh ? nullptr : c.parent.p, c.leaf_rank.p, c.frame.p, c.cen.p, c.nrm.p, c.nt,
+      hb.nodes.p, hb.tri_s.p, hb.root, c.parent.p, c.leaf_rank.p, c.frame.p, c.cen.p, c.nrm.p, c.nt,
       nphi, dc.p, ds.p, dtree.p, (int)tree.size(), (float)offset, slots, entries, c.H.p, c.derr.p);
   ILG_CUDA(cudaGetLastError());
   c.nphi = nphi;
@@ -1773,9 +1801,11 @@ static int cast_visibility(Context& c, GroupBufs& g, const int* src, int a, int 
   k_vis_units<<<div_up(b - a, 256), 256, 0, s>>>(g.cnt.p, a, b, part, g.units.p, nunits);
   ILG_CUDA(cudaGetLastError());
   const int blocks = (int)std::min<int64_t>((cap + warps - 1) / warps, most);
-  const int entries = path_entries(c);
+  const bool near = rays_near(c, offset);
+  const int entries = near ? path_entries(c) : 1;
   const size_t smem = (size_t)warps * entries * sizeof(PathEntry);
-  k_vis_rays<<<blocks, VIS_THREADS, smem, s>>>(c.nodes.p, c.tri_s.p, c.parent.p, c.leaf_rank.p, g.G, c.cen.p, c.nrm.p,
+  auto kern = near ? k_vis_rays<true> : k_vis_rays<false>;
+  kern<<<blocks, VIS_THREADS, smem, s>>>(c.nodes.p, c.tri_s.p, c.root, c.parent.p, c.leaf_rank.p, g.G, c.cen.p, c.nrm.p,
                                                src, g.units.p, nunits, part, offset, bits, entries, nunits + 1,
                                                ukeys, counters, c.derr.p);
   ILG_CUDA(cudaGetLastError());

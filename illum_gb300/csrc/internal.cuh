@@ -194,6 +194,7 @@ struct Context {
   cudaStream_t stream = nullptr;   // = owned_stream.s
   StepPipe pipe;
   float scene_mag = 1.0f;   // max |coordinate|
+  float nrm_max = 1.0f;     // longest facet normal (1 unless the caller gave longer ones)
   float r_max = 0.0f;       // max facet bounding radius
 
   dbuf<float4> tri_o, cen, nrm;
