@@ -408,33 +408,53 @@ static StepPlan solo_plan(Context& c, const ilg_run_opts& o) {
   return p;
 }
 
-// A large result array is fresh memory without pages (the C library maps
-// blocks above 32 MB anew each time; smaller ones usually come from memory it
-// has used before), and the copy into it stops at every page: 264 MB arrive in
-// 10.5 ms, 1.5 ms where the pages exist (GB300 / Grace, 64 KB pages).
-// MADV_POPULATE_WRITE maps a whole range in one call, contents kept: 3.9 ms in
-// all with four threads, 9.9 with one, 5.5 with eight. The form factors of a
-// 256 x 256 terrain 48.3 -> 43.6 ms; for the 4 MB arrays of a terrain's outputs
-// the calls cost more than they saved (four steps 3.41 -> 3.62 ms), hence the
-// line at 32 MB. Only a hint: where the kernel does not know it (or the memory
-// is not ordinary memory), the copy maps the pages as before.
+// A result array may be fresh memory without pages (always above 32 MB, where
+// the C library maps blocks anew each time; below, when a program's first
+// results make the heap grow), and the copy into it stops at every page: 264
+// MB arrive in 10.5 ms, 1.5 ms where the pages exist (GB300 / Grace, 64 KB
+// pages). MADV_POPULATE_WRITE maps a whole range in one call, contents kept:
+// 3.9 ms in all with four threads, 9.9 with one, 5.5 with eight. The form
+// factors of a 256 x 256 terrain 48.3 -> 43.6 ms. Below 32 MB one call without
+// threads, if the first, middle or last page does not exist: fresh arrays of
+// 0.66 and 4.1 MB 180 -> 60 and 310 -> 175 us (40 and 55 us where the pages
+// exist), the first outputs of a program with a 512 x 512 terrain 4.5 -> 0.35
+// ms (four arrays; later ones 0.15 -> 0.17 ms). Only a hint: where the kernel
+// does not know it (or the memory is not ordinary memory), the copy maps the
+// pages as before.
 #ifndef MADV_POPULATE_WRITE
 #define MADV_POPULATE_WRITE 23
 #endif
-constexpr size_t FAULT_MIN = 32 << 20, FAULT_PARTS = 4;
+constexpr size_t FAULT_MIN = 128 << 10, FAULT_LARGE = 32 << 20, FAULT_PARTS = 4;
 
 void fault_in(std::initializer_list<HostRange> ranges) {
-  size_t large = 0;
-  for (const HostRange& r : ranges)
-    if (r.p && r.bytes >= FAULT_MIN) ++large;
-  if (!large) return;
   const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
-  auto part = [&ranges, page](size_t k) {   // the k-th part of every large range
+  auto pages = [page](const HostRange& r, uintptr_t& first) {   // the range's pages
+    first = (uintptr_t)r.p / page;
+    return ((uintptr_t)r.p + r.bytes - 1) / page + 1 - first;
+  };
+  auto populate = [page](uintptr_t a, uintptr_t b) {
+    if (a < b) (void)madvise((void*)(a * page), (b - a) * page, MADV_POPULATE_WRITE);
+  };
+  size_t large = 0;
+  for (const HostRange& r : ranges) {
+    if (!r.p || r.bytes < FAULT_MIN) continue;
+    if (r.bytes >= FAULT_LARGE) { ++large; continue; }
+    uintptr_t a;
+    const size_t n = pages(r, a);
+    bool there = true;
+    for (const size_t k : {n - 1, n / 2, (size_t)0}) {
+      unsigned char in = 1;
+      if (mincore((void*)((a + k) * page), page, &in) == 0 && !(in & 1)) there = false;
+    }
+    if (!there) populate(a, a + n);
+  }
+  if (!large) return;
+  auto part = [&](size_t k) {   // the k-th part of every large range
     for (const HostRange& r : ranges) {
-      if (!r.p || r.bytes < FAULT_MIN) continue;
-      const uintptr_t a = (uintptr_t)r.p / page, n = ((uintptr_t)r.p + r.bytes - 1) / page + 1 - a;
-      const uintptr_t x = a + n * k / FAULT_PARTS, y = a + n * (k + 1) / FAULT_PARTS;
-      if (x < y) (void)madvise((void*)(x * page), (y - x) * page, MADV_POPULATE_WRITE);
+      if (!r.p || r.bytes < FAULT_LARGE) continue;
+      uintptr_t a;
+      const size_t n = pages(r, a);
+      populate(a + n * k / FAULT_PARTS, a + n * (k + 1) / FAULT_PARTS);
     }
   };
   std::thread helper[FAULT_PARTS - 1];
