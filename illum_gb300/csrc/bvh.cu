@@ -587,11 +587,12 @@ __device__ __forceinline__ bool in_box(const RayF& r, float lx, float ly, float 
 // Whether the ray's stretch [tn, tf] (inside the node's box) meets its slab:
 // the heights at the two ends, mo + t m . d, bound it. Within the box every
 // term is below ~2 sqrt(3) of the scene's magnitude, so the heights' rounding
-// stays below ~1.2e-6 of it; the slabs are widened by 2e-6.
+// stays below ~1.2e-6 of it; the slabs are widened by 2e-6. A direction that
+// is not a number enters every slab, as it does every box.
 __device__ __forceinline__ bool in_slab(const RayF& r, f3 m, float mo, float dmin, float dmax, float tn, float tf) {
   const float md = dotf(m, r.d);
   const float a = __fmaf_rn(tn, md, mo), b = __fmaf_rn(tf, md, mo);
-  return fminf(a, b) <= dmax && fmaxf(a, b) >= dmin;
+  return !(fminf(a, b) > dmax) && !(fmaxf(a, b) < dmin);
 }
 template <bool NEAR>
 __device__ __forceinline__ bool in_entry(const RayF& r, const PathEntry& e, float tmax) {
