@@ -1738,13 +1738,9 @@ struct FNorms {
   unsigned max_abs, row_sum;    // rounded up, as the bits of floats, whose order is theirs (a NaN counts as largest)
   unsigned long long col_sum;   // in units
 };
-__global__ void k_col_sums(const int32_t* __restrict__ col, const double* __restrict__ val, int64_t nnz,
-                           const FNorms* norms, unsigned long long* sums) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nnz) return;
-  const float m = __uint_as_float(norms->max_abs);
-  const float units = __fmul_ru(__fdiv_ru(__double2float_ru(fabs(val[k])), m), 4294967296.f);
-  atomicAdd(sums + col[k], __float2ull_ru(units));
+// An entry's |F| in units.
+__device__ __forceinline__ unsigned long long norm_units(double f, const FNorms* norms) {
+  return __float2ull_ru(__fmul_ru(__fdiv_ru(__double2float_ru(fabs(f)), __uint_as_float(norms->max_abs)), 4294967296.f));
 }
 __global__ void k_col_max(const unsigned long long* __restrict__ sums, int nt, FNorms* norms) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1773,9 +1769,10 @@ __global__ void k_row_scale(const int64_t* __restrict__ rowptr, const double* __
   }
   if (lane == 0) {
     rscale[i] = m > 0.0 ? (float)m : 1.f;
-    if (sum != 0.f) {
-      atomicMax(&norms->max_abs, __float_as_uint(__double2float_ru(m)));
-      atomicMax(&norms->row_sum, __float_as_uint(fabsf(sum)));
+    if (sum != 0.f) {   // (most rows are not the largest so far)
+      const unsigned mb = __float_as_uint(__double2float_ru(m)), sb = __float_as_uint(fabsf(sum));
+      if (mb > *(volatile unsigned*)&norms->max_abs) atomicMax(&norms->max_abs, mb);
+      if (sb > *(volatile unsigned*)&norms->row_sum) atomicMax(&norms->row_sum, sb);
     }
   }
 }
@@ -1837,9 +1834,23 @@ __global__ void k_tile_slots(const unsigned long long* __restrict__ key, const u
                              int64_t n, int rb, const unsigned long long* __restrict__ skey,
                              const uint32_t* __restrict__ ssrc, const int64_t* __restrict__ rowptr,
                              const int* __restrict__ rowoff, const RowTile* __restrict__ tiles, uint16_t* cf,
-                             uint32_t* esrc, uint32_t* efac) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+                             uint32_t* esrc, uint32_t* efac, const double* __restrict__ val,
+                             const uint32_t* __restrict__ order, const FNorms* norms, unsigned long long* col_sums) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const bool in = i < n;
+  {   // the column sums, a run of equal columns at a time (one atomic per entry: 0.65 ms for 22 M)
+    unsigned long long u = in ? norm_units(val[ssrc[idx[i]]], norms) : 0ull;
+    const unsigned heads = __ballot_sync(0xffffffffu, !in || flag[i] || lane == 0);
+    const int start = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long y = __shfl_up_sync(0xffffffffu, u, o);
+      if (lane - o >= start) u += y;
+    }
+    const bool last = lane == 31 || ((heads >> (lane + 1)) & 1);
+    if (in && last) atomicAdd(col_sums + order[key[i] & ((1ull << rb) - 1ull)], u);
+  }
+  if (!in) return;
   const int t = (int)(key[i] >> rb);
   const RowTile T = tiles[t];
   const int64_t run = (int64_t)before[i] + flag[i] - 1;
@@ -2053,14 +2064,6 @@ int radiosity_prepare(Context& c) {
   ILG_CUDA(cudaMemsetAsync(col_sums.p, 0, (size_t)nt * 8, s));
   k_row_scale<<<div_up((int64_t)nt * 32, 256), 256, 0, s>>>(c.rowptr.p, c.val.p, nt, c.row_scale.p, norms.p);
   ILG_CUDA(cudaGetLastError());
-  if (nnz > 0) {
-    k_col_sums<<<div_up(nnz, 256), 256, 0, s>>>(c.col.p, c.val.p, nnz, norms.p, col_sums.p);
-    ILG_CUDA(cudaGetLastError());
-    k_col_max<<<div_up(nt, 256), 256, 0, s>>>(col_sums.p, nt, norms.p);
-    ILG_CUDA(cudaGetLastError());
-  }
-  FNorms norms_h;
-  ILG_CUDA(cudaMemcpyAsync(&norms_h, norms.p, sizeof(FNorms), cudaMemcpyDeviceToHost, s));
   ILG_TRY(c.rperm.alloc(nt));
   ILG_CUDA(cudaMemcpyAsync(c.rperm.p, c.morton_order.p, (size_t)nt * 4, cudaMemcpyDeviceToDevice, s));
 
@@ -2302,20 +2305,6 @@ int radiosity_prepare(Context& c) {
     if (!split) break;
     if (iter > 40) { set_error("row tiles: halos do not fit after %d splits", iter); return ILG_ERR_CUDA; }
   }
-  // errors of a change sweep's row sums: a row's entries in its threads' runs,
-  // then the runs, and the rounding of the values (see FNorms)
-  int64_t chain = 0;
-  for (int t = 0; t < ntile; ++t) {
-    int64_t longest = 0;
-    for (int q = 0; q < tiles[t].nrows; ++q) longest = std::max(longest, rlen(tile_a[t] + q));
-    const int64_t lam = tiles[t].lam;
-    chain = std::max(chain, std::min(longest, lam) + (longest + lam - 1) / lam + 3);
-  }
-  float max_abs, row_sum;
-  std::memcpy(&max_abs, &norms_h.max_abs, 4);
-  std::memcpy(&row_sum, &norms_h.row_sum, 4);
-  const double col_sum = (double)norms_h.col_sum * ((double)max_abs / 4294967296.0);
-  c.rad_err = (float)((double)chain * std::ldexp(1.02, -24) * std::sqrt((double)row_sum * col_sum));
   if (ntile > 0) {
     c.ntiles = ntile;
     c.tile_elems = stored_total;
@@ -2348,7 +2337,10 @@ int radiosity_prepare(Context& c) {
     ILG_CUDA(cudaMemsetAsync(dsrc.p, 0xff, (size_t)ns * 4, s));
     ILG_CUDA(cudaMemsetAsync(dfac.p, 0, (size_t)ns * 4, s));
     k_tile_slots<<<div_up(nnz, 256), 256, 0, s>>>(key2.p, idx2.p, flag.p, before.p, nnz, rb, dkey.p, dsv.p,
-                                                  c.rowptr.p, drowoff.p, c.tiles.p, c.t_cf.p, dsrc.p, dfac.p);
+                                                  c.rowptr.p, drowoff.p, c.tiles.p, c.t_cf.p, dsrc.p, dfac.p,
+                                                  c.val.p, c.morton_order.p, norms.p, col_sums.p);
+    ILG_CUDA(cudaGetLastError());
+    k_col_max<<<div_up(nt, 256), 256, 0, s>>>(col_sums.p, nt, norms.p);
     ILG_CUDA(cudaGetLastError());
     k_tile_banks<<<div_up((int64_t)ntile * (RAD_THREADS / 32), 4), 128, 0, s>>>(c.tiles.p, ntile, c.t_cf.p, dsrc.p);
     ILG_CUDA(cudaGetLastError());
@@ -2361,13 +2353,32 @@ int radiosity_prepare(Context& c) {
     k_tile_scale<<<div_up((int64_t)trow.size(), 256), 256, 0, s>>>(c.t_row.p, c.rperm.p, (int)trow.size(),
                                                                   c.row_scale.p, c.t_scale.p);
     ILG_CUDA(cudaGetLastError());
+    FNorms norms_h;
+    ILG_CUDA(cudaMemcpyAsync(&norms_h, norms.p, sizeof(FNorms), cudaMemcpyDeviceToHost, s));
     ILG_CUDA(cudaStreamSynchronize(s));
+    // errors of a change sweep's row sums: a row's entries in its threads' runs,
+    // then the runs, and the rounding of the values (see FNorms)
+    int64_t chain = 0;
+    for (int t = 0; t < ntile; ++t) {
+      int64_t longest = 0;
+      const int* j0 = rowj0.data() + tiles[t].r0;
+      for (int q = 1; q < tiles[t].nrows; ++q) longest = std::max<int64_t>(longest, j0[q] - j0[q - 1]);
+      longest = std::max(longest, tile_ne[t] - j0[tiles[t].nrows - 1]);
+      const int64_t lam = tiles[t].lam;
+      chain = std::max(chain, std::min(longest, lam) + (longest + lam - 1) / lam + 3);
+    }
+    float max_abs, row_sum;
+    std::memcpy(&max_abs, &norms_h.max_abs, 4);
+    std::memcpy(&row_sum, &norms_h.row_sum, 4);
+    const double col_sum = (double)norms_h.col_sum * ((double)max_abs / 4294967296.0);
+    c.rad_err = (float)((double)chain * std::ldexp(1.02, -24) * std::sqrt((double)row_sum * col_sum));
     c.sched_grid = radiosity_grid(ntile, ILG_PREC_FP64);
     ILG_TRY(radiosity_schedule(tiles, c.sched_grid, c.sched_start, c.sched_tile, s));
   } else {
     c.sched_grid = radiosity_grid(0, ILG_PREC_FP64);
     ILG_TRY(radiosity_schedule({}, c.sched_grid, c.sched_start, c.sched_tile, s));
     c.ntiles = 0;
+    c.rad_err = 0.f;
     c.tile_elems = 0;
     c.tiles_h.clear();
     ILG_TRY(c.tiles.alloc(1));
