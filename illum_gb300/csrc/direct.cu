@@ -401,8 +401,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_direct_beside(StepV
   __shared__ DxFacet fs[DXB_FACETS];
   __shared__ int list[DXB_LIST];
   __shared__ int work[DXB_FACETS + THREADS];   // undecided facets
-  __shared__ int nlist, nwork;
-  if (threadIdx.x == 0) nwork = 0;
+  __shared__ int nlist, nwork, ndone;   // ndone: undecided facets that have been through the exact test
+  if (threadIdx.x == 0) nwork = ndone = 0;
   __syncthreads();
   for (int64_t f0 = (int64_t)blockIdx.x * THREADS; f0 < v.nt; f0 += (int64_t)gridDim.x * THREADS) {
     const int f = (int)min(f0 + threadIdx.x, (int64_t)v.nt);
@@ -414,11 +414,26 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_direct_beside(StepV
       n -= DXB_FACETS;
     }
     __syncthreads();
-    if (threadIdx.x == 0) nwork = n;
+    if (threadIdx.x == 0) {
+      ndone += nwork - n;
+      nwork = n;
+    }
     __syncthreads();
   }
   const int n = nwork;
   if (n > 0) exact_facets<THREADS, DXB_LIST>(v, fs, list, nlist, work, n, 0, mu32_flux, ahead);
+  // the launch's count, as the two launches leave it in counters[0]: blocks add
+  // (1, count) to counters[3], counters[2], the last one takes the sum and
+  // clears it for the next launch
+  if (threadIdx.x == 0) {
+    unsigned long long* sum = reinterpret_cast<unsigned long long*>(v.counters + 2);
+    const unsigned found = (unsigned)(ndone + nwork);
+    const unsigned long long was = atomicAdd(sum, (1ull << 32) + found);
+    if ((unsigned)(was >> 32) == gridDim.x - 1) {
+      v.counters[0] = (int)((unsigned)was + found);
+      *sum = 0ull;
+    }
+  }
 }
 
 }  // namespace

@@ -289,7 +289,7 @@ struct Context {
   int ndisk = 0;
   double disk_rmax = 0.0;
   dbuf<int> work;                 // ambiguous facets
-  dbuf<int> counters;             // [0] work count, [1] step (sun index), [2] frame, [3] sweeps
+  dbuf<int> counters;             // [0] undecided facets; [2], [3] their sum so far and blocks done (k_direct_beside)
   dbuf<int> derr;                 // DERR_COUNT error flags
   dbuf<unsigned> barrier;         // grid barrier state of the radiosity kernel
   dbuf<float> x32;                // mixed-precision radiosity iterates (3 x N)
