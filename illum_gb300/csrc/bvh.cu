@@ -1697,7 +1697,10 @@ int horizons_build(Context& c, int nphi, double theta_eps, double offset, const 
   const int entries = near ? path_entries(c) : 1;
   const size_t smem = (size_t)(HZ_THREADS / 32) * slots * entries * sizeof(PathEntry);
   auto kern = near ? k_horizons<true> : k_horizons<false>;
-  ILG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // the most that any launch asks for: the attribute is the kernel's, and other
+  // contexts launch it at the same time
+  constexpr size_t most = (size_t)(HZ_THREADS / 32) * HZ_FACETS * PATH_MOST * sizeof(PathEntry);
+  ILG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
   kern<<<div_up(warps, HZ_THREADS / 32), HZ_THREADS, smem, s>>>(
       hb.nodes.p, hb.tri_s.p, hb.root, c.parent.p, c.leaf_rank.p, c.frame.p, c.cen.p, c.nrm.p, c.nt,
       nphi, dc.p, ds.p, dtree.p, (int)tree.size(), (float)offset, slots, entries, c.H.p, c.derr.p);
