@@ -389,7 +389,7 @@ def build_c2(ig, meshgen, precision, nmesh=None, nsteps=None):
         ctx.set_insolation(1, 0, CFG["solar"])
         ctx.compute_F(albedo=BATCH["albedo"], fetch=False)
         # tiles for the batch: all members together, not one, fill the GPU
-        ctx.set_radiosity_blocks(ig.radiosity_blocks_for(ctx.F_info()["nnz"]))
+        ctx.set_radiosity_blocks(ig.radiosity_blocks_for(ctx.F_info()["nnz"], 200_000))
         period = q["period_h"] * 3600.0
         dt = period / q["steps_per_rot"]
         n = nsteps or q["steps_per_rot"]
@@ -475,7 +475,7 @@ def nested_batch(ig, meshgen, K, W):
             "dtype": mixed_dtype(),
             "config": {"workload": "64 meshes seeds 2-65, icosphere L3-L6, Poisson craters 0.0025/facet, nz 30-80, "
                                    "ti log-U[50,2000], P U[2,12] h, 360/720 steps per rotation, nphi 32, albedo 0.1, "
-                                   "one batch, one launch per phase, CUDA graph per step, radiosity row tiles of <= 64k "
+                                   "one batch, one launch per phase, CUDA graph per step, radiosity row tiles of ~200k "
                                    "entries per member; FP64 arm radiosity tol 1e-10; mixed arm "
                                    + mixed_solve_label(),
                        "facets": nf, "l2": "256 MB flush before every timed step"},

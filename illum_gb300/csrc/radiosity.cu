@@ -88,17 +88,6 @@ constexpr int RAD_MAX_MESH = 1024;
 constexpr int RAD_MESH_BYTES = 13;       // shared memory per mesh of the view (MeshState)
 constexpr int RAD_INNER = 2;             // most fp32 sweeps per refinement of the mixed solve: the bf16 error
                                          // (~4e-3 of the correction) already dominates rho^(k+1), rho ~ 0.013
-// Largest tile, in entries, of a mesh that is cut for fewer blocks than the
-// device holds, to be solved beside others: a 24th of its entries, between
-// 20,000 and 64,000. Blocks take several meshes' tiles, longest first, and
-// with few of them per block the longest block decides; but a tile costs as
-// much as 26,000 entries besides its own. FP64 / mixed solves of a step, us,
-// with a largest tile of 200,000, 128,000, 64,000 entries and with this rule:
-// 64 meshes (156 M entries) 1962 2067 2191 2149 / 292 301 319 322; 16 meshes
-// (36.7 M) 711 546 592 574 / 98 86 96 90; 7 meshes 381 315 336 328 / 67 56 61
-// 59; 3 meshes 381 276 185 188 / 63 52 39 43; 12 meshes of at most 20,480
-// facets (2.3 M) 214 216 145 99 / 53 53 41 30.
-constexpr int64_t RAD_SHARED_TILES = 24, RAD_SHARED_MIN = 20000, RAD_SHARED_MAX = 64000;
 constexpr int64_t RAD_SPLIT_MIN = 131072;  // entries: tiles above twice the split target are halved
 // Tile balance, in stored entries: a block's sweep time is about
 // c + 1.35e-4 us per stored entry + 8.8e-4 us per row + 1.5e-4 us per halo
@@ -2120,10 +2109,7 @@ int radiosity_prepare(Context& c) {
   // halo exceeds the shared-memory capacity is split in two, until none
   // does.
   const int Gdev = g_rad_nsm * std::min(g_rad_per_sm64, g_rad_per_smm);
-  const int64_t shared = std::min(RAD_SHARED_MAX, std::max(RAD_SHARED_MIN, nnz / RAD_SHARED_TILES));
-  const int G = c.tile_blocks > 0
-                    ? (int)std::min<int64_t>(Gdev, std::max<int64_t>(c.tile_blocks, (nnz + shared - 1) / shared))
-                    : Gdev;
+  const int G = c.tile_blocks > 0 ? std::min(Gdev, c.tile_blocks) : Gdev;
   std::vector<RowTile> tiles;
   std::vector<size_t> tile_a;   // first active row of each tile
   std::vector<int64_t> tile_ne;  // entries of each tile

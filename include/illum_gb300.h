@@ -176,7 +176,9 @@ int ilg_radiosity_solve(ilg_ctx* ctx, const double* E, double tol, int max_sweep
 
 /* Cut the context's radiosity row tiles for `blocks` blocks (0: every block
  * the device holds at once, the default), rebuilding them if form factors
- * exist. Fewer, larger tiles suit a mesh that is solved beside others (a
+ * exist. A tile holds at most 3,072 rows and 8,192 halo facets, and one above
+ * twice max(131,072, entries / (4 blocks)) entries is halved, so there may be
+ * more tiles than blocks. Fewer, larger tiles suit a mesh that is solved beside others (a
  * batch or the serving loop): each tile costs a fixed set-up besides its
  * entries. A context's results depend on its tiling in the last bits only,
  * and are the same alone and in a batch for a given setting. No reference
