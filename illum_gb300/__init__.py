@@ -428,7 +428,8 @@ class IllumContext:
     def autotune(self, opts, first_sun=0):
         """Times every launch shape of the step kernels on this context's
         workload (its state is left as it was) and keeps the fastest;
-        returns the chosen shapes and their measured times."""
+        returns the chosen shapes and their measured times. Which steps use
+        the direct-insolation shapes: include/illum_gb300.h ilg_tune."""
         t = Tune()
         _check(lib().ilg_autotune(self._h, C.byref(opts), int(first_sun), C.byref(t)))
         return t.as_dict()

@@ -1365,6 +1365,7 @@ int ilg_autotune(ilg_ctx* ctx, const ilg_run_opts* opts, int first_sun, ilg_tune
   v.tune.classify_threads = best.classify_threads;
   v.tune.exact_facets = best.exact_facets;
   for (int bs : {32, 64, 128}) {
+    if (bs > conduction_most_threads(o.precision, c.nz)) continue;   // (would run as the one before)
     v.tune.conduct_threads = bs;
     ILG_TRY(time_launches(c, [&] { return conduction_launch(v, v.rad, o.precision, 1, c.nz, s); }, reps, &us));
     if (us < best_c) { best_c = us; best.conduct_threads = bs; }

@@ -783,6 +783,9 @@ int launch_conduct(const StepView& v, const double* Q, int upd, int nz_max, cuda
 // Opt the shared-memory kernels into SMEM_LIMIT bytes (once per process,
 // before any capture).
 int conduction_step_threads() { return COND_STEP_THREADS; }
+int conduction_most_threads(int precision, int nz) {
+  return precision == ILG_PREC_MIXED && nz <= COL_MAX ? COL_THREADS : 128;
+}
 
 int conduction_setup() {
   static std::mutex mu;

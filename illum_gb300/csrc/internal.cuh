@@ -424,6 +424,7 @@ constexpr int REC_W = 15;
 constexpr int REC_PART = 18;
 int record_launch(const StepView& v, int precision, int ncblocks, cudaStream_t s);
 int conduction_step_threads();   // facets per conduction block of a scene step
+int conduction_most_threads(int precision, int nz);   // most that conduct_threads can be for single-mesh steps
 // Q: heat flux at the new time level per facet (global index); upd: also
 // update rad_avg / therm_avg / therm_max; nz_max: deepest mesh of the view.
 int conduction_launch(const StepView& v, const double* Q, int precision, int upd, int nz_max, cudaStream_t s,

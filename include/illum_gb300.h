@@ -304,12 +304,17 @@ int ilg_debug_ff_chunk(long long pairs);
 /* ---- launch-shape autotuner (no reference counterpart) ------------------------ */
 /* Launch shapes of the step kernels. No result depends on them (every
  * facet's work is independent of the block it runs in, and the sums are
- * per facet), only the step's speed. */
+ * per facet), only the step's speed. The direct-insolation shapes are those
+ * of the two-launch form: runs without radiosity or in the fixed-sweep mode,
+ * a run's first frame and phase-timed steps. Other steps with radiosity
+ * compute a later frame's insolation beside the solve, in one kernel whose
+ * shape is fixed by the room the solve leaves. */
 typedef struct ilg_tune {
   int classify_threads;   /* direct-insolation pass 1, threads per block: 128, 256, 512 */
   int exact_facets;       /* direct-insolation pass 2, undecided facets per block: 4, 8, 16, 32 */
-  int conduct_threads;    /* conduction, columns per block (single-mesh steps): 32, 64, 128 */
-  double direct_us;       /* ilg_autotune: measured time of the chosen direct shapes (us per step) */
+  int conduct_threads;    /* conduction, columns per block (single-mesh steps): 32, 64, 128 (mixed
+                             precision up to 80 layers: 32 or 64, 128 counts as 64) */
+  double direct_us;       /* ilg_autotune: measured time of the chosen direct shapes (us per frame) */
   double conduct_us;      /* ilg_autotune: measured time of the chosen conduction shape */
 } ilg_tune;
 /* Times every shape on the context's own workload for opts (sun position
@@ -360,8 +365,8 @@ int ilg_batch_bench_phases(ilg_batch* batch, int nsteps, double flush_mb, double
  * with its first member's; its conduction runs on the batch's own block
  * table): every supported shape timed on the batch's own workload (no state
  * changes), the fastest kept for the batch's later steps; *chosen (may be
- * NULL) receives the shapes and their time per step (direct_us). No result
- * depends on the shapes. */
+ * NULL) receives the shapes and their time per frame (direct_us). No result
+ * depends on the shapes; see ilg_tune for the steps that use them. */
 int ilg_batch_autotune(ilg_batch* batch, ilg_tune* chosen);
 /* per member (arrays of n, any may be NULL): still active, steps done in
  * total (including before this batch), radiosity sweeps of the last step */
