@@ -176,7 +176,7 @@ static int build(Batch& b) {
   }
   const int RT = radiosity_threads();
   int64_t ntl1 = ntl > 0 ? ntl : 1, nel1 = nel > 0 ? nel : 1;
-  ILG_TRY(b.tiles.alloc(ntl1)); ILG_TRY(b.tile_d2.alloc(2 * ntl1)); ILG_TRY(b.t_start.alloc(ntl1 * RT));
+  ILG_TRY(b.tiles.alloc(ntl1 + 1)); ILG_TRY(b.tile_d2.alloc(2 * ntl1)); ILG_TRY(b.t_start.alloc(ntl1 * RT));
   ILG_TRY(b.t_cf.alloc(nel1)); ILG_TRY(b.t_vhi.alloc(nel1)); ILG_TRY(b.t_vlo.alloc(nel1)); ILG_TRY(b.t_vbf.alloc(nel1));
   ILG_TRY(b.t_row.alloc(nrow > 0 ? nrow : 1)); ILG_TRY(b.t_scale.alloc(nrow > 0 ? nrow : 1));
   ILG_TRY(b.t_halo.alloc(nhal > 0 ? nhal : 1));
@@ -205,7 +205,8 @@ static int build(Batch& b) {
   }
   if (!th.empty())
     ILG_CUDA(cudaMemcpyAsync(b.tiles.p, th.data(), th.size() * sizeof(RowTile), cudaMemcpyHostToDevice, s));
-  b.sched_grid = radiosity_grid((int)th.size(), b.precision);
+  ILG_CUDA(cudaMemsetAsync(b.tiles.p + th.size(), 0, sizeof(RowTile), s));   // the empty tile (k_radiosity64_solo)
+  b.sched_grid = radiosity_grid((int)th.size(), b.nt);
   ILG_TRY(radiosity_schedule(th, b.sched_grid, b.sched_start, b.sched_tile, s));
   ILG_CUDA(cudaMemsetAsync(b.row_act.p, 0, nt, s));
   ILG_CUDA(cudaMemsetAsync(b.counters.p, 0, 8 * sizeof(int), s));
@@ -312,7 +313,7 @@ static int build(Batch& b) {
   b.plan.precision = b.precision;
   b.plan.rad_on = b.ntiles > 0;
   b.plan.rec_on = nrec > 0;
-  b.plan.rad_grid = b.plan.rad_on ? radiosity_grid(b.ntiles, b.precision) : 1;
+  b.plan.rad_grid = b.plan.rad_on ? radiosity_grid(b.ntiles, b.nt) : 1;
   int min_sweeps = b.opts[0].max_sweeps;
   for (const ilg_run_opts& o : b.opts) min_sweeps = std::min(min_sweeps, o.max_sweeps);
   b.plan.rad_inner = radiosity_inner(min_sweeps);

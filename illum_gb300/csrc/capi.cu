@@ -395,7 +395,7 @@ static StepPlan solo_plan(Context& c, const ilg_run_opts& o) {
   StepPlan p;
   p.precision = o.precision;
   p.rad_on = o.use_radiosity && c.have_F && c.ntiles > 0;
-  p.rad_grid = p.rad_on ? radiosity_grid(c.ntiles, o.precision) : 1;
+  p.rad_grid = p.rad_on ? radiosity_grid(c.ntiles, c.nt) : 1;
   p.rad_inner = radiosity_inner(o.max_sweeps);
   p.rad_lagged = o.precision == ILG_PREC_MIXED && o.refine_every > 0;
   p.layer_sr = o.precision == ILG_PREC_MIXED && o.layer_rounding == 1;
@@ -917,7 +917,7 @@ int ilg_radiosity_solve(ilg_ctx* ctx, const double* E, double tol, int max_sweep
   ILG_CUDA(cudaMemcpyAsync(c.E.p + e_slot(M.frame) * c.nt, E, (size_t)c.nt * 8, cudaMemcpyHostToDevice,
                            c.stream));
   StepView v = solo_view(c, ILG_PREC_FP64);
-  ILG_TRY(radiosity_launch(v, c.Q.p, 0, ILG_PREC_FP64, radiosity_grid(c.ntiles, ILG_PREC_FP64), 1, false, c.stream));
+  ILG_TRY(radiosity_launch(v, c.Q.p, 0, ILG_PREC_FP64, radiosity_grid(c.ntiles, c.nt), 1, false, c.stream));
   MeshDesc out;
   ILG_CUDA(cudaMemcpyAsync(x, c.Q.p, (size_t)c.nt * 8, cudaMemcpyDeviceToHost, c.stream));
   ILG_CUDA(cudaMemcpyAsync(&out, c.md.p, sizeof(out), cudaMemcpyDeviceToHost, c.stream));

@@ -1263,7 +1263,7 @@ __global__ void __maxnreg__(RAD_REGS64) k_radiosity64(StepView v, double* x, int
   record_residuals64(v, st);
 }
 
-// ---- the FP64 solve of one mesh with one tile per block ----
+// ---- the FP64 solve of one mesh with at most one tile per block ----
 //
 // The same sweeps on the same tiles, bit for bit, for the usual single-mesh
 // solve. A sweep of such a mesh is short (about 1 us of entries per block for
@@ -1372,7 +1372,9 @@ __global__ void __maxnreg__(RAD_REGS64) k_radiosity64_solo(StepView v, double* x
   const bool producer = threadIdx.x >= RAD_THREADS;
   const int gt = blockIdx.x * RAD_THREADS + threadIdx.x;
   const int nthreads = gridDim.x * RAD_THREADS;
-  const int t = v.blk_tile[v.blk_start[blockIdx.x]];
+  // blocks beyond the tiles (which the schedule gives to the first blocks) help
+  // at the ends only: their tile is the empty one after the others
+  const int t = blockIdx.x < v.ntiles ? v.blk_tile[v.blk_start[blockIdx.x]] : v.ntiles;
   const RowTile T = v.tiles[t];
   const float unit = v.md[0].res_unit, c = v.md[0].rad_err;
   const int budget = v.md[0].max_sweeps;
@@ -1394,7 +1396,7 @@ __global__ void __maxnreg__(RAD_REGS64) k_radiosity64_solo(StepView v, double* x
   const bool has_row = !producer && threadIdx.x < T.nrows;
   if (!producer) {
     init_x(v, x, warm, gt, nthreads, false);
-    s0 = tile_start(v, t);
+    s0 = t < v.ntiles ? tile_start(v, t) : 0u;
 #pragma unroll
     for (int q = 0; q < SOLO_HALO; ++q) {
       const int h = threadIdx.x + q * RAD_THREADS;
@@ -1464,7 +1466,7 @@ __global__ void __maxnreg__(RAD_REGS64) k_radiosity64_solo(StepView v, double* x
         }
       }
       d2 = block_sum(d2, S.red);
-      if (threadIdx.x == 0) v.tile_d2[(size_t)(it & 1) * v.ntiles + t] = (double)d2;
+      if (threadIdx.x == 0 && t < v.ntiles) v.tile_d2[(size_t)(it & 1) * v.ntiles + t] = (double)d2;
     }
     if (!solo_sweep_end(v, S, it, d2, unit, c, budget)) return;
     if (S.stop) break;
@@ -2296,7 +2298,8 @@ int radiosity_prepare(Context& c) {
     c.tile_elems = stored_total;
     c.tiles_h = tiles;
     const int64_t ns = stored_total;
-    ILG_TRY(c.tiles.alloc(ntile));
+    ILG_TRY(c.tiles.alloc((size_t)ntile + 1));   // and an empty one (k_radiosity64_solo)
+    ILG_CUDA(cudaMemsetAsync(c.tiles.p + ntile, 0, sizeof(RowTile), s));
     ILG_TRY(c.t_cf.alloc(ns));
     ILG_TRY(c.t_vhi.alloc(ns));
     ILG_TRY(c.t_vlo.alloc(ns));
@@ -2358,10 +2361,10 @@ int radiosity_prepare(Context& c) {
     std::memcpy(&row_sum, &norms_h.row_sum, 4);
     const double col_sum = (double)norms_h.col_sum * ((double)max_abs / 4294967296.0);
     c.rad_err = (float)((double)chain * std::ldexp(1.02, -24) * std::sqrt((double)row_sum * col_sum));
-    c.sched_grid = radiosity_grid(ntile, ILG_PREC_FP64);
+    c.sched_grid = radiosity_grid(ntile, nt);
     ILG_TRY(radiosity_schedule(tiles, c.sched_grid, c.sched_start, c.sched_tile, s));
   } else {
-    c.sched_grid = radiosity_grid(0, ILG_PREC_FP64);
+    c.sched_grid = radiosity_grid(0, nt);
     ILG_TRY(radiosity_schedule({}, c.sched_grid, c.sched_start, c.sched_tile, s));
     c.ntiles = 0;
     c.rad_err = 0.f;
@@ -2399,13 +2402,16 @@ size_t radiosity_barrier_words(int nmesh) { return RAD_BAR_WORDS1 + 2 * 3 * RES_
 // Cooperative grid size for ntiles tiles (at most the co-resident blocks).
 // Both solves launch the same block shape and shared memory, so one grid
 // (and one tile schedule) serves either precision.
-int radiosity_grid(int ntiles, int precision) {
-  (void)precision;
-  if (radiosity_setup() != ILG_OK) return 1;
-  int per_sm = std::min(g_rad_per_smm, g_rad_per_sm64);
-  int grid = per_sm * g_rad_nsm;
-  if (ntiles < grid) grid = ntiles;
-  return grid < 1 ? 1 : grid;
+// A view of few tiles and many facets gets further blocks, without a tile: the
+// passes over all facets before and after the sweeps take RAD_ILP of them per
+// thread and turn. With one block for the one tile of a body with a single
+// small crater (81,920 facets, 134 entries) an FP64 solve took 288 us and a
+// one-pass one 391 us, 41 and 37 us with 21 blocks.
+int radiosity_grid(int ntiles, int64_t nt) {
+  if (radiosity_setup() != ILG_OK || ntiles < 1) return 1;
+  const int64_t facets = (nt + RAD_ILP * RAD_THREADS - 1) / (RAD_ILP * RAD_THREADS);
+  return (int)std::min<int64_t>((int64_t)std::min(g_rad_per_smm, g_rad_per_sm64) * g_rad_nsm,
+                                std::max<int64_t>(ntiles, facets));
 }
 
 // Tile cost in stored entries (RAD_ROW_COST per row, RAD_HALO_COST per halo
@@ -2502,9 +2508,9 @@ int radiosity_launch(const StepView& v, double* x, int warm, int precision, int 
     set_error("radiosity grid %d has no tile schedule (made for %d blocks)", grid, v.sched_grid);
     return ILG_ERR_ARG;
   }
-  // one mesh, one tile per block (the schedule gives every block one when
-  // there are as many tiles as blocks)
-  const bool solo = precision != ILG_PREC_MIXED && v.nmesh == 1 && v.ntiles == grid && grid <= RAD_MAX_GRID;
+  // one mesh, at most one tile per block (so the schedule deals them out when
+  // there are no more tiles than blocks)
+  const bool solo = precision != ILG_PREC_MIXED && v.nmesh == 1 && v.ntiles <= grid && grid <= RAD_MAX_GRID;
   ILG_CUDA(cudaMemsetAsync(v.barrier, 0, (RAD_BAR_WORDS0 + (solo ? 8 * (size_t)grid : 0)) * sizeof(unsigned), s));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
