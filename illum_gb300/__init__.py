@@ -100,6 +100,7 @@ _SIGS = {
     "ilg_radiosity_levels": (C.c_int, [C.c_void_p, C.POINTER(C.c_int)]),
     "ilg_debug_barrier_timeout": (C.c_int, [C.c_void_p, C.c_int, C.c_longlong, C.c_int]),
     "ilg_debug_ff_chunk": (C.c_int, [C.c_longlong]),
+    "ilg_debug_sort": (C.c_int, [C.c_void_p, C.c_void_p, C.c_longlong, C.c_int, C.c_int]),
     "ilg_set_radiosity_mode": (C.c_int, [C.c_void_p, C.c_int, C.c_int]),
     "ilg_thermal_init": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_double, C.c_void_p,
                                    C.c_double, C.c_double, C.c_int, C.c_int]),
@@ -594,6 +595,14 @@ def radiosity_blocks_for(nnz: int, entries_per_tile: int | None = None) -> int:
 def debug_ff_chunk(pairs):
     """Candidate pairs per form-factor build chunk (test entry; 0: default)."""
     _check(lib().ilg_debug_ff_chunk(int(pairs)))
+
+
+def debug_sort(keys, vals=None, bits=64, polls=-1):
+    """Sorted copies of keys (and vals) by the set-up's radix sort (test entry)."""
+    k = np.array(keys, np.uint64)
+    v = None if vals is None else np.array(vals, np.uint32)
+    _check(lib().ilg_debug_sort(_p(k), _p(v), k.shape[0], int(bits), int(polls)))
+    return k if v is None else (k, v)
 
 
 def device_pool_high(reset=False):

@@ -987,6 +987,28 @@ int ilg_radiosity_solve_gs(ilg_ctx* ctx, const double* E, int gs_steps, double* 
 
 int ilg_debug_ff_chunk(long long pairs) { return ff_set_chunk((int64_t)pairs); }
 
+int ilg_debug_sort(unsigned long long* keys, unsigned* vals, long long n, int bits, int polls) {
+  if (!keys || n < 1 || bits < 1 || bits > 64) { set_error("invalid sort arguments"); return ILG_ERR_ARG; }
+  ILG_TRY(alloc_pool_setup());
+  OwnedStream os;
+  ILG_CUDA(cudaStreamCreateWithFlags(&os.s, cudaStreamNonBlocking));
+  AllocOn on_(os.s);
+  dbuf<unsigned long long> k;
+  dbuf<uint32_t> v;
+  SortScratch tmp;
+  ILG_TRY(k.alloc((size_t)n));
+  ILG_CUDA(cudaMemcpyAsync(k.p, keys, (size_t)n * 8, cudaMemcpyHostToDevice, os.s));
+  if (vals) {
+    ILG_TRY(v.alloc((size_t)n));
+    ILG_CUDA(cudaMemcpyAsync(v.p, vals, (size_t)n * 4, cudaMemcpyHostToDevice, os.s));
+  }
+  ILG_TRY(radix_sort_u64(k.p, vals ? v.p : nullptr, n, bits, tmp, os.s, polls));
+  ILG_CUDA(cudaMemcpyAsync(keys, k.p, (size_t)n * 8, cudaMemcpyDeviceToHost, os.s));
+  if (vals) ILG_CUDA(cudaMemcpyAsync(vals, v.p, (size_t)n * 4, cudaMemcpyDeviceToHost, os.s));
+  ILG_CUDA(cudaStreamSynchronize(os.s));
+  return ILG_OK;
+}
+
 int ilg_debug_barrier_timeout(ilg_ctx* ctx, int blocks, long long polls, int unreachable) {
   if (!ctx) { set_error("ctx is NULL"); return ILG_ERR_ARG; }
   Context& c = ctx->c;

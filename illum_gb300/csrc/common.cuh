@@ -154,6 +154,6 @@ struct SortScratch {
   void release() { keys_alt.release(); vals_alt.release(); hist.release(); }
 };
 int radix_sort_u64(unsigned long long* keys, uint32_t* vals, int64_t n, int bits, SortScratch& tmp,
-                   cudaStream_t s);
+                   cudaStream_t s, int polls = -1);   // polls: look-back polls of a tile (< 0: the default)
 
 }  // namespace ilg

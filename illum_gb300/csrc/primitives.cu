@@ -1,7 +1,7 @@
 // primitives.cu — device prefix scan and stable LSD radix sort used by the
 // LBVH build (Morton codes) and the form-factor CSR assembly (row/column
 // keys). Reduce-then-scan with 2048-element tiles; the radix sort ranks keys
-// inside a tile with warp match masks, which keeps it stable.
+// inside a tile by warp votes on their bits, which keeps it stable.
 #include <algorithm>
 #include <utility>
 
@@ -103,7 +103,9 @@ int scan_impl(const T* in, u64* out, int64_t n, ScanScratch& tmp, cudaStream_t s
 // Stable LSD sort, 8 bits or less per pass. One launch counts the digits of
 // all passes; a pass then reads and writes every key once: a tile ranks its
 // keys, publishes its digit counts, adds up those of the tiles before it
-// (their own counts, or a running sum where one has been published: look-back)
+// (their own counts, or a running sum where one has been published: the
+// decoupled look-back of Merrill and Garland 2016, in the arrangement of
+// Adinets and Merrill's one-sweep radix sort, 2022)
 // and writes the tile out in digit order through shared memory, in runs of
 // about TILE / 128 keys. Tiles take their number from a counter, so the tiles
 // that one waits for are running or done. Bound by the ranking and the
@@ -310,7 +312,7 @@ k_radix_pass(const u64* __restrict__ kin, const uint32_t* __restrict__ vin, u64*
 }
 
 template <class R>
-int radix_passes(u64* keys, uint32_t* vals, int64_t n, int bits, SortScratch& tmp, cudaStream_t s) {
+int radix_passes(u64* keys, uint32_t* vals, int64_t n, int bits, SortScratch& tmp, cudaStream_t s, int polls) {
   const int64_t tiles = (n + R::TILE - 1) / R::TILE;
   const int passes = (bits + 7) / 8, width = (bits + passes - 1) / passes;
   // digit counts, tile counters and tile states, all zero at first
@@ -328,7 +330,7 @@ int radix_passes(u64* keys, uint32_t* vals, int64_t n, int bits, SortScratch& tm
   uint32_t *va = vals, *vb = vals ? tmp.vals_alt.p : nullptr;
   for (int p = 0; p < passes; ++p) {
     kern<<<(int)tiles, R::THREADS, R::SMEM, s>>>(ka, va, kb, vb, n, p, width, hist + (size_t)p * RS_BINS, state,
-                                                 taken + p, RS_POLLS);
+                                                 taken + p, polls);
     ILG_CUDA(cudaGetLastError());
     std::swap(ka, kb);
     std::swap(va, vb);
@@ -346,12 +348,13 @@ int scan_exclusive_u32_to_u64(const uint32_t* in, u64* out, int64_t n, ScanScrat
   return scan_impl<uint32_t>(in, out, n, tmp, s, 0);
 }
 
-int radix_sort_u64(u64* keys, uint32_t* vals, int64_t n, int bits, SortScratch& tmp, cudaStream_t s) {
+int radix_sort_u64(u64* keys, uint32_t* vals, int64_t n, int bits, SortScratch& tmp, cudaStream_t s, int polls) {
+  if (polls < 0) polls = RS_POLLS;
   if (n <= 1 || bits <= 0) return ILG_OK;
   ILG_TRY(tmp.keys_alt.reserve((size_t)n));
   if (vals) ILG_TRY(tmp.vals_alt.reserve((size_t)n));
-  return n <= RS_SMALL ? radix_passes<RadixSmall>(keys, vals, n, bits, tmp, s)
-                       : radix_passes<RadixLarge>(keys, vals, n, bits, tmp, s);
+  return n <= RS_SMALL ? radix_passes<RadixSmall>(keys, vals, n, bits, tmp, s, polls)
+                       : radix_passes<RadixLarge>(keys, vals, n, bits, tmp, s, polls);
 }
 
 }  // namespace ilg

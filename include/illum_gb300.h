@@ -300,6 +300,12 @@ int ilg_debug_barrier_timeout(ilg_ctx* ctx, int blocks, long long polls, int unr
  * small mesh through the several-chunk path, whose matrix must equal the
  * one-chunk build's. Not for concurrent use with other builds. */
 int ilg_debug_ff_chunk(long long pairs);
+/* Test entry for the radix sort of the set-up: sorts host arrays in place by
+ * the keys' low `bits` bits (keys must be zero above them), stably; vals (may
+ * be NULL) follow. polls: how often a tile of the sort looks for the digit
+ * counts of the tiles before it until it counts the keys itself (< 0: the
+ * default); the result does not depend on it. */
+int ilg_debug_sort(unsigned long long* keys, unsigned* vals, long long n, int bits, int polls);
 
 /* ---- launch-shape autotuner (no reference counterpart) ------------------------ */
 /* Launch shapes of the step kernels. No result depends on them (every
