@@ -100,6 +100,7 @@ _SIGS = {
     "ilg_radiosity_levels": (C.c_int, [C.c_void_p, C.POINTER(C.c_int)]),
     "ilg_debug_barrier_timeout": (C.c_int, [C.c_void_p, C.c_int, C.c_longlong, C.c_int]),
     "ilg_debug_ff_chunk": (C.c_int, [C.c_longlong]),
+    "ilg_debug_gs_polls": (C.c_int, [C.c_void_p, C.c_longlong]),
     "ilg_debug_sort": (C.c_int, [C.c_void_p, C.c_void_p, C.c_longlong, C.c_int, C.c_int]),
     "ilg_set_radiosity_mode": (C.c_int, [C.c_void_p, C.c_int, C.c_int]),
     "ilg_thermal_init": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_double, C.c_void_p,
@@ -364,6 +365,10 @@ class IllumContext:
         """Status of one grid-barrier wait with a `polls` limit (test entry):
         0 when the barrier opened, ILG_ERR_DEVICE when the wait ran out."""
         return lib().ilg_debug_barrier_timeout(self._h, int(blocks), int(polls), int(bool(unreachable)))
+
+    def debug_gs_polls(self, polls=0):
+        """Most polls of a Gauss-Seidel row wait (test entry; 0: the default)."""
+        _check(lib().ilg_debug_gs_polls(self._h, int(polls)))
 
     def radiosity_levels(self) -> int:
         n = C.c_int()

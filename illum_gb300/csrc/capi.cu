@@ -987,6 +987,14 @@ int ilg_radiosity_solve_gs(ilg_ctx* ctx, const double* E, int gs_steps, double* 
 
 int ilg_debug_ff_chunk(long long pairs) { return ff_set_chunk((int64_t)pairs); }
 
+int ilg_debug_gs_polls(ilg_ctx* ctx, long long polls) {
+  if (!ctx || polls < 0) { set_error("invalid arguments"); return ILG_ERR_ARG; }
+  AllocOn on_(ctx->c.stream);
+  invalidate_graph(ctx->c);   // the limit is a launch argument
+  ctx->c.gs_polls = polls;
+  return ILG_OK;
+}
+
 int ilg_debug_sort(unsigned long long* keys, unsigned* vals, long long n, int bits, int polls) {
   if (!keys || n < 1 || bits < 1 || bits > 64) { set_error("invalid sort arguments"); return ILG_ERR_ARG; }
   ILG_TRY(alloc_pool_setup());

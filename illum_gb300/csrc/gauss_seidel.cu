@@ -132,7 +132,8 @@ __global__ void __launch_bounds__(GS_THREADS) k_gs_sweep(const uint32_t* __restr
                                                          const int32_t* __restrict__ col,
                                                          const double* __restrict__ val, const int* __restrict__ nlow,
                                                          const double* __restrict__ b, GsWord* x,
-                                                         unsigned long long sweep, double* xout, int* derr) {
+                                                         unsigned long long sweep, double* xout, int* derr,
+                                                         long long polls) {
   const int lane = threadIdx.x & 31;
   const int nw = gridDim.x * (GS_THREADS / 32);
   for (int t = blockIdx.x * (GS_THREADS / 32) + (threadIdx.x >> 5); t < n; t += nw) {
@@ -175,10 +176,10 @@ __global__ void __launch_bounds__(GS_THREADS) k_gs_sweep(const uint32_t* __restr
           pos = 32;
         }
         for (; pos < end; ++pos) xi = xi + __shfl_sync(0xffffffffu, p, pos);
-        if (it > 1024 && (it & 1023) == 0) {   // give up together with the others, or alone
+        if ((it & 1023) == 1023 || it > polls) {   // give up together with the others, or alone
           int stop = 0;
           if (lane == 0) {
-            if (it > GS_POLLS) atomicExch(&derr[DERR_BARRIER], 1);
+            if (it > polls) atomicExch(&derr[DERR_BARRIER], 1);
             stop = *(volatile int*)&derr[DERR_BARRIER];
           }
           if (__shfl_sync(0xffffffffu, stop, 0)) return;
@@ -300,7 +301,7 @@ int gs_solve_launch(const Context& c, const double* E, double* x, int gs_steps, 
     double* xo = sw == gs_steps ? x : nullptr;
     ILG_CUDA(cudaLaunchKernelEx(&cfg, k_gs_sweep, (const uint32_t*)c.gs_rows.p, n, (const int64_t*)c.rowptr.p,
                                 (const int32_t*)c.col.p, (const double*)c.val.p, (const int*)c.gs_nlow.p, rhs, out,
-                                number, xo, c.derr.p));
+                                number, xo, c.derr.p, c.gs_polls > 0 ? c.gs_polls : GS_POLLS));
   }
   return ILG_OK;
 }

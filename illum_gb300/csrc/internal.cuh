@@ -254,6 +254,7 @@ struct Context {
   dbuf<int> gs_nlow;              // per row: entries left of the diagonal
   dbuf<double> gs_x;              // 6 x N: two iterates as (value, sweep) words, E + U x, the right-hand side
   int gs_grid = 0;                // co-resident blocks of a sweep
+  long long gs_polls = 0;         // most polls of a wait for a row's column (0: the default; ilg_debug_gs_polls)
 
   // thermal
   bool have_thermal = false;

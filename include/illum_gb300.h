@@ -295,6 +295,10 @@ int ilg_set_timing(ilg_ctx* ctx, int enable);
  * limit is a per-device setting for the duration of the launch: do not run
  * radiosity solves on the same device meanwhile. */
 int ilg_debug_barrier_timeout(ilg_ctx* ctx, int blocks, long long polls, int unreachable);
+/* Test entry: the most polls of a wait for a row's column in the context's
+ * fixed-sweep Gauss-Seidel solves (0 restores the default of 2^21). A solve
+ * whose wait runs out returns ILG_ERR_DEVICE and the context stays usable. */
+int ilg_debug_gs_polls(ilg_ctx* ctx, long long polls);
 /* Test entry for the form-factor build: candidate pairs per source chunk
  * (process-wide; <= 0 restores the default of 2^29). A small value runs a
  * small mesh through the several-chunk path, whose matrix must equal the
