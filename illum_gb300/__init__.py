@@ -99,6 +99,7 @@ _SIGS = {
     "ilg_radiosity_solve_gs": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.POINTER(C.c_double)]),
     "ilg_radiosity_levels": (C.c_int, [C.c_void_p, C.POINTER(C.c_int)]),
     "ilg_debug_barrier_timeout": (C.c_int, [C.c_void_p, C.c_int, C.c_longlong, C.c_int]),
+    "ilg_debug_sweep_timeout": (C.c_int, [C.c_void_p, C.c_int, C.c_longlong, C.c_int]),
     "ilg_debug_ff_chunk": (C.c_int, [C.c_longlong]),
     "ilg_debug_gs_polls": (C.c_int, [C.c_void_p, C.c_longlong]),
     "ilg_debug_sort": (C.c_int, [C.c_void_p, C.c_void_p, C.c_longlong, C.c_int, C.c_int]),
@@ -365,6 +366,11 @@ class IllumContext:
         """Status of one grid-barrier wait with a `polls` limit (test entry):
         0 when the barrier opened, ILG_ERR_DEVICE when the wait ran out."""
         return lib().ilg_debug_barrier_timeout(self._h, int(blocks), int(polls), int(bool(unreachable)))
+
+    def debug_sweep_timeout(self, blocks=4, polls=4096, unreachable=True):
+        """Return code of the wait at the end of a single mesh's FP64 sweep
+        (test entry), as debug_barrier_timeout."""
+        return lib().ilg_debug_sweep_timeout(self._h, int(blocks), int(polls), int(bool(unreachable)))
 
     def debug_gs_polls(self, polls=0):
         """Most polls of a Gauss-Seidel row wait (test entry; 0: the default)."""

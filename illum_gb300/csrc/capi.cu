@@ -1017,15 +1017,23 @@ int ilg_debug_sort(unsigned long long* keys, unsigned* vals, long long n, int bi
   return ILG_OK;
 }
 
-int ilg_debug_barrier_timeout(ilg_ctx* ctx, int blocks, long long polls, int unreachable) {
+static int debug_wait(ilg_ctx* ctx, int blocks, long long polls, int unreachable, bool words) {
   if (!ctx) { set_error("ctx is NULL"); return ILG_ERR_ARG; }
   Context& c = ctx->c;
   AllocOn on_(c.stream);
   ILG_TRY(c.barrier.reserve(radiosity_barrier_words(1)));
   ILG_TRY(c.derr.reserve(DERR_COUNT));
   ILG_CUDA(cudaMemsetAsync(c.derr.p, 0, DERR_COUNT * sizeof(int), c.stream));
-  ILG_TRY(radiosity_barrier_probe(c.barrier.p, c.derr.p, blocks, polls, unreachable, c.stream));
+  ILG_TRY(radiosity_barrier_probe(c.barrier.p, c.derr.p, blocks, polls, unreachable, words, c.stream));
   return read_device_errors(c);   // ILG_ERR_DEVICE once the wait ran out (the flags are cleared)
+}
+
+int ilg_debug_barrier_timeout(ilg_ctx* ctx, int blocks, long long polls, int unreachable) {
+  return debug_wait(ctx, blocks, polls, unreachable, false);
+}
+
+int ilg_debug_sweep_timeout(ilg_ctx* ctx, int blocks, long long polls, int unreachable) {
+  return debug_wait(ctx, blocks, polls, unreachable, true);
 }
 
 int ilg_radiosity_levels(const ilg_ctx* ctx, int* levels) {

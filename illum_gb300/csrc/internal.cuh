@@ -375,7 +375,8 @@ size_t radiosity_barrier_words(int nmesh);
 float radiosity_res_unit(double tol2);
 int radiosity_launch(const StepView& v, double* x, int warm, int precision, int grid, int inner, bool lagged,
                      cudaStream_t s);
-int radiosity_barrier_probe(unsigned* bar, int* derr, int blocks, long long polls, int unreachable, cudaStream_t s);
+int radiosity_barrier_probe(unsigned* bar, int* derr, int blocks, long long polls, int unreachable, bool words,
+                            cudaStream_t s);
 // inner sweeps of a mixed refinement round for a sweep budget (the smallest
 // budget of a view's meshes): the budget, at most radiosity_max_inner()
 int radiosity_inner(int max_sweeps);

@@ -1308,14 +1308,14 @@ struct SoloShared {
 constexpr int SOLO_HALO = 3;   // halo positions kept per thread (81,920 facets: 2,050 per tile on average)
 
 // End of sweep `it` of the block whose partial is d2 (thread 0's): publish,
-// wait for every block's, and decide. All threads; false once a wait ran out.
+// wait for every block's (nb of them: the grid's), and decide. All threads;
+// false once a wait ran out.
 // A word is written after a fence and read by an acquiring load, so what the
 // other blocks stored before theirs is visible to the loads after this (a
 // fence after the wait instead: 0.2 us a sweep more).
 __device__ __forceinline__ bool solo_sweep_end(const StepView& v, SoloShared& S, int it, float d2, float unit,
-                                               float c, int budget) {
+                                               float c, int budget, unsigned nb) {
   __syncthreads();   // the block's stores of this sweep come before its word
-  const unsigned nb = gridDim.x;
   SweepWord* words = sweep_words(v);
   if (threadIdx.x == 0) {
     int level;
@@ -1468,7 +1468,7 @@ __global__ void __maxnreg__(RAD_REGS64) k_radiosity64_solo(StepView v, double* x
       d2 = block_sum(d2, S.red);
       if (threadIdx.x == 0 && t < v.ntiles) v.tile_d2[(size_t)(it & 1) * v.ntiles + t] = (double)d2;
     }
-    if (!solo_sweep_end(v, S, it, d2, unit, c, budget)) return;
+    if (!solo_sweep_end(v, S, it, d2, unit, c, budget, gridDim.x)) return;
     if (S.stop) break;
   }
   if (!producer) {
@@ -2471,16 +2471,26 @@ __global__ void k_barrier_probe(unsigned* bar, unsigned expected, int* derr) {
   unsigned gen = 0;
   grid_barrier(bar, expected, gen, derr);
 }
+// The same for the end of a solo solve's sweep.
+__global__ void k_sweep_word_probe(StepView v, unsigned expected) {
+  __shared__ SoloShared S;
+  if (threadIdx.x == 0) {
+    S.mode = 0;
+    S.acc = S.prev = 0.f;
+  }
+  solo_sweep_end(v, S, 0, 1.f, 1.f, 0.f, 1, expected);
+}
 }  // namespace
 
-// One cooperative launch of `blocks` blocks waiting at a barrier that
-// `unreachable` keeps shut, with the poll limit set to `polls` for the
+// One cooperative launch of `blocks` blocks waiting at a barrier (words: for
+// one another's sweep words) that `unreachable` keeps shut, with the poll limit set to `polls` for the
 // launch (and restored after it). The wait's outcome is in the view's error
 // flags, read by the caller.
-int radiosity_barrier_probe(unsigned* bar, int* derr, int blocks, long long polls, int unreachable, cudaStream_t s) {
+int radiosity_barrier_probe(unsigned* bar, int* derr, int blocks, long long polls, int unreachable, bool words,
+                            cudaStream_t s) {
   if (blocks < 1 || blocks > 8 || polls < 1) { set_error("invalid barrier probe"); return ILG_ERR_ARG; }
   ILG_CUDA(cudaMemcpyToSymbolAsync(g_barrier_polls, &polls, sizeof(polls), 0, cudaMemcpyHostToDevice, s));
-  ILG_CUDA(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), s));
+  ILG_CUDA(cudaMemsetAsync(bar, 0, (RAD_BAR_WORDS0 + 8 * (blocks + 1)) * sizeof(unsigned), s));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(blocks);
   cfg.blockDim = dim3(32);
@@ -2491,7 +2501,11 @@ int radiosity_barrier_probe(unsigned* bar, int* derr, int blocks, long long poll
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   const unsigned expected = (unsigned)blocks + (unreachable ? 1u : 0u);
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_barrier_probe, bar, expected, derr);
+  StepView v{};
+  v.barrier = bar;
+  v.derr = derr;
+  const cudaError_t e = words ? cudaLaunchKernelEx(&cfg, k_sweep_word_probe, v, expected)
+                              : cudaLaunchKernelEx(&cfg, k_barrier_probe, bar, expected, derr);
   const long long standard = BARRIER_POLLS;
   const cudaError_t e2 = cudaMemcpyToSymbolAsync(g_barrier_polls, &standard, sizeof(standard), 0,
                                                  cudaMemcpyHostToDevice, s);

@@ -295,6 +295,10 @@ int ilg_set_timing(ilg_ctx* ctx, int enable);
  * limit is a per-device setting for the duration of the launch: do not run
  * radiosity solves on the same device meanwhile. */
 int ilg_debug_barrier_timeout(ilg_ctx* ctx, int blocks, long long polls, int unreachable);
+/* The same for the wait at the end of a single mesh's FP64 sweep, where each
+ * block waits for a word of every other one: with unreachable != 0 for one
+ * word that no block writes. */
+int ilg_debug_sweep_timeout(ilg_ctx* ctx, int blocks, long long polls, int unreachable);
 /* Test entry: the most polls of a wait for a row's column in the context's
  * fixed-sweep Gauss-Seidel solves (0 restores the default of 2^21). A solve
  * whose wait runs out returns ILG_ERR_DEVICE and the context stays usable. */
