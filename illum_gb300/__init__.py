@@ -102,6 +102,7 @@ _SIGS = {
     "ilg_debug_sweep_timeout": (C.c_int, [C.c_void_p, C.c_int, C.c_longlong, C.c_int]),
     "ilg_debug_ff_chunk": (C.c_int, [C.c_longlong]),
     "ilg_debug_gs_polls": (C.c_int, [C.c_void_p, C.c_longlong]),
+    "ilg_debug_path_entries": (C.c_int, [C.c_int]),
     "ilg_debug_sort": (C.c_int, [C.c_void_p, C.c_void_p, C.c_longlong, C.c_int, C.c_int]),
     "ilg_set_radiosity_mode": (C.c_int, [C.c_void_p, C.c_int, C.c_int]),
     "ilg_thermal_init": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_double, C.c_void_p,
@@ -606,6 +607,11 @@ def radiosity_blocks_for(nnz: int, entries_per_tile: int | None = None) -> int:
 def debug_ff_chunk(pairs):
     """Candidate pairs per form-factor build chunk (test entry; 0: default)."""
     _check(lib().ilg_debug_ff_chunk(int(pairs)))
+
+
+def debug_path_entries(entries=0):
+    """Most path entries per facet of the set-up's rays (test entry; 0: default)."""
+    _check(lib().ilg_debug_path_entries(int(entries)))
 
 
 def debug_sort(keys, vals=None, bits=64, polls=-1):

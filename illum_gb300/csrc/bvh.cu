@@ -1414,7 +1414,7 @@ __global__ void k_rowptr(const int32_t* __restrict__ rows, int64_t nnz, int nt, 
 
 // ====================================================================== host
 
-// Padding of the boxes (see slabf for what it has to cover).
+// Padding of the boxes (see geom.h slab and RayF for what it has to cover).
 static float box_pad(const Context& c) { return 1e-6f * c.scene_mag; }
 // Whether rays from the facets' centroids, `offset` along the normals, start
 // near the context's own tree: within a quarter of the scene's magnitude of
@@ -1424,8 +1424,14 @@ static float box_pad(const Context& c) { return 1e-6f * c.scene_mag; }
 static bool rays_near(const Context& c, float offset) {
   return std::fabs(offset) * c.nrm_max <= 0.25f * c.scene_mag && c.scene_mag < 1e19f;
 }
-// Most path entries of a facet: one per level, as many as the mask's bits.
-static int path_entries(const Context& c) { return std::max(1, std::min(c.bvh_longest, PATH_MOST)); }
+// Most path entries of a facet: one per level, as many as the mask's bits (a
+// test entry may lower it to exercise paths that end with the whole tree).
+static std::atomic<int> g_path_most{PATH_MOST};
+int path_set_most(int entries) {
+  g_path_most.store(entries > 0 ? std::min(entries, PATH_MOST) : PATH_MOST);
+  return ILG_OK;
+}
+static int path_entries(const Context& c) { return std::max(1, std::min(c.bvh_longest, g_path_most.load())); }
 
 int bvh_build(Context& c, const float* verts_h, int nv, const int32_t* tris_h, const float* normals_h) {
   int nt = c.nt;

@@ -985,6 +985,8 @@ int ilg_radiosity_solve_gs(ilg_ctx* ctx, const double* E, int gs_steps, double* 
   return ILG_OK;
 }
 
+int ilg_debug_path_entries(int entries) { return path_set_most(entries); }
+
 int ilg_debug_ff_chunk(long long pairs) { return ff_set_chunk((int64_t)pairs); }
 
 int ilg_debug_gs_polls(ilg_ctx* ctx, long long polls) {

@@ -359,6 +359,7 @@ int direct_beside_launch(const StepView& v, int mu32_flux, int ahead, cudaStream
 // ---- radiosity.cu ----
 int radiosity_prepare(Context& c);
 int radiosity_grid(int ntiles, int64_t nt);
+int path_set_most(int entries);
 int ff_set_chunk(int64_t pairs);   // candidate pairs per form-factor chunk (<= 0: the default)
 // Balanced assignment of row tiles to the grid's blocks (longest tiles
 // first, each to the least loaded block); uploads it to start/order.

@@ -308,6 +308,11 @@ int ilg_debug_gs_polls(ilg_ctx* ctx, long long polls);
  * small mesh through the several-chunk path, whose matrix must equal the
  * one-chunk build's. Not for concurrent use with other builds. */
 int ilg_debug_ff_chunk(long long pairs);
+/* Test entry for the rays from facets: the most path entries per facet
+ * (process-wide; <= 0 restores the default of 64, more than any but
+ * degenerate meshes need). A longer path ends with the whole tree; results do
+ * not depend on it. Not for concurrent use with other set-ups. */
+int ilg_debug_path_entries(int entries);
 /* Test entry for the radix sort of the set-up: sorts host arrays in place by
  * the keys' low `bits` bits (keys must be zero above them), stably; vals (may
  * be NULL) follow. polls: how often a tile of the sort looks for the digit
