@@ -901,13 +901,13 @@ def main():
     peak, peak_kind = _peaks()
     bytes_cond = N * (2 * nz * 8 + 6 * 8)
     nnz = W["setup"]["nnz"]
-    # a full sweep (the first, and one about six sweeps in) reads F as 64-bit
-    # values, a change sweep as 32-bit ones
-    full = min(2.0, sweeps_per_step)
-    bytes_rad = (full * (nnz * (8 + 4) + N * (4 + 8 + 8 + 8)) +
-                 (sweeps_per_step - full) * (nnz * (4 + 4) + N * (4 + 4 + 8 + 8)))
+    # a full sweep reads F as 64-bit values with 16-bit columns, a change sweep
+    # as 32-bit ones (counted by the solve); and the facets' vectors
+    full = st["full_sweeps"] / nph
+    bytes_rad = (full * (nnz * (8 + 2) + N * (4 + 8 + 8 + 8)) +
+                 (sweeps_per_step - full) * (nnz * (4 + 2) + N * (4 + 4 + 8 + 8)))
     kern = {"conduction": (bytes_cond, ph["conduction"], "k_conduct_dfloat_c1"),
-            "radiosity": (bytes_rad, ph["radiosity"], "k_radiosity64_c1")}
+            "radiosity": (bytes_rad, ph["radiosity"], "k_radiosity64_solo_c1")}
     dom = max(kern, key=lambda k: kern[k][1])
     b, ms, prof = kern[dom]
     achieved = b / (ms / 1000.0) / 1e9
@@ -977,7 +977,8 @@ def main():
                        "parallelism": f"replicas x{world}"},
             "e2e": e2e, "gpu_launches": 4 * args.steps, "roofline": roofline, "cpu_baseline": cpu,
             "clocks": clk, "parity_vs_oracle": parity,
-            "phases_ms_per_step": ph, "radiosity_sweeps_per_step": sweeps_per_step, "autotune": tune,
+            "phases_ms_per_step": ph, "radiosity_sweeps_per_step": sweeps_per_step,
+            "radiosity_full_sweeps_per_step": full, "autotune": tune,
             "ambiguous_facets_per_step": amb_per_step,
             "direct_samples_per_s": (N * (len(W["disk"]) - 1) / (ph["direct"] * 1e-3) if ph.get("direct") else None),
             "visibility_rays_per_s": su["visibility_rays"] / su["form_factors_s"],

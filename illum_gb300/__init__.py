@@ -119,6 +119,7 @@ _SIGS = {
     "ilg_autotune": (C.c_int, [C.c_void_p, C.POINTER(RunOpts), C.c_int, C.POINTER(Tune)]),
     "ilg_set_tune": (C.c_int, [C.c_void_p, C.POINTER(Tune)]),
     "ilg_get_tune": (C.c_int, [C.c_void_p, C.POINTER(Tune)]),
+    "ilg_get_full_sweeps": (C.c_int, [C.c_void_p, C.POINTER(C.c_int64)]),
     "ilg_get_stats": (C.c_int, [C.c_void_p, C.POINTER(C.c_double), C.POINTER(C.c_double), C.POINTER(C.c_double),
                                 C.POINTER(C.c_int64), C.POINTER(C.c_int64)]),
     "ilg_batch_create": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.POINTER(C.c_void_p)]),
@@ -458,10 +459,11 @@ class IllumContext:
 
     def stats(self):
         a, b, c = C.c_double(), C.c_double(), C.c_double()
-        amb, sw = C.c_int64(), C.c_int64()
+        amb, sw, full = C.c_int64(), C.c_int64(), C.c_int64()
         _check(lib().ilg_get_stats(self._h, C.byref(a), C.byref(b), C.byref(c), C.byref(amb), C.byref(sw)))
+        _check(lib().ilg_get_full_sweeps(self._h, C.byref(full)))
         return {"ms_direct": a.value, "ms_radiosity": b.value, "ms_conduction": c.value,
-                "ambiguous_facets": amb.value, "radiosity_sweeps": sw.value}
+                "ambiguous_facets": amb.value, "radiosity_sweeps": sw.value, "full_sweeps": full.value}
 
 
 class ThermalModel:

@@ -537,6 +537,7 @@ static int collect_stats(Context& c, bool phases) {
   ILG_CUDA(cudaStreamSynchronize(c.stream));
   c.stats_ambiguous += h0;
   c.stats_sweeps += md.sweeps;
+  c.stats_full += md.full_sweeps;
   if (phases) {
     float a, b, d;
     ILG_CUDA(cudaEventElapsedTime(&a, c.ev[0], c.ev[1]));
@@ -1457,7 +1458,7 @@ int ilg_set_timing(ilg_ctx* ctx, int enable) {
   AllocOn on_(c.stream);
   c.timing = enable != 0;
   c.ms_direct = c.ms_rad = c.ms_cond = 0.f;
-  c.stats_ambiguous = c.stats_sweeps = 0;
+  c.stats_ambiguous = c.stats_sweeps = c.stats_full = 0;
   return ILG_OK;
 }
 
@@ -1471,6 +1472,12 @@ int ilg_get_stats(ilg_ctx* ctx, double* ms_direct, double* ms_radiosity, double*
   if (ms_conduction) *ms_conduction = c.ms_cond;
   if (ambiguous) *ambiguous = c.stats_ambiguous;
   if (sweeps) *sweeps = c.stats_sweeps;
+  return ILG_OK;
+}
+
+int ilg_get_full_sweeps(ilg_ctx* ctx, int64_t* full_sweeps) {
+  if (!ctx || !full_sweeps) { set_error("invalid arguments"); return ILG_ERR_ARG; }
+  *full_sweeps = ctx->c.stats_full;
   return ILG_OK;
 }
 

@@ -107,6 +107,7 @@ struct MeshDesc {
                                // pass per step, with fl(F) every K-th step (k_radiosity_lagged)
   int ref_age;                 // that solve: steps since its reference pass (-1: none yet)
   int sweeps;                  // out: sweeps of the last solve
+  int full_sweeps;             // out: those of them in double-float (FP64 solve)
   double res2;                 // out: squared residual bound of the last solve
   int active;                  // 0: skipped by the step kernels
   int done_steps;              // steps taken since the run started
@@ -301,7 +302,7 @@ struct Context {
   dbuf<int> mesh_flag;
   double* pinned_tsurf = nullptr;        // 2 x N surface temperatures (alternating slots)
   cudaEvent_t slot_ev[2] = {nullptr, nullptr};
-  int64_t stats_ambiguous = 0, stats_sweeps = 0;
+  int64_t stats_ambiguous = 0, stats_sweeps = 0, stats_full = 0;
   bool timing = false;
   float ms_direct = 0, ms_rad = 0, ms_cond = 0;
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};

@@ -822,6 +822,7 @@ __device__ __forceinline__ void init_meshes64(const StepView& v, MeshState64& st
     st.mode[m] = (M.active && M.ntiles > 0) ? 0 : 1 << MODE_DONE;
     st.sweeps[m] = 0;
     st.acc[m] = st.prev[m] = 0.f;
+    if (blockIdx.x == 0) v.md[m].full_sweeps = 0;
   }
   const int gt = blockIdx.x * blockDim.x + threadIdx.x;
   for (int m = gt; m < RES_LEVELS * v.nmesh; m += gridDim.x * blockDim.x) res_acc(v, 0)[m] = 0ull;
@@ -850,7 +851,10 @@ __device__ __forceinline__ int decide_meshes64(const StepView& v, MeshState64& s
         run = false;
         st.acc[m] = dec.err;   // for record_residuals64
       }
-      if (blockIdx.x == 0) v.md[m].sweeps = sw;
+      if (blockIdx.x == 0) {
+        v.md[m].sweeps = sw;
+        if (!change) atomicAdd(&v.md[m].full_sweeps, 1);   // (nothing waits for it)
+      }
     }
     running += __syncthreads_count(run);
   }
@@ -1301,7 +1305,7 @@ __device__ __forceinline__ SweepWord word_load(const SweepWord* p) {
 
 struct SoloShared {
   float red[32];
-  int bad, ok, mode, stop;   // mode as MeshState64::mode
+  int bad, ok, mode, stop, full;   // mode as MeshState64::mode; full sweeps so far
   float acc, prev, err;
 };
 
@@ -1359,6 +1363,7 @@ __device__ __forceinline__ bool solo_sweep_end(const StepView& v, SoloShared& S,
       S.acc = dec.acc;
       S.prev = dec.dn;
       S.err = dec.err;
+      S.full += change ? 0 : 1;
       S.ok = ok;
     }
   }
@@ -1383,7 +1388,7 @@ __global__ void __maxnreg__(RAD_REGS64) k_radiosity64_solo(StepView v, double* x
   // (every group of a sweep is taken before the next sweep's first copy)
   Pipe pipe = make_pipe(sm, &S.bad);
   if (threadIdx.x == 0) {
-    S.mode = 0;
+    S.mode = S.full = 0;
     S.acc = S.prev = 0.f;
   }
   const RadBufs B(v);
@@ -1480,6 +1485,7 @@ __global__ void __maxnreg__(RAD_REGS64) k_radiosity64_solo(StepView v, double* x
       r2 = warp_sum(r2);
       if (threadIdx.x == 0) {
         v.md[0].sweeps = it + 1;
+        v.md[0].full_sweeps = S.full;
         v.md[0].res2 = with_errors(r2, S.err, v.md[0].tol2);
       }
     }
@@ -2475,7 +2481,7 @@ __global__ void k_barrier_probe(unsigned* bar, unsigned expected, int* derr) {
 __global__ void k_sweep_word_probe(StepView v, unsigned expected) {
   __shared__ SoloShared S;
   if (threadIdx.x == 0) {
-    S.mode = 0;
+    S.mode = S.full = 0;
     S.acc = S.prev = 0.f;
   }
   solo_sweep_end(v, S, 0, 1.f, 1.f, 0.f, 1, expected);

@@ -358,6 +358,9 @@ int ilg_record_thermal(ilg_ctx* ctx, int capacity);
 int ilg_get_thermal_records(ilg_ctx* ctx, double* out, int* count);
 int ilg_get_stats(ilg_ctx* ctx, double* ms_direct, double* ms_radiosity, double* ms_conduction,
                   int64_t* ambiguous_facets, int64_t* radiosity_sweeps);
+/* Those of the counted radiosity sweeps that evaluated F x in double-float (FP64
+ * solves; the others evaluated F of the last change in FP32). */
+int ilg_get_full_sweeps(ilg_ctx* ctx, int64_t* full_sweeps);
 
 /* ---- batches: many meshes stepped together ---------------------------------- */
 /* A batch steps its member contexts (each with horizons, suns set by
