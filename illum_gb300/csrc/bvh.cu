@@ -722,7 +722,8 @@ __device__ __forceinline__ void walk_nodes(Walk& w, int* stack, const float4* __
 // waited for its longest. A ray first tests the triangle its lane's last ray
 // hit: the next angle of the bisection often hits it again.
 // Bound by issue and node-load latency (rays of one facet differ most in
-// length); 8 blocks per SM hide the loads best (7 were 6% slower, 9 spill).
+// length); 8 blocks per SM hide the loads best, at 28 bytes of spills (7 were
+// 6% slower, 9 spill more).
 // 81,920 facets x 64 azimuths: 23.6 ms with a root-to-leaf walk over boxes
 // alone, 18.9 ms with one azimuth per lane, 16.5 ms this way; 20,480 x 32
 // 1.03 -> 0.79 ms; a 256 x 256 terrain x 128 68 -> 60 ms. With two or four
@@ -1095,7 +1096,8 @@ __global__ void __launch_bounds__(128) k_count_pairs(LeafGroups G, const float4*
 // against a candidate list in device memory (a counting and a filling walk per
 // source, 0.4 and 0.17 of the ray kernel's time) and one root-to-leaf walk
 // over boxes per ray. The enumeration waits in shared memory, which leaves the
-// walk without spills at seven blocks per SM (five: 13% slower, six 4%).
+// walk with 12 bytes of spills at seven blocks per SM (five: 13% slower, six
+// 4%).
 constexpr int VIS_THREADS = 128;
 constexpr int VIS_QUEUE = 64;      // candidates waiting (at most 31 + 32)
 constexpr int VIS_KEYS = 64;       // keys waiting to be written (at most 31 + 32)

@@ -123,7 +123,7 @@ struct RadixTile {
   static constexpr int BLOCKS = BLOCKS_, THREADS = THREADS_, ITEMS = ITEMS_, WARPS = THREADS / 32, TILE = THREADS * ITEMS;
   static constexpr size_t SMEM = (size_t)TILE * 12;   // keys and values in digit order
 };
-typedef RadixTile<512, 12, 2> RadixLarge;
+typedef RadixTile<512, 12, 2> RadixLarge;   // spills 44 bytes, 96 with values
 typedef RadixTile<256, 8, 2> RadixSmall;   // up to RS_SMALL keys: more tiles than a few
 constexpr int64_t RS_SMALL = 1 << 19;
 

@@ -78,7 +78,9 @@ constexpr int RAD_THREADS = 992;             // consumer threads (31 warps): one
 // Registers per thread: 1,024 threads leave 8,192 of the SM's in the FP64 and
 // 16,384 in the mixed solve, one block of 128 or 256 threads of the direct
 // insolation that runs beside it (direct.cu k_direct_beside). The FP64 solves
-// are long enough to hide the smaller block and lose 8% at 48 registers.
+// are long enough to hide the smaller block and lose 8% at 48 registers. At 48
+// the one-pass solve's first pass spills 160 bytes per thread (the others
+// none).
 #define RAD_REGS64 56
 #define RAD_REGSM 48
 constexpr int RAD_BLOCK = RAD_THREADS + 32;  // and one producer warp that issues the entry-stream copies
@@ -1150,7 +1152,6 @@ __device__ __forceinline__ MeshState64::MeshState64(int nmesh) {
 // The ring's barriers, set up by thread 0 before the launch's first block
 // barrier (inside init_meshes' caller): full counts the producer's one
 // arrival plus the copied bytes, empty one arrival per consumer warp.
-// first: the first of its barriers (pipes that share the ring take turns).
 __device__ __forceinline__ Pipe make_pipe(const RadSmem& m, int* bad) {
   if (threadIdx.x == 0) {
     for (int s = 0; s < RAD_STAGES; ++s) {
@@ -1529,7 +1530,7 @@ __global__ void __maxnreg__(RAD_REGSM) k_radiosity_mixed(StepView v, double* x, 
       __syncwarp();
     } else {
       for (int k = v.blk_start[blockIdx.x]; k < v.blk_start[blockIdx.x + 1]; ++k) {
-    const int t = v.blk_tile[k];
+        const int t = v.blk_tile[k];
         const RowTile T = v.tiles[t];
         if (st.done[T.mesh]) continue;
         const uint32_t s0 = tile_start(v, t);
@@ -1564,7 +1565,7 @@ __global__ void __maxnreg__(RAD_REGSM) k_radiosity_mixed(StepView v, double* x, 
         __syncwarp();
       } else {
         for (int k = v.blk_start[blockIdx.x]; k < v.blk_start[blockIdx.x + 1]; ++k) {
-    const int t = v.blk_tile[k];
+          const int t = v.blk_tile[k];
           const RowTile T = v.tiles[t];
           if (st.done[T.mesh]) continue;
           const uint32_t s0 = tile_start(v, t);
@@ -1643,9 +1644,8 @@ __global__ void __maxnreg__(RAD_REGSM) k_radiosity_lagged(StepView v, double* x,
   __shared__ float red[32];
   __shared__ int bad;
   // each mesh's kind of pass (0: bf16 step, 1: reference step, 2: reference
-  // step without an earlier reference) lives in st.now until the pass is
-  // over (the static shared memory has no room for another array beside the
-  // ring)
+  // step without an earlier reference) lives in st.now, unused until the pass
+  // is over
   unsigned char* kind = st.now;
   const RadSmem sm = rad_smem();
   const bool producer = threadIdx.x >= RAD_THREADS;
