@@ -810,11 +810,11 @@ __device__ __forceinline__ Sweep64 sweep_decision(unsigned long long q0, unsigne
   r.dn = sqrtf((float)q0 + cap * ((float)q1 + cap * (float)q2)) * (1.f / 1024.f);
   r.err = change ? c * acc : 0.f;
   r.acc = change ? acc + r.dn : r.dn;
-  r.stop = change ? r.dn + r.err <= 1023.f / 1024.f : q1 == 0 && q2 == 0 && q0 <= RES_UNITS;
+  r.stop = change ? r.dn + r.err <= 1023.f / 1024.f : ((q1 | q2) == 0) & (q0 <= RES_UNITS);
   const float e = c * r.acc;   // the errors after another change sweep
-  const bool last = r.dn <= 1.f || (e > 0.5f && r.dn * r.dn <= (prev > 0.f ? prev : 8.f * r.dn));
-  const bool renew = e > 1.f && 16.f * c * r.dn * prev <= prev - r.dn;
-  r.next_change = !last && !renew && r.dn > 4.f * e && r.dn < CHG_RANGE;
+  const bool last = (r.dn <= 1.f) | ((e > 0.5f) & (r.dn * r.dn <= (prev > 0.f ? prev : 8.f * r.dn)));
+  const bool renew = (e > 1.f) & (r.dn * (16.f * c * prev) <= prev - r.dn);
+  r.next_change = !last & !renew & (r.dn > 4.f * e) & (r.dn < CHG_RANGE);
   return r;
 }
 
@@ -838,13 +838,15 @@ __device__ __forceinline__ int decide_meshes64(const StepView& v, MeshState64& s
     const int m = m0 + threadIdx.x;
     bool run = m < v.nmesh && !(st.mode[m] >> MODE_DONE);
     if (run) {
+      // every load before the first store (one trip to L2 instead of three)
       const unsigned long long q0 = __ldcg(res_acc(v, k, 0) + m), q1 = __ldcg(res_acc(v, k, 1) + m),
                                q2 = __ldcg(res_acc(v, k, 2) + m);
-      const bool change = st.mode[m] & 1;
-      const int sw = ++st.sweeps[m];
-      const Sweep64 dec = sweep_decision(q0, q1, q2, change, v.md[m].rad_err, st.acc[m], st.prev[m]);
-      const int in_s1 = change ? st.mode[m] & 2 : (st.mode[m] & 2) ^ 2;
+      const float c = v.md[m].rad_err;
       const int budget = v.md[m].max_sweeps;
+      const bool change = st.mode[m] & 1;
+      const Sweep64 dec = sweep_decision(q0, q1, q2, change, c, st.acc[m], st.prev[m]);
+      const int sw = ++st.sweeps[m];
+      const int in_s1 = change ? st.mode[m] & 2 : (st.mode[m] & 2) ^ 2;
       st.mode[m] = in_s1 | (dec.next_change && sw + 1 < budget ? 1 : 0);
       st.acc[m] = dec.acc;
       st.prev[m] = dec.dn;
@@ -1306,7 +1308,7 @@ __device__ __forceinline__ SweepWord word_load(const SweepWord* p) {
 
 struct SoloShared {
   float red[32];
-  int bad, ok, mode, stop, full;   // mode as MeshState64::mode; full sweeps so far
+  int bad, ok, mode, stop;   // mode as MeshState64::mode
   float acc, prev, err;
 };
 
@@ -1364,7 +1366,6 @@ __device__ __forceinline__ bool solo_sweep_end(const StepView& v, SoloShared& S,
       S.acc = dec.acc;
       S.prev = dec.dn;
       S.err = dec.err;
-      S.full += change ? 0 : 1;
       S.ok = ok;
     }
   }
@@ -1389,7 +1390,7 @@ __global__ void __maxnreg__(RAD_REGS64) k_radiosity64_solo(StepView v, double* x
   // (every group of a sweep is taken before the next sweep's first copy)
   Pipe pipe = make_pipe(sm, &S.bad);
   if (threadIdx.x == 0) {
-    S.mode = S.full = 0;
+    S.mode = 0;
     S.acc = S.prev = 0.f;
   }
   const RadBufs B(v);
@@ -1413,9 +1414,10 @@ __global__ void __maxnreg__(RAD_REGS64) k_radiosity64_solo(StepView v, double* x
   unsigned gen = 0;
   if (!grid_barrier(v.barrier, gridDim.x, gen, v.derr)) return;
   float2 sown = has_row ? ld_it(B.S0 + rpos) : make_float2(0.f, 0.f);
-  int it = 0;
+  int it = 0, full = 0;
   for (;; ++it) {
     const int mode = S.mode;
+    full += 1 - (mode & 1);
     float d2 = 0.f;
     if (producer) {
       if ((threadIdx.x & 31) == 0) {
@@ -1486,7 +1488,7 @@ __global__ void __maxnreg__(RAD_REGS64) k_radiosity64_solo(StepView v, double* x
       r2 = warp_sum(r2);
       if (threadIdx.x == 0) {
         v.md[0].sweeps = it + 1;
-        v.md[0].full_sweeps = S.full;
+        v.md[0].full_sweeps = full;
         v.md[0].res2 = with_errors(r2, S.err, v.md[0].tol2);
       }
     }
@@ -2481,7 +2483,7 @@ __global__ void k_barrier_probe(unsigned* bar, unsigned expected, int* derr) {
 __global__ void k_sweep_word_probe(StepView v, unsigned expected) {
   __shared__ SoloShared S;
   if (threadIdx.x == 0) {
-    S.mode = S.full = 0;
+    S.mode = 0;
     S.acc = S.prev = 0.f;
   }
   solo_sweep_end(v, S, 0, 1.f, 1.f, 0.f, 1, expected);
