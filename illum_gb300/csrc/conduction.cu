@@ -37,6 +37,7 @@
 #include <cstring>
 #include <mutex>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "geom.h"
@@ -1033,6 +1034,42 @@ __global__ void __launch_bounds__(256) k_relayout(const double* __restrict__ in,
   }
 }
 
+// The pool of the standalone columns' buffers on the current device: its own,
+// because these calls must not keep what the contexts' pool would (a call
+// with large arrays left all of its device memory with the process), and
+// bounded: it keeps at most COL_POOL_KEEP between calls, enough that small
+// calls map nothing.
+constexpr uint64_t COL_POOL_KEEP = 64 << 20;
+static int columns_pool(cudaMemPool_t* pool) {
+  static std::mutex mu;
+  static std::vector<std::pair<int, cudaMemPool_t>> pools;
+  int dev = 0;
+  ILG_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lock(mu);
+  for (const auto& p : pools)
+    if (p.first == dev) { *pool = p.second; return ILG_OK; }
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  ILG_CUDA(cudaMemPoolCreate(pool, &props));
+  uint64_t keep = COL_POOL_KEEP;
+  ILG_CUDA(cudaMemPoolSetAttribute(*pool, cudaMemPoolAttrReleaseThreshold, &keep));
+  pools.push_back({dev, *pool});
+  return ILG_OK;
+}
+struct ColumnsBuffer {   // freed on its stream, which outlives it
+  unsigned char* p = nullptr;
+  cudaStream_t s;
+  explicit ColumnsBuffer(cudaStream_t st) : s(st) {}
+  ColumnsBuffer(const ColumnsBuffer&) = delete;
+  ~ColumnsBuffer() {
+    if (!p) return;
+    cudaFreeAsync(p, s);
+    cudaStreamSynchronize(s);   // what the pool does not keep goes back here
+  }
+};
+
 // Standalone batched columns (host arrays, reference layout: column-major
 // nz x ncol). Runs on the current device with a private stream and one
 // stream-ordered allocation, which holds
@@ -1052,17 +1089,24 @@ static int run_columns(int ncol, int nz, const double* z, double dt, const doubl
   CondScalars cs;
   ILG_TRY(build_tables(nz, z, ti, rhoc, dt, emiss, Fgeo, bc, tab, cs));
   ILG_TRY(conduction_setup());
-  ILG_TRY(alloc_pool_setup());
+  cudaMemPool_t pool;
+  ILG_TRY(columns_pool(&pool));
   OwnedStream os;   // destroyed after the buffer, which is freed on it
   ILG_CUDA(cudaStreamCreateWithFlags(&os.s, cudaStreamNonBlocking));
   cudaStream_t s = os.s;
-  AllocOn on(s);
   const size_t n = (size_t)nz * ncol, nc = (size_t)ncol;
   const size_t tab_b = (tab.size() * 8 + 255) & ~(size_t)255, md_b = (sizeof(MeshDesc) + 255) & ~(size_t)255;
   const size_t head_b = tab_b + md_b + 256;
   const bool deep = (size_t)nz * COL_HOST_THREADS * sizeof(double) > SMEM_LIMIT;
-  dbuf<unsigned char> buf;
-  ILG_TRY(buf.alloc(head_b + (4 * nc + (deep ? 3 : 2) * n) * 8));
+  ColumnsBuffer buf(s);
+  const size_t bytes = head_b + (4 * nc + (deep ? 3 : 2) * n) * 8;
+  const cudaError_t ea = cudaMallocFromPoolAsync((void**)&buf.p, bytes, pool, s);
+  if (ea != cudaSuccess) {
+    buf.p = nullptr;
+    cudaGetLastError();   // an allocation failure is not sticky
+    set_error("device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(ea));
+    return ILG_ERR_NOMEM;
+  }
   double* const dtab = reinterpret_cast<double*>(buf.p);
   MeshDesc* const dmd = reinterpret_cast<MeshDesc*>(buf.p + tab_b);
   int* const derr = reinterpret_cast<int*>(buf.p + tab_b + md_b);
