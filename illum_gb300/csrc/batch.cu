@@ -554,6 +554,7 @@ int ilg_batch_get_tsurf(ilg_batch* batch, int member, double* out) {
   if (!batch || !out || member < 0 || member >= (int)batch->b.members.size()) { set_error("invalid member"); return ILG_ERR_ARG; }
   Batch& b = batch->b;
   const MeshDesc& M = b.mh[member];
+  fault_in({{out, (size_t)M.nfacet * 8}});
   ILG_CUDA(cudaMemcpyAsync(out, b.Tsurf.p + M.facet0, (size_t)M.nfacet * 8, cudaMemcpyDeviceToHost, b.stream));
   ILG_CUDA(cudaStreamSynchronize(b.stream));
   return ILG_OK;

@@ -421,9 +421,11 @@ static StepPlan solo_plan(Context& c, const ilg_run_opts& o) {
 // threads, if the first, middle or last page does not exist: fresh arrays of
 // 0.66 and 4.1 MB 180 -> 60 and 310 -> 175 us (40 and 55 us where the pages
 // exist), the first outputs of a program with a 512 x 512 terrain 4.5 -> 0.35
-// ms (four arrays; later ones 0.15 -> 0.17 ms). Only a hint: where the kernel
-// does not know it (or the memory is not ordinary memory), the copy maps the
-// pages as before.
+// ms (four arrays; later ones 0.15 -> 0.17 ms). A byte of each page is then
+// written back: now and then a copy into pages that exist took 0.9 ms per 4 MB
+// (about 13 us a page; in three of ten runs of that terrain, none with the
+// bytes written). Only a hint: where the kernel does not know the calls (or the
+// memory is not ordinary memory), the copy maps the pages as before.
 #ifndef MADV_POPULATE_WRITE
 #define MADV_POPULATE_WRITE 23
 #endif
@@ -450,6 +452,11 @@ void fault_in(std::initializer_list<HostRange> ranges) {
       if (mincore((void*)((a + k) * page), page, &in) == 0 && !(in & 1)) there = false;
     }
     if (!there) populate(a, a + n);
+    // a byte of every page written back: pages that exist can still stop the
+    // device (those that the kernel has marked for its page placement), the
+    // processor passes them at once
+    volatile unsigned char* const q = static_cast<volatile unsigned char*>(r.p);
+    for (size_t k = 0; k < r.bytes; k += page - ((uintptr_t)r.p + k) % page) q[k] = q[k];
   }
   if (!large) return;
   auto part = [&](size_t k) {   // the k-th part of every large range
@@ -893,6 +900,7 @@ int ilg_direct_radiosity(ilg_ctx* ctx, const double* sun, const double* disk_xy,
   M.host_sun = 1;
   ILG_TRY(upload_desc(c, M));
   ILG_TRY(direct_launch(solo_view(c, ILG_PREC_FP64), 1, 0, 0, c.stream));
+  fault_in({{out, (size_t)c.nt * 8}});
   ILG_CUDA(cudaMemcpyAsync(out, c.E.p, (size_t)c.nt * 8, cudaMemcpyDeviceToHost, c.stream));
   ILG_CUDA(cudaStreamSynchronize(c.stream));
   return read_device_errors(c);
@@ -923,6 +931,7 @@ int ilg_radiosity_solve(ilg_ctx* ctx, const double* E, double tol, int max_sweep
   StepView v = solo_view(c, ILG_PREC_FP64);
   ILG_TRY(radiosity_launch(v, c.Q.p, 0, ILG_PREC_FP64, radiosity_grid(c.ntiles, c.nt), 1, false, c.stream));
   MeshDesc out;
+  fault_in({{x, (size_t)c.nt * 8}});   // while the solve runs
   ILG_CUDA(cudaMemcpyAsync(x, c.Q.p, (size_t)c.nt * 8, cudaMemcpyDeviceToHost, c.stream));
   ILG_CUDA(cudaMemcpyAsync(&out, c.md.p, sizeof(out), cudaMemcpyDeviceToHost, c.stream));
   ILG_CUDA(cudaStreamSynchronize(c.stream));
@@ -973,6 +982,7 @@ int ilg_radiosity_solve_gs(ilg_ctx* ctx, const double* E, int gs_steps, double* 
   double* Ed = gs_rhs(c);
   ILG_CUDA(cudaMemcpyAsync(Ed, E, (size_t)c.nt * 8, cudaMemcpyHostToDevice, c.stream));
   ILG_TRY(gs_solve_launch(c, Ed, c.Q.p, gs_steps, c.stream));
+  fault_in({{x, (size_t)c.nt * 8}});   // while the solve runs
   std::vector<double> r2;
   if (res) {
     ILG_TRY(gs_residual_launch(c, Ed, c.Q.p, c.gs_x.p, c.stream));
